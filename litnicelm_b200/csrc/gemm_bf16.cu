@@ -4,9 +4,14 @@
 // Persistent kernel, one CTA per SM, tiles of 128 x BN taken round robin:
 //   warp 0      one lane issues the TMA loads of the A and W tiles (64 k per stage, 128-byte swizzle)
 //   warp 1      owns tensor memory (two accumulators of BN columns); one lane issues tcgen05.mma
-//   warps 2-5   read a finished accumulator and store the tile while the next one is multiplied:
-//               32 columns at a time through a padded shared-memory patch, so that global reads and
-//               writes are whole rows of 128 bytes
+//   warps 2-9   read a finished accumulator and store the tile while the next one is multiplied: two warps
+//               to each 32 rows, 32 columns at a time through a swizzled shared-memory patch that a TMA store
+//               (or, for results that are added, a TMA reduction) carries out, clipped at the result's edges
+// Bound: the tensor pipe for long k (an instruction of 128 x 256 x 16 takes about 160 clocks), the store for short k and
+// for GELU (erff: about 35 instructions an element). The store used to be four warps with whole-row global accesses behind a
+// padded patch, residuals read back inside it: about 12 us a tile of 128 x 256 whatever the activation, against 1 us of
+// products at k = 256 and 4 us at k = 1024. Prompts of 4 x 2048 tokens through six Mitilix layers of width 1024, 30 of these
+// products: 3.06 ms a pass before, 1.97 ms with eight warps and TMA stores.
 // Rows and columns outside the operands load as zeros (k need not be a multiple of 64) and are not
 // stored. Every mbarrier wait is bounded; a wait that runs out sets the error word and ends the kernel
 // after its copies have landed and tensor memory is freed. No clusters, no multicast.
@@ -25,26 +30,27 @@ namespace {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int GB_THREADS = 192;
-constexpr int GB_PATCH_LD = 36;  // floats per row of a warp's staging patch
-constexpr int GB_PATCH = 32 * GB_PATCH_LD * 4;
+constexpr int GB_STORE_WARPS = 8;
+constexpr int GB_THREADS = 64 + 32 * GB_STORE_WARPS;
+constexpr int GB_PATCH = 32 * 32 * 4;  // a warp's staging patch: 32 rows of 32 floats, or two buffers of 32 rows of 32 bfloat16
 constexpr int GB_GROUP = 16;     // row tiles that share a sweep over the columns (W tiles stay in L2)
 
 template <int BN>
 struct GbSmem {
-  static constexpr int STAGES = BN == 256 ? 4 : BN == 128 ? 5 : 6;
+  static constexpr int STAGES = BN == 256 ? 4 : BN == 128 ? 6 : 8;
   static constexpr int A_BYTES = TC_BM * 128;
   static constexpr int B_BYTES = BN * 128;
   static constexpr int STAGE = A_BYTES + B_BYTES;
   static constexpr int PATCH_OFF = STAGES * STAGE;
-  static constexpr int BAR_OFF = PATCH_OFF + 4 * GB_PATCH;
+  static constexpr int BAR_OFF = PATCH_OFF + GB_STORE_WARPS * GB_PATCH;
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
-template <int BN>
+template <int BN, int GATED>
 __global__ void __launch_bounds__(GB_THREADS, 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, Bf16Product p, int m,
-                 int m_tiles, int n_tiles, DevErr *err) {
+gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
+                 const __grid_constant__ CUtensorMap map_half, const __grid_constant__ CUtensorMap map_float, int half_tma,
+                 int float_tma, const __grid_constant__ Bf16Product p, int m, int m_tiles, int n_tiles, DevErr *err) {
   using L = GbSmem<BN>;
   constexpr int S = L::STAGES;
   extern __shared__ unsigned char smem_raw[];
@@ -73,7 +79,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull(b), 1);
-      mbar_init(tempty(b), 4);
+      mbar_init(tempty(b), GB_STORE_WARPS);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -157,13 +163,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         if (global_timer() - t0 > WAIT_LIMIT_NS) break;
     }
   } else {
-    const int q = warp & 3;
-    float *patch = reinterpret_cast<float *>(base_ptr + L::PATCH_OFF + (warp - 2) * GB_PATCH);
-    const bool half_vec = p.half_out != nullptr && (p.half_ld & 3) == 0 && (reinterpret_cast<uintptr_t>(p.half_out) & 7) == 0;
-    const bool float_vec = p.float_out != nullptr && (p.float_ld & 3) == 0 &&
-                           (reinterpret_cast<uintptr_t>(p.float_out) & 15) == 0 && (p.n_half & 3) == 0;
-    const int sub = lane >> 3, c4 = (lane & 7) * 4;
-    int use = 0;
+    const int q = warp & 3, part = (warp - 2) >> 2;  // lanes of tensor memory, share of the columns
+    unsigned char *patch = base_ptr + L::PATCH_OFF + (warp - 2) * GB_PATCH;
+    const unsigned patch_u = base + (unsigned)(L::PATCH_OFF + (warp - 2) * GB_PATCH);
+    int use = 0, turn = 0;
+    bool wide = false;  // the last store read the whole patch
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++use) {
       const int buf = use & 1;
       if (!mbar_wait_warp(tfull(buf), (unsigned)(use >> 1) & 1u, abort_flag, err, 14)) break;
@@ -172,70 +176,100 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       place(tile, m0, n0);
       const int row0 = m0 + q * 32;
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      for (int c0 = part * (BN / 2); c0 < (part + 1) * (BN / 2); c0 += 32) {
         unsigned r[32];
         tc_ld32(tmem + ((unsigned)(q * 32) << 16) + (unsigned)(buf * BN + c0), r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (c0 + 32 == BN) {
+        if (c0 + 32 == (part + 1) * (BN / 2)) {
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0) mbar_arrive(tempty(buf));
         }
-        if (n0 + c0 >= p.n) continue;
+        const int col = n0 + c0;
+        if (col >= p.n || row0 >= m) continue;
+        const bool to_half = col + 32 <= p.n_half || (col < p.n_half && p.n_half == p.n);
+        if (to_half && half_tma) {
+          if (p.act == ACT_GELU_ERF) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 1 + GATED) r[j] = __float_as_uint(activate(__uint_as_float(r[j]), ACT_GELU_ERF));
+          } else if (p.act == ACT_GELU_TANH) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 1 + GATED) r[j] = __float_as_uint(activate(__uint_as_float(r[j]), ACT_GELU_TANH));
+          }
+          constexpr int PIECES = GATED ? 2 : 4;  // 16-byte pieces of a row
+          unsigned h[4 * PIECES];
+#pragma unroll
+          for (int j = 0; j < 4 * PIECES; ++j) {
+            __nv_bfloat162 v;
+            if (GATED)
+              v = __floats2bfloat162_rn(__uint_as_float(r[4 * j]) * __uint_as_float(r[4 * j + 1]),
+                                        __uint_as_float(r[4 * j + 2]) * __uint_as_float(r[4 * j + 3]));
+            else
+              v = __floats2bfloat162_rn(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+            h[j] = *reinterpret_cast<const unsigned *>(&v);
+          }
+          if (lane == 0) {
+            if (wide) bulk_wait_read<0>();
+            else bulk_wait_read<1>();
+          }
+          __syncwarp();
+          const unsigned at = (unsigned)(turn * (GB_PATCH / 2));
+          const int turned = GATED ? (lane >> 2) & 1 : (lane >> 1) & 3;
+#pragma unroll
+          for (int j = 0; j < PIECES; ++j)
+            *reinterpret_cast<uint4 *>(patch + at + lane * (16 * PIECES) + ((j ^ turned) << 4)) =
+                make_uint4(h[4 * j], h[4 * j + 1], h[4 * j + 2], h[4 * j + 3]);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) tma_store_2d(&map_half, patch_u + at, GATED ? col >> 1 : col, row0);
+          turn ^= 1;
+          wide = false;
+          continue;
+        }
+        if (lane == 0) bulk_wait_read<0>();
         __syncwarp();
+        if (col >= p.n_half && float_tma) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<uint4 *>(patch + lane * GB_PATCH_LD + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4 *>(patch + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) {
+            if (p.accumulate) tma_add_2d(&map_float, patch_u, col - p.n_half, row0);
+            else tma_store_2d(&map_float, patch_u, col - p.n_half, row0);
+          }
+          wide = true;
+          continue;
+        }
+        // columns on both sides of n_half, or a result no tensor map can address: a row at a time, lane = column
+        float *plain = reinterpret_cast<float *>(patch);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          *reinterpret_cast<uint4 *>(patch + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+              make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
         __syncwarp();
-        const int col = n0 + c0 + c4;
-        const bool to_half = col < p.n_half;
-        const bool whole = col + 4 <= (to_half ? p.n_half : p.n);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int rr = i * 4 + sub, row = row0 + rr;
-          if (row >= m || col >= p.n) continue;
-          float4 v = *reinterpret_cast<const float4 *>(patch + rr * GB_PATCH_LD + c4);
-          if (whole && to_half && p.gated) {  // two pairs
-            const __nv_bfloat162 a = __floats2bfloat162_rn(activate(v.x, p.act) * v.y, activate(v.z, p.act) * v.w);
-            *reinterpret_cast<__nv_bfloat162 *>(static_cast<bf16 *>(p.half_out) + (long long)row * p.half_ld + (col >> 1)) = a;
-          } else if (whole && to_half && half_vec) {
-            if (p.act != ACT_NONE)
-              v = make_float4(activate(v.x, p.act), activate(v.y, p.act), activate(v.z, p.act), activate(v.w, p.act));
-            const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-            uint2 o;
-            o.x = *reinterpret_cast<const unsigned *>(&a);
-            o.y = *reinterpret_cast<const unsigned *>(&b);
-            *reinterpret_cast<uint2 *>(static_cast<bf16 *>(p.half_out) + (long long)row * p.half_ld + col) = o;
-          } else if (whole && !to_half && float_vec) {
-            float4 *o = reinterpret_cast<float4 *>(p.float_out + (long long)row * p.float_ld + (col - p.n_half));
-            if (p.accumulate) {
-              const float4 x = *o;
-              v = make_float4(x.x + v.x, x.y + v.y, x.z + v.z, x.w + v.w);
-            }
-            *o = v;
-          } else {
-            const float e[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (col + j >= p.n) continue;
-              if (col + j < p.n_half) {
-                if (p.gated) {
-                  if ((j & 1) == 0)  // n_half is even
-                    static_cast<bf16 *>(p.half_out)[(long long)row * p.half_ld + ((col + j) >> 1)] =
-                        __float2bfloat16_rn(activate(e[j], p.act) * e[j + 1]);
-                } else {
-                  static_cast<bf16 *>(p.half_out)[(long long)row * p.half_ld + col + j] =
-                      __float2bfloat16_rn(activate(e[j], p.act));
-                }
-              } else {
-                float *o = p.float_out + (long long)row * p.float_ld + (col + j - p.n_half);
-                *o = p.accumulate ? *o + e[j] : e[j];
-              }
+        const int mine = col + lane, rows = min(32, m - row0);
+        if (mine < p.n) {
+          for (int rr = 0; rr < rows; ++rr) {
+            const float v = plain[rr * 32 + ((((lane >> 2) ^ (rr & 7)) << 2) | (lane & 3))];
+            const long long row = row0 + rr;
+            if (mine >= p.n_half) {
+              float *o = p.float_out + row * p.float_ld + (mine - p.n_half);
+              *o = p.accumulate ? *o + v : v;
+            } else if (!GATED) {
+              static_cast<bf16 *>(p.half_out)[row * p.half_ld + mine] = __float2bfloat16_rn(activate(v, p.act));
+            } else if ((lane & 1) == 0) {  // n_half is even
+              const float f = plain[rr * 32 + ((((lane >> 2) ^ (rr & 7)) << 2) | ((lane & 3) + 1))];
+              static_cast<bf16 *>(p.half_out)[row * p.half_ld + (mine >> 1)] = __float2bfloat16_rn(activate(v, p.act) * f);
             }
           }
         }
+        __syncwarp();
+        wide = false;
       }
     }
+    if (lane == 0) bulk_wait_all();  // the stores are part of the grid's results
   }
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -257,17 +291,32 @@ int device_sms() {
   return n;
 }
 
-template <int BN>
+template <int BN, int GATED>
 void launch_bn(const Bf16Product &p, int m, cudaStream_t st, DevErr *err) {
   using L = GbSmem<BN>;
-  CUtensorMap ma, mw;
+  CUtensorMap ma, mw, mh{}, mf{};
   tc_make_map_bf16(&ma, p.a, (unsigned long long)m, (unsigned long long)p.k, (unsigned long long)p.a_ld, TC_BM);
   tc_make_map_bf16(&mw, p.w, (unsigned long long)p.n, (unsigned long long)p.k, (unsigned long long)p.w_ld, BN);
-  LB_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+  const int halves = GATED ? p.n_half / 2 : p.n_half, floats = p.n - p.n_half;
+  const bool half_tma = halves > 0 && p.half_ld % 8 == 0 && (reinterpret_cast<uintptr_t>(p.half_out) & 15) == 0;
+  const bool float_tma = floats > 0 && p.float_ld % 4 == 0 && p.n_half % 4 == 0 &&
+                         (reinterpret_cast<uintptr_t>(p.float_out) & 15) == 0;
+  if (half_tma) tc_make_store_map(&mh, p.half_out, true, (unsigned long long)m, (unsigned long long)halves,
+                                  (unsigned long long)p.half_ld, GATED ? 16 : 32);
+  if (float_tma) tc_make_store_map(&mf, p.float_out, false, (unsigned long long)m, (unsigned long long)floats,
+                                   (unsigned long long)p.float_ld, 32);
+  LB_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<BN, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
   const int mt = (m + TC_BM - 1) / TC_BM, nt = (p.n + BN - 1) / BN;
   const long long tiles = (long long)mt * nt;
   const unsigned grid = (unsigned)(tiles < device_sms() ? tiles : device_sms());
-  launch_pdl(gemm_bf16_kernel<BN>, dim3(grid), dim3(GB_THREADS), L::TOTAL, st, false, ma, mw, p, m, mt, nt, err);
+  launch_pdl(gemm_bf16_kernel<BN, GATED>, dim3(grid), dim3(GB_THREADS), L::TOTAL, st, false, ma, mw, mh, mf, half_tma ? 1 : 0,
+             float_tma ? 1 : 0, p, m, mt, nt, err);
+}
+
+template <int BN>
+void launch_form(const Bf16Product &p, int m, cudaStream_t st, DevErr *err) {
+  if (p.gated) launch_bn<BN, 1>(p, m, st, err);
+  else launch_bn<BN, 0>(p, m, st, err);
 }
 
 }  // namespace
@@ -278,9 +327,9 @@ void launch_gemm_bf16(const Bf16Product &p, int m, cudaStream_t st, DevErr *err)
   // the widest tile that still gives most SMs one
   const long long mt = (m + TC_BM - 1) / TC_BM;
   const long long sms = device_sms();
-  if (p.n > 128 && mt * ((p.n + 255) / 256) >= sms * 3 / 4) launch_bn<256>(p, m, st, err);
-  else if (p.n > 64 && mt * ((p.n + 127) / 128) >= sms * 3 / 4) launch_bn<128>(p, m, st, err);
-  else launch_bn<64>(p, m, st, err);
+  if (p.n > 128 && mt * ((p.n + 255) / 256) >= sms * 3 / 4) launch_form<256>(p, m, st, err);
+  else if (p.n > 64 && mt * ((p.n + 127) / 128) >= sms * 3 / 4) launch_form<128>(p, m, st, err);
+  else launch_form<64>(p, m, st, err);
 }
 
 }  // namespace lb

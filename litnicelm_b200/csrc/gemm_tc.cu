@@ -664,6 +664,27 @@ void tc_make_map_bf16(CUtensorMap *map, const void *base, unsigned long long row
     throw std::runtime_error("litnice_b200: cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
 }
 
+// Results that leave by TMA: boxes of 32 rows, their rows swizzled over the row's own length.
+void tc_make_store_map(CUtensorMap *map, void *base, bool half, unsigned long long rows, unsigned long long cols,
+                       unsigned long long ld, unsigned box_cols) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (fn == nullptr) throw std::runtime_error("litnice_b200: cuTensorMapEncodeTiled is not available");
+  const unsigned size = half ? 2 : 4, row = box_cols * size;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (ld * size) % 16 != 0 || cols > ld || rows == 0 || cols == 0 ||
+      (row != 32 && row != 64 && row != 128))
+    throw std::invalid_argument("litnice_b200: a result stored by TMA must have 16-byte aligned rows");
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {ld * size};
+  const cuuint32_t box[2] = {box_cols, 32};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = fn(map, half ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides,
+                        box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        row == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : row == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    throw std::runtime_error("litnice_b200: cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
+}
+
 // How many clusters of 2..8 CTAs of these kernels the device holds at once (a cluster sits inside
 // one GPC); -1 where the runtime cannot say. Every configuration runs one CTA per SM, so one of them
 // stands for all.

@@ -104,6 +104,8 @@ void tc_make_map_plain(CUtensorMap *map, const float *base, unsigned long long r
 // [rows, cols] reads as zero.
 void tc_make_map_bf16(CUtensorMap *map, const void *base, unsigned long long rows, unsigned long long cols,
                       unsigned long long ld, unsigned box_rows);
+void tc_make_store_map(CUtensorMap *map, void *base, bool half, unsigned long long rows, unsigned long long cols,
+                       unsigned long long ld, unsigned box_cols);
 
 // How one product is tiled: tile width (64, 128 or 256 columns), how many CTAs share
 // the k range of a tile, and the scratch that sharing needs (floats of partial

@@ -90,6 +90,28 @@ __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap *map
 __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap *map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
+// Tiles from this CTA's shared memory to global memory, and the same added to what is there (32-bit floats, each
+// sum rounded once). Issued by one thread, in groups of its own: the box must stay in shared memory until
+// bulk_wait_read says so. Starts at non-negative coordinates, x on a 16-byte boundary; clipped at the map's extents.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, unsigned src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
+               ::"l"(map), "r"(x), "r"(y), "r"(src)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void tma_add_2d(const CUtensorMap *map, unsigned src, int x, int y) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
+               ::"l"(map), "r"(x), "r"(y), "r"(src)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() {  // at most N of this thread's newest groups still read shared memory
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void bulk_wait_all() {  // this thread's groups are complete
+  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
 // Untiled bulk copy global -> this CTA's shared memory, completion counted in bytes on an
 // mbarrier. Both addresses 16-byte aligned, the size a multiple of 16 bytes.
 __device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigned bytes, unsigned bar) {

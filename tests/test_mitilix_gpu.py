@@ -70,6 +70,28 @@ def test_product_over_many_tiles_and_a_long_k():
         assert rms_rel(bf16_product_host(a, w, 1), a.astype(np.float64) @ w.T.astype(np.float64)) < 1e-4
 
 
+@pytest.mark.parametrize("m,n,n_half", [(1000, 3600, 3600), (1000, 3600, 1808), (1000, 3601, 2008), (1025, 3590, 36),
+                                        (2080, 1030, 0), (1999, 1040, 520)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_product_stored_by_tile(m, n, n_half, gated):
+    """Every way a tile's columns leave: bfloat16, pairs, floats stored and added, the border between them inside a group of
+    32 columns, rows no tensor map can address. Sums of 72 products in 32 bits: 72 * 2^-24 of the terms' size, and bfloat16's
+    half unit in the last place."""
+    rng = np.random.default_rng(m + n + n_half)
+    k = 72
+    a, w = rounded(rng.standard_normal((m, k))), rounded(rng.standard_normal((n, k)) * k ** -0.5)
+    c = a.astype(np.float64) @ w.T.astype(np.float64)
+    first = om.gelu_exact(c[:, :n_half])
+    if gated:
+        first = om.gelu_exact(c[:, 0:n_half:2]) * c[:, 1:n_half:2]
+    old = rng.standard_normal((m, first.shape[1] + n - n_half)).astype(np.float32)
+    for acc in (None, old):
+        got = bf16_product_host(a, w, 1, n_half=n_half, act="gelu", gated=gated, c=acc)
+        rest = c[:, n_half:] + (0.0 if acc is None else old[:, first.shape[1]:])
+        assert n_half == 0 or np.abs(got[:, :first.shape[1]] - first).max() < 2 ** -8 * np.abs(first).max()
+        assert n_half == n or np.abs(got[:, first.shape[1]:] - rest).max() < 2e-5
+
+
 @pytest.mark.parametrize("taps", [1, 2, 3, 4, 5, 9, 13])
 @pytest.mark.parametrize("n,d,portions", [(1, 24, None), (37, 100, None), (37, 100, [1, 2, 3, 2, 11, 8, 9, 1]),
                                           (40, 260, [2] * 20), (40, 33, [16, 24])])
