@@ -34,6 +34,7 @@ struct Backend {
   long long launches = 0;
   void *scratch = nullptr;  // partial sums and row statistics of the training entries
   size_t scratch_bytes = 0;
+  SplitScratch split;  // operands of the large products
 
   // Deferred operators. The host issues one table call per operator and per attention head
   // (self_attention_fused_inplace.cpp:82-94: three calls per head; transformer_layer.cpp:79-86 and
@@ -155,6 +156,7 @@ void *api_create(uint32_t device_kind) {
   auto *b = new Backend();
   try {
     b->device = dev;
+    b->split.pdl = true;
     if (const char *env = std::getenv("LITNICE_B200_READ_AHEAD")) b->read_ahead = env[0] != '0';
     if (const char *env = std::getenv("LITNICE_B200_ABI_QUEUE")) b->queue_on = env[0] != '0';
     bind(b);
@@ -607,8 +609,7 @@ void run_gemm(Backend *b, const MatView &a, const MatView &bm, const MatView &c,
               const GemmEpilogue &ep = GemmEpilogue{}) {
   check_gemm(a, bm, c, who);
   bind(b);
-  launch_gemm_simt(a, bm, c, c.rows, c.cols, a.cols, ep, b->st);
-  ++b->launches;
+  b->launches += launch_gemm_f32(a, bm, c, false, ep, b->split, b->st, b->err_dev);
 }
 
 // device_backend.cpp:1096-1110
@@ -817,12 +818,11 @@ bool issue_heads_grouped(Backend *b, size_t at, long long n) {
     dense_sx.cs = 4;
     sx_all = with_heads(dense_sx, n, (long long)per_head * 4);
   }
-  launch_gemm_simt(with_heads(qa, n, dq), with_heads(kb, n, dk), sc_all, sc.rows, sc.cols, qa.cols, GemmEpilogue{},
-                   b->st);
+  b->launches += launch_gemm_f32(with_heads(qa, n, dq), with_heads(kb, n, dk), sc_all, false, GemmEpilogue{}, b->split, b->st,
+                                 b->err_dev);
   launch_softmax_rows(sx_all, with_heads(so, n, dw), 1, q[1].scale, b->st);
-  launch_gemm_simt(with_heads(wa, n, dw), with_heads(vb, n, dv), with_heads(co, n, dc), co.rows, co.cols, wa.cols,
-                   GemmEpilogue{}, b->st);
-  b->launches += 3;
+  b->launches += 1 + launch_gemm_f32(with_heads(wa, n, dw), with_heads(vb, n, dv), with_heads(co, n, dc), false,
+                                     GemmEpilogue{}, b->split, b->st, b->err_dev);
   if (shared_scores) {
     RowView last{};
     last.data = reinterpret_cast<char *>(b->queue_scratch + (size_t)(n - 1) * sc.rows * sc.cols);
@@ -1015,7 +1015,7 @@ void api_gemm_ranked_matrix_rhs_t(void *h, LitniceView a, LitniceView bb, Litnic
 }
 
 // device_backend.cpp:1154-1173: out[r, c] = sum over p and k of a[p, k, r] * b[p, k, c] (weight
-// gradients). One product per leading index, each added to the sum of those before it.
+// gradients).
 void api_gemm_ranked_reduce_lhs_t(void *h, LitniceView a, LitniceView bb, LitniceView out) {
   Backend *b = self(h);
   require_gpu_f32(a, "litnice_b200::gemm_ranked_reduce_lhs_t(a)");
@@ -1026,17 +1026,7 @@ void api_gemm_ranked_reduce_lhs_t(void *h, LitniceView a, LitniceView bb, Litnic
   if (av.batch != bv.batch || av.rows != bv.rows || ov.batch != 1 || ov.rows != av.cols || ov.cols != bv.cols)
     throw std::runtime_error("litnice_b200::gemm_ranked_reduce_lhs_t: shape mismatch");
   bind(b);
-  for (long long p = 0; p < av.batch; ++p) {
-    MatView ap = av, bp = bv;
-    ap.data = av.data + batch_offset(av, p);
-    bp.data = bv.data + batch_offset(bv, p);
-    ap.nb = bp.nb = 0;
-    ap.batch = bp.batch = 1;
-    GemmEpilogue ep;
-    if (p > 0) ep.residual = reinterpret_cast<const float *>(ov.data);  // in place: every element by one thread
-    launch_gemm_simt(transposed(ap), bp, ov, ov.rows, ov.cols, av.rows, ep, b->st);
-    ++b->launches;
-  }
+  b->launches += launch_gemm_f32(transposed(av), bv, ov, true, GemmEpilogue{}, b->split, b->st, b->err_dev);
 }
 
 // device_backend.cpp:1195-1214: out[p] = a[p]^T * b[p]

@@ -1,0 +1,628 @@
+// fp32-grade matrix products on the tensor cores for operands of any strides (sm_100a, tcgen05 + TMEM + TMA):
+//     C[b] = A[b] B[b] (+ bias) (+ residual) (ReLU),    or C = sum over p of A[p] B[p]
+// the products of the plugin table (litnicelm src/model/backend/device_backend.cpp:1096-1235) and of the 32-bit form of the
+// registered designs, where they are large enough (gemm_f32_scratch_bytes).
+//
+// Two kernels. split_operands_kernel writes both operands as TF32 pairs x = hi + lo (22 bits, any exponent) in K-major rows,
+// which TMA can address whatever the operands' strides were. gemm_split_kernel adds a_lo b_hi + a_hi b_lo + a_hi b_hi. The
+// tensor pipe truncates when it accumulates, so a chain in tensor memory is one block of 32 k (12 instructions); the chains are
+// added in registers with rounding to nearest. Where an operand holds a value that a pair cannot (infinite, NaN, or so large
+// that it rounds to infinity) the product is computed with plain fused multiply-adds in the order of k instead, so such values
+// come out as they do there. Parts below 2^-126 count as zero.
+//
+// gemm_split_kernel: persistent, one CTA of 10 warps per SM, tiles of 128 x BN:
+//   warp 0      one lane issues the TMA loads (a ring of 3 or 4 stages of four operand tiles)
+//   warp 1      owns tensor memory; one lane issues tcgen05.mma
+//   warps 2-9   add finished chains (lane = row, half of the columns) and store the tile while the next one is multiplied
+// Few tiles: k is cut into ranges, the CTAs of a tile form a cluster and each stores a share of the rows from the sums of all,
+// read over distributed shared memory in rank order. Every wait is bounded.
+//
+// Bound: shared memory (a block of 32 k of a 128 x 128 tile is read 12 x 8 KB and written 64 KB, 1280 clocks at 128 bytes; 1630
+// measured) and, for short k, the first loads and the last store of a CTA. 4096^3: 180 TFLOP/s (41 on the tile kernel). A training
+// step of 8 x 250 tokens (width 512, two layers) takes 3.8 ms, 7.0 with the tile kernel. Splitting inside the product's own
+// loading warps instead of a kernel in front (one launch less) measured 134 TFLOP/s at 4096^3 and 52 us against 39 at
+// 2000 x 1536 x 512: two loading warps per scheduler do not hide their latency, four leave too few registers.
+#include "gemm_tc.cuh"
+#include "tc_ptx.cuh"
+
+namespace lb {
+
+namespace {
+
+constexpr int GS_BM = 128, GS_BK = 32, GS_SMS = 148;
+constexpr int GS_ADDERS = 8;
+constexpr int GS_THREADS = 64 + 32 * GS_ADDERS;
+constexpr int GS_CHAINS = 4;  // accumulation chains in flight
+
+template <int BN>
+struct GsSmem {
+  static constexpr int STAGES = BN == 128 ? 3 : 4;
+  static constexpr int A_BYTES = GS_BM * 128;
+  static constexpr int B_BYTES = BN * 128;
+  static constexpr int STAGE = 2 * (A_BYTES + B_BYTES);
+  static constexpr int LD = BN + 4;  // floats per row of a finished range of k, which overlays the stages
+  static constexpr int PATCH_OFF = STAGES * STAGE;  // 2 KB per adding warp: 32 rows of 16 columns
+  static constexpr int BAR_OFF = PATCH_OFF + GS_ADDERS * 2048;
+  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+  static_assert(GS_BM * LD * 4 <= STAGES * STAGE, "the finished range lies over the stages");
+};
+
+struct GsOperand {
+  const float *p;
+  long long outer, k;  // element strides
+  int n;               // outer extent
+  int vec;             // rows of k on 16-byte boundaries
+  float *hi, *lo;      // [batch or 1][n][ld]
+  MatView view;        // batch axes
+  int batch;
+};
+
+struct GsArgs {
+  GsOperand a, b;
+  float *c;
+  const float *residual, *bias;
+  long long c_rs, c_cs;
+  int m, n, k, kp, sums;  // k of one summand, padded to a multiple of 32, and the number of summands
+  int kblocks, relu, c_vec, splits, m_tiles, n_tiles, tiles;
+  MatView cv;
+  int *bad, seq;  // *bad == seq: an operand of this product holds a value that a pair cannot
+};
+
+// x = hi + lo, both rounded to nearest at 11 bits (the tensor pipe ignores the 13 bits below). The integer addition rounds as
+// cvt.rna.tf32 does and issues at full rate.
+__device__ __forceinline__ void gs_split(float x, float &hi, float &lo) {
+  hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
+  lo = __uint_as_float(__float_as_uint(x - hi) + 0x1000u);
+}
+
+// One tile of 32 rows x 64 k of one operand: read along whichever axis is contiguous, written as rows of k.
+__global__ void __launch_bounds__(256) split_operands_kernel(const __grid_constant__ GsArgs g, int a_blocks) {
+  __shared__ float tile[32][65];
+  pdl_launch_dependents();
+  pdl_wait();
+  const bool first = (int)blockIdx.x < a_blocks;
+  const GsOperand &o = first ? g.a : g.b;
+  const int k_tiles = (g.kp + 63) / 64, r_tiles = (o.n + 31) / 32;
+  int at = (int)blockIdx.x - (first ? 0 : a_blocks);
+  const int k0 = at % k_tiles * 64;
+  at /= k_tiles;
+  const int r0 = at % r_tiles * 32, batch = at / r_tiles, tid = threadIdx.x;
+  const float *src = reinterpret_cast<const float *>(reinterpret_cast<const char *>(o.p) + batch_offset(o.view, batch));
+  const long long ld = (long long)g.kp * g.sums;
+  const long long to0 = g.sums > 1 ? (long long)batch * g.kp : (long long)batch * o.n * ld;
+  float4 x[2];
+  const int piece = tid & 15, k = k0 + piece * 4;
+  if (o.vec && o.k == 1) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = r0 + (tid >> 4) + i * 16;
+      x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < o.n) {
+        const float *p = src + (long long)r * o.outer + k;
+        if (k + 4 <= g.k) {
+          x[i] = *reinterpret_cast<const float4 *>(p);
+        } else {
+          if (k < g.k) x[i].x = p[0];
+          if (k + 1 < g.k) x[i].y = p[1];
+          if (k + 2 < g.k) x[i].z = p[2];
+        }
+      }
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int e = tid + i * 256;
+      const int r = o.k == 1 ? e >> 6 : e & 31, kk = o.k == 1 ? e & 63 : e >> 5;
+      tile[r][kk] = r0 + r < o.n && k0 + kk < g.k ? src[(long long)(r0 + r) * o.outer + (long long)(k0 + kk) * o.k] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float *p = &tile[(tid >> 4) + i * 16][piece * 4];
+      x[i] = make_float4(p[0], p[1], p[2], p[3]);
+    }
+  }
+  float bad = 0.f;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = r0 + (tid >> 4) + i * 16;
+    if (r >= o.n || k >= g.kp) continue;
+    float4 h, l;
+    gs_split(x[i].x, h.x, l.x);
+    gs_split(x[i].y, h.y, l.y);
+    gs_split(x[i].z, h.z, l.z);
+    gs_split(x[i].w, h.w, l.w);
+    bad = fmaf(l.x, 0.f, fmaf(l.y, 0.f, fmaf(l.z, 0.f, fmaf(l.w, 0.f, bad))));  // not a number where lo is not finite
+    const long long to = to0 + (long long)r * ld + k;
+    *reinterpret_cast<float4 *>(o.hi + to) = h;
+    *reinterpret_cast<float4 *>(o.lo + to) = l;
+  }
+  if (bad != bad) *g.bad = g.seq;
+}
+
+// Four results of a row, from column col on, through the epilogue to C.
+__device__ __forceinline__ void gs_store4(const GsArgs &g, float *C, const float *R, int row, int col, float4 x) {
+  float v[4] = {x.x, x.y, x.z, x.w};
+  const long long at = (long long)row * g.c_rs;
+  if (g.c_vec && col + 3 < g.n) {
+    if (g.bias) {
+      const float4 t = *reinterpret_cast<const float4 *>(g.bias + col);
+      v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
+    }
+    if (R) {
+      const float4 t = *reinterpret_cast<const float4 *>(R + at + col);
+      v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
+    }
+    if (g.relu) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = v[j] > 0.f ? v[j] : 0.f;
+    }
+    *reinterpret_cast<float4 *>(C + at + col) = make_float4(v[0], v[1], v[2], v[3]);
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (col + j >= g.n) break;
+    const long long to = at + (long long)(col + j) * g.c_cs;
+    float o = v[j];
+    if (g.bias) o += g.bias[col + j];
+    if (R) o += R[to];
+    if (g.relu) o = o > 0.f ? o : 0.f;
+    C[to] = o;
+  }
+}
+
+// Four elements of a row the way they would be without pairs.
+__device__ __noinline__ float4 gs_plain4(const GsArgs &g, long long batch, int row, int col) {
+  float v[4];
+  for (int j = 0; j < 4; ++j) {
+    float s = 0.f;
+    for (int of = 0; of < g.sums && col + j < g.n; ++of) {
+      const long long at = g.sums > 1 ? of : batch;
+      const float *x = reinterpret_cast<const float *>(reinterpret_cast<const char *>(g.a.p) + batch_offset(g.a.view, at)) +
+                       (long long)row * g.a.outer;
+      const float *y = reinterpret_cast<const float *>(reinterpret_cast<const char *>(g.b.p) + batch_offset(g.b.view, at)) +
+                       (long long)(col + j) * g.b.outer;
+      for (int k = 0; k < g.k; ++k) s = fmaf(x[(long long)k * g.a.k], y[(long long)k * g.b.k], s);
+    }
+    v[j] = s;
+  }
+  return make_float4(v[0], v[1], v[2], v[3]);
+}
+
+template <int BN>
+__global__ void __launch_bounds__(GS_THREADS, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ CUtensorMap a_lo,
+                  const __grid_constant__ CUtensorMap b_hi, const __grid_constant__ CUtensorMap b_lo,
+                  const __grid_constant__ GsArgs g, DevErr *err) {
+  using L = GsSmem<BN>;
+  constexpr int S = L::STAGES, CW = BN / 2;  // columns of an adding warp
+  extern __shared__ unsigned char smem_raw[];
+  const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  unsigned char *base_ptr = smem_raw + (base - smem_u32(smem_raw));
+  const unsigned bars = base + L::BAR_OFF;
+  auto full = [&](int s) { return bars + 8u * s; };
+  auto empty = [&](int s) { return bars + 8u * (S + s); };
+  auto chain_full = [&](int b) { return bars + 8u * (2 * S + b); };
+  auto chain_empty = [&](int b) { return bars + 8u * (2 * S + GS_CHAINS + b); };
+  const unsigned done = bars + 8u * (2 * S + 2 * GS_CHAINS);
+  volatile unsigned *tmem_holder = reinterpret_cast<volatile unsigned *>(base_ptr + L::BAR_OFF + 192);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(base_ptr + L::BAR_OFF + 196);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)blockIdx.x % g.splits, cta = (int)blockIdx.x / g.splits, ctas = (int)gridDim.x / g.splits;
+  const int each = (g.kblocks + g.splits - 1) / g.splits;
+  const int first = min(g.kblocks, rank * each), count = min(g.kblocks, first + each) - first;
+  auto place = [&](int tile, int &batch, int &m0, int &n0) {
+    const int per = g.m_tiles * g.n_tiles, rest = tile % per;
+    batch = tile / per;
+    m0 = rest % g.m_tiles * GS_BM;
+    n0 = rest / g.m_tiles * BN;
+  };
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(full(s), 1);
+      mbar_init(empty(s), 1);
+    }
+    for (int b = 0; b < GS_CHAINS; ++b) {
+      mbar_init(chain_full(b), 1);
+      mbar_init(chain_empty(b), GS_ADDERS);
+    }
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void *)tmem_holder)),
+                 "r"((unsigned)(GS_CHAINS * BN))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const unsigned tmem = *tmem_holder;
+  pdl_launch_dependents();
+  pdl_wait();
+  const bool plain = *g.bad == g.seq;
+
+  if (warp == 0) {
+    int it = 0;
+    bool ok = true;
+    for (int tile = cta; tile < g.tiles && ok; tile += ctas) {
+      int batch, m0, n0;
+      place(tile, batch, m0, n0);
+      if (g.sums == 1) {
+        m0 += batch * g.m;
+        if (g.b.batch > 1) n0 += batch * g.n;
+      }
+      for (int kb = first; kb < first + count; ++kb, ++it) {
+        const int s = it % S;
+        ok = mbar_wait_warp(empty(s), ((unsigned)(it / S) & 1u) ^ 1u, abort_flag, err, 51);
+        if (!ok) break;
+        if (lane == 0) {
+          const unsigned st = base + (unsigned)(s * L::STAGE);
+          mbar_expect_tx(full(s), (unsigned)L::STAGE);
+          tma_load_2d(st, &a_hi, kb * GS_BK, m0, full(s));
+          tma_load_2d(st + L::A_BYTES, &a_lo, kb * GS_BK, m0, full(s));
+          tma_load_2d(st + 2 * L::A_BYTES, &b_hi, kb * GS_BK, n0, full(s));
+          tma_load_2d(st + 2 * L::A_BYTES + L::B_BYTES, &b_lo, kb * GS_BK, n0, full(s));
+        }
+        __syncwarp();
+      }
+    }
+    if (*abort_flag) {  // copies in flight must land before the shared memory goes away
+      for (int j = it > S ? it - S : 0; j < it; ++j) {
+        const unsigned long long t0 = global_timer();
+        while (!mbar_try_wait(full(j % S), (unsigned)(j / S) & 1u))
+          if (global_timer() - t0 > WAIT_LIMIT_NS) break;
+      }
+    }
+  } else if (warp == 1) {
+    constexpr unsigned idesc = umma_idesc_tf32(BN);
+    int it = 0;
+    bool ok = true;
+    for (int tile = cta; tile < g.tiles && ok; tile += ctas) {
+      for (int kb = 0; kb < count; ++kb, ++it) {
+        const int s = it % S, buf = it % GS_CHAINS;
+        ok = mbar_wait_warp(chain_empty(buf), ((unsigned)(it / GS_CHAINS) & 1u) ^ 1u, abort_flag, err, 52) &&
+             mbar_wait_warp(full(s), (unsigned)(it / S) & 1u, abort_flag, err, 53);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (lane == 0) {
+          const unsigned st = base + (unsigned)(s * L::STAGE), d = tmem + (unsigned)(buf * BN);
+          const unsigned long long ah = umma_desc_k128(st), al = umma_desc_k128(st + L::A_BYTES),
+                                   bh = umma_desc_k128(st + 2 * L::A_BYTES),
+                                   bl = umma_desc_k128(st + 2 * L::A_BYTES + L::B_BYTES);
+#pragma unroll
+          for (unsigned ks = 0; ks < 8; ks += 2) tc_mma_tf32(d, al + ks, bh + ks, idesc, ks ? 1u : 0u);
+#pragma unroll
+          for (unsigned ks = 0; ks < 8; ks += 2) tc_mma_tf32(d, ah + ks, bl + ks, idesc, 1u);
+#pragma unroll
+          for (unsigned ks = 0; ks < 8; ks += 2) tc_mma_tf32(d, ah + ks, bh + ks, idesc, 1u);
+          tc_commit(empty(s));
+          tc_commit(chain_full(buf));
+        }
+        __syncwarp();
+      }
+    }
+    if (!ok) {  // what was issued ends, within the limit, before the shared memory goes away
+      if (lane == 0) tc_commit(done);
+      __syncwarp();
+      const unsigned long long t0 = global_timer();
+      while (!mbar_try_wait(done, 0u))
+        if (global_timer() - t0 > WAIT_LIMIT_NS) break;
+    }
+  } else {
+    const int q = warp & 3, half = (warp - 2) >> 2, piece = lane & 3;
+    float4 *patch = reinterpret_cast<float4 *>(base_ptr + L::PATCH_OFF) + (warp - 2) * 128;
+    int it = 0;
+    bool ok = true;
+    for (int tile = cta; tile < g.tiles && ok; tile += ctas) {
+      float acc[CW];
+#pragma unroll
+      for (int j = 0; j < CW; ++j) acc[j] = 0.f;
+      for (int kb = 0; kb < count; ++kb, ++it) {
+        const int buf = it % GS_CHAINS;
+        ok = mbar_wait_warp(chain_full(buf), (unsigned)(it / GS_CHAINS) & 1u, abort_flag, err, 54);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int c0 = 0; c0 < CW; c0 += 32) {
+          unsigned r[32];
+          tc_ld32(tmem + ((unsigned)(q * 32) << 16) + (unsigned)(buf * BN + half * CW + c0), r);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 32; ++j) acc[c0 + j] = __fadd_rn(acc[c0 + j], __uint_as_float(r[j]));
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(chain_empty(buf));
+      }
+      if (g.splits > 1) {  // every product has been read: the range's sums may lie over the stages
+        float *sums = reinterpret_cast<float *>(base_ptr) + (q * 32 + lane) * L::LD + half * CW;
+#pragma unroll
+        for (int j = 0; j < CW; j += 4)
+          *reinterpret_cast<float4 *>(sums + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+        break;
+      }
+      int batch, m0, n0;
+      place(tile, batch, m0, n0);
+      const long long c_off = batch_offset(g.cv, batch);
+      float *C = reinterpret_cast<float *>(reinterpret_cast<char *>(g.c) + c_off);
+      const float *R = g.residual ? reinterpret_cast<const float *>(reinterpret_cast<const char *>(g.residual) + c_off) : nullptr;
+#pragma unroll
+      for (int c0 = 0; c0 < CW; c0 += 16) {  // 16 columns at a time, turned so that four lanes store a row's 64 bytes
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          patch[lane * 4 + (j ^ ((lane >> 1) & 3))] =
+              make_float4(acc[c0 + 4 * j], acc[c0 + 4 * j + 1], acc[c0 + 4 * j + 2], acc[c0 + 4 * j + 3]);
+        __syncwarp();
+        const int col = n0 + half * CW + c0 + piece * 4;
+#pragma unroll 1
+        for (int pass = 0; pass < 4; ++pass) {
+          const int rr = pass * 8 + (lane >> 2), row = m0 + q * 32 + rr;
+          if (row >= g.m || col >= g.n) continue;
+          float4 x = patch[rr * 4 + (piece ^ ((rr >> 1) & 3))];
+          if (plain) x = gs_plain4(g, batch, row, col);
+          gs_store4(g, C, R, row, col, x);
+        }
+        __syncwarp();
+      }
+    }
+  }
+  __syncwarp();
+  if (g.splits > 1) {  // one tile, its ranges of k over the CTAs of the cluster
+    cluster_sync_all();
+    int batch, m0, n0;
+    place(cta, batch, m0, n0);
+    const long long c_off = batch_offset(g.cv, batch);
+    float *C = reinterpret_cast<float *>(reinterpret_cast<char *>(g.c) + c_off);
+    const float *R = g.residual ? reinterpret_cast<const float *>(reinterpret_cast<const char *>(g.residual) + c_off) : nullptr;
+    const int rows_each = (GS_BM + g.splits - 1) / g.splits;
+    const int row_end = min(min(GS_BM, (rank + 1) * rows_each), g.m - m0);
+    constexpr int LANES = BN / 4;  // threads to a row
+    const int c4 = ((int)threadIdx.x % LANES) * 4, col = n0 + c4;
+    for (int row = rank * rows_each + (int)threadIdx.x / LANES; row < row_end && col < g.n; row += GS_THREADS / LANES) {
+      const unsigned at = base + (unsigned)(row * L::LD + c4) * 4u;
+      float4 x = ld_cluster_f4(cluster_map(at, 0u));
+      for (int r = 1; r < g.splits; ++r) {
+        const float4 y = ld_cluster_f4(cluster_map(at, (unsigned)r));
+        x = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+      }
+      if (plain) x = gs_plain4(g, batch, m0 + row, col);
+      gs_store4(g, C, R, m0 + row, col, x);
+    }
+    __syncwarp();
+    cluster_sync_all();  // no peer reads these sums any more
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((unsigned)(GS_CHAINS * BN)));
+  }
+}
+
+bool on16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+bool batch_on16(const MatView &v) {
+  for (int i = 0; i < v.nb; ++i)
+    if ((v.bs[i] & 15) != 0) return false;
+  return true;
+}
+
+GsOperand operand(const MatView &v, long long outer, long long k, int n) {
+  GsOperand o{};
+  o.p = reinterpret_cast<const float *>(v.data);
+  o.outer = outer / 4;
+  o.k = k / 4;
+  o.n = n;
+  o.vec = on16(v.data) && batch_on16(v) && (o.outer & 3) == 0;
+  o.view = v;
+  o.batch = (int)v.batch;
+  return o;
+}
+
+// The innermost batch axis becomes rows where it continues them in both operands.
+void fold(MatView &a, MatView &c) {
+  while (a.nb > 0 && a.nb == c.nb && a.bd[a.nb - 1] == c.bd[c.nb - 1] && a.bs[a.nb - 1] == a.rows * a.rs &&
+         c.bs[c.nb - 1] == c.rows * c.rs && a.rows * a.bd[a.nb - 1] < (1ll << 30)) {
+    const long long n = a.bd[a.nb - 1];
+    for (MatView *v : {&a, &c}) {
+      v->rows *= n;
+      v->batch /= n;
+      --v->nb;
+    }
+  }
+}
+
+void turn(MatView &v) {
+  std::swap(v.rows, v.cols);
+  std::swap(v.rs, v.cs);
+}
+
+// Tile width and ranges of k by the time of the longest CTA: blocks of k at what they were measured to take (in clocks: 1630
+// at 128 columns, 1100 at 64), the store of the last tile, and for ranges the exchange of their sums.
+struct Plan {
+  int bn, splits, tiles;
+};
+Plan make_plan(long long batch, int m, int n, int kblocks) {
+  Plan best{64, 1, 0};
+  double least = 1e30;
+  const long long mt = (m + GS_BM - 1) / GS_BM;
+  for (int bn : {64, 128}) {
+    if (bn == 128 && n <= 64) continue;
+    const long long tiles = batch * mt * ((n + bn - 1) / bn);
+    if (tiles > (1 << 30)) throw std::invalid_argument("litnice_b200: product too large");
+    const double block = bn == 128 ? 1630 : 1100;
+    for (int s = 1; s <= 8; ++s) {
+      if (s > 1 && (tiles * s > GS_SMS || kblocks < 3 * s)) break;
+      const int each = (kblocks + s - 1) / s;
+      if ((kblocks + each - 1) / each != s) continue;  // no empty range
+      const double waves = s > 1 ? 1.0 : (double)((tiles + GS_SMS - 1) / GS_SMS);
+      const double t = waves * each * block + 3000 + (s > 1 ? 2500 + 500 * s : 0);
+      if (t < least) {
+        least = t;
+        best = Plan{bn, s, (int)tiles};
+      }
+    }
+  }
+  return best;
+}
+
+template <int BN>
+void launch_tile(const GsArgs &g, bool pdl, cudaStream_t st, DevErr *err) {
+  CUtensorMap ah, al, bh, bl;
+  const unsigned long long ld = (unsigned long long)g.kp * g.sums;
+  const unsigned long long ra = (unsigned long long)g.m * (g.sums > 1 ? 1 : g.a.batch), rb = (unsigned long long)g.n * (g.sums > 1 ? 1 : g.b.batch);
+  tc_make_map(&ah, g.a.hi, ra, ld, GS_BM);
+  tc_make_map(&al, g.a.lo, ra, ld, GS_BM);
+  tc_make_map(&bh, g.b.hi, rb, ld, BN);
+  tc_make_map(&bl, g.b.lo, rb, ld, BN);
+  LB_CUDA(cudaFuncSetAttribute(gemm_split_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, GsSmem<BN>::TOTAL));
+  const int ctas = g.splits > 1 || g.tiles < GS_SMS ? g.tiles : GS_SMS;
+  launch_pdl_cluster_x(gemm_split_kernel<BN>, dim3((unsigned)(ctas * g.splits)), dim3(GS_THREADS), (size_t)GsSmem<BN>::TOTAL,
+                       st, pdl, (unsigned)g.splits, ah, al, bh, bl, g, err);
+}
+
+constexpr long long GS_ROWS = 16384;  // rows of A per launch: bounds the pairs' memory
+
+void launch_gemm_split(MatView a, MatView b, MatView c, bool sum_batches, const GemmEpilogue &ep, void *scratch, int seq,
+                       bool pdl, cudaStream_t st, DevErr *err) {
+  GsArgs g{};
+  g.m = (int)a.rows;
+  g.n = (int)b.cols;
+  g.k = (int)a.cols;
+  g.kp = (g.k + GS_BK - 1) / GS_BK * GS_BK;
+  g.sums = sum_batches ? (int)a.batch : 1;
+  g.a = operand(a, a.rs, a.cs, g.m);
+  g.b = operand(b, b.cs, b.rs, g.n);
+  g.bad = static_cast<int *>(scratch);
+  g.seq = seq;
+  float *pairs = reinterpret_cast<float *>(static_cast<char *>(scratch) + 256);
+  const long long na = (long long)g.m * g.kp * g.a.batch, nb = (long long)g.n * g.kp * g.b.batch;
+  g.a.hi = pairs;
+  g.a.lo = pairs + na;
+  g.b.hi = pairs + 2 * na;
+  g.b.lo = pairs + 2 * na + nb;
+  g.c = reinterpret_cast<float *>(c.data);
+  g.residual = ep.residual;
+  g.bias = ep.bias;
+  g.relu = ep.relu;
+  g.c_rs = c.rs / 4;
+  g.c_cs = c.cs / 4;
+  g.cv = c;
+  g.c_vec = g.c_cs == 1 && (g.c_rs & 3) == 0 && on16(c.data) && batch_on16(c) && (!ep.residual || on16(ep.residual)) &&
+            (!ep.bias || on16(ep.bias));
+  g.kblocks = g.kp / GS_BK * g.sums;
+  const Plan plan = make_plan(c.batch, g.m, g.n, g.kblocks);
+  g.splits = plan.splits;
+  g.tiles = plan.tiles;
+  g.m_tiles = (g.m + GS_BM - 1) / GS_BM;
+  g.n_tiles = (g.n + plan.bn - 1) / plan.bn;
+  const long long k_tiles = (g.kp + 63) / 64;
+  const long long a_blocks = (g.m + 31) / 32 * k_tiles * g.a.batch, b_blocks = (g.n + 31) / 32 * k_tiles * g.b.batch;
+  launch_pdl(split_operands_kernel, dim3((unsigned)(a_blocks + b_blocks)), dim3(256), 0, st, pdl, g, (int)a_blocks);
+  if (plan.bn == 128) launch_tile<128>(g, pdl, st, err);
+  else launch_tile<64>(g, pdl, st, err);
+}
+
+}  // namespace
+
+SplitScratch::~SplitScratch() {
+  if (p) cudaFree(p);
+}
+
+bool SplitScratch::ensure(size_t need, cudaStream_t st) {
+  if (need <= bytes) return true;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) return false;
+  if (p) {
+    LB_CUDA(cudaStreamSynchronize(st));
+    cudaFree(p);
+    p = nullptr;
+    bytes = 0;
+  }
+  const size_t grown = need + need / 4;
+  if (cudaMalloc(&p, grown) != cudaSuccess) {
+    p = nullptr;
+    (void)cudaGetLastError();
+    return false;
+  }
+  bytes = grown;
+  LB_CUDA(cudaMemsetAsync(p, 0, 256, st));
+  return true;
+}
+
+// Measured on one B200, both ways, launches back to back in us (tile kernel -> two launches here): 64 x 64 x 64 6 -> 8,
+// 100 x 100 x 64 of 8 batches 7 -> 8.5, 128 x 128 x 128 9 -> 10, 256 x 256 x 256 16 -> 11, 250 x 250 x 64 of 64 batches
+// 32 -> 24, 64 x 512 x 512 29 -> 11, 613 x 3072 x 512 83 -> 25, 2000 x 512 x 2048 297 -> 59, 4096^3 3356 -> 763. The tile kernel is
+// bound by the latency of its k loop (0.05 us a k) where there are few tiles and by the FMA pipe where there are many; here the two
+// launches cost about 8 us and a block of 32 k about 0.6 us. Few rows against a large matrix: splitting the matrix costs more
+// than reading it (16 x 32000 x 1024 would write 262 MB). Below 128 k a sequential sum in 32 bits is as exact as pairs are
+// (k = 64: 1.05e-7 against 1.17e-7 on operands of one sign); from there on the pairs are (k = 250: 2.9e-7 against 1.5e-7,
+// k = 2048: 8.1e-7 against 1.7e-7; gradients of a training step, width 512: 1.12e-7 against 1.03e-7).
+size_t gemm_f32_scratch_bytes(long long m, long long n, long long k, long long a_batch, long long b_batch, bool sum_batches) {
+  const long long batch = a_batch, total_k = sum_batches ? k * a_batch : k;
+  if (m <= 0 || n <= 0 || k <= 0 || batch <= 0) return 0;
+  const double work = (double)m * n * k * batch;
+  if (total_k < 128) return 0;
+  if (work < 1 << 24 && !(total_k >= 256 && work >= 1 << 21)) return 0;
+  const double small = (double)(m < n ? m : n);
+  if (small < 64 && (double)(m < n ? n : m) * k > 4e6) return 0;
+  const long long kp = (k + GS_BK - 1) / GS_BK * GS_BK;
+  if ((double)m * a_batch > 1e9 || (double)n * b_batch > 1e9 || (double)kp * (sum_batches ? a_batch : 1) > 1e9) return 0;
+  const long long rows = sum_batches || b_batch > 1 || m < GS_ROWS ? m : GS_ROWS;
+  const double floats = 2.0 * kp * ((double)rows * a_batch + (double)n * b_batch);
+  if (floats * 4 > 4e9) return 0;
+  return (size_t)floats * 4 + 256;
+}
+
+int launch_gemm_f32(const MatView &a, const MatView &b, const MatView &c, bool sum_batches, const GemmEpilogue &ep,
+                    SplitScratch &scratch, cudaStream_t st, DevErr *err) {
+  if (a.rows <= 0 || b.cols <= 0) return 0;
+  MatView fa = a, fb = b, fc = c;
+  if (sum_batches) {  // summands may lie one behind another along k
+    turn(fa);
+    fold(fa, fb);
+    turn(fa);
+  } else if (b.batch == 1) {
+    fold(fa, fc);
+  }
+  const size_t need = gemm_f32_scratch_bytes(fa.rows, fb.cols, fa.cols, fa.batch, fb.batch, sum_batches);
+  if (need > 0 && scratch.ensure(need, st)) {
+    int launched = 0;
+    const long long part = fa.batch > 1 || sum_batches ? fa.rows : GS_ROWS;
+    for (long long r = 0; r < fa.rows; r += part) {
+      MatView pa = fa, pc = fc;
+      pa.rows = pc.rows = fa.rows - r < part ? fa.rows - r : part;
+      pa.data += r * fa.rs;
+      pc.data += r * fc.rs;
+      GemmEpilogue pe = ep;
+      if (pe.residual) pe.residual = reinterpret_cast<const float *>(reinterpret_cast<const char *>(pe.residual) + r * fc.rs);
+      if (++scratch.seq <= 0) scratch.seq = 1;
+      launch_gemm_split(pa, fb, pc, sum_batches, pe, scratch.p, scratch.seq, scratch.pdl || g_pdl_enabled, st, err);
+      launched += 2;
+    }
+    return launched;
+  }
+  if (!sum_batches) {
+    launch_gemm_simt(a, b, c, c.rows, c.cols, a.cols, ep, st);
+    return 1;
+  }
+  for (long long p = 0; p < a.batch; ++p) {  // each summand added to the sum of those before it
+    MatView ap = a, bp = b;
+    ap.data += batch_offset(a, p);
+    bp.data += batch_offset(b, p);
+    ap.nb = bp.nb = 0;
+    ap.batch = bp.batch = 1;
+    GemmEpilogue pe = ep;
+    if (p > 0) pe.residual = reinterpret_cast<const float *>(c.data);  // in place: every element by one thread
+    launch_gemm_simt(ap, bp, c, c.rows, c.cols, a.cols, pe, st);
+  }
+  return (int)a.batch;
+}
+
+}  // namespace lb

@@ -325,6 +325,13 @@ class Gobesun final : public DecoderModel {
         }
       }
       moved |= scratch_.ensure(need * 4 + 16, st);
+      moved |= reserve_split(split_, rows, width_, vocab_, st);
+      for (const Layer &l : layers_) {
+        moved |= reserve_split(split_, rows, width_, in_ld(l), st);
+        moved |= reserve_split(split_, rows, l.o_cols(), width_, st);
+        if (l.ff) moved |= reserve_split(split_, rows, width_, l.ff, st);
+        if (l.ff) moved |= reserve_split(split_, rows, l.ff, width_, st);
+      }
     }
     return moved;
   }
@@ -374,7 +381,7 @@ class Gobesun final : public DecoderModel {
   // out[m, n] = a[m, k] w^T in float
   void product(const void *a, int a_ld, int k, const DevBuf &w, int n, float *out, int m, cudaStream_t st, DevErr *err) {
     if (prec_ == Precision::F32) {
-      launches_ += product_f32(static_cast<const float *>(a), m, k, w.f(), n, nullptr, out, scratch_.f(), st, err);
+      launches_ += product_f32(static_cast<const float *>(a), m, k, w.f(), n, nullptr, out, scratch_.f(), split_, st, err);
       return;
     }
     Bf16Product p;
@@ -396,7 +403,7 @@ class Gobesun final : public DecoderModel {
   void project(const Layer &l, const RowBatch &b, cudaStream_t st, DevErr *err) {
     const int m = (int)b.rows();
     if (prec_ == Precision::F32) {
-      launches_ += product_f32(h_.f(), m, width_, l.in.f(), in_ld(l), nullptr, in_.f(), scratch_.f(), st, err);
+      launches_ += product_f32(h_.f(), m, width_, l.in.f(), in_ld(l), nullptr, in_.f(), scratch_.f(), split_, st, err);
       return;
     }
     Bf16Product p;
@@ -476,8 +483,8 @@ class Gobesun final : public DecoderModel {
   void feed_forward(const Layer &l, const RowBatch &b, cudaStream_t st, DevErr *err) {
     const int m = (int)b.rows();
     if (prec_ == Precision::F32) {
-      launches_ += product_f32(h_.f(), m, width_, l.gate_up.f(), l.ff, nullptr, hidden_.f(), scratch_.f(), st, err);
-      launches_ += product_f32(h_.f(), m, width_, l.up.f(), l.ff, nullptr, factor_.f(), scratch_.f(), st, err);
+      launches_ += product_f32(h_.f(), m, width_, l.gate_up.f(), l.ff, nullptr, hidden_.f(), scratch_.f(), split_, st, err);
+      launches_ += product_f32(h_.f(), m, width_, l.up.f(), l.ff, nullptr, factor_.f(), scratch_.f(), split_, st, err);
       launch_activation_f32(hidden_.f(), factor_.f(), (long long)m * l.ff, ACT_GELU_TANH, st);
       ++launches_;
       product(hidden_.p, l.ff, l.ff, l.down, width_, y_.f(), m, st, err);
@@ -505,6 +512,7 @@ class Gobesun final : public DecoderModel {
   int in_max_ = 0, o_max_ = 0, ff_max_ = 0, q_max_ = 0, heads_max_ = 0;
   DevBuf embed_, head_, final_norm_;
   int slots_ = 0, cap_ = 0, launches_ = 0;
+  SplitScratch split_;
   DevBuf x_, y_, h_, in_, ba_, q_, mix_, hidden_, factor_, delta_, scratch_;
 };
 

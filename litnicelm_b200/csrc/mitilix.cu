@@ -221,6 +221,14 @@ class Mitilix final : public DecoderModel {
                          l.ff ? gemv_scratch_floats(8, width_, l.ff) : 0})
           need = n > need ? n : need;
       moved |= scratch_.ensure(need * 4 + 16, st);
+      moved |= reserve_split(split_, rows, width_, vocab_, st);
+      for (const Layer &l : layers_) {
+        moved |= reserve_split(split_, rows, width_, l.q_cols(), st);
+        moved |= reserve_split(split_, rows, width_, l.rank, st);
+        moved |= reserve_split(split_, rows, l.o_cols(), width_, st);
+        if (l.ff) moved |= reserve_split(split_, rows, width_, l.ff, st);
+        if (l.ff) moved |= reserve_split(split_, rows, l.ff, width_, st);
+      }
     }
     return moved;
   }
@@ -387,7 +395,7 @@ class Mitilix final : public DecoderModel {
 
   void product_f32(const float *a, int m, int k, const float *w, int n, const float *residual, float *out,
                    cudaStream_t st, DevErr *err) {
-    launches_ += lb::product_f32(a, m, k, w, n, residual, out, scratch_.f(), st, err);
+    launches_ += lb::product_f32(a, m, k, w, n, residual, out, scratch_.f(), split_, st, err);
   }
 
   void layer_f32(int i, const RowBatch &b, cudaStream_t st, DevErr *err) {
@@ -421,6 +429,7 @@ class Mitilix final : public DecoderModel {
   int window_max_ = 1, q_max_ = 0, rank_max_ = 0, ff_max_ = 0, o_max_ = 0, mix_max_ = 0;
   DevBuf embed_, pos_, head_;
   int slots_ = 0, cap_ = 0, launches_ = 0;
+  SplitScratch split_;
   long long decode_rows_ = 0;
   DevBuf x_, xl_, a1_, a2_, q_, dkv_, mix_, hidden_, scratch_;
   DevBuf packed_, k_, vt_;                    // latents, keys and transposed values of a portion's window

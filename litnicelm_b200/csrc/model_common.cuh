@@ -80,12 +80,18 @@ inline int products_bf16(const Bf16Product *p, int count, int m, cudaStream_t st
 
 // out[m, n] = a[m, k] w[k, n] (+ residual) on the float products; scratch: gemv_scratch_floats(8, n, k) floats.
 inline int product_f32(const float *a, int m, int k, const float *w, int n, const float *residual, float *out,
-                       float *scratch, cudaStream_t st, DevErr *err) {
+                       float *scratch, SplitScratch &split, cudaStream_t st, DevErr *err) {
   if (m <= 8) return launch_gemv(a, m, w, k, n, nullptr, out, scratch, st, err, residual);
   GemmEpilogue ep;
   ep.residual = residual;
-  launch_gemm_simt(dense_view(a, m, k), dense_view(w, k, n), dense_view(out, m, n), m, n, k, ep, st);
-  return 1;
+  return launch_gemm_f32(dense_view(a, m, k), dense_view(w, k, n), dense_view(out, m, n), false, ep, split, st, err);
+}
+
+// Room in `split` for product_f32 of up to `rows` rows; true when it moved.
+inline bool reserve_split(SplitScratch &split, long long rows, int k, int n, cudaStream_t st) {
+  const void *before = split.p;
+  split.ensure(gemm_f32_scratch_bytes(rows, n, k, 1, 1, false), st);
+  return split.p != before;
 }
 
 }  // namespace lb

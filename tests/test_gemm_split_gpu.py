@@ -1,0 +1,107 @@
+"""The plugin table's products at sizes that run on the tensor cores, against 64-bit sums: tile edges and remainders, strides
+of every kind, summed and batched operands, cut k ranges, epilogues, values that no operand pair holds."""
+import numpy as np
+import pytest
+
+from abi_util import Buffer
+from litnicelm_b200.plugin import Backend
+from training_util import dense, read
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def be():
+    b = Backend()
+    yield b
+    b.close()
+
+
+def operand(be, a, layout):
+    """`a` in a buffer of its own as rows of k, turned, or with gaps that no 16-byte access fits."""
+    if layout == "rows":
+        return dense(be, a)[1]
+    turned = np.swapaxes(a, -1, -2)
+    if layout == "turned":
+        t = dense(be, np.ascontiguousarray(turned))[1]
+        s = list(t.strides)
+        return type(t)(t.ptr, a.shape, tuple(s[:-2] + [s[-1], s[-2]]), t.dtype, t.device)
+    pitch = a.shape[-1] + 3
+    wide = np.full(a.shape[:-1] + (pitch,), -7.0, np.float32)
+    wide[..., 1:1 + a.shape[-1]] = a
+    t = dense(be, wide)[1]
+    return type(t)(t.ptr + 4, a.shape, t.strides, t.dtype, t.device)
+
+
+def bound(a, b):
+    """Pairs leave 2^-22 of each product's size, a sum of k such parts rounded in chains of 32: below 2^-21 |a| |b| in all. Short
+    sums run one after another in 32 bits: 2^-24 a step."""
+    k = a.shape[-1]
+    return max(2.0 ** -21, k * 2.0 ** -24 if k < 128 else 0.0) * (np.abs(a.astype(np.float64)) @ np.abs(b.astype(np.float64))) + 1e-30
+
+
+@pytest.mark.parametrize("m,n,k", [(128, 128, 1024), (129, 130, 1030), (1, 500, 5000), (300, 64, 900), (2000, 96, 512),
+                                   (127, 2050, 260), (1500, 1290, 72), (640, 3000, 33), (24, 40, 4096)])
+@pytest.mark.parametrize("left,right", [("rows", "rows"), ("turned", "gaps"), ("gaps", "turned")])
+def test_product(be, m, n, k, left, right):
+    rng = np.random.default_rng(m + n + k)
+    a = (rng.standard_normal((m, k)) * 10.0 ** rng.uniform(-6, 6, (m, 1))).astype(np.float32)
+    b = (rng.standard_normal((k, n)) * 10.0 ** rng.uniform(-6, 6, (1, n))).astype(np.float32)
+    ob, ov = dense(be, np.zeros((m, n), np.float32))
+    be.call("gemm", operand(be, a, left), operand(be, b, right), ov)
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    assert (np.abs(read(ob, ov) - want) <= bound(a, b)).all()
+
+
+@pytest.mark.parametrize("batch,m,n,k", [(8, 250, 250, 64), (3, 130, 70, 513), (64, 100, 64, 100), (2, 300, 700, 96)])
+def test_batches_sums_and_epilogues(be, batch, m, n, k):
+    rng = np.random.default_rng(batch + m + n + k)
+    a = rng.standard_normal((batch, m, k)).astype(np.float32)
+    b = rng.standard_normal((batch, k, n)).astype(np.float32)
+    ob, ov = dense(be, np.zeros((batch, m, n), np.float32))
+    be.call("gemm_batched", operand(be, a, "gaps"), operand(be, b, "rows"), ov)
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    assert (np.abs(read(ob, ov) - want) <= bound(a, b)).all()
+    # sum over the batch of turned left operands, with rows one behind another and with gaps
+    for layout in ("rows", "gaps"):
+        ob, ov = dense(be, np.zeros((m, n), np.float32))
+        at = np.ascontiguousarray(np.swapaxes(a, -1, -2))
+        be.call("gemm_ranked_reduce_lhs_t", operand(be, at, layout), operand(be, b, layout), ov)
+        assert (np.abs(read(ob, ov) - want.sum(0)) <= bound(a, b).sum(0)).all()
+    w, bias = b[0], rng.standard_normal((1, n)).astype(np.float32)
+    ob, ov = dense(be, np.zeros((batch, m, n), np.float32))
+    _, wv = dense(be, w)
+    be.call("gemm_ranked_matrix_rhs", operand(be, a, "rows"), wv, ov)
+    be.call("add_bias_relu_rowwise_inplace", ov, dense(be, bias)[1])
+    want = np.maximum(a.astype(np.float64) @ w.astype(np.float64) + bias, 0.0)
+    assert (np.abs(read(ob, ov) - want) <= bound(a, w) + 2.0 ** -23 * np.abs(bias) + 2.0 ** -23 * want).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(300, 200, 512), (64, 96, 2048)])
+def test_values_no_pair_holds(be, m, n, k):
+    rng = np.random.default_rng(m)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    a[3, 7], a[5, 9], a[6, 1], a[9, :] = np.inf, np.nan, -np.inf, 0.0
+    b[11, 2], a[:, 11] = 3.4028e38, np.float32(0.5)
+    with np.errstate(all="ignore"):
+        want = a.astype(np.float64) @ b.astype(np.float64)
+    ob, ov = dense(be, np.zeros((m, n), np.float32))
+    be.call("gemm", dense(be, a)[1], dense(be, b)[1], ov)
+    got = read(ob, ov)
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    fine = np.isfinite(want)
+    assert (np.abs(got[fine] - want[fine]) <= 1e-5 * np.abs(want[fine]) + 1e-4).all()
+    a[~np.isfinite(a)] = 1.0
+    b[11, 2] = 1.0
+    be.call("gemm", dense(be, a)[1], dense(be, b)[1], ov)  # and the next product is back on its way
+    assert (np.abs(read(ob, ov) - a.astype(np.float64) @ b) <= bound(a, b)).all()
+
+
+def test_small_and_tiny_values(be):
+    rng = np.random.default_rng(5)
+    a = (rng.standard_normal((256, 512)) * 1e-30).astype(np.float32)
+    b = (rng.standard_normal((512, 256)) * 1e20).astype(np.float32)
+    ob, ov = dense(be, np.zeros((256, 256), np.float32))
+    be.call("gemm", dense(be, a)[1], dense(be, b)[1], ov)
+    assert (np.abs(read(ob, ov) - a.astype(np.float64) @ b.astype(np.float64)) <= bound(a, b)).all()
