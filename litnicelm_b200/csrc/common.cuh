@@ -267,13 +267,14 @@ struct LoopState {
   int max_seq;
 };
 
-// embed.cu
+// embed.cu; newest: only the last position of every stream, row b of the outputs = stream b
 void launch_embed_pos(const float *tok_emb, const float *pos_emb, const int *ids, int ids_ld,
                       const LoopState *state, int n_streams, int s_host, int d, int vocab,
                       float *x, DevErr *err, cudaStream_t st, float *x_hi = nullptr, float *x_lo = nullptr,
-                      double2 *stats = nullptr, const struct TcPairF16 *x_f16 = nullptr);
+                      double2 *stats = nullptr, const struct TcPairF16 *x_f16 = nullptr, bool newest = false);
 // head_greedy.cu: final norm + output head + first-max selection + append +
-// state advance in one launch (greedy, few streams, vocabulary up to 1024).
+// state advance in one launch (greedy, few streams or a small vocabulary); state == nullptr: the
+// norm and the logits only.
 // `done` is a zero-initialised counter the kernel returns to zero.
 bool head_greedy_supports(int n_streams, int d, int vocab);
 void launch_head_greedy(const float *x, const float *gamma, const float *beta, const float *w, int d, int vocab,
@@ -337,9 +338,11 @@ void launch_embed_last_ln(const float *tok_emb, const float *pos_emb, const int 
 void launch_kv_store(const float *qkv, const LoopState *state, int s_host, int n_streams, int d, int cap, float *kc,
                      float *vc, cudaStream_t st);
 // counters: one zero-resting int per (stream, head), needed when the keys are cut into chunks.
-// Returns the number of kernels launched.
+// The context rows leave as fp32, as a TF32 pair (ctx, ctx_lo) or as the fp16 pair ctx_f16 (head
+// dimension 64). Returns the number of kernels launched.
 int launch_attn_decode(const float *qkv, float *kc, float *vc, int cap, int d_model, int n_heads, int n_streams,
-                       const LoopState *state, int s_host, float *part, int *counters, float *ctx, cudaStream_t st);
+                       const LoopState *state, int s_host, float *part, int *counters, float *ctx, cudaStream_t st,
+                       float *ctx_lo = nullptr, const struct TcPairF16 *ctx_f16 = nullptr);
 
 // decode_persistent.cu: cached mode, greedy, up to 8 streams: `steps` tokens in one resident kernel
 // (cooperative launch, one CTA per SM, grid-wide barriers between the operators).

@@ -10,6 +10,7 @@
 // live in [n_streams, ...] buffers: x (residual stream), ln, qkv [.., 3 d_model],
 // ctx, h [.., d_ff].
 #include "common.cuh"
+#include "gemm_tc.cuh"
 
 namespace lb {
 
@@ -85,24 +86,69 @@ __global__ void kv_store_kernel(const float *__restrict__ qkv, const LoopState *
   }
 }
 
+// Where the context row goes: fp32 (lo == nullptr), a TF32 pair (ctx, lo), or the fp16 pair a
+// projection on fp16 pairs reads (one scale per 64 columns; head dimension 64).
+struct DecodeCtx {
+  float *ctx, *lo;
+  TcPairF16 pair;
+};
+
+// Column tid of head h of stream b's context row (threads tid < DH hold one each). All 128 threads
+// call it together.
+template <int DH>
+__device__ __forceinline__ void store_context(const DecodeCtx &o, float v, int b, int h, int d_model, int tid, float *red) {
+  const long long at = (long long)b * d_model + h * DH + tid;
+  if (DH == 64 && o.pair.hi != nullptr) {
+    float am = tid < DH ? fabsf(v) : 0.f;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, s));
+    if ((tid & 31) == 0) red[tid >> 5] = am;
+    __syncthreads();
+    if (tid >= DH) return;
+    float inv;
+    const float a = v * f16_block_scale(fmaxf(red[0], red[1]), &inv);
+    const __half hi = __float2half_rn(a);
+    o.pair.hi[at] = hi;
+    o.pair.lo[at] = __float2half_rn(a - __half2float(hi));
+    if (tid == 0) o.pair.inv_scale[(long long)b * (d_model / TC_F16_SLOT) + h] = inv;
+    return;
+  }
+  if (tid >= DH) return;
+  if (o.lo != nullptr) {
+    float hi, lo;
+    split_tf32(v, hi, lo);
+    o.ctx[at] = hi;
+    o.lo[at] = lo;
+  } else {
+    o.ctx[at] = v;
+  }
+}
+
 // Attention of the newest row of stream b, head h, over the keys of one chunk of positions:
 // scores q.k / sqrt(dh) in fp32, their maximum, e = expf(score - max), the sum of e in double
 // (scaled_causal_softmax_rows, device_backend.cpp:1554-1592, restricted to one row) and
 // o = sum e_j v_j. The CTA whose chunk holds the newest position first appends that position's K
 // and V (this step's QKV row) to the caches. With one chunk the normalised context row is
 // written directly; otherwise (o, max, sum) go to `part` and the chunk that finishes last joins them.
+//
+// Bound by the cache bytes (8 * s * d_model per layer and stream), so what counts is bytes in
+// flight: both products read 16 bytes per lane and issue DEC_UNROLL keys' loads before the first
+// is used (DEC_UNROLL x 32 bytes per thread of keys, x 16 of values): 64 streams of 128 .. 191
+// positions at d_model 512 take 19.5 us, 27.4 us with 4-byte loads of values and one key at a time.
+constexpr int DEC_UNROLL = 4;
 template <int DH>
 __global__ void __launch_bounds__(128)
-attn_decode_kernel(const float *__restrict__ qkv, float *__restrict__ kc, float *__restrict__ vc, int cap,
-                   int d_model, const LoopState *state, int s_host, int keys_per_chunk, float scale,
-                   float *__restrict__ part, float *__restrict__ ctx, int *__restrict__ counters) {
+attn_decode_kernel(const float *__restrict__ qkv, float *kc, float *vc, int cap, int d_model, const LoopState *state,
+                   int s_host, int keys_per_chunk, float scale, float *__restrict__ part, DecodeCtx ctx,
+                   int *__restrict__ counters) {
   constexpr int LPK = DH / 8;      // lanes that share one key: 8 floats of the head each
   constexpr int KPI = 128 / LPK;   // keys per trip of the CTA
-  constexpr int PARTS = 128 / DH;  // threads per output column in the second product
+  constexpr int VPR = DH / 4;      // lanes that share one row of values: 4 floats each
+  constexpr int VPI = 128 / VPR;   // rows of values per trip of the CTA
   extern __shared__ float sc[];    // scores, then e, of the chunk's keys
   __shared__ float red_f[4];
   __shared__ double red_d[4];
-  __shared__ float o_part[128];
+  __shared__ __align__(16) float o_part[512];  // [VPI][DH]
   __shared__ int is_last;
   pdl_launch_dependents();
   pdl_wait();
@@ -119,76 +165,101 @@ attn_decode_kernel(const float *__restrict__ qkv, float *__restrict__ kc, float 
       out[DH + 1] = 0.f;
     }
   } else {
-  const float *row = qkv + (long long)b * 3 * d_model;
-  if (p >= c0 && p < c1 && tid < DH / 4) {
-    const float4 k4 = *reinterpret_cast<const float4 *>(row + d_model + h * DH + tid * 4);
-    const float4 v4 = *reinterpret_cast<const float4 *>(row + 2 * d_model + h * DH + tid * 4);
-    *reinterpret_cast<float4 *>(kc + ((long long)b * cap + p) * d_model + h * DH + tid * 4) = k4;
-    *reinterpret_cast<float4 *>(vc + ((long long)b * cap + p) * d_model + h * DH + tid * 4) = v4;
-  }
-  __syncthreads();
-  const int sub = tid % LPK;
-  const float4 q0 = *reinterpret_cast<const float4 *>(row + h * DH + sub * 8);
-  const float4 q1 = *reinterpret_cast<const float4 *>(row + h * DH + sub * 8 + 4);
-  for (int base = c0; base < c1; base += KPI) {  // uniform trip count: the shuffles need whole warps
-    const int j = base + tid / LPK;
-    float dot = 0.f;
-    if (j < c1) {
-      const float *kp = kc + ((long long)b * cap + j) * d_model + h * DH + sub * 8;
-      const float4 k0 = *reinterpret_cast<const float4 *>(kp), k1 = *reinterpret_cast<const float4 *>(kp + 4);
-      dot = q0.x * k0.x;
-      dot = fmaf(q0.y, k0.y, dot);
-      dot = fmaf(q0.z, k0.z, dot);
-      dot = fmaf(q0.w, k0.w, dot);
-      dot = fmaf(q1.x, k1.x, dot);
-      dot = fmaf(q1.y, k1.y, dot);
-      dot = fmaf(q1.z, k1.z, dot);
-      dot = fmaf(q1.w, k1.w, dot);
+    const float *row = qkv + (long long)b * 3 * d_model;
+    if (p >= c0 && p < c1 && tid < DH / 4) {
+      const float4 k4 = *reinterpret_cast<const float4 *>(row + d_model + h * DH + tid * 4);
+      const float4 v4 = *reinterpret_cast<const float4 *>(row + 2 * d_model + h * DH + tid * 4);
+      *reinterpret_cast<float4 *>(kc + ((long long)b * cap + p) * d_model + h * DH + tid * 4) = k4;
+      *reinterpret_cast<float4 *>(vc + ((long long)b * cap + p) * d_model + h * DH + tid * 4) = v4;
     }
+    __syncthreads();
+    const int sub = tid % LPK;
+    const float4 q0 = *reinterpret_cast<const float4 *>(row + h * DH + sub * 8);
+    const float4 q1 = *reinterpret_cast<const float4 *>(row + h * DH + sub * 8 + 4);
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float *kb = kc + (long long)b * cap * d_model + h * DH + sub * 8;
+    for (int base = c0; base < c1; base += DEC_UNROLL * KPI) {  // uniform trip count: the shuffles need whole warps
+      float4 k0[DEC_UNROLL], k1[DEC_UNROLL];
 #pragma unroll
-    for (int o = LPK >> 1; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-    if (j < c1 && sub == 0) sc[j - c0] = dot * scale;
-  }
-  __syncthreads();
-  const int nk = c1 - c0;
-  float m = -INFINITY;
-  for (int i = tid; i < nk; i += 128) m = fmaxf(m, sc[i]);
+      for (int u = 0; u < DEC_UNROLL; ++u) {
+        const int j = base + u * KPI + tid / LPK;
+        const float4 *kp = reinterpret_cast<const float4 *>(kb + (long long)j * d_model);
+        k0[u] = j < c1 ? kp[0] : zero4;
+        k1[u] = j < c1 ? kp[1] : zero4;
+      }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) red_f[wid] = m;
-  __syncthreads();
-  m = fmaxf(fmaxf(red_f[0], red_f[1]), fmaxf(red_f[2], red_f[3]));
-  double l = 0.0;
-  for (int i = tid; i < nk; i += 128) {
-    const float e = expf(sc[i] - m);
-    sc[i] = e;
-    l += (double)e;
-  }
-  l = warp_sum_d(l);
-  if (lane == 0) red_d[wid] = l;
-  __syncthreads();
-  l = ((red_d[0] + red_d[1]) + red_d[2]) + red_d[3];
-  // second product: thread -> (column d of the head, every PARTS-th key)
-  const int d = tid % DH, pt = tid / DH;
-  float o = 0.f;
-  const float *vp = vc + ((long long)b * cap + c0) * d_model + h * DH + d;
-  for (int i = pt; i < nk; i += PARTS) o = fmaf(sc[i], vp[(long long)i * d_model], o);
-  o_part[tid] = o;
-  __syncthreads();
-  if (tid < DH) {
-    float t = o_part[tid];
+      for (int u = 0; u < DEC_UNROLL; ++u) {
+        const int j = base + u * KPI + tid / LPK;
+        float dot = q0.x * k0[u].x;
+        dot = fmaf(q0.y, k0[u].y, dot);
+        dot = fmaf(q0.z, k0[u].z, dot);
+        dot = fmaf(q0.w, k0[u].w, dot);
+        dot = fmaf(q1.x, k1[u].x, dot);
+        dot = fmaf(q1.y, k1[u].y, dot);
+        dot = fmaf(q1.z, k1[u].z, dot);
+        dot = fmaf(q1.w, k1[u].w, dot);
 #pragma unroll
-    for (int q = 1; q < PARTS; ++q) t += o_part[q * DH + tid];
+        for (int o = LPK >> 1; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        if (j < c1 && sub == 0) sc[j - c0] = dot * scale;
+      }
+    }
+    __syncthreads();
+    const int nk = c1 - c0;
+    float m = -INFINITY;
+    for (int i = tid; i < nk; i += 128) m = fmaxf(m, sc[i]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) red_f[wid] = m;
+    __syncthreads();
+    m = fmaxf(fmaxf(red_f[0], red_f[1]), fmaxf(red_f[2], red_f[3]));
+    double l = 0.0;
+    for (int i = tid; i < nk; i += 128) {
+      const float e = expf(sc[i] - m);
+      sc[i] = e;
+      l += (double)e;
+    }
+    l = warp_sum_d(l);
+    if (lane == 0) red_d[wid] = l;
+    __syncthreads();
+    l = ((red_d[0] + red_d[1]) + red_d[2]) + red_d[3];
+    // second product: thread -> (four columns of the head, every VPI-th key)
+    const int vr = tid / VPR, vq = tid % VPR;
+    float4 o = zero4;
+    const float *vp = vc + ((long long)b * cap + c0) * d_model + h * DH + vq * 4;
+    for (int i0 = vr; i0 < nk; i0 += DEC_UNROLL * VPI) {
+      float4 v[DEC_UNROLL];
+#pragma unroll
+      for (int u = 0; u < DEC_UNROLL; ++u) {
+        const int i = i0 + u * VPI;
+        v[u] = i < nk ? *reinterpret_cast<const float4 *>(vp + (long long)i * d_model) : zero4;
+      }
+#pragma unroll
+      for (int u = 0; u < DEC_UNROLL; ++u) {
+        const int i = i0 + u * VPI;
+        const float e = i < nk ? sc[i] : 0.f;
+        o.x = fmaf(e, v[u].x, o.x);
+        o.y = fmaf(e, v[u].y, o.y);
+        o.z = fmaf(e, v[u].z, o.z);
+        o.w = fmaf(e, v[u].w, o.w);
+      }
+    }
+    *reinterpret_cast<float4 *>(o_part + vr * DH + vq * 4) = o;
+    __syncthreads();
+    float t = 0.f;
+    if (tid < DH) {
+      t = o_part[tid];
+#pragma unroll
+      for (int q = 1; q < VPI; ++q) t += o_part[q * DH + tid];
+    }
     if (out == nullptr) {
-      ctx[(long long)b * d_model + h * DH + tid] = t * (float)(1.0 / l);
-    } else {
+      store_context<DH>(ctx, t * (float)(1.0 / l), b, h, d_model, tid, red_f);
+    } else if (tid < DH) {
       out[tid] = t;
       if (tid == 0) {
         out[DH] = m;
         out[DH + 1] = (float)l;
       }
     }
-  }
   }  // chunk with keys
   if (out == nullptr) return;
   // The chunk that finishes last joins all chunks of its (stream, head) in chunk order: the common
@@ -202,6 +273,7 @@ attn_decode_kernel(const float *__restrict__ qkv, float *__restrict__ kc, float 
   __syncthreads();
   if (!is_last) return;
   __threadfence();
+  float v = 0.f;
   if (tid < DH) {
     const float *pp = part + ((long long)b * gridDim.y + h) * chunks * (DH + 2);
     float mm = -INFINITY;
@@ -215,9 +287,10 @@ attn_decode_kernel(const float *__restrict__ qkv, float *__restrict__ kc, float 
       ll += (double)__ldcg(&pp[q * (DH + 2) + DH + 1]) * (double)w;
       oo = fmaf(__ldcg(&pp[q * (DH + 2) + tid]), w, oo);
     }
-    ctx[(long long)b * d_model + h * DH + tid] = oo * (float)(1.0 / ll);
+    v = oo * (float)(1.0 / ll);
     if (tid == 0) counters[b * gridDim.y + h] = 0;
   }
+  store_context<DH>(ctx, v, b, h, d_model, tid, red_f);
 }
 
 }  // namespace
@@ -257,7 +330,7 @@ DecodeAttnPlan attn_decode_plan(int n_streams, int s, int n_heads, int dh) {
 template <int DH>
 static void launch_attn_decode_dh(const float *qkv, float *kc, float *vc, int cap, int d_model, int n_heads,
                                   int n_streams, const LoopState *state, int s_host, const DecodeAttnPlan &plan,
-                                  float *part, int *counters, float *ctx, cudaStream_t st) {
+                                  float *part, int *counters, const DecodeCtx &ctx, cudaStream_t st) {
   const float scale = 1.0f / sqrtf((float)DH);
   dim3 grid((unsigned)plan.chunks, (unsigned)n_heads, (unsigned)n_streams);
   float *pp = plan.chunks > 1 ? part : nullptr;
@@ -266,11 +339,15 @@ static void launch_attn_decode_dh(const float *qkv, float *kc, float *vc, int ca
 }
 
 int launch_attn_decode(const float *qkv, float *kc, float *vc, int cap, int d_model, int n_heads, int n_streams,
-                       const LoopState *state, int s_host, float *part, int *counters, float *ctx, cudaStream_t st) {
+                       const LoopState *state, int s_host, float *part, int *counters, float *ctx_out, cudaStream_t st,
+                       float *ctx_lo, const TcPairF16 *ctx_f16) {
+  const DecodeCtx ctx{ctx_out, ctx_lo, ctx_f16 ? *ctx_f16 : TcPairF16{}};
   const int dh = d_model / n_heads;
   const DecodeAttnPlan plan = attn_decode_plan(n_streams, s_host, n_heads, dh);
   if (plan.chunks > 1 && (part == nullptr || counters == nullptr))
     throw std::invalid_argument("litnice_b200: decode attention needs scratch");
+  if (ctx_f16 != nullptr && dh != TC_F16_SLOT)
+    throw std::invalid_argument("litnice_b200: decode attention stores fp16 pairs for head dimension 64 only");
   switch (dh) {
     case 16: launch_attn_decode_dh<16>(qkv, kc, vc, cap, d_model, n_heads, n_streams, state, s_host, plan, part, counters, ctx, st); break;
     case 32: launch_attn_decode_dh<32>(qkv, kc, vc, cap, d_model, n_heads, n_streams, state, s_host, plan, part, counters, ctx, st); break;

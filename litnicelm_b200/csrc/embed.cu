@@ -20,13 +20,13 @@ __global__ void embed_pos_kernel(const float *__restrict__ tok_emb,
                                  int ids_ld, const LoopState *state, int n_streams, int s_cap, int d,
                                  int vocab, float *__restrict__ x, float *__restrict__ x_hi,
                                  float *__restrict__ x_lo, double2 *__restrict__ stats, TcPairF16 x_f16,
-                                 DevErr *err) {
+                                 int newest, DevErr *err) {
   pdl_launch_dependents();
   pdl_wait();
   const int s = state ? state->s : s_cap;
   const long long r = blockIdx.x;
-  if (r >= (long long)n_streams * s) return;
-  const int b = (int)(r / s), t = (int)(r - (long long)b * s);
+  if (r >= (newest ? (long long)n_streams : (long long)n_streams * s)) return;
+  const int b = newest ? (int)r : (int)(r / s), t = newest ? s - 1 : (int)(r - (long long)b * s);
   int id = ids[(long long)b * ids_ld + t];
   const bool bad = id < 0 || id >= vocab;
   if (bad) {
@@ -171,11 +171,12 @@ __global__ void embed_rows_kernel(const T *__restrict__ table, const T *__restri
 void launch_embed_pos(const float *tok_emb, const float *pos_emb, const int *ids, int ids_ld,
                       const LoopState *state, int n_streams, int s_host, int d, int vocab,
                       float *x, DevErr *err, cudaStream_t st, float *x_hi, float *x_lo, double2 *stats,
-                      const TcPairF16 *x_f16) {
-  const long long rows = (long long)n_streams * s_host;
+                      const TcPairF16 *x_f16, bool newest) {
+  const long long rows = newest ? n_streams : (long long)n_streams * s_host;
   if (rows <= 0) return;
   launch_pdl(embed_pos_kernel, dim3((unsigned)rows), dim3(d >= 512 ? 128 : 32), 0, st, g_pdl_enabled, tok_emb, pos_emb,
-             ids, ids_ld, state, n_streams, s_host, d, vocab, x, x_hi, x_lo, stats, x_f16 ? *x_f16 : TcPairF16{}, err);
+             ids, ids_ld, state, n_streams, s_host, d, vocab, x, x_hi, x_lo, stats, x_f16 ? *x_f16 : TcPairF16{},
+             newest ? 1 : 0, err);
 }
 
 void launch_gather_last_ln(const float *x, const float *gamma, const float *beta,

@@ -61,6 +61,11 @@ struct TcEpilogue {
   __half *qk16_hi = nullptr, *qk16_lo = nullptr;
   __half *vt16_hi = nullptr, *vt16_lo = nullptr;
   const float *col_scale = nullptr;  // [N / 64]
+  // Cached mode, pass over the prompt: the K columns [vt_col0 - vt_rows, vt_col0) and the V columns
+  // also leave as fp32 to the caches, element (row r = stream * s + t, column c of the third) to
+  // kcache / vcache[(stream * kv_cap + t) * vt_rows + c].
+  float *kcache = nullptr, *vcache = nullptr;
+  int kv_cap = 0;
   __host__ __device__ bool has_vt() const { return vt_hi != nullptr || vt16_hi != nullptr; }
   // LayerNorm folded into the product. With W' = diag(gamma) W the reference's
   // LN(x) W + b (layernorm_forward then gemm_ranked_matrix_rhs + add_bias_rowwise)

@@ -64,6 +64,7 @@ constexpr unsigned TC_EP_FORM_QKV = TC_EP_FOLD | TC_EP_BIAS | TC_EP_QK16;
 constexpr unsigned TC_EP_FORM_W1 = TC_EP_FOLD | TC_EP_BIAS | TC_EP_RELU | TC_EP_F16;
 constexpr unsigned TC_EP_FORM_RES = TC_EP_BIAS | TC_EP_RESIDUAL | TC_EP_C | TC_EP_F16 | TC_EP_STATS;
 __device__ __forceinline__ unsigned tc_ep_form(const TcEpilogue &ep) {
+  if (ep.kcache != nullptr) return TC_EP_GENERIC;
   return (ep.ln_u != nullptr ? TC_EP_FOLD : 0u) | (ep.relu ? TC_EP_RELU : 0u) | (ep.residual != nullptr ? TC_EP_RESIDUAL : 0u) |
          (ep.c != nullptr ? TC_EP_C : 0u) | (ep.c_hi != nullptr ? TC_EP_SPLIT : 0u) | (ep.qk16_hi != nullptr ? TC_EP_QK16 : 0u) |
          (ep.c_f16.hi != nullptr ? TC_EP_F16 : 0u) | (ep.stats_out != nullptr ? TC_EP_STATS : 0u) |
@@ -154,6 +155,11 @@ __device__ __forceinline__ void tc_store_rows(const TcEpilogue &ep, int m, int n
         split_tf32(v[g].w, hh.w, ll.w);
         *reinterpret_cast<float4 *>(ep.c_hi + off) = hh;
         *reinterpret_cast<float4 *>(ep.c_lo + off) = ll;
+      }
+      if (GEN && ep.kcache != nullptr && col >= ep.vt_col0 - ep.vt_rows) {
+        const int s_now = ep.state ? ep.state->s : ep.vt_s, stream = (m0 + rg) / s_now, tok = (m0 + rg) - stream * s_now;
+        if (stream < ep.vt_streams)
+          *reinterpret_cast<float4 *>(ep.kcache + ((long long)stream * ep.kv_cap + tok) * ep.vt_rows + col - (ep.vt_col0 - ep.vt_rows)) = v[g];
       }
       if (out_qk16) {  // fp16 pair under the head's fixed scale
         uint2 hi, lo;
@@ -346,6 +352,13 @@ __device__ __forceinline__ void tc_store_vt(const TcEpilogue &ep, int m, int m0,
     if (!act) continue;
     const float vals[4] = {t.x, t.y, t.z, t.w}, us[4] = {u4.x, u4.y, u4.z, u4.w}, bs[4] = {b4.x, b4.y, b4.z, b4.w};
     const long long at0 = ((long long)v_stream * ep.vt_rows + (col - ep.vt_col0)) * ep.vt_pitch + v_tok;
+    if (ep.vcache != nullptr) {
+      float f[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) f[e] = (fold ? __fmul_rn(st.y, __fmaf_rn(-st.x, us[e], vals[e])) : vals[e]) + bs[e];
+      *reinterpret_cast<float4 *>(ep.vcache + ((long long)v_stream * ep.kv_cap + v_tok) * ep.vt_rows + (col - ep.vt_col0)) =
+          make_float4(f[0], f[1], f[2], f[3]);
+    }
     if (ep.vt16_hi != nullptr) {  // fp16 pair under the head's fixed scale (the four columns share a head)
       const float cs = __ldg(ep.col_scale + col / 64);
 #pragma unroll

@@ -206,8 +206,10 @@ struct litnice_b200_session {
 
   // Opt-in cached mode (LITNICE_B200_KV_CACHE=1, an extension: the reference keeps no cache). Keys
   // and values of earlier positions stay in HBM, [n_layers][kv_streams][kv_cap][d_model] each, and a
-  // step computes one new row per stream (decode.cu). Runs on the fp32 kernels: the whole-context
-  // pass over the prompt that fills the caches on the SIMT path, the steps on the few-row products.
+  // step computes one new row per stream (decode.cu). The whole-context pass over the prompt that
+  // fills the caches runs as in the loop without a cache; the steps of up to 8 streams on the few-row
+  // products in fp32 (bound by the weight bytes), those of more streams on the tensor cores, as a
+  // whole-context pass of one row per stream with the attention over the caches in its place.
   bool kv = false;
   bool kv_fuse = true;  // LayerNorms inside the products, one-launch greedy tail (LITNICE_B200_KV_FUSE=0: kernels of their own)
   float *kcache = nullptr, *vcache = nullptr;
@@ -525,18 +527,23 @@ void projection_f16(litnice_b200_session *s, PairKind pk, long long rows, int k,
 
 // Transformer::forward over all rows up to the last layer's output
 // (transformer.cpp:70-114, transformer_layer.cpp:50-92); leaves the final
-// hidden state in s->x.
-void enqueue_body(litnice_b200_session *s, int B, int sl, const LoopState *dstate = nullptr) {
+// hidden state in s->x. newest (cached mode, tensor-core path): only the newest row of every
+// stream, row b of every buffer = stream b, attention over the cached positions and the new one;
+// sl then is the (bound of the) context length.
+void enqueue_body(litnice_b200_session *s, int B, int sl, const LoopState *dstate = nullptr, bool newest = false) {
   const litnice_b200_dims &d = s->dims;
-  const long long R = (long long)B * sl;
+  const long long R = newest ? B : (long long)B * sl;
   const int D = d.d_model, F = d.d_ff;
+  const LoopState *rows_state = newest ? nullptr : dstate;  // what shortens a launch's row count
+  const size_t cache_layer = (size_t)s->kv_streams * s->kv_cap * D;
   // With the LayerNorms folded into the QKV and W1 products, the kernels that
   // produce x and y also store them as TF32 pairs in (ln, ln_lo) with per-row
   // partial sums in row_stats, and no LayerNorm kernel runs in the layers.
   const bool fold = s->ln_fold;
   launch_embed_pos(P(s, s->lay.tok_emb), P(s, s->lay.pos_emb), s->ids, d.max_seq_len, dstate, B, sl, D,
                    d.vocab_size, s->x, s->err_dev, s->st, fold && !s->f16 ? s->ln : nullptr,
-                   fold && !s->f16 ? s->ln_lo : nullptr, fold ? s->row_stats : nullptr, s->f16 ? &s->pair_ln : nullptr);
+                   fold && !s->f16 ? s->ln_lo : nullptr, fold ? s->row_stats : nullptr, s->f16 ? &s->pair_ln : nullptr,
+                   newest);
   ++s->launches;
   for (int l = 0; l < d.n_layers; ++l) {
     const LayerOff &o = s->lay.layer[l];
@@ -549,21 +556,31 @@ void enqueue_body(litnice_b200_session *s, int B, int sl, const LoopState *dstat
       consume1.ln_slots = consume2.ln_slots = D / 64;
       produce.stats_out = s->row_stats;
     } else {
-      launch_layernorm_dense(s->x, P(s, o.ln1_g), P(s, o.ln1_b), R, D, s->ln, s->tc ? s->ln_lo : nullptr, dstate, B,
+      launch_layernorm_dense(s->x, P(s, o.ln1_g), P(s, o.ln1_b), R, D, s->ln, s->tc ? s->ln_lo : nullptr, rows_state, B,
                              s->st);
       ++s->launches;
+    }
+    float *kc = s->kv ? s->kcache + l * cache_layer : nullptr, *vc = s->kv ? s->vcache + l * cache_layer : nullptr;
+    if (s->kv_store && s->tc_attn) {  // cached mode, pass over the prompt: this layer's K and V of every position
+      consume1.kcache = kc;
+      consume1.vcache = vc;
+      consume1.kv_cap = s->kv_cap;
     }
     const float *qkv_bias = fold ? (*tw)[0].ln_v : P(s, o.qkv_b);
     if (s->f16) {
       // every projection input is an fp16 pair written by the kernel that produced it
-      consume1.vt_col0 = 2 * D;
-      consume1.vt_rows = D;
-      consume1.vt_pitch = s->vt_pitch;
-      consume1.vt_s = sl;
-      consume1.vt_streams = B;
-      consume1.state = dstate;
       consume1.bias = qkv_bias;
-      if (s->attn16) {  // Q, K and V^T as fp16 pairs under the heads' fixed scales
+      if (!newest) {
+        consume1.vt_col0 = 2 * D;
+        consume1.vt_rows = D;
+        consume1.vt_pitch = s->vt_pitch;
+        consume1.vt_s = sl;
+        consume1.vt_streams = B;
+        consume1.state = dstate;
+      }
+      if (newest) {
+        consume1.c = s->dqkv;
+      } else if (s->attn16) {  // Q, K and V^T as fp16 pairs under the heads' fixed scales
         consume1.qk16_hi = s->qk16_hi;
         consume1.qk16_lo = s->qk16_lo;
         consume1.vt16_hi = s->vt16_hi;
@@ -582,7 +599,10 @@ void enqueue_body(litnice_b200_session *s, int B, int sl, const LoopState *dstat
                                   s->attn_timeline_used < litnice_b200_session::kTimelineSlots)
                                      ? s->attn_timeline + 32 * s->attn_timeline_used++
                                      : nullptr;
-        if (s->attn16)
+        if (newest)
+          launch_attn_decode(s->dqkv, kc, vc, s->kv_cap, D, d.n_heads, B, dstate, sl, s->dec_part, s->dec_counters, nullptr,
+                             s->st, nullptr, &s->pair_ctx);
+        else if (s->attn16)
           launch_attention_tc16(s->qk16_map, s->vt16_map, (*tw)[0].head_inv, B, sl, d.n_heads, D, s->attn_scratch,
                                 s->attn_counters, dstate, s->err_dev, s->st, tl, s->pair_ctx);
         else
@@ -608,7 +628,14 @@ void enqueue_body(litnice_b200_session *s, int B, int sl, const LoopState *dstat
       projection_f16(s, PAIR_H, R, F, &(*tw)[3], D, e_w2);
       continue;
     }
-    if (s->tc_attn) {
+    if (newest) {  // the context leaves as the TF32 pair the out-projection reads
+      projection(s, A_LN, R, D, P(s, o.qkv_w), &(*tw)[0], 3 * D, qkv_bias, nullptr, 0, s->dqkv, nullptr,
+                 fold ? &consume1 : nullptr);
+      ClassTimer t(s, &s->attn_ev);
+      launch_attn_decode(s->dqkv, kc, vc, s->kv_cap, D, d.n_heads, B, dstate, sl, s->dec_part, s->dec_counters, s->ctx,
+                         s->st, s->ctx_lo);
+      ++s->launches;
+    } else if (s->tc_attn) {
       // Q and K as TF32 pairs, V transposed: what the tensor-core attention reads
       consume1.vt_hi = s->vt_hi;
       consume1.vt_lo = s->vt_lo;
@@ -632,8 +659,7 @@ void enqueue_body(litnice_b200_session *s, int B, int sl, const LoopState *dstat
       projection(s, A_LN, R, D, P(s, o.qkv_w), tw ? &(*tw)[0] : nullptr, 3 * D, qkv_bias, nullptr, 0, s->qkv,
                  nullptr, fold ? &consume1 : nullptr);
       if (s->kv_store) {  // cached mode, pass over the prompt: this layer's K and V of every position
-        const size_t layer = (size_t)s->kv_streams * s->kv_cap * D;
-        launch_kv_store(s->qkv, dstate, sl, B, D, s->kv_cap, s->kcache + l * layer, s->vcache + l * layer, s->st);
+        launch_kv_store(s->qkv, dstate, sl, B, D, s->kv_cap, kc, vc, s->st);
         ++s->launches;
       }
       ClassTimer t(s, &s->attn_ev);
@@ -648,7 +674,7 @@ void enqueue_body(litnice_b200_session *s, int B, int sl, const LoopState *dstat
       continue;
     }
     projection(s, A_CTX, R, D, P(s, o.out_w), tw ? &(*tw)[1] : nullptr, D, P(s, o.out_b), s->x, 0, s->y, nullptr);
-    launch_layernorm_dense(s->y, P(s, o.ln2_g), P(s, o.ln2_b), R, D, s->ln, s->tc ? s->ln_lo : nullptr, dstate, B,
+    launch_layernorm_dense(s->y, P(s, o.ln2_g), P(s, o.ln2_b), R, D, s->ln, s->tc ? s->ln_lo : nullptr, rows_state, B,
                            s->st);
     ++s->launches;
     projection(s, A_LN, R, D, P(s, o.w1), tw ? &(*tw)[2] : nullptr, F, P(s, o.b1), nullptr, 1, s->h,
@@ -662,6 +688,13 @@ void enqueue_body(litnice_b200_session *s, int B, int sl, const LoopState *dstat
 void enqueue_head_last(litnice_b200_session *s, int B, int sl, const LoopState *dstate = nullptr) {
   const litnice_b200_dims &d = s->dims;
   const bool head_tc = s->tc && B > 8 && s->tc_head.usable();
+  if (B > 8 && !head_tc && s->fused_tail && head_greedy_supports(B, d.d_model, d.vocab_size)) {
+    // norm and logits in one launch
+    launch_head_greedy(s->x, P(s, s->lay.lnf_g), P(s, s->lay.lnf_b), P(s, s->lay.lm_head), d.d_model, d.vocab_size, B, sl,
+                       dstate, nullptr, nullptr, nullptr, 0, nullptr, 0, s->logits, s->st);
+    ++s->launches;
+    return;
+  }
   launch_gather_last_ln(s->x, P(s, s->lay.lnf_g), P(s, s->lay.lnf_b), dstate, B, sl, d.d_model, s->xl,
                         head_tc ? s->xl_lo : nullptr, s->st);
   ++s->launches;
@@ -676,7 +709,7 @@ void enqueue_head_last(litnice_b200_session *s, int B, int sl, const LoopState *
 
 // Cached mode: one projection of the step's rows, out[B, n] = LN?(a)[B, k] W + bias (+ residual) (ReLU):
 // the few-row kernels up to 8 streams (with the LayerNorm in front of the product applied inside the
-// kernel where its shape allows), the fp32 tile kernel beyond. ln_g / ln_b: that LayerNorm, or null;
+// kernel where its shape allows), the fp32 tile kernel beyond (models the tensor-core path does not take). ln_g / ln_b: that LayerNorm, or null;
 // ln_out: where its rows go when it has to run as a kernel of its own.
 void decode_projection(litnice_b200_session *s, const float *a, int B, int k, const float *w, int n, const float *bias,
                        const float *residual, int relu, float *out, const float *ln_g = nullptr,
@@ -707,6 +740,13 @@ void decode_projection(litnice_b200_session *s, const float *a, int B, int k, co
 void enqueue_decode_step(litnice_b200_session *s, int B, int sl, const LoopState *dstate, bool with_head) {
   const litnice_b200_dims &d = s->dims;
   const int D = d.d_model, F = d.d_ff, V = d.vocab_size;
+  // Beyond the few-row products' 8 rows: 64 streams at 6 layers of width 512 take 0.33 ms a step here
+  // (a product 10 us), 1.77 ms on the fp32 tile kernel (55 us: few tiles, a serial k loop).
+  if (s->tc && B > 8) {
+    enqueue_body(s, B, sl, dstate, true);
+    if (with_head) enqueue_head_last(s, B, 1);
+    return;
+  }
   const size_t layer = (size_t)s->kv_streams * s->kv_cap * D;
   // the newest row's embedding; its first LayerNorm only when the QKV product cannot apply it itself
   const bool ln_in_qkv = B <= 8 && s->kv_fuse && gemv_fuses_layernorm(3 * D, D);
@@ -1290,7 +1330,7 @@ static int session_create_impl(const litnice_b200_dims *dims, int32_t max_stream
       must(cudaMalloc(reinterpret_cast<void **>(&s->pk_barrier), 16));
     }
     const char *tc_env = std::getenv("LITNICE_B200_TC");
-    s->tc = !s->kv && !(tc_env && tc_env[0] == '0') && tc_runtime_available() && d.d_model % 64 == 0 &&
+    s->tc = !(tc_env && tc_env[0] == '0') && tc_runtime_available() && d.d_model % 64 == 0 &&
             d.d_ff % 64 == 0;
     // Attention on the tensor cores needs head dimension 64; LITNICE_B200_TC_ATTN=0
     // keeps the fp32 SIMT attention kernel.
@@ -1525,6 +1565,7 @@ int litnice_b200_run(litnice_b200_session *s, int32_t max_new, const litnice_b20
       // cached mode: whole-context buffers only for the pass over the prompt that fills the caches
       if (steps > 0) {
         ensure_kv(s, B, s_last_cap);
+        if (s->tc && B > 8) ensure_rows(s, B);
         if (s->kv_len != s0 - 1) {
           ensure_rows(s, (long long)B * s0);
           ensure_attention_scratch(s, B, s0, s0);
@@ -1604,7 +1645,7 @@ int litnice_b200_run(litnice_b200_session *s, int32_t max_new, const litnice_b20
       } else if (decode) {
         enqueue_decode_step(s, B, sl_cap, dstate, !decode_tail);
         if (decode_tail) {  // the step's rows are the last rows: one row per stream
-          launch_head_greedy(s->dx, P(s, s->lay.lnf_g), P(s, s->lay.lnf_b), P(s, s->lay.lm_head), s->dims.d_model, V, B,
+          launch_head_greedy(s->tc && B > 8 ? s->x : s->dx, P(s, s->lay.lnf_g), P(s, s->lay.lnf_b), P(s, s->lay.lm_head), s->dims.d_model, V, B,
                              1, nullptr, s->state, reinterpret_cast<unsigned *>(s->state + 1), s->ids,
                              s->dims.max_seq_len, s->out_tokens, s->out_cap, s->logits, s->st);
           ++s->launches;

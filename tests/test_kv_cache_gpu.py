@@ -114,3 +114,33 @@ def test_streams_resume_and_many_streams(oracle):
     assert np.array_equal(parts, few)
     for b in range(3):
         assert rel_err(lg[:, b, :], ref[b][1]) < LOGIT_RTOL
+
+
+# More than 8 streams: steps on the tensor cores. Every head dimension (64: fp16 pairs, others: TF32 pairs), one and several
+# key chunks, contexts that cross a 64-position bucket, heads on the tensor cores (vocabulary % 64 == 0), in the one-launch
+# tail, and on the tile kernel.
+@pytest.mark.parametrize("dims,streams,prompt,new", [
+    ((2, 2, 128, 256, 64, 160), 9, 60, 20),
+    ((1, 3, 192, 192, 50, 300), 33, 40, 12),
+    ((2, 4, 128, 256, 52, 96), 12, 1, 9),
+    ((1, 1, 128, 128, 96, 200), 9, 130, 10),
+    ((1, 8, 128, 192, 128, 80), 129, 62, 6),
+])
+def test_many_streams_step_on_the_tensor_cores(oracle, dims, streams, prompt, new):
+    d = formats.ModelDims(*dims)
+    arena = formats.make_param_arena(d, 7, bias_std=0.02, ln_std=0.1)
+    prompts = np.stack([formats.zipf_prompt(d.vocab, prompt, 70 + i) for i in range(streams)])
+    with Session(d, streams) as s:
+        s.load_params(arena)
+        fast = s.generate(prompts, new)
+        s.keep_step_logits(True)
+        toks = s.generate(prompts, new)
+        lg = s.read_step_logits(new, streams)
+    for b in sorted({0, 7, 8, streams // 2, streams - 1}):
+        ref_tokens, ref_logits = oracle.generate(d, arena, prompts[b], new, want_logits=True)
+        srt = np.sort(ref_logits.astype(np.float64), axis=1)
+        gaps = srt[:, -1] - srt[:, -2]
+        n = agreed_prefix(toks[b], ref_tokens, gaps)
+        # operands of 22 bits (2^-22 per product), sums of at most 256 terms in fp32 on either side, a handful of layers
+        assert rel_err(lg[:n, b, :], ref_logits[:n]) < 2e-5
+        agreed_prefix(fast[b], ref_tokens, gaps)
