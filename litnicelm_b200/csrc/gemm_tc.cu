@@ -404,7 +404,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_consta
   if (go && !(ep.has_vt() && n0 >= ep.vt_col0)) {  // a tile of V columns only has left already
     // the token loop's three forms with their terms fixed at compile time (a loop body that stays in
     // the instruction cache), everything else through the general form
-    const unsigned form = tc_ep_form(ep);
+    const unsigned form = ep.kcache != nullptr ? TC_EP_GENERIC : tc_ep_form(ep);
     if (F16 && form == TC_EP_FORM_QKV)
       tc_store_rows<BN, tc_threads(BN), TC_EP_FORM_QKV>(ep, m, n, m0, n0, (int)threadIdx.x, stage, row_stats, cluster_splits,
                                                         rows_each, row_begin, row_end, first);
@@ -727,6 +727,15 @@ TcPlan tc_plan(int m, int n, int k, bool has64, bool has128, bool has256, int k_
   // single-stream shapes.
   p.bn = (has128 && (!has64 || mt * (n / 128) >= 74)) ? 128 : 64;
   if (has256 && mt * (n / 256) >= 2 * 148) p.bn = 256;
+  if (has256 && k_block == TC_F16_SLOT && p.bn == 128) {
+    // fp16 pairs in 256-column tiles run on resident CTAs (gemm_tc_many.cu), whose store phase and start
+    // hide behind the next tile's chains: the wider tile is taken where its waves are cheaper (tenths of a
+    // microsecond: a chain of 256 columns 1.0, of 128 columns 0.6; a store phase exposed 4 and 8, and 2
+    // of it per tile of a resident CTA). 2048 rows of width 512 (6 layers, a forward pass): 626 -> 548 us,
+    // 9216 rows: 2002 -> 1597 us; 1024 rows keep the narrow tiles (406 us).
+    const long long kbs = k / k_block, w256 = (mt * (n / 256) + 147) / 148, w128 = (mt * (n / 128) + 147) / 148;
+    if (w256 * (10 * kbs + 20) + 40 < w128 * (6 * kbs + 80)) p.bn = 256;
+  }
   const long long ctas = mt * (n / p.bn);
   const int kb = k / k_block;
   // Few tiles (a short single stream): cut k over several CTAs per tile so the
@@ -803,6 +812,8 @@ void launch_gemm_tc_f16(const TcMatrix &a, const float *a_inv_scale, const TcMat
     const char *e = std::getenv("LITNICE_B200_TC_WIDE");
     return (e && e[0] >= '0' && e[0] <= '2') ? e[0] - '0' : 1;
   }();
+  // many rows in one of the token loop's forms: resident CTAs; every other form of a 256-column plan below
+  if (bn == 256 && plan.splits == 1 && launch_gemm_tc_many(a, a_inv_scale, b, b_inv_scale, m, n, k, ep, err, st)) return;
   if (bn == 256)
     launch_cfg<256, 2, true>(a, b, m, n, k, ep, plan.splits, scratch, counters, err, st, a_inv_scale, b_inv_scale);
   else if (bn == 128 && wide >= 2)

@@ -52,6 +52,8 @@ struct TcEpilogue {
   float *vt_hi = nullptr;
   float *vt_lo = nullptr;
   int vt_col0 = 0, vt_rows = 0, vt_pitch = 0, vt_s = 0, vt_streams = 0;
+  // Graph replay: m is a bound, the rows in use are vt_streams * state->s (of every form; only
+  // launch_gemm_tc_many leaves the tiles behind them out).
   const LoopState *state = nullptr;
   // The same outputs as fp16 pairs under fixed scales, for the fp16-pair attention kernel: every
   // 64-column block of the result (one head of Q, K or V) is multiplied by col_scale[column / 64],
@@ -137,6 +139,10 @@ void launch_gemm_tc(const TcMatrix &a, const TcMatrix &b, int m, int n, int k, c
 void launch_gemm_tc_f16(const TcMatrix &a, const float *a_inv_scale, const TcMatrix &b, const float *b_inv_scale,
                         int m, int n, int k, const TcPlan &plan, const TcEpilogue &ep, float *scratch, int *counters,
                         DevErr *err, cudaStream_t st);
+// gemm_tc_many.cu: the same for the three epilogue forms of the token loop (QKV, W1, out-projection / W2) in tiles of
+// 128 x 256; false: a form, shape or alignment it does not take, and nothing was launched.
+bool launch_gemm_tc_many(const TcMatrix &a, const float *a_inv_scale, const TcMatrix &b, const float *b_inv_scale, int m, int n,
+                         int k, const TcEpilogue &ep, DevErr *err, cudaStream_t st);
 // Row-major W [k, n] (rows optionally scaled) -> K-major fp16 pair [n, k] with one
 // scale for the matrix; *inv_scale_dev (device float) receives its inverse.
 // amax_scratch: one int of device memory.

@@ -63,8 +63,7 @@ constexpr unsigned TC_EP_FOLD = 1u, TC_EP_RELU = 2u, TC_EP_RESIDUAL = 4u, TC_EP_
 constexpr unsigned TC_EP_FORM_QKV = TC_EP_FOLD | TC_EP_BIAS | TC_EP_QK16;
 constexpr unsigned TC_EP_FORM_W1 = TC_EP_FOLD | TC_EP_BIAS | TC_EP_RELU | TC_EP_F16;
 constexpr unsigned TC_EP_FORM_RES = TC_EP_BIAS | TC_EP_RESIDUAL | TC_EP_C | TC_EP_F16 | TC_EP_STATS;
-__device__ __forceinline__ unsigned tc_ep_form(const TcEpilogue &ep) {
-  if (ep.kcache != nullptr) return TC_EP_GENERIC;
+__host__ __device__ inline unsigned tc_ep_form(const TcEpilogue &ep) {
   return (ep.ln_u != nullptr ? TC_EP_FOLD : 0u) | (ep.relu ? TC_EP_RELU : 0u) | (ep.residual != nullptr ? TC_EP_RESIDUAL : 0u) |
          (ep.c != nullptr ? TC_EP_C : 0u) | (ep.c_hi != nullptr ? TC_EP_SPLIT : 0u) | (ep.qk16_hi != nullptr ? TC_EP_QK16 : 0u) |
          (ep.c_f16.hi != nullptr ? TC_EP_F16 : 0u) | (ep.stats_out != nullptr ? TC_EP_STATS : 0u) |

@@ -555,6 +555,11 @@ void enqueue_body(litnice_b200_session *s, int B, int sl, const LoopState *dstat
       consume1.ln_stats = consume2.ln_stats = s->row_stats;
       consume1.ln_slots = consume2.ln_slots = D / 64;
       produce.stats_out = s->row_stats;
+      if (!newest)
+        for (TcEpilogue *e : {&consume1, &consume2, &produce}) {
+          e->state = dstate;
+          e->vt_streams = B;
+        }
     } else {
       launch_layernorm_dense(s->x, P(s, o.ln1_g), P(s, o.ln1_b), R, D, s->ln, s->tc ? s->ln_lo : nullptr, rows_state, B,
                              s->st);
@@ -575,8 +580,6 @@ void enqueue_body(litnice_b200_session *s, int B, int sl, const LoopState *dstat
         consume1.vt_rows = D;
         consume1.vt_pitch = s->vt_pitch;
         consume1.vt_s = sl;
-        consume1.vt_streams = B;
-        consume1.state = dstate;
       }
       if (newest) {
         consume1.c = s->dqkv;

@@ -44,8 +44,8 @@ __device__ __forceinline__ unsigned mbar_try_wait(unsigned bar, unsigned parity)
 // execute still costs instruction-cache space.
 // err may be null (a caller without an error word): the wait still ends and
 // the abort flag still tells the other roles.
-static __device__ __noinline__ bool mbar_wait_limit(unsigned bar, unsigned parity, volatile int *abort_flag, DevErr *err,
-                                                    int where, unsigned long long limit_ns) {
+__device__ __forceinline__ bool mbar_wait_body(unsigned bar, unsigned parity, volatile int *abort_flag, DevErr *err, int where,
+                                               unsigned long long limit_ns) {
   const unsigned long long t0 = global_timer();
   unsigned spins = 0;
   while (true) {
@@ -63,6 +63,10 @@ static __device__ __noinline__ bool mbar_wait_limit(unsigned bar, unsigned parit
     }
   }
 }
+static __device__ __noinline__ bool mbar_wait_limit(unsigned bar, unsigned parity, volatile int *abort_flag, DevErr *err,
+                                                    int where, unsigned long long limit_ns) {
+  return mbar_wait_body(bar, parity, abort_flag, err, where, limit_ns);
+}
 static __device__ __forceinline__ bool mbar_wait_slow(unsigned bar, unsigned parity, volatile int *abort_flag,
                                                       DevErr *err, int where) {
   return mbar_wait_limit(bar, parity, abort_flag, err, where, WAIT_LIMIT_NS);
@@ -71,6 +75,12 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatil
                                           int where) {
   if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow(bar, parity, abort_flag, err, where);
+}
+// Without the call: for kernels that re-divide their registers with setmaxnreg (the allocation of a
+// register share does not go through a function's calling convention).
+__device__ __forceinline__ bool mbar_wait_inline(unsigned bar, unsigned parity, volatile int *abort_flag, DevErr *err, int where) {
+  if (mbar_try_wait(bar, parity)) return true;
+  return mbar_wait_body(bar, parity, abort_flag, err, where, WAIT_LIMIT_NS);
 }
 // The same for a whole converged warp: every lane learns the common outcome,
 // so the warp cannot split on a wait that runs out for some lanes only.
