@@ -2,9 +2,9 @@
 // queries, keys and values, and the gated norm of each head's output.
 //
 //   delta_conv_kernel   convolution of a portion's rows, its last inputs kept as the slot's history
-//   delta_step_kernel   the recurrence, state in registers: CTA = one head (and 32 to 128 of its value columns)
-//                       of one stream, warps share the state's rows. FUSED (one new row per stream): convolution,
-//                       recurrence, norm and gate in one launch; otherwise any number of rows in order
+//   delta_step_kernel   one new row per stream: convolution, recurrence, norm and gate in one launch. CTA = one head
+//                       (or 32 to 128 of its value columns) of one stream, warps share the state's rows
+//   delta_rows_kernel   the recurrence of any number of rows in order, a value column in eight lanes' registers
 //   delta_norm_kernel   norm and gate of rows whose outputs lie in memory
 //
 // With the unscaled vectors k', q' and r = 1 / |k'|, r' = dim^-1/2 / |q'| (norms of what the matrix products
@@ -226,14 +226,14 @@ __device__ __forceinline__ void store_cols(float *p, const float (&s)[VPT]) {
   else *p = s[0];
 }
 
-// WARPS warps share the state's rows, DPW each; a lane holds VPT value columns. FUSED: the CTAs of a head are a
+// WARPS warps share the state's rows, DPW each; a lane holds VPT value columns. The CTAs of a head are a
 // cluster (one CTA: none); the squares of its outputs meet in shared memory while each stores its part of the state.
-template <typename T, int WARPS, int DPW, int VPT, bool FUSED>
+template <typename T, int WARPS, int DPW, int VPT>
 __global__ void __launch_bounds__(WARPS * 32, 512 / (WARPS * 32))
-delta_step_kernel(StepArgs a, const T *in, T *history, float *o_rows, T *out, DeltaRows g) {
+delta_step_kernel(StepArgs a, const T *in, T *history, T *out, DeltaRows g) {
   constexpr int THREADS = WARPS * 32, VT = 32 * VPT, DIMS = WARPS * DPW;
   constexpr int FILL = (2 * DIMS + VT + THREADS - 1) / THREADS;
-  __shared__ __align__(16) float vec[2][2 * DIMS + VT];  // q', k', v of a token
+  __shared__ __align__(16) float vec[2 * DIMS + VT];  // q', k', v
   __shared__ __align__(16) float red[WARPS][2][VT];
   __shared__ float squares;
   pdl_launch_dependents();
@@ -272,136 +272,241 @@ delta_step_kernel(StepArgs a, const T *in, T *history, float *o_rows, T *out, De
     return e < 2 * DIMS + VT && v < a.vdim ? 2 * a.groups * a.dim + h * a.vdim + v : -1;
   };
   const int channels = 2 * a.groups * a.dim + a.heads * a.vdim;
-  float next[FILL], next_b, next_a;
-  auto fetch = [&](int t) {
-    const long long r = (long long)b * g.n + t;
+  const T *x_row = in + (long long)b * a.in_ld;
 #pragma unroll
-    for (int i = 0; i < FILL; ++i) {
-      const int c = channel(tid + i * THREADS);
-      next[i] = 0.f;
-      if (c < 0) continue;
-      if constexpr (FUSED) {  // t == 0: the convolution of the one new row
-        T *hist = history + (long long)(g.slot0 + b) * a.taps * channels + c;
-        const T x = in[r * a.in_ld + c];
-        float y = 0.f;
-        for (int j = 0; j + 1 < a.taps; ++j) {
-          const int p = p0 - a.taps + 1 + j;
-          if (p >= 0) y = fmaf(a.conv[(long long)j * channels + c], to_f(hist[(long long)(p % a.taps) * channels]), y);
-        }
-        y = fmaf(a.conv[(long long)(a.taps - 1) * channels + c], to_f(x), y);
-        next[i] = to_f(from_f<T>(Wide<T>::silu(y)));
-        if (tid + i * THREADS >= 2 * DIMS || (vt == 0 && h % (a.heads / a.groups) == 0)) hist[(long long)(p0 % a.taps) * channels] = x;
-      } else {
-        next[i] = to_f(in[r * a.rows_ld + c]);
+  for (int i = 0; i < FILL; ++i) {  // the convolution of the new row
+    const int e = tid + i * THREADS, c = channel(e);
+    if (e >= 2 * DIMS + VT) continue;
+    float value = 0.f;
+    if (c >= 0) {
+      T *hist = history + (long long)(g.slot0 + b) * a.taps * channels + c;
+      const T x = x_row[c];
+      float y = 0.f;
+      for (int j = 0; j + 1 < a.taps; ++j) {
+        const int p = p0 - a.taps + 1 + j;
+        if (p >= 0) y = fmaf(a.conv[(long long)j * channels + c], to_f(hist[(long long)(p % a.taps) * channels]), y);
       }
+      y = fmaf(a.conv[(long long)(a.taps - 1) * channels + c], to_f(x), y);
+      value = to_f(from_f<T>(Wide<T>::silu(y)));
+      if (e >= 2 * DIMS || (vt == 0 && h % (a.heads / a.groups) == 0)) hist[(long long)(p0 % a.taps) * channels] = x;
     }
-    next_b = a.ba[r * a.ba_ld + h];
-    next_a = a.ba[r * a.ba_ld + a.heads + h];
-  };
-  fetch(0);
-  for (int t = 0; t < g.n; ++t) {
-    float *q = vec[t & 1], *k = q + DIMS, *v = k + DIMS;
+    vec[e] = value;
+  }
+  const float beta = sigmoid_f32(a.ba[(long long)b * a.ba_ld + h]);
+  const float decay = expf(delta_log_decay(a.ba[(long long)b * a.ba_ld + a.heads + h], a_exp_log, bias));
+  const float *q = vec, *k = q + DIMS, *v = k + DIMS;
+  __syncthreads();
+  float qq = 0.f, kk = 0.f, kq = 0.f;
+  for (int d = lane; d < DIMS; d += 32) {
+    qq = fmaf(q[d], q[d], qq);
+    kk = fmaf(k[d], k[d], kk);
+    kq = fmaf(k[d], q[d], kq);
+  }
+  float sa[VPT] = {}, sq[VPT] = {};
 #pragma unroll
-    for (int i = 0; i < FILL; ++i)
-      if (tid + i * THREADS < 2 * DIMS + VT) q[tid + i * THREADS] = next[i];
-    const float beta = sigmoid_f32(next_b), decay = expf(delta_log_decay(next_a, a_exp_log, bias));
-    if (!FUSED && t + 1 < g.n) fetch(t + 1);
-    __syncthreads();
-    float qq = 0.f, kk = 0.f, kq = 0.f;
-    for (int d = lane; d < DIMS; d += 32) {
-      qq = fmaf(q[d], q[d], qq);
-      kk = fmaf(k[d], k[d], kk);
-      kq = fmaf(k[d], q[d], kq);
-    }
-    float sa[VPT] = {}, sq[VPT] = {};
-#pragma unroll
-    for (int i = 0; i < DPW; ++i) {
-      const float kd = k[d0 + i], qd = q[d0 + i];
-#pragma unroll
-      for (int j = 0; j < VPT; ++j) {
-        sa[j] = fmaf(kd, s[i][j], sa[j]);
-        sq[j] = fmaf(qd, s[i][j], sq[j]);
-      }
-    }
+  for (int i = 0; i < DPW; ++i) {
+    const float kd = k[d0 + i], qd = q[d0 + i];
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
-      red[wid][0][lane * VPT + j] = sa[j];
-      red[wid][1][lane * VPT + j] = sq[j];
+      sa[j] = fmaf(kd, s[i][j], sa[j]);
+      sq[j] = fmaf(qd, s[i][j], sq[j]);
     }
-    const float rk = 1.0f / sqrtf(warp_sum(kk) + DELTA_UNIT_EPS);
-    const float rq = a.q_scale / sqrtf(warp_sum(qq) + DELTA_UNIT_EPS);
-    kq = warp_sum(kq) * rk * rq;
-    __syncthreads();
-    float u[VPT];
+  }
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) {
+    red[wid][0][lane * VPT + j] = sa[j];
+    red[wid][1][lane * VPT + j] = sq[j];
+  }
+  const float rk = 1.0f / sqrtf(warp_sum(kk) + DELTA_UNIT_EPS);
+  const float rq = a.q_scale / sqrtf(warp_sum(qq) + DELTA_UNIT_EPS);
+  kq = warp_sum(kq) * rk * rq;
+  __syncthreads();
+  float u[VPT];
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) {
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) sum += red[w][0][lane * VPT + j];
+    u[j] = beta * (v[lane * VPT + j] - decay * rk * sum);
+  }
+  float o[VPT];
+  if (wid == 0) {
+    float ss = 0.f;
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
       float sum = 0.f;
 #pragma unroll
-      for (int w = 0; w < WARPS; ++w) sum += red[w][0][lane * VPT + j];
-      u[j] = beta * (v[lane * VPT + j] - decay * rk * sum);
+      for (int w = 0; w < WARPS; ++w) sum += red[w][1][lane * VPT + j];
+      o[j] = decay * rq * sum + kq * u[j];
+      ss = fmaf(o[j], o[j], ss);
     }
-    float o[VPT];
-    if (wid == 0) {
-      float ss = 0.f;
+    ss = warp_sum(ss);  // padding columns are zeros
+    if (lane == 0) squares = ss;
+  }
+  if (tiles > 1) {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  }
 #pragma unroll
-      for (int j = 0; j < VPT; ++j) {
-        float sum = 0.f;
+  for (int i = 0; i < DPW; ++i) {
+    const float kd = k[d0 + i] * rk;
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w) sum += red[w][1][lane * VPT + j];
-        o[j] = decay * rq * sum + kq * u[j];
-        ss = fmaf(o[j], o[j], ss);
-      }
-      if constexpr (FUSED) {  // padding columns are zeros
-        ss = warp_sum(ss);
-        if (lane == 0) squares = ss;
-      } else if (v_in) {
-        const long long r = (long long)b * g.n + t;
-#pragma unroll
-        for (int j = 0; j < VPT; ++j) o_rows[(r * a.heads + h) * a.vdim + v0 + j] = o[j];
-      }
-    }
-    if (FUSED && tiles > 1) {
-      __syncwarp();
-      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    }
-#pragma unroll
-    for (int i = 0; i < DPW; ++i) {
-      const float kd = k[d0 + i] * rk;
-#pragma unroll
-      for (int j = 0; j < VPT; ++j) s[i][j] = fmaf(kd, u[j], decay * s[i][j]);
-    }
-    if constexpr (FUSED) {
-#pragma unroll
-      for (int i = 0; i < DPW; ++i)
-        if (v_in && d0 + i < a.dim) store_cols(S + (long long)(d0 + i) * a.vdim + v0, s[i]);
-      if (tiles > 1) {
-        __syncwarp();
-        cluster_wait();
-      }
-      if (wid == 0) {
-        __syncwarp();
-        float ss = tiles == 1 ? squares : 0.f;
-        if (tiles > 1)
-          for (int i = 0; i < tiles; ++i) ss += ld_cluster_f32(cluster_map(smem_u32(&squares), (unsigned)i));
-        const float inv = 1.0f / sqrtf(ss / a.count + a.eps);
-        const T *gate = in + (long long)b * a.in_ld + channels + h * a.vdim;
-        T *y = out + (long long)b * a.out_ld + h * a.vdim;
-        if (v_in) {
-#pragma unroll
-          for (int j = 0; j < VPT; ++j)
-            y[v0 + j] = from_f<T>(o[j] * inv * a.norm[v0 + j] * Wide<T>::silu(to_f(gate[v0 + j])));
-        }
-      }
-      if (tiles > 1) {  // a CTA's shared memory stays until every other has read it
-        __syncwarp();
-        cluster_sync_all();
-      }
-      return;
-    }
+    for (int j = 0; j < VPT; ++j) s[i][j] = fmaf(kd, u[j], decay * s[i][j]);
   }
 #pragma unroll
   for (int i = 0; i < DPW; ++i)
     if (v_in && d0 + i < a.dim) store_cols(S + (long long)(d0 + i) * a.vdim + v0, s[i]);
+  if (tiles > 1) {
+    __syncwarp();
+    cluster_wait();
+  }
+  if (wid == 0) {
+    __syncwarp();
+    float ss = tiles == 1 ? squares : 0.f;
+    if (tiles > 1)
+      for (int i = 0; i < tiles; ++i) ss += ld_cluster_f32(cluster_map(smem_u32(&squares), (unsigned)i));
+    const float inv = 1.0f / sqrtf(ss / a.count + a.eps);
+    const T *gate = in + (long long)b * a.in_ld + channels + h * a.vdim;
+    T *y = out + (long long)b * a.out_ld + h * a.vdim;
+    if (v_in) {
+#pragma unroll
+      for (int j = 0; j < VPT; ++j)
+        y[v0 + j] = from_f<T>(o[j] * inv * a.norm[v0 + j] * Wide<T>::silu(to_f(gate[v0 + j])));
+    }
+  }
+  if (tiles > 1) {  // a CTA's shared memory stays until every other has read it
+    __syncwarp();
+    cluster_sync_all();
+  }
+}
+
+// The rows of a portion in order. A value column's recurrence needs nothing of the others but the token's vectors: here
+// eight lanes hold one column of the state (DPL rows of it each), so a token costs 2 * DPL products and three shuffles per
+// sum and no barrier; four warps take 16 columns of one head of one stream. A tile of tokens comes to shared memory while
+// the one before is used, with the scalars of its tokens (norms, gate, decay), which no token's state enters. Bound by
+// that chain: 0.16 us a token at dim 64 (8 heads, portions of 9 to 613 rows); with the state's rows over eight warps and
+// two barriers per token it was 1.04 us.
+template <typename T, int DPL>
+__global__ void __launch_bounds__(128)
+delta_rows_kernel(StepArgs a, const T *in, float *o_rows, DeltaRows g) {
+  constexpr int DIMS = 8 * DPL, TT = 2048 / DIMS;  // tokens per tile
+  constexpr int ROW4 = 2 * DIMS / 4, FILL = TT * ROW4 / 128;
+  static_assert(TT >= 4 && TT <= 32 && FILL == 8, "");
+  __shared__ __align__(16) float vec[TT][2 * DIMS];  // q', k'
+  __shared__ __align__(16) float vs[TT][16], os[TT][16];
+  __shared__ __align__(16) float fac[TT][8];  // beta, g r, g r', r r' (k' . q'), r, g
+  __shared__ float ba[2][TT];
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, sub = lane & 7, col = wid * 4 + (lane >> 3);
+  const int tiles = a.vdim / 16;
+  const int h = blockIdx.x / tiles, vt = (blockIdx.x - h * tiles) * 16, b = blockIdx.y;
+  const int grp = h / (a.heads / a.groups);
+  float *S = a.state + ((long long)(g.slot0 + b) * a.heads + h) * a.dim * a.vdim + vt + col;
+  const float a_exp_log = a.a_log[h], bias = a.dt_bias[h];
+  pdl_wait();
+  const bool fresh = g.first_position() == 0;  // a new sequence
+  // row i of a lane: piece i / 4 of 32 rows, four rows per lane
+  auto row_of = [&](int i) { return (i >> 2) * 32 + sub * 4 + (i & 3); };
+  float s[DPL];
+#pragma unroll
+  for (int i = 0; i < DPL; ++i) s[i] = !fresh && row_of(i) < a.dim ? S[(long long)row_of(i) * a.vdim] : 0.f;
+  float4 next[FILL], next_v;
+  float next_b = 0.f, next_a = 0.f;
+  auto fetch = [&](int t0) {
+#pragma unroll
+    for (int i = 0; i < FILL; ++i) {
+      const int e = tid + i * 128, tk = e / ROW4, d = (e - tk * ROW4) * 4, dd = d < DIMS ? d : d - DIMS;
+      const bool ok = t0 + tk < g.n && dd < a.dim;
+      next[i] = ok ? load4(in + ((long long)b * g.n + t0 + tk) * a.rows_ld + (d < DIMS ? grp : a.groups + grp) * a.dim + dd)
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (tid < TT * 4 && t0 + tid / 4 < g.n)
+      next_v = load4(in + ((long long)b * g.n + t0 + tid / 4) * a.rows_ld + 2 * a.groups * a.dim + h * a.vdim + vt + (tid & 3) * 4);
+    if (tid < TT && t0 + tid < g.n) {
+      const float *p = a.ba + ((long long)b * g.n + t0 + tid) * a.ba_ld + h;
+      next_b = p[0];
+      next_a = p[a.heads];
+    }
+  };
+  fetch(0);
+  for (int t0 = 0; t0 < g.n; t0 += TT) {
+    const int nt = min(TT, g.n - t0);
+#pragma unroll
+    for (int i = 0; i < FILL; ++i) reinterpret_cast<float4 *>(&vec[0][0])[tid + i * 128] = next[i];
+    if (tid < TT * 4) reinterpret_cast<float4 *>(&vs[0][0])[tid] = next_v;
+    if (tid < TT) {
+      ba[0][tid] = next_b;
+      ba[1][tid] = next_a;
+    }
+    if (t0 + TT < g.n) fetch(t0 + TT);
+    __syncthreads();
+    for (int tk = tid >> 3; tk < TT; tk += 16) {  // whole warps: TT is a multiple of 4
+      float qq = 0.f, kk = 0.f, kq = 0.f;
+#pragma unroll 4
+      for (int i = 0; i < DPL; i += 4) {
+        const float4 q = load4(&vec[tk][row_of(i)]), k = load4(&vec[tk][DIMS + row_of(i)]);
+        qq = fmaf(q.x, q.x, fmaf(q.y, q.y, fmaf(q.z, q.z, fmaf(q.w, q.w, qq))));
+        kk = fmaf(k.x, k.x, fmaf(k.y, k.y, fmaf(k.z, k.z, fmaf(k.w, k.w, kk))));
+        kq = fmaf(k.x, q.x, fmaf(k.y, q.y, fmaf(k.z, q.z, fmaf(k.w, q.w, kq))));
+      }
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        qq += __shfl_xor_sync(0xffffffffu, qq, o);
+        kk += __shfl_xor_sync(0xffffffffu, kk, o);
+        kq += __shfl_xor_sync(0xffffffffu, kq, o);
+      }
+      if (sub == 0) {
+        const float rk = 1.0f / sqrtf(kk + DELTA_UNIT_EPS), rq = a.q_scale / sqrtf(qq + DELTA_UNIT_EPS);
+        const float decay = expf(delta_log_decay(ba[1][tk], a_exp_log, bias));
+        *reinterpret_cast<float4 *>(&fac[tk][0]) = make_float4(sigmoid_f32(ba[0][tk]), decay * rk, decay * rq, kq * rk * rq);
+        *reinterpret_cast<float2 *>(&fac[tk][4]) = make_float2(rk, decay);
+      }
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (int tk = 0; tk < nt; ++tk) {
+      const float4 f = load4(&fac[tk][0]);
+      const float2 f2 = *reinterpret_cast<const float2 *>(&fac[tk][4]);
+      const float v = vs[tk][col];
+      float4 k[DPL / 4];
+      float sa[4] = {}, sq[4] = {};
+#pragma unroll
+      for (int i = 0; i < DPL; i += 4) {
+        k[i / 4] = load4(&vec[tk][DIMS + row_of(i)]);
+        const float4 q = load4(&vec[tk][row_of(i)]);
+        sa[0] = fmaf(k[i / 4].x, s[i], sa[0]);
+        sa[1] = fmaf(k[i / 4].y, s[i + 1], sa[1]);
+        sa[2] = fmaf(k[i / 4].z, s[i + 2], sa[2]);
+        sa[3] = fmaf(k[i / 4].w, s[i + 3], sa[3]);
+        sq[0] = fmaf(q.x, s[i], sq[0]);
+        sq[1] = fmaf(q.y, s[i + 1], sq[1]);
+        sq[2] = fmaf(q.z, s[i + 2], sq[2]);
+        sq[3] = fmaf(q.w, s[i + 3], sq[3]);
+      }
+      float sum_a = (sa[0] + sa[1]) + (sa[2] + sa[3]), sum_q = (sq[0] + sq[1]) + (sq[2] + sq[3]);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        sum_a += __shfl_xor_sync(0xffffffffu, sum_a, o);
+        sum_q += __shfl_xor_sync(0xffffffffu, sum_q, o);
+      }
+      const float u = f.x * (v - f.y * sum_a), ru = f2.x * u;
+      if (sub == 0) os[tk][col] = f.z * sum_q + f.w * u;
+#pragma unroll
+      for (int i = 0; i < DPL; i += 4) {
+        s[i] = fmaf(k[i / 4].x, ru, f2.y * s[i]);
+        s[i + 1] = fmaf(k[i / 4].y, ru, f2.y * s[i + 1]);
+        s[i + 2] = fmaf(k[i / 4].z, ru, f2.y * s[i + 2]);
+        s[i + 3] = fmaf(k[i / 4].w, ru, f2.y * s[i + 3]);
+      }
+    }
+    __syncthreads();
+    if (tid < nt * 4)
+      *reinterpret_cast<float4 *>(o_rows + (((long long)b * g.n + t0 + tid / 4) * a.heads + h) * a.vdim + vt + (tid & 3) * 4) =
+          load4(&os[0][0] + tid * 4);
+  }
+#pragma unroll
+  for (int i = 0; i < DPL; ++i)
+    if (row_of(i) < a.dim) S[(long long)row_of(i) * a.vdim] = s[i];
 }
 
 // One warp per row and head.
@@ -471,24 +576,24 @@ int launch_t(const DeltaMixer &m, void *scratch, Precision type, const RowBatch 
   a.in_ld = m.in_ld;
   a.out_ld = m.out_ld;
   a.rows_ld = m.conv_channels();
-  auto step = [&](auto kernel, int threads, int vt, const T *src, bool cluster) {
+  auto step = [&](auto kernel, int threads, int vt) {
     const int tiles = (m.vdim + vt - 1) / vt;
     launch_pdl_cluster_x(kernel, dim3((unsigned)(m.heads * tiles), (unsigned)b.streams), dim3((unsigned)threads), 0, st,
-                         g_pdl_enabled, cluster ? (unsigned)tiles : 1u, a, src, static_cast<T *>(m.history), o, out, g);
+                         g_pdl_enabled, (unsigned)tiles, a, in, static_cast<T *>(m.history), out, g);
   };
   if (b.n == 1 && m.dim <= 256 && m.vdim <= 256) {
     // the fewest value columns per lane that let one CTA hold a head: splitting a head further gained nothing at any size
     auto fused = [&](auto one, auto two, auto four, int threads) {
-      if (m.vdim <= 32) step(one, threads, 32, in, true);
-      else if (m.vdim <= 64) step(two, threads, 64, in, true);
-      else step(four, threads, 128, in, true);
+      if (m.vdim <= 32) step(one, threads, 32);
+      else if (m.vdim <= 64) step(two, threads, 64);
+      else step(four, threads, 128);
     };
     if (m.dim <= 64)
-      fused(delta_step_kernel<T, 8, 8, 1, true>, delta_step_kernel<T, 8, 8, 2, true>, delta_step_kernel<T, 8, 8, 4, true>, 256);
+      fused(delta_step_kernel<T, 8, 8, 1>, delta_step_kernel<T, 8, 8, 2>, delta_step_kernel<T, 8, 8, 4>, 256);
     else if (m.dim <= 128)
-      fused(delta_step_kernel<T, 8, 16, 1, true>, delta_step_kernel<T, 8, 16, 2, true>, delta_step_kernel<T, 8, 16, 4, true>, 256);
+      fused(delta_step_kernel<T, 8, 16, 1>, delta_step_kernel<T, 8, 16, 2>, delta_step_kernel<T, 8, 16, 4>, 256);
     else
-      fused(delta_step_kernel<T, 16, 16, 1, true>, delta_step_kernel<T, 16, 16, 2, true>, delta_step_kernel<T, 16, 16, 4, true>,
+      fused(delta_step_kernel<T, 16, 16, 1>, delta_step_kernel<T, 16, 16, 2>, delta_step_kernel<T, 16, 16, 4>,
             512);
     return 1;
   }
@@ -512,11 +617,14 @@ int launch_t(const DeltaMixer &m, void *scratch, Precision type, const RowBatch 
     launches += launch_delta_chunks(m, conv, o, at + part.conv + part.o, b, &normed, st, err);
     if (normed) return launches;
   } else {
-    const T *src = conv;
-    if (m.dim <= 64) step(delta_step_kernel<T, 8, 8, 4, false>, 256, 128, src, false);
-    else if (m.dim <= 128) step(delta_step_kernel<T, 8, 16, 4, false>, 256, 128, src, false);
-    else if (m.dim <= 256) step(delta_step_kernel<T, 16, 16, 4, false>, 512, 128, src, false);
-    else step(delta_step_kernel<T, 16, 32, 2, false>, 512, 64, src, false);
+    auto rows = [&](auto kernel) {
+      launch_pdl(kernel, dim3((unsigned)(m.heads * (m.vdim / 16)), (unsigned)b.streams), dim3(128), 0, st, g_pdl_enabled, a,
+                 (const T *)conv, o, g);
+    };
+    if (m.dim <= 64) rows(delta_rows_kernel<T, 8>);
+    else if (m.dim <= 128) rows(delta_rows_kernel<T, 16>);
+    else if (m.dim <= 256) rows(delta_rows_kernel<T, 32>);
+    else rows(delta_rows_kernel<T, 64>);
     ++launches;
   }
   const long long total = b.rows() * m.heads;
