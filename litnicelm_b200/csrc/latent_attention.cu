@@ -326,7 +326,7 @@ template <int NT, bool CLUSTER>
 __global__ void __launch_bounds__(LD_THREADS)
 latent_chunk_kernel(LdShape g, const bf16 *q_hi, const bf16 *q_lo, const bf16 *cache,
                     int cap, int ld, int stages, float *part_o, float2 *part_ml, const bf16 *__restrict__ w_uv, int w_ld,
-                    bf16 *out, int out_ld) {
+                    int uv_resident, bf16 *out, int out_ld) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int rk = g.rk, pitch = rk + 8;               // 16-byte rows whose fragments hit distinct banks
   bf16 *qh = reinterpret_cast<bf16 *>(smraw);        // [16][pitch] high and low terms of the query
@@ -338,13 +338,20 @@ latent_chunk_kernel(LdShape g, const bf16 *q_hi, const bf16 *q_lo, const bf16 *c
   float *fac = sc + LD_HEADS * SP;                   // [16] factors of what has been summed so far
   bf16 *tiles = reinterpret_cast<bf16 *>(fac + LD_HEADS);     // [stages][LD_KEYS][pitch]
   pdl_launch_dependents();
-  if constexpr (CLUSTER) {  // the value rows this CTA maps its heads through depend on nothing: towards L2 now
+  bf16 *uv = tiles + stages * LD_KEYS * pitch;       // [share][vdim][w_ld] value rows, where uv_resident
+  if constexpr (CLUSTER) {  // the value rows this CTA maps its heads through depend on nothing: on their way now
     const int nh = min(LD_HEADS, g.heads - (int)blockIdx.y * LD_HEADS);
     for (int hh = blockIdx.x; hh < nh; hh += g.splits) {
       const char *rows = reinterpret_cast<const char *>(w_uv + (long long)(blockIdx.y * LD_HEADS + hh) * g.vdim * w_ld);
+      if (uv_resident) {
+        char *to = reinterpret_cast<char *>(uv) + (size_t)(hh / g.splits) * g.vdim * w_ld * 2;
+        for (int at = threadIdx.x * 16; at < g.vdim * w_ld * 2; at += LD_THREADS * 16) copy16(to + at, rows + at, 16);
+        continue;
+      }
       for (int at = threadIdx.x * 128; at < g.vdim * w_ld * 2; at += LD_THREADS * 128)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(rows + at));
     }
+    copy_commit();
   }
   pdl_wait();
   const long long r = blockIdx.z;
@@ -536,7 +543,8 @@ latent_chunk_kernel(LdShape g, const bf16 *q_hi, const bf16 *q_lo, const bf16 *c
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int k = min(k0 + u, n_rows - 1), i = k / g.vdim, e = k - i * g.vdim;
-        wr[u] = w_uv + ((long long)(h0 + (int)blockIdx.x + i * ranks) * g.vdim + e) * w_ld;
+        wr[u] = uv_resident ? uv + (i * g.vdim + e) * w_ld
+                            : w_uv + ((long long)(h0 + (int)blockIdx.x + i * ranks) * g.vdim + e) * w_ld;
         x[u] = ol + i * r8;
       }
       for (int c = lane * 8; c < r8; c += 256) {
@@ -792,14 +800,20 @@ int launch_latent_decode(const LatentAttention &a, const LatentFresh &fresh, flo
   if (rows < LD_ROWS) query(latent_query_kernel<1>, 1);
   else query(latent_query_kernel<LD_ROWS>, LD_ROWS);
   const int stages = g.span > LD_KEYS && chunk_smem(g.rank, 2) <= LD_SMEM_LIMIT ? 2 : 1;
-  const size_t smem = chunk_smem(g.rank, stages);
+  size_t smem = chunk_smem(g.rank, stages);
   const bool cluster = g.splits <= LD_CLUSTER;
+  // Where every CTA has an SM to itself, the value rows of its heads come to shared memory while the queries and scores
+  // are formed (and while the predecessor ends); read from L2 behind them, four rows a warp at a time, they cost 4 us of a
+  // layer's 37 (8 rows, 16 heads of 64, rank 256, 350 keys: 459 -> 410 us a token in 12 layers).
+  const size_t uv = (size_t)((a.heads < LD_HEADS ? a.heads : LD_HEADS) + g.splits - 1) / g.splits * a.vdim * a.w_ld * 2;
+  const bool uv_resident = cluster && (long long)g.splits * (g.heads16 / LD_HEADS) * rows <= 148 && smem + uv <= LD_SMEM_LIMIT;
+  if (uv_resident) smem += uv;
   auto chunk = [&](auto kernel) {
     if (smem > 48 * 1024) LB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     launch_pdl_cluster_x(kernel, dim3((unsigned)g.splits, (unsigned)(g.heads16 / LD_HEADS), (unsigned)rows), dim3(LD_THREADS),
                          smem, st, g_pdl_enabled, cluster ? (unsigned)g.splits : 1u, g, (const bf16 *)qh, (const bf16 *)ql,
                          cache, a.cache.cap, a.cache.ld, stages, po, ml, static_cast<const bf16 *>(a.w_uv), a.w_ld,
-                         static_cast<bf16 *>(a.out), a.out_ld);
+                         uv_resident ? 1 : 0, static_cast<bf16 *>(a.out), a.out_ld);
   };
   if (cluster) {
     if (g.rk <= 128) chunk(latent_chunk_kernel<2, true>);
