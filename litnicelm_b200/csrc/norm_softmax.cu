@@ -145,6 +145,43 @@ __global__ void softmax_rows_kernel(RowView x, RowView out, int causal, float sc
   }
 }
 
+// The same for rows of up to 32 * NP columns, a warp per row with the row in registers: every load of a row in flight
+// together, no barrier, one pass over memory. 16000 rows of 250 columns, causal: 26 us,
+// 87 us with a CTA per row.
+template <int NP>
+__global__ void __launch_bounds__(256) softmax_rows_warp_kernel(RowView x, RowView out, int causal, float scale) {
+  const long long row = blockIdx.x * 8LL + (threadIdx.x >> 5);
+  if (row >= x.rows) return;
+  const int n = (int)x.cols, lane = threadIdx.x & 31, last = causal ? (int)(row % n) : n - 1;
+  const char *xp = x.data + row_offset(x, row);
+  char *op = out.data + row_offset(out, row);
+  float v[NP], mx = -3.402823466e+38f;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int c = lane + 32 * i;
+    v[i] = c <= last ? *reinterpret_cast<const float *>(xp + c * x.cs) : 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    if (causal) v[i] = __fmul_rn(v[i], scale);
+    if (lane + 32 * i <= last) mx = fmaxf(mx, v[i]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  double sum = 0.0;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    v[i] = lane + 32 * i <= last ? expf(__fsub_rn(v[i], mx)) : 0.f;
+    sum += (double)v[i];
+  }
+  const float inv = (float)(1.0 / warp_sum(sum));
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int c = lane + 32 * i;
+    if (c < n) *reinterpret_cast<float *>(op + c * out.cs) = c <= last ? v[i] * inv : 0.f;
+  }
+}
+
 }  // namespace
 
 void launch_layernorm(const RowView &x, const float *gamma, long long gamma_cs, const float *beta,
@@ -171,7 +208,16 @@ void launch_layernorm_dense(const float *x, const float *gamma, const float *bet
 void launch_softmax_rows(const RowView &x, const RowView &out, int causal, float scale,
                          cudaStream_t st) {
   if (x.rows <= 0) return;
-  const int threads = x.cols >= 512 ? 256 : (x.cols >= 128 ? 128 : 32);
+  const unsigned warps = (unsigned)((x.rows + 7) / 8);
+  if (x.cols >= 1 && x.cols <= 1024) {
+    if (x.cols <= 128) softmax_rows_warp_kernel<4><<<warps, 256, 0, st>>>(x, out, causal, scale);
+    else if (x.cols <= 256) softmax_rows_warp_kernel<8><<<warps, 256, 0, st>>>(x, out, causal, scale);
+    else if (x.cols <= 512) softmax_rows_warp_kernel<16><<<warps, 256, 0, st>>>(x, out, causal, scale);
+    else softmax_rows_warp_kernel<32><<<warps, 256, 0, st>>>(x, out, causal, scale);
+    LB_LAUNCH_CHECK();
+    return;
+  }
+  const int threads = 256;
   softmax_rows_kernel<<<(unsigned)x.rows, threads, 0, st>>>(x, out, causal, scale);
   LB_LAUNCH_CHECK();
 }

@@ -265,3 +265,54 @@ be.call("adamw_step", pv, pv, pv, pv, 0, 0.002, 0.9, 0.999, 0.01, 0)
 _, sv = dense(be, np.ones((1, 4, 4), np.float32))
 be.call("softmax_backward_causal_rows_exec_context", sv, sv, sv)
 """, "no exec context group is open")
+
+
+# more ids than classes, and more tokens than a piece, so that rows' sums are put down and taken up again; a column tile's remainder
+@pytest.mark.parametrize("rows,cols,vocab,width", [(5, 700, 11, 130), (3, 341, 1000, 64), (1, 1024, 257, 33), (2, 513, 1, 128)])
+def test_embedding_gradients_bit_exact_over_pieces_and_classes(be, rows, cols, vocab, width):
+    rng = np.random.default_rng(rows * cols)
+    ids = np.minimum(rng.geometric(min(0.9, 8.0 / vocab), size=(rows, cols)) - 1, vocab - 1)
+    d_cur = rng.standard_normal((rows, cols, width)).astype(np.float32)
+    tok0 = rng.standard_normal((vocab, width)).astype(np.float32)
+    pos0 = rng.standard_normal((cols, width)).astype(np.float32)
+    tok_w, pos_w = T.accumulate_embedding_grads(ids, d_cur, tok0, pos0)
+    for p in (be,):
+        _, iv = dense(p, ids.astype(np.int32), dtype=1)
+        _, cv = dense(p, d_cur)
+        tb, tv = dense(p, tok0)
+        pb, pv = dense(p, pos0)
+        p.call("accumulate_embedding_grads", iv, cv, tv, pv)
+        assert np.array_equal(read(tb, tv), tok_w)
+        assert np.array_equal(read(pb, pv), pos_w)
+
+
+# rows a warp holds in registers (up to 512 and 1024 columns) and rows beyond; the row's own end, and a causal row's
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 128, 129, 256, 257, 512, 513, 1024, 1025])
+@pytest.mark.parametrize("causal", [False, True])
+def test_softmax_rows_of_every_size(be, n, causal):
+    rng = np.random.default_rng(n)
+    rows = n if causal else 11
+    x = (rng.standard_normal((1, rows, n)) * 3).astype(np.float32)
+    g = rng.standard_normal((1, rows, n)).astype(np.float32)
+    scale = 0.37
+    z = x.astype(np.float64) * (scale if causal else 1.0)
+    if causal:
+        z = np.where(np.arange(n)[None] <= np.arange(rows)[:, None], z, -np.inf)
+    w = np.exp(z - z.max(-1, keepdims=True))
+    w /= w.sum(-1, keepdims=True)
+    for p in (be,):
+        xb, xv = dense(p, x)
+        ob, ov = dense(p, np.full_like(x, 7.0))
+        if causal:
+            p.call("scaled_causal_softmax_rows", xv, scale, ov)
+        else:
+            p.call("softmax_rows", xv, ov)
+        got = read(ob, ov)
+        # one rounding each of scale, difference, expf (2 ulp) and the product with the inverse: below 2^-20 of the weight
+        assert np.all(np.abs(got - w) <= 2.0 ** -20 * w + 1e-30 + 2.0 ** -22 * np.abs(z.clip(-1e3, None)) * w)
+        _, gv = dense(p, g)
+        db, dv = dense(p, np.full_like(x, 7.0))
+        p.call("softmax_backward_causal_rows" if causal else "softmax_backward_rows", ov, gv, dv)
+        s64 = got.astype(np.float64)
+        want = s64 * (g - (s64 * g).sum(-1, keepdims=True))
+        assert np.abs(read(db, dv) - want).max() < 2.0 ** -20 * max(1.0, float(np.abs(g).max()))
