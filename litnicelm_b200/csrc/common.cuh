@@ -155,10 +155,17 @@ struct MatView {
   long long rs, cs;     // bytes
 };
 
+// a / b of two non-negative numbers: in 32 bits where both fit, which is nearly always (a 64-bit division is a call of
+// about a hundred instructions, and an element of a view costs up to eight of them; a training step of 265 launches
+// went from 3.28 to 3.24 ms).
+__host__ __device__ __forceinline__ long long div_index(long long a, long long b) {
+  return (unsigned long long)(a | b) >> 32 == 0 ? (long long)((unsigned)a / (unsigned)b) : a / b;
+}
+
 __host__ __device__ inline long long row_offset(const RowView &v, long long row) {
   long long off = 0;
   for (int i = v.np - 1; i >= 0; --i) {
-    const long long q = row / v.pd[i];
+    const long long q = div_index(row, v.pd[i]);
     off += (row - q * v.pd[i]) * v.ps[i];
     row = q;
   }
@@ -168,7 +175,7 @@ __host__ __device__ inline long long row_offset(const RowView &v, long long row)
 __host__ __device__ inline long long batch_offset(const MatView &v, long long b) {
   long long off = 0;
   for (int i = v.nb - 1; i >= 0; --i) {
-    const long long q = b / v.bd[i];
+    const long long q = div_index(b, v.bd[i]);
     off += (b - q * v.bd[i]) * v.bs[i];
     b = q;
   }

@@ -34,13 +34,13 @@ __global__ void rowwise_kernel(RowView a, RowView b, long long b_mod_rows, float
   constexpr bool HAS_B = OP == EW_ADD || OP == EW_ADD_BIAS || OP == EW_ADD_BIAS_RELU || OP == EW_RELU_BWD;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total_chunks;
        idx += (long long)gridDim.x * blockDim.x) {
-    const long long row = idx / chunks_per_row;
+    const long long row = div_index(idx, chunks_per_row);
     const long long c0 = (idx - row * chunks_per_row) * VEC;
     char *op = out.data + row_offset(out, row) + c0 * out.cs;
     const char *ap = HAS_A ? a.data + row_offset(a, row) + c0 * a.cs : nullptr;
     const char *bp = nullptr;
     if (HAS_B) {
-      const long long br = b_mod_rows > 0 ? row % b_mod_rows : row;
+      const long long br = b_mod_rows > 0 ? row - div_index(row, b_mod_rows) * b_mod_rows : row;
       bp = b.data + row_offset(b, br) + c0 * b.cs;
     }
     if (VEC == 4) {
@@ -100,9 +100,9 @@ __global__ void causal_mask_kernel(MatView sc, float neg_inf, long long total) {
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     const long long per = sc.rows * sc.cols;
-    const long long b = idx / per;
+    const long long b = div_index(idx, per);
     const long long rem = idx - b * per;
-    const long long i = rem / sc.cols, j = rem - i * sc.cols;
+    const long long i = div_index(rem, sc.cols), j = rem - i * sc.cols;
     if (j > i)
       *reinterpret_cast<float *>(sc.data + batch_offset(sc, b) + i * sc.rs + j * sc.cs) = neg_inf;
   }
@@ -114,7 +114,7 @@ __global__ void causal_mask_kernel(MatView sc, float neg_inf, long long total) {
 __global__ void embedding_kernel(RowView table, const char *ids_data, int ids_is_f32,
                                  RowView ids_rows, RowView out, long long vocab, DevErr *err) {
   const long long t = blockIdx.x;
-  const long long ir = t / ids_rows.cols, ic = t - ir * ids_rows.cols;
+  const long long ir = div_index(t, ids_rows.cols), ic = t - ir * ids_rows.cols;
   const char *ip = ids_data + row_offset(ids_rows, ir) + ic * ids_rows.cs;
   long long id = ids_is_f32 ? (long long)(*reinterpret_cast<const float *>(ip))
                             : (long long)(*reinterpret_cast<const int *>(ip));
@@ -135,7 +135,7 @@ __global__ void embedding_kernel(RowView table, const char *ids_data, int ids_is
 __global__ void transpose_kernel(MatView x, MatView out, long long total) {
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
-    const long long r = idx / x.cols, c = idx - r * x.cols;
+    const long long r = div_index(idx, x.cols), c = idx - r * x.cols;
     *reinterpret_cast<float *>(out.data + c * out.rs + r * out.cs) =
         *reinterpret_cast<const float *>(x.data + r * x.rs + c * x.cs);
   }

@@ -224,7 +224,7 @@ __global__ void ln_bwd_join_kernel(const float *__restrict__ partial, int chunks
 // receives its rows of d_cur in the CPU order.
 
 __device__ __forceinline__ long long load_index(const char *ids, int is_f32, const RowView &iv, long long t) {
-  const long long r = t / iv.cols, c = t - r * iv.cols;
+  const long long r = div_index(t, iv.cols), c = t - r * iv.cols;
   const char *p = ids + row_offset(iv, r) + c * iv.cs;
   return is_f32 ? (long long)*reinterpret_cast<const float *>(p) : (long long)*reinterpret_cast<const int *>(p);
 }
@@ -233,7 +233,7 @@ __global__ void embedding_grad_pos_kernel(RowView d_cur, long long tokens, long 
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long d = d_cur.cols;
   if (idx >= seq * d) return;
-  const long long pos = idx / d, c = idx - pos * d;
+  const long long pos = div_index(idx, d), c = idx - pos * d;
   const long long po = row_offset(d_pos, pos);
   float acc = ld(d_pos, po, c);
   for (long long t = pos; t < tokens; t += seq) acc += ld(d_cur, row_offset(d_cur, t), c);
