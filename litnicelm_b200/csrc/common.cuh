@@ -144,6 +144,10 @@ struct RowView {
   long long cs;         // stride of the last axis in bytes
 };
 
+// Kernels take views as `const __grid_constant__`: their axes are walked with a variable index, for which a plain
+// by-value parameter is first copied to every thread's local memory (240 to 360 bytes, more than the thread's data: the
+// adds of 2000 rows of 512 took 16.7 us, 6.7 without).
+
 // A batch of matrices: the last two axes are (rows, cols), the rest is batch.
 struct MatView {
   char *data;

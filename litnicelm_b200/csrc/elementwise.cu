@@ -28,8 +28,8 @@ __device__ __forceinline__ float ew_apply(float a, float b, float s) {
 // device_backend.cpp:715-732 (copy), :734-750 (fill), :752-813 (add),
 // :840-940 (bias variants), :942-964 (mul_scalar), :978-1001 (relu).
 template <int OP, int VEC>
-__global__ void rowwise_kernel(RowView a, RowView b, long long b_mod_rows, float scalar,
-                               RowView out, long long chunks_per_row, long long total_chunks) {
+__global__ void rowwise_kernel(const __grid_constant__ RowView a, const __grid_constant__ RowView b, long long b_mod_rows,
+                               float scalar, const __grid_constant__ RowView out, long long chunks_per_row, long long total_chunks) {
   constexpr bool HAS_A = OP != EW_FILL;
   constexpr bool HAS_B = OP == EW_ADD || OP == EW_ADD_BIAS || OP == EW_ADD_BIAS_RELU || OP == EW_RELU_BWD;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total_chunks;
@@ -96,7 +96,7 @@ void launch_rowwise_op(const RowView &a, const RowView *b, long long b_mod_rows,
 }
 
 // device_backend.cpp:1675-1697: scores[.., i, j] = neg_inf for j > i.
-__global__ void causal_mask_kernel(MatView sc, float neg_inf, long long total) {
+__global__ void causal_mask_kernel(const __grid_constant__ MatView sc, float neg_inf, long long total) {
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     const long long per = sc.rows * sc.cols;
@@ -111,8 +111,9 @@ __global__ void causal_mask_kernel(MatView sc, float neg_inf, long long total) {
 // device_backend.cpp:1345-1366: out[t, :] = table[ids[t], :]. The CPU backend
 // throws on an id outside [0, vocab); here the row is zero-filled and the error
 // word is set, and the host raises at its next synchronisation.
-__global__ void embedding_kernel(RowView table, const char *ids_data, int ids_is_f32,
-                                 RowView ids_rows, RowView out, long long vocab, DevErr *err) {
+__global__ void embedding_kernel(const __grid_constant__ RowView table, const char *ids_data, int ids_is_f32,
+                                 const __grid_constant__ RowView ids_rows, const __grid_constant__ RowView out,
+                                 long long vocab, DevErr *err) {
   const long long t = blockIdx.x;
   const long long ir = div_index(t, ids_rows.cols), ic = t - ir * ids_rows.cols;
   const char *ip = ids_data + row_offset(ids_rows, ir) + ic * ids_rows.cs;
@@ -132,7 +133,7 @@ __global__ void embedding_kernel(RowView table, const char *ids_data, int ids_is
 }
 
 // device_backend.cpp:1237-1245.
-__global__ void transpose_kernel(MatView x, MatView out, long long total) {
+__global__ void transpose_kernel(const __grid_constant__ MatView x, const __grid_constant__ MatView out, long long total) {
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     const long long r = div_index(idx, x.cols), c = idx - r * x.cols;

@@ -105,7 +105,7 @@ __global__ void ordered_sum_kernel(const double *__restrict__ partial, int count
 
 constexpr int CS_COLS = 32, CS_LANES = 8;
 
-__global__ void column_sum_kernel(RowView x, long long rows_per_chunk, float *__restrict__ partial) {
+__global__ void column_sum_kernel(const __grid_constant__ RowView x, long long rows_per_chunk, float *__restrict__ partial) {
   __shared__ float red[CS_LANES][CS_COLS];
   const int cx = threadIdx.x % CS_COLS, ry = threadIdx.x / CS_COLS;
   const long long c = blockIdx.x * (long long)CS_COLS + cx;
@@ -137,7 +137,8 @@ __global__ void column_join_kernel(const float *__restrict__ partial, int chunks
 // Columns: dgamma[c] = sum_rows float(dy * xhat), dbeta[c] = sum_rows dy, float sums, by the
 // chunked column reduction above with xhat rebuilt from the saved row statistics.
 
-__global__ void ln_bwd_rows_kernel(RowView x, const char *gamma, long long gamma_cs, RowView dout, RowView dx,
+__global__ void ln_bwd_rows_kernel(const __grid_constant__ RowView x, const char *gamma, long long gamma_cs,
+                                   const __grid_constant__ RowView dout, const __grid_constant__ RowView dx,
                                    double2 *__restrict__ row_stats) {
   const long long row = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= x.rows) return;
@@ -174,7 +175,8 @@ __global__ void ln_bwd_rows_kernel(RowView x, const char *gamma, long long gamma
   if (lane == 0) row_stats[row] = make_double2(mean, inv_std);
 }
 
-__global__ void ln_bwd_columns_kernel(RowView x, RowView dout, const double2 *__restrict__ row_stats,
+__global__ void ln_bwd_columns_kernel(const __grid_constant__ RowView x, const __grid_constant__ RowView dout,
+                                      const double2 *__restrict__ row_stats,
                                       long long rows_per_chunk, float *__restrict__ partial) {
   __shared__ float red_g[CS_LANES][CS_COLS], red_b[CS_LANES][CS_COLS];
   const int cx = threadIdx.x % CS_COLS, ry = threadIdx.x / CS_COLS;
@@ -229,7 +231,8 @@ __device__ __forceinline__ long long load_index(const char *ids, int is_f32, con
   return is_f32 ? (long long)*reinterpret_cast<const float *>(p) : (long long)*reinterpret_cast<const int *>(p);
 }
 
-__global__ void embedding_grad_pos_kernel(RowView d_cur, long long tokens, long long seq, RowView d_pos) {
+__global__ void embedding_grad_pos_kernel(const __grid_constant__ RowView d_cur, long long tokens, long long seq,
+                                          const __grid_constant__ RowView d_pos) {
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long d = d_cur.cols;
   if (idx >= seq * d) return;
@@ -244,10 +247,11 @@ __global__ void embedding_grad_pos_kernel(RowView d_cur, long long tokens, long 
 // class are picked out in order, a piece at a time, and every element of d_tok receives its additions in token order
 // as the CPU loop does: the running sum of the row at hand in a register, EG_AHEAD tokens' gradients in flight. (With
 // each addition read and written back in memory, 64 classes and texts that repeat their common tokens, 2000 tokens of
-// 96 took 459 us, a chain of round trips; now 92 us.)
+// 96 took 459 us, a chain of round trips; now 80 us.)
 constexpr int EG_THREADS = 128, EG_PIECE = 1024, EG_AHEAD = 16;
 __global__ void __launch_bounds__(EG_THREADS)
-embedding_grad_tok_kernel(const char *ids, int ids_is_f32, RowView iv, RowView d_cur, long long tokens, RowView d_tok,
+embedding_grad_tok_kernel(const char *ids, int ids_is_f32, const __grid_constant__ RowView iv,
+                          const __grid_constant__ RowView d_cur, long long tokens, const __grid_constant__ RowView d_tok,
                           long long vocab, DevErr *err) {
   constexpr int PER_WARP = EG_PIECE / (EG_THREADS / 32), TRIPS = PER_WARP / 32;
   __shared__ int s_id[EG_PIECE];         // the class's tokens of the piece: id, and offset of the gradient's row (found by
@@ -330,7 +334,8 @@ embedding_grad_tok_kernel(const char *ids, int ids_is_f32, RowView iv, RowView d
 // ordered_sum_kernel. BACKWARD: logits[t, c] <- (softmax - onehot) / tokens, in place.
 
 template <bool LOSS, bool BACKWARD>
-__global__ void cross_entropy_kernel(RowView logits, const char *targets, int targets_is_f32, RowView tv,
+__global__ void cross_entropy_kernel(const __grid_constant__ RowView logits, const char *targets, int targets_is_f32,
+                                     const __grid_constant__ RowView tv,
                                      double *__restrict__ row_loss, float inv_rows, DevErr *err) {
   __shared__ float red_f[8];
   __shared__ double red_d[8];
@@ -368,7 +373,8 @@ __global__ void cross_entropy_kernel(RowView logits, const char *targets, int ta
 // part and the others receive zero. One warp per row.
 
 template <bool CAUSAL>
-__global__ void softmax_bwd_kernel(RowView sm, RowView dout, RowView dx) {
+__global__ void softmax_bwd_kernel(const __grid_constant__ RowView sm, const __grid_constant__ RowView dout,
+                                   const __grid_constant__ RowView dx) {
   const long long row = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= sm.rows) return;
   const int lane = threadIdx.x & 31;
@@ -387,7 +393,9 @@ __global__ void softmax_bwd_kernel(RowView sm, RowView dout, RowView dx) {
 
 // The same with the rows in registers (up to 32 * NP columns): all loads of a row in flight together, one pass.
 template <bool CAUSAL, int NP>
-__global__ void __launch_bounds__(256) softmax_bwd_row_kernel(RowView sm, RowView dout, RowView dx) {
+__global__ void __launch_bounds__(256)
+softmax_bwd_row_kernel(const __grid_constant__ RowView sm, const __grid_constant__ RowView dout,
+                       const __grid_constant__ RowView dx) {
   const long long row = blockIdx.x * 8LL + (threadIdx.x >> 5);
   if (row >= sm.rows) return;
   const int lane = threadIdx.x & 31, cols = (int)sm.cols, live = CAUSAL ? (int)(row % cols) + 1 : cols;
