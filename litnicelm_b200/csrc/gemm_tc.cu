@@ -404,7 +404,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_consta
   if (go && !(ep.has_vt() && n0 >= ep.vt_col0)) {  // a tile of V columns only has left already
     // the token loop's three forms with their terms fixed at compile time (a loop body that stays in
     // the instruction cache), everything else through the general form
-    const unsigned form = ep.kcache != nullptr ? TC_EP_GENERIC : tc_ep_form(ep);
+    const unsigned form = tc_ep_form(ep);
     if (F16 && form == TC_EP_FORM_QKV)
       tc_store_rows<BN, tc_threads(BN), TC_EP_FORM_QKV>(ep, m, n, m0, n0, (int)threadIdx.x, stage, row_stats, cluster_splits,
                                                         rows_each, row_begin, row_end, first);
@@ -814,6 +814,7 @@ void launch_gemm_tc_f16(const TcMatrix &a, const float *a_inv_scale, const TcMat
   }();
   // many rows in one of the token loop's forms: resident CTAs; every other form of a 256-column plan below
   if (bn == 256 && plan.splits == 1 && launch_gemm_tc_many(a, a_inv_scale, b, b_inv_scale, m, n, k, ep, err, st)) return;
+  if (ep.kcache != nullptr) throw std::invalid_argument("litnice_b200: caches are filled by launch_gemm_tc_many only");
   if (bn == 256)
     launch_cfg<256, 2, true>(a, b, m, n, k, ep, plan.splits, scratch, counters, err, st, a_inv_scale, b_inv_scale);
   else if (bn == 128 && wide >= 2)

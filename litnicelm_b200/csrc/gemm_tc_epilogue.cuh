@@ -155,11 +155,6 @@ __device__ __forceinline__ void tc_store_rows(const TcEpilogue &ep, int m, int n
         *reinterpret_cast<float4 *>(ep.c_hi + off) = hh;
         *reinterpret_cast<float4 *>(ep.c_lo + off) = ll;
       }
-      if (GEN && ep.kcache != nullptr && col >= ep.vt_col0 - ep.vt_rows) {
-        const int s_now = ep.state ? ep.state->s : ep.vt_s, stream = (m0 + rg) / s_now, tok = (m0 + rg) - stream * s_now;
-        if (stream < ep.vt_streams)
-          *reinterpret_cast<float4 *>(ep.kcache + ((long long)stream * ep.kv_cap + tok) * ep.vt_rows + col - (ep.vt_col0 - ep.vt_rows)) = v[g];
-      }
       if (out_qk16) {  // fp16 pair under the head's fixed scale
         uint2 hi, lo;
         f16_pair4(v[g], cs16, hi, lo);
@@ -351,13 +346,6 @@ __device__ __forceinline__ void tc_store_vt(const TcEpilogue &ep, int m, int m0,
     if (!act) continue;
     const float vals[4] = {t.x, t.y, t.z, t.w}, us[4] = {u4.x, u4.y, u4.z, u4.w}, bs[4] = {b4.x, b4.y, b4.z, b4.w};
     const long long at0 = ((long long)v_stream * ep.vt_rows + (col - ep.vt_col0)) * ep.vt_pitch + v_tok;
-    if (ep.vcache != nullptr) {
-      float f[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) f[e] = (fold ? __fmul_rn(st.y, __fmaf_rn(-st.x, us[e], vals[e])) : vals[e]) + bs[e];
-      *reinterpret_cast<float4 *>(ep.vcache + ((long long)v_stream * ep.kv_cap + v_tok) * ep.vt_rows + (col - ep.vt_col0)) =
-          make_float4(f[0], f[1], f[2], f[3]);
-    }
     if (ep.vt16_hi != nullptr) {  // fp16 pair under the head's fixed scale (the four columns share a head)
       const float cs = __ldg(ep.col_scale + col / 64);
 #pragma unroll

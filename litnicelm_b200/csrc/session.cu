@@ -310,6 +310,7 @@ void ensure_rows(litnice_b200_session *s, long long rows) {
   // With fp16-pair operands the attention context, the FFN hidden rows and the QKV
   // output exist only in the formats their consumers read (pair_ctx, pair_h,
   // qkv_hi/qkv_lo + vt), not as fp32 arrays.
+  if (s->f16 && s->kv) alloc(&s->qkv, rows * 3 * D);  // the prompt pass leaves keys and values there for the caches
   if (!s->f16) {
     alloc(&s->ctx, rows * D);
     alloc(&s->qkv, rows * 3 * D);
@@ -600,12 +601,24 @@ void enqueue_body(litnice_b200_session *s, int B, int sl, const LoopState *dstat
       ++s->launches;
     }
     float *kc = s->kv ? s->kcache + l * cache_layer : nullptr, *vc = s->kv ? s->vcache + l * cache_layer : nullptr;
-    if (s->kv_store && s->tc_attn) {  // cached mode, pass over the prompt: this layer's K and V of every position
-      consume1.kcache = kc;
-      consume1.vcache = vc;
-      consume1.kv_cap = s->kv_cap;
-    }
     const float *qkv_bias = fold ? (*tw)[0].ln_v : P(s, o.qkv_b);
+    if (s->kv_store && s->tc_attn) {  // cached mode, pass over the prompt: this layer's K and V of every position
+      const TcWeight &w = (*tw)[0];
+      const TcPlan plan = tc_plan((int)R, 3 * D, D, w.has64, w.has128, w.has256, TC_F16_SLOT);
+      if (s->attn16 && plan.bn == 256 && plan.splits == 1) {  // many rows: the product itself stores them
+        consume1.kcache = kc;
+        consume1.vcache = vc;
+        consume1.kv_cap = s->kv_cap;
+      } else {  // few rows: from a product of their own with a plain fp32 result
+        TcEpilogue plain = consume1;
+        plain.bias = qkv_bias;
+        plain.c = s->qkv;
+        if (s->f16) projection_f16(s, PAIR_LN, R, D, &w, 3 * D, plain);
+        else projection(s, A_LN, R, D, P(s, o.qkv_w), &w, 3 * D, qkv_bias, nullptr, 0, s->qkv, nullptr, fold ? &consume1 : nullptr);
+        launch_kv_store(s->qkv, dstate, sl, B, D, s->kv_cap, kc, vc, s->st);
+        ++s->launches;
+      }
+    }
     if (s->f16) {
       // every projection input is an fp16 pair written by the kernel that produced it
       consume1.bias = qkv_bias;
