@@ -75,6 +75,10 @@ __device__ __forceinline__ void gs_split(float x, float &hi, float &lo) {
   lo = __uint_as_float(__float_as_uint(x - hi) + 0x1000u);
 }
 
+// Infinite, not a number, or rounded to infinity by the first part. Asked of the operand itself: what the integer additions
+// above make of such a value may be finite (a NaN's bits can carry into the sign).
+__device__ __forceinline__ bool gs_no_pair(float x) { return (__float_as_uint(x) & 0x7fffffffu) >= 0x7f7ff000u; }
+
 // One tile of 32 rows x 64 k of one operand: read along whichever axis is contiguous, written as rows of k.
 __global__ void __launch_bounds__(256) split_operands_kernel(const __grid_constant__ GsArgs g, int a_blocks) {
   __shared__ float tile[32][65];
@@ -122,22 +126,22 @@ __global__ void __launch_bounds__(256) split_operands_kernel(const __grid_consta
       x[i] = make_float4(p[0], p[1], p[2], p[3]);
     }
   }
-  float bad = 0.f;
+  bool bad = false;
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int r = r0 + (tid >> 4) + i * 16;
     if (r >= o.n || k >= g.kp) continue;
+    bad |= gs_no_pair(x[i].x) | gs_no_pair(x[i].y) | gs_no_pair(x[i].z) | gs_no_pair(x[i].w);
     float4 h, l;
     gs_split(x[i].x, h.x, l.x);
     gs_split(x[i].y, h.y, l.y);
     gs_split(x[i].z, h.z, l.z);
     gs_split(x[i].w, h.w, l.w);
-    bad = fmaf(l.x, 0.f, fmaf(l.y, 0.f, fmaf(l.z, 0.f, fmaf(l.w, 0.f, bad))));  // not a number where lo is not finite
     const long long to = to0 + (long long)r * ld + k;
     *reinterpret_cast<float4 *>(o.hi + to) = h;
     *reinterpret_cast<float4 *>(o.lo + to) = l;
   }
-  if (bad != bad) *g.bad = g.seq;
+  if (bad) *g.bad = g.seq;
 }
 
 // Four results of a row, from column col on, through the epilogue to C.

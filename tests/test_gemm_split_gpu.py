@@ -105,3 +105,37 @@ def test_small_and_tiny_values(be):
     ob, ov = dense(be, np.zeros((256, 256), np.float32))
     be.call("gemm", dense(be, a)[1], dense(be, b)[1], ov)
     assert (np.abs(read(ob, ov) - a.astype(np.float64) @ b.astype(np.float64)) <= bound(a, b)).all()
+
+
+@pytest.mark.parametrize("where", ["a", "b"])
+@pytest.mark.parametrize("bits", [0x7fc00000, 0x7fffffff, 0xffffffff, 0x7f800000, 0xff800000, 0x7f7fffff, 0xff7ffff0])
+@pytest.mark.parametrize("m,n,k", [(300, 200, 512), (64, 96, 2048)])
+def test_one_value_no_pair_holds(be, m, n, k, bits, where):
+    """One NaN (as numpy writes it, as arithmetic on the GPU does, either sign), one infinity or one value beside infinity among
+    values of all lengths: where the result is NaN, where infinite, and the rest within the bound."""
+    rng = np.random.default_rng(bits % 1000 + m)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    a[:, ::3], b[::2] = np.round(a[:, ::3] * 4) / 4, np.round(b[::2] * 8) / 8  # few bits, zeros among them
+    one = np.uint32(bits).view(np.float32)
+    if where == "a":
+        a[17, 33], b[33] = one, np.where(b[33] == 0, 0.5, b[33])
+        b[33, :2] = 0.5, -1.25
+    else:
+        b[33, 17], a[:, 33] = one, np.where(a[:, 33] == 0, 0.5, a[:, 33])
+        a[:2, 33] = 0.5, -1.25
+    with np.errstate(all="ignore"):
+        want = a.astype(np.float64) @ b.astype(np.float64)
+        within = bound(a, b)
+    near = (bits & 0x7fffffff) < 0x7f800000
+    if near:  # sums beside the largest number may come out either way
+        sure = np.abs(want) < 3.0e38
+    else:
+        sure = np.ones_like(want, bool)
+    ob, ov = dense(be, np.zeros((m, n), np.float32))
+    be.call("gemm", dense(be, a)[1], dense(be, b)[1], ov)
+    got = read(ob, ov)
+    assert np.array_equal(np.isnan(got)[sure], np.isnan(want)[sure])
+    fine = np.isfinite(want) & sure
+    assert np.array_equal(got[sure & np.isinf(want)], want[sure & np.isinf(want)])
+    # the sums in the order of k that such operands get round k times
+    assert (np.abs(got[fine] - want[fine]) <= within[fine] * max(1.0, k * 2.0 ** -24 / 2.0 ** -21)).all()
