@@ -491,7 +491,12 @@ void launch_tile(const GsArgs &g, bool pdl, cudaStream_t st, DevErr *err) {
                        st, pdl, (unsigned)g.splits, ah, al, bh, bl, g, err);
 }
 
-constexpr long long GS_ROWS = 16384;  // rows of A per launch: bounds the pairs' memory
+// Rows of each A that one launch takes, by which the pairs' memory is sized too: of a single matrix at most GS_ROWS, which
+// bounds that memory; of batches and sums all.
+constexpr long long GS_ROWS = 16384;
+long long rows_at_once(long long m, long long a_batch, bool sum_batches) {
+  return a_batch > 1 || sum_batches || m < GS_ROWS ? m : GS_ROWS;
+}
 
 void launch_gemm_split(MatView a, MatView b, MatView c, bool sum_batches, const GemmEpilogue &ep, void *scratch, int seq,
                        bool pdl, cudaStream_t st, DevErr *err) {
@@ -578,8 +583,7 @@ size_t gemm_f32_scratch_bytes(long long m, long long n, long long k, long long a
   if (small < 64 && (double)(m < n ? n : m) * k > 4e6) return 0;
   const long long kp = (k + GS_BK - 1) / GS_BK * GS_BK;
   if ((double)m * a_batch > 1e9 || (double)n * b_batch > 1e9 || (double)kp * (sum_batches ? a_batch : 1) > 1e9) return 0;
-  const long long rows = sum_batches || b_batch > 1 || m < GS_ROWS ? m : GS_ROWS;
-  const double floats = 2.0 * kp * ((double)rows * a_batch + (double)n * b_batch);
+  const double floats = 2.0 * kp * ((double)rows_at_once(m, a_batch, sum_batches) * a_batch + (double)n * b_batch);
   if (floats * 4 > 4e9) return 0;
   return (size_t)floats * 4 + 256;
 }
@@ -598,7 +602,7 @@ int launch_gemm_f32(const MatView &a, const MatView &b, const MatView &c, bool s
   const size_t need = gemm_f32_scratch_bytes(fa.rows, fb.cols, fa.cols, fa.batch, fb.batch, sum_batches);
   if (need > 0 && scratch.ensure(need, st)) {
     int launched = 0;
-    const long long part = fa.batch > 1 || sum_batches ? fa.rows : GS_ROWS;
+    const long long part = rows_at_once(fa.rows, fa.batch, sum_batches);
     for (long long r = 0; r < fa.rows; r += part) {
       MatView pa = fa, pc = fc;
       pa.rows = pc.rows = fa.rows - r < part ? fa.rows - r : part;

@@ -5,7 +5,7 @@ import pytest
 
 from abi_util import Buffer
 from litnicelm_b200.plugin import Backend
-from training_util import dense, read
+from training_util import dense, read, sliced
 
 pytestmark = pytest.mark.gpu
 
@@ -139,3 +139,24 @@ def test_one_value_no_pair_holds(be, m, n, k, bits, where):
     assert np.array_equal(got[sure & np.isinf(want)], want[sure & np.isinf(want)])
     # the sums in the order of k that such operands get round k times
     assert (np.abs(got[fine] - want[fine]) <= within[fine] * max(1.0, k * 2.0 ** -24 / 2.0 ** -21)).all()
+
+
+@pytest.mark.parametrize("rows,k,n", [(24000, 512, 512), (40001, 130, 66)])
+def test_many_rows_of_batches_with_gaps(be, rows, k, n):
+    """Two left operands that do not lie one behind another, more rows each than a launch takes of a single one: the pairs of all
+    of them have room. The rows' results against the same rows as one matrix, and against 64-bit sums."""
+    rng = np.random.default_rng(rows)
+    a = rng.standard_normal((2, rows, k)).astype(np.float32)
+    w = rng.standard_normal((k, n)).astype(np.float32)
+    _, av = sliced(be, a, rows + 3)
+    ob, ov = dense(be, np.zeros((2, rows, n), np.float32))
+    _, wv = dense(be, w)
+    be.call("gemm_ranked_matrix_rhs", av, wv, ov)
+    got = read(ob, ov)
+    some = rng.integers(0, rows, 500)
+    some[:3] = 0, rows - 1, 16384
+    want = a[:, some].astype(np.float64) @ w.astype(np.float64)
+    assert (np.abs(got[:, some] - want) <= bound(a[:, some], w)).all()
+    ob, ov = dense(be, np.zeros((2 * rows, n), np.float32))
+    be.call("gemm", dense(be, a.reshape(2 * rows, k))[1], wv, ov)
+    assert (np.abs(got.reshape(2 * rows, n) - read(ob, ov)).max(0) <= 2.0 * bound(a.reshape(2 * rows, k), w).max(0)).all()
