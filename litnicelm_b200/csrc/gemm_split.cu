@@ -176,22 +176,89 @@ __device__ __forceinline__ void gs_store4(const GsArgs &g, float *C, const float
   }
 }
 
-// Four elements of a row the way they would be without pairs.
-__device__ __noinline__ float4 gs_plain4(const GsArgs &g, long long batch, int row, int col) {
-  float v[4];
-  for (int j = 0; j < 4; ++j) {
-    float s = 0.f;
-    for (int of = 0; of < g.sums && col + j < g.n; ++of) {
-      const long long at = g.sums > 1 ? of : batch;
-      const float *x = reinterpret_cast<const float *>(reinterpret_cast<const char *>(g.a.p) + batch_offset(g.a.view, at)) +
-                       (long long)row * g.a.outer;
-      const float *y = reinterpret_cast<const float *>(reinterpret_cast<const char *>(g.b.p) + batch_offset(g.b.view, at)) +
-                       (long long)(col + j) * g.b.outer;
-      for (int k = 0; k < g.k; ++k) s = fmaf(x[(long long)k * g.a.k], y[(long long)k * g.b.k], s);
+// A tile of the product without pairs, rows m0 .. m_end - 1: fused multiply-adds in the order of k, as in gemm_simt.cu. 256
+// threads with 4 H x BN / 16 elements each (H = 1: up to 64 rows), 16 of k at a time through two buffers of shared memory, the next
+// 16 on their way in registers. All threads of the block come here. A value no pair holds may be in all operands of a step that
+// has diverged, so this is about as fast as gemm_simt.cu (2000 x 512 x 2048: 187 us, there 175; 300 x 200 x 512: 34 and 33; 4096 x
+// 4096 x 1024: 1270 and 865).
+template <int BN, int H>
+__device__ __noinline__ void gs_plain_tile(const GsArgs &g, float *sm, int batch, int m0, int m_end, int n0) {
+  constexpr int PK = 16, BM = 64 * H, LDA = BM + 4, LDB = BN + 4, TM = 4 * H, TN = BN / 16;
+  constexpr int NA = BM * PK / 256, NB = BN * PK / 256;
+  float *as = sm, *bs = sm + 2 * PK * LDA;
+  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+  const bool on = tid < 256;
+  const int per = (g.k + PK - 1) / PK, trips = per * g.sums;
+  // A thread's share: elements i of a column of places one step apart, lanes along whichever axis is contiguous
+  const bool a_k = g.a.k == 1, b_k = g.b.k == 1;
+  const int ar = a_k ? tid / PK : tid % BM, ak = a_k ? tid % PK : tid / BM, ar1 = a_k ? 256 / PK : 0, ak1 = a_k ? 0 : 256 / BM;
+  const int br = b_k ? tid / PK : tid % BN, bk = b_k ? tid % PK : tid / BN, br1 = b_k ? 256 / PK : 0, bk1 = b_k ? 0 : 256 / BN;
+  const long long a_step = ar1 * g.a.outer + ak1 * g.a.k, b_step = br1 * g.b.outer + bk1 * g.b.k;
+  const long long a_at = (long long)(m0 + ar) * g.a.outer + ak * g.a.k, b_at = (long long)(n0 + br) * g.b.outer + bk * g.b.k;
+  const float *x = nullptr, *y = nullptr;
+  int left = 0, of = 0;  // of k in this summand
+  float ra[NA], rb[NB];
+  auto load = [&]() {
+    if (left <= 0) {  // the next summand
+      const long long at = g.sums > 1 ? of++ : batch;
+      x = reinterpret_cast<const float *>(reinterpret_cast<const char *>(g.a.p) + batch_offset(g.a.view, at)) + a_at;
+      y = reinterpret_cast<const float *>(reinterpret_cast<const char *>(g.b.p) + batch_offset(g.b.view, at)) + b_at;
+      left = g.k;
     }
-    v[j] = s;
+#pragma unroll
+    for (int i = 0; i < NA; ++i) ra[i] = m0 + ar + i * ar1 < m_end && ak + i * ak1 < left ? x[i * a_step] : 0.f;
+#pragma unroll
+    for (int i = 0; i < NB; ++i) rb[i] = n0 + br + i * br1 < g.n && bk + i * bk1 < left ? y[i * b_step] : 0.f;
+    x += PK * g.a.k;
+    y += PK * g.b.k;
+    left -= PK;
+  };
+  float acc[TM][TN] = {};
+  if (on) load();
+  for (int t = 0; t < trips; ++t) {
+    float *at = as + (t & 1) * PK * LDA, *bt = bs + (t & 1) * PK * LDB;
+    if (on) {
+#pragma unroll
+      for (int i = 0; i < NA; ++i) at[(ak + i * ak1) * LDA + ar + i * ar1] = ra[i];
+#pragma unroll
+      for (int i = 0; i < NB; ++i) bt[(bk + i * bk1) * LDB + br + i * br1] = rb[i];
+    }
+    __syncthreads();  // (a buffer is written again only behind the barrier of the trip after)
+    if (!on) continue;
+    if (t + 1 < trips) load();
+#pragma unroll
+    for (int kk = 0; kk < PK; ++kk) {
+      float u[TM], v[TN];
+#pragma unroll
+      for (int i = 0; i < TM; i += 4) {
+        const float4 f = *reinterpret_cast<const float4 *>(at + kk * LDA + i / 4 * 64 + ty * 4);
+        u[i] = f.x; u[i + 1] = f.y; u[i + 2] = f.z; u[i + 3] = f.w;
+      }
+#pragma unroll
+      for (int j = 0; j < TN; j += 4) {
+        const float4 f = *reinterpret_cast<const float4 *>(bt + kk * LDB + j / 4 * 64 + tx * 4);
+        v[j] = f.x; v[j + 1] = f.y; v[j + 2] = f.z; v[j + 3] = f.w;
+      }
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(u[i], v[j], acc[i][j]);
+    }
   }
-  return make_float4(v[0], v[1], v[2], v[3]);
+  if (on) {
+    const long long c_off = batch_offset(g.cv, batch);
+    float *C = reinterpret_cast<float *>(reinterpret_cast<char *>(g.c) + c_off);
+    const float *R = g.residual ? reinterpret_cast<const float *>(reinterpret_cast<const char *>(g.residual) + c_off) : nullptr;
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; j += 4) {
+        const int row = m0 + i / 4 * 64 + ty * 4 + (i & 3), col = n0 + j / 4 * 64 + tx * 4;
+        if (row < m_end && col < g.n)
+          gs_store4(g, C, R, row, col, make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]));
+      }
+  }
+  __syncthreads();  // the buffers are free for the next tile
 }
 
 template <int BN>
@@ -251,7 +318,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constan
   pdl_wait();
   const bool plain = *g.bad == g.seq;
 
-  if (warp == 0) {
+  if (plain) {  // the CTAs of a tile take a share of its rows each
+    const int share = (GS_BM + g.splits - 1) / g.splits;
+    for (int tile = cta; tile < g.tiles; tile += ctas) {
+      int batch, m0, n0;
+      place(tile, batch, m0, n0);
+      const int row = m0 + rank * share;
+      const int end = min(g.m, min(m0 + GS_BM, row + share));
+      float *sm = reinterpret_cast<float *>(base_ptr);
+      if (end - row <= 64) gs_plain_tile<BN, 1>(g, sm, batch, row, end, n0);
+      else gs_plain_tile<BN, 2>(g, sm, batch, row, end, n0);
+    }
+  } else if (warp == 0) {
     int it = 0;
     bool ok = true;
     for (int tile = cta; tile < g.tiles && ok; tile += ctas) {
@@ -368,16 +446,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constan
         for (int pass = 0; pass < 4; ++pass) {
           const int rr = pass * 8 + (lane >> 2), row = m0 + q * 32 + rr;
           if (row >= g.m || col >= g.n) continue;
-          float4 x = patch[rr * 4 + (piece ^ ((rr >> 1) & 3))];
-          if (plain) x = gs_plain4(g, batch, row, col);
-          gs_store4(g, C, R, row, col, x);
+          gs_store4(g, C, R, row, col, patch[rr * 4 + (piece ^ ((rr >> 1) & 3))]);
         }
         __syncwarp();
       }
     }
   }
   __syncwarp();
-  if (g.splits > 1) {  // one tile, its ranges of k over the CTAs of the cluster
+  if (g.splits > 1 && !plain) {  // one tile, its ranges of k over the CTAs of the cluster
     cluster_sync_all();
     int batch, m0, n0;
     place(cta, batch, m0, n0);
@@ -395,7 +471,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constan
         const float4 y = ld_cluster_f4(cluster_map(at, (unsigned)r));
         x = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
       }
-      if (plain) x = gs_plain4(g, batch, m0 + row, col);
       gs_store4(g, C, R, m0 + row, col, x);
     }
     __syncwarp();

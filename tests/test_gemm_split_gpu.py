@@ -1,5 +1,7 @@
 """The plugin table's products at sizes that run on the tensor cores, against 64-bit sums: tile edges and remainders, strides
 of every kind, summed and batched operands, cut k ranges, epilogues, values that no operand pair holds."""
+import time
+
 import numpy as np
 import pytest
 
@@ -160,3 +162,28 @@ def test_many_rows_of_batches_with_gaps(be, rows, k, n):
     ob, ov = dense(be, np.zeros((2 * rows, n), np.float32))
     be.call("gemm", dense(be, a.reshape(2 * rows, k))[1], wv, ov)
     assert (np.abs(got.reshape(2 * rows, n) - read(ob, ov)).max(0) <= 2.0 * bound(a.reshape(2 * rows, k), w).max(0)).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(2000, 512, 2048), (300, 200, 512)])
+def test_a_product_no_pair_holds_takes_its_time_but_no_more(be, m, n, k):
+    """A step that has diverged has such values everywhere: its products take up to 5 times as long as others (2000 x 512 x 2048: 42
+    and 187 us), which is what fused multiply-adds take (175 us), not a multiple of that."""
+    rng = np.random.default_rng(m)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    ob, ov = dense(be, np.zeros((m, n), np.float32))
+    bv = dense(be, b)[1]
+
+    def least(av):
+        times = []
+        for _ in range(5):
+            read(ob, ov)  # (waits)
+            t = time.perf_counter()
+            for _ in range(30):
+                be.call("gemm", av, bv, ov)
+            read(ob, ov)
+            times.append(time.perf_counter() - t)
+        return min(times)
+
+    usual = least(dense(be, a)[1])
+    a[3, 5] = np.nan
+    assert least(dense(be, a)[1]) < 9.0 * usual
