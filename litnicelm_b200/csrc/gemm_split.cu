@@ -65,7 +65,7 @@ struct GsArgs {
   int m, n, k, kp, sums;  // k of one summand, padded to a multiple of 32, and the number of summands
   int kblocks, relu, c_vec, splits, m_tiles, n_tiles, tiles;
   MatView cv;
-  int *bad, seq;  // *bad == seq: an operand of this product holds a value that a pair cannot
+  int *bad;  // [0] nonzero: an operand of this product holds a value that a pair cannot; [1] blocks that know. At rest zero
 };
 
 // x = hi + lo, both rounded to nearest at 11 bits (the tensor pipe ignores the 13 bits below). The integer addition rounds as
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(256) split_operands_kernel(const __grid_consta
     *reinterpret_cast<float4 *>(o.hi + to) = h;
     *reinterpret_cast<float4 *>(o.lo + to) = l;
   }
-  if (bad) *g.bad = g.seq;
+  if (bad) *g.bad = 1;
 }
 
 // Four results of a row, from column col on, through the epilogue to C.
@@ -316,9 +316,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constan
   const unsigned tmem = *tmem_holder;
   pdl_launch_dependents();
   pdl_wait();
-  const bool plain = *g.bad == g.seq;
+  const bool plain = *static_cast<const volatile int *>(g.bad) != 0;
 
   if (plain) {  // the CTAs of a tile take a share of its rows each
+    __syncthreads();
+    if (threadIdx.x == 0) {  // the last block to have seen the mark takes it away: the next product, or replay, starts without
+      __threadfence();
+      if (atomicInc(reinterpret_cast<unsigned *>(g.bad) + 1, gridDim.x - 1) == gridDim.x - 1) *static_cast<volatile int *>(g.bad) = 0;
+    }
     const int share = (GS_BM + g.splits - 1) / g.splits;
     for (int tile = cta; tile < g.tiles; tile += ctas) {
       int batch, m0, n0;
@@ -573,7 +578,7 @@ long long rows_at_once(long long m, long long a_batch, bool sum_batches) {
   return a_batch > 1 || sum_batches || m < GS_ROWS ? m : GS_ROWS;
 }
 
-void launch_gemm_split(MatView a, MatView b, MatView c, bool sum_batches, const GemmEpilogue &ep, void *scratch, int seq,
+void launch_gemm_split(MatView a, MatView b, MatView c, bool sum_batches, const GemmEpilogue &ep, void *scratch,
                        bool pdl, cudaStream_t st, DevErr *err) {
   GsArgs g{};
   g.m = (int)a.rows;
@@ -584,7 +589,6 @@ void launch_gemm_split(MatView a, MatView b, MatView c, bool sum_batches, const 
   g.a = operand(a, a.rs, a.cs, g.m);
   g.b = operand(b, b.cs, b.rs, g.n);
   g.bad = static_cast<int *>(scratch);
-  g.seq = seq;
   float *pairs = reinterpret_cast<float *>(static_cast<char *>(scratch) + 256);
   const long long na = (long long)g.m * g.kp * g.a.batch, nb = (long long)g.n * g.kp * g.b.batch;
   g.a.hi = pairs;
@@ -685,8 +689,7 @@ int launch_gemm_f32(const MatView &a, const MatView &b, const MatView &c, bool s
       pc.data += r * fc.rs;
       GemmEpilogue pe = ep;
       if (pe.residual) pe.residual = reinterpret_cast<const float *>(reinterpret_cast<const char *>(pe.residual) + r * fc.rs);
-      if (++scratch.seq <= 0) scratch.seq = 1;
-      launch_gemm_split(pa, fb, pc, sum_batches, pe, scratch.p, scratch.seq, scratch.pdl || g_pdl_enabled, st, err);
+      launch_gemm_split(pa, fb, pc, sum_batches, pe, scratch.p, scratch.pdl || g_pdl_enabled, st, err);
       launched += 2;
     }
     return launched;

@@ -6,7 +6,9 @@ import numpy as np
 import pytest
 
 from abi_util import Buffer
-from litnicelm_b200.plugin import Backend
+from litnicelm_b200 import formats
+from litnicelm_b200.plugin import Backend, ModelSession
+from mitilix_util import layer
 from training_util import dense, read, sliced
 
 pytestmark = pytest.mark.gpu
@@ -187,3 +189,35 @@ def test_a_product_no_pair_holds_takes_its_time_but_no_more(be, m, n, k):
     usual = least(dense(be, a)[1])
     a[3, 5] = np.nan
     assert least(dense(be, a)[1]) < 9.0 * usual
+
+
+def test_a_replayed_step_forgets_what_it_met(tmp_path):
+    """A step of a 32-bit model, captured once and replayed: after tokens whose hidden state is not finite its products are as
+    fast as before them."""
+    cfg = formats.mitilix_config(512, 4000, 128, [layer(4, 32, 32, 64, 64, ff=256)], taps=2, eps=1e-5)
+    w = formats.mitilix_random_weights(cfg, 3)
+    # column 0 of the stream is zero but for token 7, whose feed-forward sums there leave the range
+    w["embed"][:, 0] = w["pos"][:, 0] = 0.0
+    w["l0.mix.o"][0] = 0.0
+    w["embed"][7], w["embed"][7, 0] = 0.0, 32.0
+    w["l0.mlp.up"][:16], w["l0.mlp.up"][:16, 0] = 0.0, 2.0 ** 60
+    w["l0.mlp.down"][:, :16] = w["l0.mlp.down"][0] = 0.0
+    w["l0.mlp.down"][0, :16] = 2.0 ** 62
+    w["head"][7] = 0.0
+    formats.write_model_folder(str(tmp_path / "m"), cfg, w)
+    prompts = np.random.default_rng(4).integers(8, 4000, (64, 8)).astype(np.int32)
+    bad = prompts.copy()
+    bad[:, -1] = 7
+    with ModelSession(str(tmp_path / "m"), "float32", 64) as s:
+        def least_ms():
+            times = []
+            for _ in range(4):
+                s.generate(prompts, 40)
+                times.append(s.stats().device_ms)
+            return min(times)
+
+        before = least_ms()
+        assert not np.isfinite(s.forward(bad)).any()
+        s.generate(bad, 40)
+        after = least_ms()
+    assert after < 1.15 * before, (before, after)
