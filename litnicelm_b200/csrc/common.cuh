@@ -350,6 +350,8 @@ struct DecodeAttnPlan {
   size_t scratch_floats;
 };
 DecodeAttnPlan attn_decode_plan(int n_streams, int s, int n_heads, int dh);
+// Floats of `part` for every context of up to `cap` positions.
+size_t attn_decode_scratch_floats(int n_streams, int cap, int n_heads, int dh);
 void launch_embed_last_ln(const float *tok_emb, const float *pos_emb, const int *ids, int ids_ld,
                           const LoopState *state, int s_host, int n_streams, int d, int vocab, const float *gamma,
                           const float *beta, float *x, float *ln, DevErr *err, cudaStream_t st);

@@ -327,6 +327,17 @@ DecodeAttnPlan attn_decode_plan(int n_streams, int s, int n_heads, int dh) {
   return p;
 }
 
+// The number of chunks is not monotone in the context (their length grows in steps of 32): of 48 heads, 192 positions are cut
+// into 6, 224 into 7 and 256 into 4. At most as many as are wanted, or as chunks of 32 (or, where wanted chunks would be longer
+// than that, of 1024) there are in the longest context.
+size_t attn_decode_scratch_floats(int n_streams, int cap, int n_heads, int dh) {
+  const long long heads = (long long)n_streams * n_heads, want = (2 * 148 + heads - 1) / heads;
+  const long long shortest = (cap + 31) / 32, longest = (cap + 1023) / 1024;
+  long long chunks = want < shortest ? want : shortest;
+  if (chunks < longest) chunks = longest;
+  return chunks > 1 ? (size_t)heads * chunks * (dh + 2) : 0;
+}
+
 template <int DH>
 static void launch_attn_decode_dh(const float *qkv, float *kc, float *vc, int cap, int d_model, int n_heads,
                                   int n_streams, const LoopState *state, int s_host, const DecodeAttnPlan &plan,

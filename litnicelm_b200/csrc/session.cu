@@ -843,11 +843,7 @@ void ensure_kv(litnice_b200_session *s, int B, int cap) {
     s->kv_cap = cap;
     ++s->generation;
   }
-  size_t need = 0;
-  for (int sl = 64; sl <= (cap + 63) / 64 * 64; sl += 64) {
-    const size_t f = attn_decode_plan(B, sl, d.n_heads, d.d_model / d.n_heads).scratch_floats;
-    if (f > need) need = f;
-  }
+  const size_t need = attn_decode_scratch_floats(B, cap, d.n_heads, d.d_model / d.n_heads);
   if (s->kv_persist && B <= 8 && decode_persistent_supports(B, d.n_heads, d.d_model, d.d_ff, d.vocab_size)) {
     const size_t need_pk = decode_persistent_scratch_floats(B, d.n_heads, d.d_model, d.d_ff, d.vocab_size, s->sm_count);
     if (need_pk > s->pk_scratch_floats) {

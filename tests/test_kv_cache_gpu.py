@@ -144,3 +144,28 @@ def test_many_streams_step_on_the_tensor_cores(oracle, dims, streams, prompt, ne
         # operands of 22 bits (2^-22 per product), sums of at most 256 terms in fp32 on either side, a handful of layers
         assert rel_err(lg[:n, b, :], ref_logits[:n]) < 2e-5
         agreed_prefix(fast[b], ref_tokens, gaps)
+
+
+# Steps launched one by one (their logits are kept) see contexts between the multiples of 64 that a replayed step is sized for:
+# 48 heads cut 193 .. 224 positions into more chunks than any multiple up to 256, 16 heads 577 .. 608.
+@pytest.mark.parametrize("dims,streams,prompt,new", [
+    ((2, 2, 64, 128, 24, 300), 24, 200, 24),
+    ((1, 2, 128, 128, 30, 640), 8, 590, 20),
+])
+def test_contexts_between_the_buckets(oracle, dims, streams, prompt, new):
+    d = formats.ModelDims(*dims)
+    arena = formats.make_param_arena(d, 7, bias_std=0.02, ln_std=0.1)
+    prompts = np.stack([formats.zipf_prompt(d.vocab, prompt, 70 + i) for i in range(streams)])
+    with Session(d, streams) as s:
+        s.load_params(arena)
+        fast = s.generate(prompts, new)
+        s.keep_step_logits(True)
+        toks = s.generate(prompts, new)
+        lg = s.read_step_logits(new, streams)
+    for b in range(streams):
+        ref_tokens, ref_logits = oracle.generate(d, arena, prompts[b], new, want_logits=True)
+        srt = np.sort(ref_logits.astype(np.float64), axis=1)
+        gaps = srt[:, -1] - srt[:, -2]
+        n = agreed_prefix(toks[b], ref_tokens, gaps)
+        assert rel_err(lg[:n, b, :], ref_logits[:n]) < 2e-5  # as above
+        agreed_prefix(fast[b], ref_tokens, gaps)
