@@ -66,14 +66,16 @@ __device__ __forceinline__ double sb_warp_sum(double v) {
 }
 
 // LayerNorm of eight rows [SB_ROWS][d], a warp each, to out [d][SB_ROWS] (device_backend.cpp:1247-1279). Both sums in one
-// pass, in double: what var = E[x^2] - mean^2 loses is far below the variance's rounding to float.
+// pass, in double, of the values less one of the row's own: its distance from the mean squared is at most d variances, so the
+// variance loses d * 2^-52 of itself however far the row lies from zero.
 __device__ __forceinline__ void sb_layernorm(const float *rows, const float *gamma, const float *beta, int d, double inv_d,
                                              float *out) {
   const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;
   const float *x = rows + r * d;
+  const double at = (double)x[0];
   double sum = 0.0, sq = 0.0;
   for (int c = lane; c < d; c += 32) {
-    const double v = (double)x[c];
+    const double v = (double)x[c] - at;
     sum += v;
     sq = fma(v, v, sq);
   }
@@ -82,8 +84,8 @@ __device__ __forceinline__ void sb_layernorm(const float *rows, const float *gam
     sum += __shfl_xor_sync(0xffffffffu, sum, o);
     sq += __shfl_xor_sync(0xffffffffu, sq, o);
   }
-  const double mean = sum * inv_d, var = fmax(fma(-mean, mean, sq * inv_d), 0.0);
-  const float inv_std = 1.0f / sqrtf((float)var + 1e-5f), fmean = (float)mean;
+  const double off = sum * inv_d, mean = at + off, spread = fma(-off, off, sq * inv_d), var = spread < 0.0 ? 0.0 : spread;
+  const float inv_std = 1.0f / sqrtf((float)var + 1e-5f), fmean = (float)mean;  // (not a number where a value is not finite)
   for (int c = lane; c < d; c += 32) out[c * SB_ROWS + r] = __fadd_rn(__fmul_rn((x[c] - fmean) * inv_std, gamma[c]), beta[c]);
   __syncthreads();
 }

@@ -48,3 +48,40 @@ def test_bad_ids_are_errors():
         s.load_params(formats.make_param_arena(d, 5))
         with pytest.raises(Exception, match="id out of range"):
             s.forward(np.array([[1, 2, 9]], np.int32))
+
+
+@pytest.mark.parametrize("width,heads", [(32, 2), (64, 2), (96, 3)])
+def test_rows_far_from_zero(oracle, width, heads):
+    """Embeddings a million away from zero, half apart: the first LayerNorm's variance comes out of such rows as the host's two
+    passes give it. What it feeds is scaled up so that the stream's own rounding (1/16 at a million) does not count."""
+    d = formats.ModelDims(1, heads, width, 2 * width, 20, 48)
+    arena = formats.make_param_arena(d, 5)
+    layout = formats.ParamLayout.build(d)
+    rng = np.random.default_rng(width)
+    layout.view(arena, "tok_embedding")[...] = 1.0e6 + np.round(4.0 * rng.standard_normal((20, width))) / 8.0
+    layout.view(arena, "pos_embedding")[...] = 0.0
+    layout.view(arena, "layer0.attn_out_w")[...] *= 1e8
+    layout.view(arena, "layer0.ffn_w2")[...] *= 1e4
+    ids = rng.integers(0, 20, (2, 19)).astype(np.int32)
+    with Session(d, 2) as s:
+        s.load_params(arena)
+        got = s.forward(ids, all_rows=True)
+    for b in range(2):
+        want = oracle.forward(d, arena, ids[b])
+        assert float(np.abs(got[b] - want).max() / np.abs(want).max()) < 2e-5
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("place", [0, 37])
+def test_values_that_are_not_finite_stay_visible(oracle, value, place):
+    """One of them in a token's embedding: the logits of its row and of those behind it are not numbers, as the host's are."""
+    d = formats.ModelDims(2, 2, 64, 128, 20, 48)
+    arena = formats.make_param_arena(d, 5)
+    formats.ParamLayout.build(d).view(arena, "tok_embedding")[3, place] = value
+    ids = np.array([1, 2, 4, 5, 3, 6, 7, 8, 9, 10, 11], np.int32)
+    with Session(d, 1) as s:
+        s.load_params(arena)
+        got = s.forward(ids, all_rows=True)[0]
+    assert np.isnan(oracle.forward(d, arena, ids)[4:]).all() and np.isnan(got[4:]).all()
+    before = oracle.forward(d, arena, ids[:4])
+    assert float(np.abs(got[:4] - before).max() / np.abs(before).max()) < 2e-5
