@@ -225,7 +225,7 @@ struct GemmEpilogue {
 // come from the three MatViews' batch axes (b_batch may be null for a shared B).
 void launch_gemm_simt(const MatView &a, const MatView &bmat, const MatView &c, long long m,
                       long long n, long long k, const GemmEpilogue &ep, cudaStream_t st);
-// The same on the tensor cores (gemm_split.cu). SplitScratch: the operands' pairs, owned by whoever issues products on one
+// The same on the tensor cores (gemm_split.cu). SplitScratch: the operands' parts, owned by whoever issues products on one
 // stream; it grows with the products (never while the stream is being captured).
 struct SplitScratch {
   void *p = nullptr;
@@ -240,7 +240,7 @@ struct SplitScratch {
 // Bytes that launch_gemm_f32 uses for a product of these extents (0: it runs on launch_gemm_simt).
 size_t gemm_f32_scratch_bytes(long long m, long long n, long long k, long long a_batch, long long b_batch, bool sum_batches);
 // C[b] = A[b] B[b], or with sum_batches C = sum over b of A[b] B[b], by the kernel that suits the extents; falls back to
-// launch_gemm_simt where there is no memory for the pairs. Returns the kernels launched.
+// launch_gemm_simt where there is no memory for the parts. Returns the kernels launched.
 int launch_gemm_f32(const MatView &a, const MatView &b, const MatView &c, bool sum_batches, const GemmEpilogue &ep,
                     SplitScratch &scratch, cudaStream_t st, DevErr *err);
 

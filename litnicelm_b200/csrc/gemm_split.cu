@@ -3,48 +3,56 @@
 // the products of the plugin table (litnicelm src/model/backend/device_backend.cpp:1096-1235) and of the 32-bit form of the
 // registered designs, where they are large enough (gemm_f32_scratch_bytes).
 //
-// Two kernels. split_operands_kernel writes both operands as TF32 pairs x = hi + lo (22 bits, any exponent) in K-major rows,
-// which TMA can address whatever the operands' strides were. gemm_split_kernel adds a_lo b_hi + a_hi b_lo + a_hi b_hi. The
-// tensor pipe truncates when it accumulates, so a chain in tensor memory is one block of 32 k (12 instructions); the chains are
-// added in registers with rounding to nearest. Where an operand holds a value that a pair cannot (infinite, NaN, or so large
-// that it rounds to infinity) the product is computed with plain fused multiply-adds in the order of k instead, so such values
-// come out as they do there. Parts below 2^-126 count as zero.
+// Two kernels. split_operands_kernel writes both operands in three bfloat16 parts, x = x0 + 2^-8 x1 + 2^-16 x2, each the part
+// before it left over, rounded to nearest: all 24 bits of any finite x, since no part is smaller than bfloat16 can hold. The rows
+// are K-major, which TMA can address whatever the operands' strides were. gemm_split_kernel adds the products of the parts,
+// (1,2) (2,1) | (0,2) (1,1) (2,0) | (0,1) (1,0) in one accumulator, scaled by 2^-8 from one group to the next by the
+// instruction that starts it, and (0,0) in another. What is left out, (2,2), is below 2^-32 of a product. The tensor pipe
+// truncates when it accumulates, so a chain in tensor memory is one block of 64 k; the two accumulators are added, and the chains,
+// in registers with rounding to nearest. A sum of one term is therefore rounded to within 2^-24 of itself as a fused multiply-add
+// is, and exact where that is. Where an operand holds a value that is infinite, NaN or 2^63 and more the product is computed with
+// plain fused multiply-adds in the order of k instead, so such values come out as they do there.
 //
 // gemm_split_kernel: persistent, one CTA of 10 warps per SM, tiles of 128 x BN:
-//   warp 0      one lane issues the TMA loads (a ring of 3 or 4 stages of four operand tiles)
+//   warp 0      one lane issues the TMA loads (a ring of 2 or 3 stages of six operand tiles)
 //   warp 1      owns tensor memory; one lane issues tcgen05.mma
 //   warps 2-9   add finished chains (lane = row, half of the columns) and store the tile while the next one is multiplied
 // Few tiles: k is cut into ranges, the CTAs of a tile form a cluster and each stores a share of the rows from the sums of all,
 // read over distributed shared memory in rank order. Every wait is bounded.
 //
-// Bound: shared memory (a block of 32 k of a 128 x 128 tile is read 12 x 8 KB and written 64 KB, 1280 clocks at 128 bytes; 1630
-// measured) and, for short k, the first loads and the last store of a CTA. 4096^3: 180 TFLOP/s (41 on the tile kernel). A training
-// step of 8 x 250 tokens (width 512, two layers) takes 3.8 ms, 7.0 with the tile kernel. Splitting inside the product's own
-// loading warps instead of a kernel in front (one launch less) measured 134 TFLOP/s at 4096^3 and 52 us against 39 at
-// 2000 x 1536 x 512: two loading warps per scheduler do not hide their latency, four leave too few registers.
+// Bound: shared memory (a block of 64 k of a 128 x 128 tile is read 32 x 8 KB and written 96 KB, 2816 clocks at 128 bytes; 2930
+// measured) and, for short k, the first loads and the last store of a CTA. 4096^3: 742 us, 185 TFLOP/s (41 on the tile kernel;
+// 191 with operands as TF32 pairs, three products and 22 bits; 153 with blocks of 32 k in 64-byte rows). A training step of
+// 8 x 250 tokens (width 512, two layers) takes 2.80 ms, 2.79 with pairs. Splitting inside the product's own loading warps instead
+// of a kernel in front (one launch less) was slower with pairs, 52 us against 39 at 2000 x 1536 x 512: two loading warps per
+// scheduler do not hide their latency, four leave too few registers.
 #include "gemm_tc.cuh"
 #include "tc_ptx.cuh"
+
+#include <cuda_bf16.h>
 
 namespace lb {
 
 namespace {
 
-constexpr int GS_BM = 128, GS_BK = 32, GS_SMS = 148;
+constexpr int GS_BM = 128, GS_BK = 64, GS_SMS = 148;
 constexpr int GS_ADDERS = 8;
 constexpr int GS_THREADS = 64 + 32 * GS_ADDERS;
-constexpr int GS_CHAINS = 4;  // accumulation chains in flight
 
 template <int BN>
 struct GsSmem {
-  static constexpr int STAGES = BN == 128 ? 3 : 4;
+  static constexpr int STAGES = BN == 128 ? 2 : 3;
+  static constexpr int CHAINS = 512 / (2 * BN);  // in flight, two accumulators each
   static constexpr int A_BYTES = GS_BM * 128;
   static constexpr int B_BYTES = BN * 128;
-  static constexpr int STAGE = 2 * (A_BYTES + B_BYTES);
+  static constexpr int STAGE = 3 * (A_BYTES + B_BYTES);
   static constexpr int LD = BN + 4;  // floats per row of a finished range of k, which overlays the stages
-  static constexpr int PATCH_OFF = STAGES * STAGE;  // 2 KB per adding warp: 32 rows of 16 columns
-  static constexpr int BAR_OFF = PATCH_OFF + GS_ADDERS * 2048;
+  static constexpr int PATCH_OFF = STAGES * STAGE;
+  static constexpr int PIECES = BN / 32;  // 32 rows of as many float4s per adding warp
+  static constexpr int BAR_OFF = PATCH_OFF + GS_ADDERS * 512 * PIECES;
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
   static_assert(GS_BM * LD * 4 <= STAGES * STAGE, "the finished range lies over the stages");
+  static_assert(TOTAL <= 227 * 1024 && 8 * (2 * STAGES + 2 * CHAINS + 1) <= 192, "");
 };
 
 struct GsOperand {
@@ -52,7 +60,8 @@ struct GsOperand {
   long long outer, k;  // element strides
   int n;               // outer extent
   int vec;             // rows of k on 16-byte boundaries
-  float *hi, *lo;      // [batch or 1][n][ld]
+  __nv_bfloat16 *part;  // [3][batch or 1][n][ld]
+  long long each;       // elements of a part
   MatView view;        // batch axes
   int batch;
 };
@@ -62,22 +71,23 @@ struct GsArgs {
   float *c;
   const float *residual, *bias;
   long long c_rs, c_cs;
-  int m, n, k, kp, sums;  // k of one summand, padded to a multiple of 32, and the number of summands
+  int m, n, k, kp, sums;  // k of one summand, padded to a multiple of 64, and the number of summands
   int kblocks, relu, c_vec, splits, m_tiles, n_tiles, tiles;
   MatView cv;
-  int *bad;  // [0] nonzero: an operand of this product holds a value that a pair cannot; [1] blocks that know. At rest zero
+  int *bad;  // [0] nonzero: an operand of this product holds a value that three parts cannot; [1] blocks that know. At rest zero
 };
 
-// x = hi + lo, both rounded to nearest at 11 bits (the tensor pipe ignores the 13 bits below). The integer addition rounds as
-// cvt.rna.tf32 does and issues at full rate.
-__device__ __forceinline__ void gs_split(float x, float &hi, float &lo) {
-  hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
-  lo = __uint_as_float(__float_as_uint(x - hi) + 0x1000u);
+// x = x0 + 2^-8 x1 + 2^-16 x2, exactly: what a part leaves has at most 15, then 7 bits.
+__device__ __forceinline__ void gs_split(float x, __nv_bfloat16 (&part)[3]) {
+  part[0] = __float2bfloat16_rn(x);
+  const float r = (x - __bfloat162float(part[0])) * 256.f;
+  part[1] = __float2bfloat16_rn(r);
+  part[2] = __float2bfloat16_rn((r - __bfloat162float(part[1])) * 256.f);
 }
 
-// Infinite, not a number, or rounded to infinity by the first part. Asked of the operand itself: what the integer additions
-// above make of such a value may be finite (a NaN's bits can carry into the sign).
-__device__ __forceinline__ bool gs_no_pair(float x) { return (__float_as_uint(x) & 0x7fffffffu) >= 0x7f7ff000u; }
+// Infinite, not a number, or from 2^63 on: products of lesser ones leave the accumulator of the scaled parts, which reaches twice
+// the product, in range.
+__device__ __forceinline__ bool gs_no_parts(float x) { return (__float_as_uint(x) & 0x7fffffffu) >= 0x5f000000u; }
 
 // One tile of 32 rows x 64 k of one operand: read along whichever axis is contiguous, written as rows of k.
 __global__ void __launch_bounds__(256) split_operands_kernel(const __grid_constant__ GsArgs g, int a_blocks) {
@@ -131,15 +141,18 @@ __global__ void __launch_bounds__(256) split_operands_kernel(const __grid_consta
   for (int i = 0; i < 2; ++i) {
     const int r = r0 + (tid >> 4) + i * 16;
     if (r >= o.n || k >= g.kp) continue;
-    bad |= gs_no_pair(x[i].x) | gs_no_pair(x[i].y) | gs_no_pair(x[i].z) | gs_no_pair(x[i].w);
-    float4 h, l;
-    gs_split(x[i].x, h.x, l.x);
-    gs_split(x[i].y, h.y, l.y);
-    gs_split(x[i].z, h.z, l.z);
-    gs_split(x[i].w, h.w, l.w);
+    bad |= gs_no_parts(x[i].x) | gs_no_parts(x[i].y) | gs_no_parts(x[i].z) | gs_no_parts(x[i].w);
+    const float v[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+    __nv_bfloat16 part[4][3];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) gs_split(v[j], part[j]);
     const long long to = to0 + (long long)r * ld + k;
-    *reinterpret_cast<float4 *>(o.hi + to) = h;
-    *reinterpret_cast<float4 *>(o.lo + to) = l;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const __nv_bfloat162 lo{part[0][q], part[1][q]}, hi{part[2][q], part[3][q]};
+      *reinterpret_cast<uint2 *>(o.part + q * o.each + to) =
+          make_uint2(*reinterpret_cast<const unsigned *>(&lo), *reinterpret_cast<const unsigned *>(&hi));
+    }
   }
   if (bad) *g.bad = 1;
 }
@@ -176,9 +189,27 @@ __device__ __forceinline__ void gs_store4(const GsArgs &g, float *C, const float
   }
 }
 
-// A tile of the product without pairs, rows m0 .. m_end - 1: fused multiply-adds in the order of k, as in gemm_simt.cu. 256
+// D = A B, D += A B, or D = 2^-8 D + A B.
+constexpr int GS_NEW = 0, GS_ADD = 1, GS_SCALED = 2;
+__device__ __forceinline__ void gs_mma(unsigned d, unsigned long long a, unsigned long long b, unsigned idesc, int how) {
+  if (how == GS_SCALED)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, 1, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, 8;\n\t}"
+        ::"r"(d), "l"(a), "l"(b), "r"(idesc)
+        : "memory");
+  else
+    tc_mma_f16(d, a, b, idesc, how == GS_ADD ? 1u : 0u);
+}
+
+struct GsMaps {
+  CUtensorMap a[3], b[3];
+};
+
+// A tile of the product without parts, rows m0 .. m_end - 1: fused multiply-adds in the order of k, as in gemm_simt.cu. 256
 // threads with 4 H x BN / 16 elements each (H = 1: up to 64 rows), 16 of k at a time through two buffers of shared memory, the next
-// 16 on their way in registers. All threads of the block come here. A value no pair holds may be in all operands of a step that
+// 16 on their way in registers. All threads of the block come here. A value the parts cannot hold may be in all operands of a step that
 // has diverged, so this is about as fast as gemm_simt.cu (2000 x 512 x 2048: 187 us, there 175; 300 x 200 x 512: 34 and 33; 4096 x
 // 4096 x 1024: 1270 and 865).
 template <int BN, int H>
@@ -263,11 +294,9 @@ __device__ __noinline__ void gs_plain_tile(const GsArgs &g, float *sm, int batch
 
 template <int BN>
 __global__ void __launch_bounds__(GS_THREADS, 1)
-gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ CUtensorMap a_lo,
-                  const __grid_constant__ CUtensorMap b_hi, const __grid_constant__ CUtensorMap b_lo,
-                  const __grid_constant__ GsArgs g, DevErr *err) {
+gemm_split_kernel(const __grid_constant__ GsMaps maps, const __grid_constant__ GsArgs g, DevErr *err) {
   using L = GsSmem<BN>;
-  constexpr int S = L::STAGES, CW = BN / 2;  // columns of an adding warp
+  constexpr int S = L::STAGES, CHAINS = L::CHAINS, CW = BN / 2;  // columns of an adding warp
   extern __shared__ unsigned char smem_raw[];
   const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char *base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -275,8 +304,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constan
   auto full = [&](int s) { return bars + 8u * s; };
   auto empty = [&](int s) { return bars + 8u * (S + s); };
   auto chain_full = [&](int b) { return bars + 8u * (2 * S + b); };
-  auto chain_empty = [&](int b) { return bars + 8u * (2 * S + GS_CHAINS + b); };
-  const unsigned done = bars + 8u * (2 * S + 2 * GS_CHAINS);
+  auto chain_empty = [&](int b) { return bars + 8u * (2 * S + CHAINS + b); };
+  const unsigned done = bars + 8u * (2 * S + 2 * CHAINS);
   volatile unsigned *tmem_holder = reinterpret_cast<volatile unsigned *>(base_ptr + L::BAR_OFF + 192);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(base_ptr + L::BAR_OFF + 196);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -295,7 +324,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constan
       mbar_init(full(s), 1);
       mbar_init(empty(s), 1);
     }
-    for (int b = 0; b < GS_CHAINS; ++b) {
+    for (int b = 0; b < CHAINS; ++b) {
       mbar_init(chain_full(b), 1);
       mbar_init(chain_empty(b), GS_ADDERS);
     }
@@ -306,7 +335,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constan
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void *)tmem_holder)),
-                 "r"((unsigned)(GS_CHAINS * BN))
+                 "r"(512u)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -351,10 +380,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constan
         if (lane == 0) {
           const unsigned st = base + (unsigned)(s * L::STAGE);
           mbar_expect_tx(full(s), (unsigned)L::STAGE);
-          tma_load_2d(st, &a_hi, kb * GS_BK, m0, full(s));
-          tma_load_2d(st + L::A_BYTES, &a_lo, kb * GS_BK, m0, full(s));
-          tma_load_2d(st + 2 * L::A_BYTES, &b_hi, kb * GS_BK, n0, full(s));
-          tma_load_2d(st + 2 * L::A_BYTES + L::B_BYTES, &b_lo, kb * GS_BK, n0, full(s));
+#pragma unroll
+          for (int q = 2; q >= 0; --q) {
+            tma_load_2d(st + q * L::A_BYTES, &maps.a[q], kb * GS_BK, m0, full(s));
+            tma_load_2d(st + 3 * L::A_BYTES + q * L::B_BYTES, &maps.b[q], kb * GS_BK, n0, full(s));
+          }
         }
         __syncwarp();
       }
@@ -367,27 +397,33 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    constexpr unsigned idesc = umma_idesc_tf32(BN);
+    constexpr unsigned idesc = umma_idesc_bf16(BN);
     int it = 0;
     bool ok = true;
     for (int tile = cta; tile < g.tiles && ok; tile += ctas) {
       for (int kb = 0; kb < count; ++kb, ++it) {
-        const int s = it % S, buf = it % GS_CHAINS;
-        ok = mbar_wait_warp(chain_empty(buf), ((unsigned)(it / GS_CHAINS) & 1u) ^ 1u, abort_flag, err, 52) &&
+        const int s = it % S, buf = it % CHAINS;
+        ok = mbar_wait_warp(chain_empty(buf), ((unsigned)(it / CHAINS) & 1u) ^ 1u, abort_flag, err, 52) &&
              mbar_wait_warp(full(s), (unsigned)(it / S) & 1u, abort_flag, err, 53);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (lane == 0) {
-          const unsigned st = base + (unsigned)(s * L::STAGE), d = tmem + (unsigned)(buf * BN);
-          const unsigned long long ah = umma_desc_k128(st), al = umma_desc_k128(st + L::A_BYTES),
-                                   bh = umma_desc_k128(st + 2 * L::A_BYTES),
-                                   bl = umma_desc_k128(st + 2 * L::A_BYTES + L::B_BYTES);
+          const unsigned st = base + (unsigned)(s * L::STAGE), d = tmem + (unsigned)(buf * 2 * BN);
+          auto times = [&](unsigned to, int i, int j, int start) {  // 64 k of parts i and j; start: see gs_mma
+            const unsigned long long a = umma_desc_k128(st + i * L::A_BYTES),
+                                     b = umma_desc_k128(st + 3 * L::A_BYTES + j * L::B_BYTES);
+            gs_mma(to, a, b, idesc, start);
 #pragma unroll
-          for (unsigned ks = 0; ks < 8; ks += 2) tc_mma_tf32(d, al + ks, bh + ks, idesc, ks ? 1u : 0u);
-#pragma unroll
-          for (unsigned ks = 0; ks < 8; ks += 2) tc_mma_tf32(d, ah + ks, bl + ks, idesc, 1u);
-#pragma unroll
-          for (unsigned ks = 0; ks < 8; ks += 2) tc_mma_tf32(d, ah + ks, bh + ks, idesc, 1u);
+            for (unsigned ks = 2; ks < 8; ks += 2) gs_mma(to, a + ks, b + ks, idesc, GS_ADD);
+          };
+          times(d + BN, 1, 2, GS_NEW);
+          times(d + BN, 2, 1, GS_ADD);
+          times(d + BN, 0, 2, GS_SCALED);
+          times(d + BN, 1, 1, GS_ADD);
+          times(d + BN, 2, 0, GS_ADD);
+          times(d + BN, 0, 1, GS_SCALED);
+          times(d + BN, 1, 0, GS_ADD);
+          times(d, 0, 0, GS_NEW);
           tc_commit(empty(s));
           tc_commit(chain_full(buf));
         }
@@ -402,8 +438,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constan
         if (global_timer() - t0 > WAIT_LIMIT_NS) break;
     }
   } else {
-    const int q = warp & 3, half = (warp - 2) >> 2, piece = lane & 3;
-    float4 *patch = reinterpret_cast<float4 *>(base_ptr + L::PATCH_OFF) + (warp - 2) * 128;
+    constexpr int PIECES = L::PIECES, ROWS = 32 / PIECES;  // a warp stores ROWS rows at a time
+    const int q = warp & 3, half = (warp - 2) >> 2, piece = lane % PIECES;
+    auto turned = [](int row) { return PIECES == 4 ? (row >> 1) & 3 : (row >> 2) & 1; };  // distinct banks
+    float4 *patch = reinterpret_cast<float4 *>(base_ptr + L::PATCH_OFF) + (warp - 2) * (32 * PIECES);
     int it = 0;
     bool ok = true;
     for (int tile = cta; tile < g.tiles && ok; tile += ctas) {
@@ -411,17 +449,19 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constan
 #pragma unroll
       for (int j = 0; j < CW; ++j) acc[j] = 0.f;
       for (int kb = 0; kb < count; ++kb, ++it) {
-        const int buf = it % GS_CHAINS;
-        ok = mbar_wait_warp(chain_full(buf), (unsigned)(it / GS_CHAINS) & 1u, abort_flag, err, 54);
+        const int buf = it % CHAINS;
+        ok = mbar_wait_warp(chain_full(buf), (unsigned)(it / CHAINS) & 1u, abort_flag, err, 54);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int c0 = 0; c0 < CW; c0 += 32) {
-          unsigned r[32];
-          tc_ld32(tmem + ((unsigned)(q * 32) << 16) + (unsigned)(buf * BN + half * CW + c0), r);
+          unsigned r[32], t[32];
+          tc_ld32(tmem + ((unsigned)(q * 32) << 16) + (unsigned)(buf * 2 * BN + half * CW + c0), r);
+          tc_ld32(tmem + ((unsigned)(q * 32) << 16) + (unsigned)(buf * 2 * BN + BN + half * CW + c0), t);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int j = 0; j < 32; ++j) acc[c0 + j] = __fadd_rn(acc[c0 + j], __uint_as_float(r[j]));
+          for (int j = 0; j < 32; ++j)
+            acc[c0 + j] = __fadd_rn(acc[c0 + j], __fmaf_rn(__uint_as_float(t[j]), 0x1p-8f, __uint_as_float(r[j])));
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
@@ -440,18 +480,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constan
       float *C = reinterpret_cast<float *>(reinterpret_cast<char *>(g.c) + c_off);
       const float *R = g.residual ? reinterpret_cast<const float *>(reinterpret_cast<const char *>(g.residual) + c_off) : nullptr;
 #pragma unroll
-      for (int c0 = 0; c0 < CW; c0 += 16) {  // 16 columns at a time, turned so that four lanes store a row's 64 bytes
+      for (int c0 = 0; c0 < CW; c0 += 4 * PIECES) {  // turned so that PIECES lanes store a row's bytes
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          patch[lane * 4 + (j ^ ((lane >> 1) & 3))] =
+        for (int j = 0; j < PIECES; ++j)
+          patch[lane * PIECES + (j ^ turned(lane))] =
               make_float4(acc[c0 + 4 * j], acc[c0 + 4 * j + 1], acc[c0 + 4 * j + 2], acc[c0 + 4 * j + 3]);
         __syncwarp();
         const int col = n0 + half * CW + c0 + piece * 4;
 #pragma unroll 1
-        for (int pass = 0; pass < 4; ++pass) {
-          const int rr = pass * 8 + (lane >> 2), row = m0 + q * 32 + rr;
+        for (int pass = 0; pass < PIECES; ++pass) {
+          const int rr = pass * ROWS + lane / PIECES, row = m0 + q * 32 + rr;
           if (row >= g.m || col >= g.n) continue;
-          gs_store4(g, C, R, row, col, patch[rr * 4 + (piece ^ ((rr >> 1) & 3))]);
+          gs_store4(g, C, R, row, col, patch[rr * PIECES + (piece ^ turned(rr))]);
         }
         __syncwarp();
       }
@@ -485,7 +525,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constan
   __syncthreads();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((unsigned)(GS_CHAINS * BN)));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
   }
 }
 
@@ -527,8 +567,10 @@ void turn(MatView &v) {
   std::swap(v.rs, v.cs);
 }
 
-// Tile width and ranges of k by the time of the longest CTA: blocks of k at what they were measured to take (in clocks: 1630
-// at 128 columns, 1100 at 64), the store of the last tile, and for ranges the exchange of their sums.
+// Tile width and ranges of k by the time of the longest CTA: blocks of 64 k at what they were measured to take (in clocks: 2930
+// at 128 columns, 2450 at 64), the store of the last tile, and for ranges the exchange of their sums. The clusters of a tile's
+// ranges sit inside a GPC each; more of them than fit at once take a second wave (512 x 1536 x 2000: 48 clusters of three 55.8 us,
+// of two 40.4; 613 x 512 x 2048: 20 of six 23.2, of eight 35.5).
 struct Plan {
   int bn, splits, tiles;
 };
@@ -536,16 +578,18 @@ Plan make_plan(long long batch, int m, int n, int kblocks) {
   Plan best{64, 1, 0};
   double least = 1e30;
   const long long mt = (m + GS_BM - 1) / GS_BM;
+  const int *fit = tc_cluster_capacity();
   for (int bn : {64, 128}) {
     if (bn == 128 && n <= 64) continue;
     const long long tiles = batch * mt * ((n + bn - 1) / bn);
     if (tiles > (1 << 30)) throw std::invalid_argument("litnice_b200: product too large");
-    const double block = bn == 128 ? 1630 : 1100;
+    const double block = bn == 128 ? 2930 : 2450;
     for (int s = 1; s <= 8; ++s) {
-      if (s > 1 && (tiles * s > GS_SMS || kblocks < 3 * s)) break;
+      if (s > 1 && (tiles * s > GS_SMS || kblocks < 2 * s)) break;
+      if (s > 1 && fit[s] <= 0) continue;
       const int each = (kblocks + s - 1) / s;
       if ((kblocks + each - 1) / each != s) continue;  // no empty range
-      const double waves = s > 1 ? 1.0 : (double)((tiles + GS_SMS - 1) / GS_SMS);
+      const double waves = (double)(s > 1 ? (tiles + fit[s] - 1) / fit[s] : (tiles + GS_SMS - 1) / GS_SMS);
       const double t = waves * each * block + 3000 + (s > 1 ? 2500 + 500 * s : 0);
       if (t < least) {
         least = t;
@@ -558,20 +602,20 @@ Plan make_plan(long long batch, int m, int n, int kblocks) {
 
 template <int BN>
 void launch_tile(const GsArgs &g, bool pdl, cudaStream_t st, DevErr *err) {
-  CUtensorMap ah, al, bh, bl;
+  GsMaps maps;
   const unsigned long long ld = (unsigned long long)g.kp * g.sums;
   const unsigned long long ra = (unsigned long long)g.m * (g.sums > 1 ? 1 : g.a.batch), rb = (unsigned long long)g.n * (g.sums > 1 ? 1 : g.b.batch);
-  tc_make_map(&ah, g.a.hi, ra, ld, GS_BM);
-  tc_make_map(&al, g.a.lo, ra, ld, GS_BM);
-  tc_make_map(&bh, g.b.hi, rb, ld, BN);
-  tc_make_map(&bl, g.b.lo, rb, ld, BN);
+  for (int q = 0; q < 3; ++q) {
+    tc_make_map_bf16(&maps.a[q], g.a.part + q * g.a.each, ra, ld, ld, GS_BM);
+    tc_make_map_bf16(&maps.b[q], g.b.part + q * g.b.each, rb, ld, ld, BN);
+  }
   LB_CUDA(cudaFuncSetAttribute(gemm_split_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, GsSmem<BN>::TOTAL));
   const int ctas = g.splits > 1 || g.tiles < GS_SMS ? g.tiles : GS_SMS;
   launch_pdl_cluster_x(gemm_split_kernel<BN>, dim3((unsigned)(ctas * g.splits)), dim3(GS_THREADS), (size_t)GsSmem<BN>::TOTAL,
-                       st, pdl, (unsigned)g.splits, ah, al, bh, bl, g, err);
+                       st, pdl, (unsigned)g.splits, maps, g, err);
 }
 
-// Rows of each A that one launch takes, by which the pairs' memory is sized too: of a single matrix at most GS_ROWS, which
+// Rows of each A that one launch takes, by which the parts' memory is sized too: of a single matrix at most GS_ROWS, which
 // bounds that memory; of batches and sums all.
 constexpr long long GS_ROWS = 16384;
 long long rows_at_once(long long m, long long a_batch, bool sum_batches) {
@@ -589,12 +633,10 @@ void launch_gemm_split(MatView a, MatView b, MatView c, bool sum_batches, const 
   g.a = operand(a, a.rs, a.cs, g.m);
   g.b = operand(b, b.cs, b.rs, g.n);
   g.bad = static_cast<int *>(scratch);
-  float *pairs = reinterpret_cast<float *>(static_cast<char *>(scratch) + 256);
-  const long long na = (long long)g.m * g.kp * g.a.batch, nb = (long long)g.n * g.kp * g.b.batch;
-  g.a.hi = pairs;
-  g.a.lo = pairs + na;
-  g.b.hi = pairs + 2 * na;
-  g.b.lo = pairs + 2 * na + nb;
+  g.a.each = (long long)g.m * g.kp * g.a.batch;
+  g.b.each = (long long)g.n * g.kp * g.b.batch;
+  g.a.part = reinterpret_cast<__nv_bfloat16 *>(static_cast<char *>(scratch) + 256);
+  g.b.part = g.a.part + 3 * g.a.each;
   g.c = reinterpret_cast<float *>(c.data);
   g.residual = ep.residual;
   g.bias = ep.bias;
@@ -644,14 +686,14 @@ bool SplitScratch::ensure(size_t need, cudaStream_t st) {
   return true;
 }
 
-// Measured on one B200, both ways, launches back to back in us (tile kernel -> two launches here): 64 x 64 x 64 6 -> 8,
-// 100 x 100 x 64 of 8 batches 7 -> 8.5, 128 x 128 x 128 9 -> 10, 256 x 256 x 256 16 -> 11, 250 x 250 x 64 of 64 batches
-// 32 -> 24, 64 x 512 x 512 29 -> 11, 613 x 3072 x 512 83 -> 25, 2000 x 512 x 2048 297 -> 59, 4096^3 3356 -> 763. The tile kernel is
-// bound by the latency of its k loop (0.05 us a k) where there are few tiles and by the FMA pipe where there are many; here the two
-// launches cost about 8 us and a block of 32 k about 0.6 us. Few rows against a large matrix: splitting the matrix costs more
-// than reading it (16 x 32000 x 1024 would write 262 MB). Below 128 k a sequential sum in 32 bits is as exact as pairs are
-// (k = 64: 1.05e-7 against 1.17e-7 on operands of one sign); from there on the pairs are (k = 250: 2.9e-7 against 1.5e-7,
-// k = 2048: 8.1e-7 against 1.7e-7; gradients of a training step, width 512: 1.12e-7 against 1.03e-7).
+// Measured on one B200, both ways, calls back to back in us (tile kernel -> two launches here): 128 x 128 x 128 10 -> 10,
+// 256 x 256 x 256 17 -> 10.5, 250 x 250 x 250 of 8 batches 19.5 -> 17, 64 x 512 x 512 31 -> 11, 613 x 3072 x 512 83 -> 25,
+// 2000 x 512 x 2048 174 -> 40, 4096^3 3352 -> 742. The tile kernel is bound by the latency of its k loop (0.05 us a k) where there
+// are few tiles and by the FMA pipe where there are many; here the two launches cost about 8 us where they are short (the split
+// alone takes 14 us on average in a training step, of which it writes a third more than it reads) and a block of 64 k 1.5 us. Few
+// rows against a large matrix: splitting the matrix costs more than reading it (16 x 32000 x 1024 would write 196 MB). Errors
+// against 64-bit sums, 2-norm (tile kernel, here): k = 256 2.9e-7, 8.0e-8; k = 2048 8.1e-7, 9.9e-8, on operands of one sign 7.0e-7,
+// 9.2e-8, on factors over twelve decades 3.5e-7, 1.3e-7. Below 128 k the tile kernel is near enough and faster.
 size_t gemm_f32_scratch_bytes(long long m, long long n, long long k, long long a_batch, long long b_batch, bool sum_batches) {
   const long long batch = a_batch, total_k = sum_batches ? k * a_batch : k;
   if (m <= 0 || n <= 0 || k <= 0 || batch <= 0) return 0;
@@ -662,9 +704,9 @@ size_t gemm_f32_scratch_bytes(long long m, long long n, long long k, long long a
   if (small < 64 && (double)(m < n ? n : m) * k > 4e6) return 0;
   const long long kp = (k + GS_BK - 1) / GS_BK * GS_BK;
   if ((double)m * a_batch > 1e9 || (double)n * b_batch > 1e9 || (double)kp * (sum_batches ? a_batch : 1) > 1e9) return 0;
-  const double floats = 2.0 * kp * ((double)rows_at_once(m, a_batch, sum_batches) * a_batch + (double)n * b_batch);
-  if (floats * 4 > 4e9) return 0;
-  return (size_t)floats * 4 + 256;
+  const double parts = 3.0 * kp * ((double)rows_at_once(m, a_batch, sum_batches) * a_batch + (double)n * b_batch);
+  if (parts * 2 > 4e9) return 0;
+  return (size_t)parts * 2 + 256;
 }
 
 int launch_gemm_f32(const MatView &a, const MatView &b, const MatView &c, bool sum_batches, const GemmEpilogue &ep,

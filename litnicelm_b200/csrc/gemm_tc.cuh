@@ -140,6 +140,8 @@ void launch_gemm_tc(const TcMatrix &a, const TcMatrix &b, int m, int n, int k, c
 void launch_gemm_tc_f16(const TcMatrix &a, const float *a_inv_scale, const TcMatrix &b, const float *b_inv_scale,
                         int m, int n, int k, const TcPlan &plan, const TcEpilogue &ep, float *scratch, int *counters,
                         DevErr *err, cudaStream_t st);
+// Clusters of 2 .. 8 CTAs (index) that the device holds at once, of kernels that run one CTA per SM; -1 unknown.
+const int *tc_cluster_capacity();
 // gemm_tc_many.cu: the same for the three epilogue forms of the token loop (QKV, W1, out-projection / W2) in tiles of
 // 128 x 256; false: a form, shape or alignment it does not take, and nothing was launched.
 bool launch_gemm_tc_many(const TcMatrix &a, const float *a_inv_scale, const TcMatrix &b, const float *b_inv_scale, int m, int n,

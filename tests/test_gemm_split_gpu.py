@@ -221,3 +221,68 @@ def test_a_replayed_step_forgets_what_it_met(tmp_path):
         s.generate(bad, 40)
         after = least_ms()
     assert after < 1.15 * before, (before, after)
+
+
+def hits(rng, k, n):
+    """A k x n matrix with a single one per column."""
+    e = np.zeros((k, n), np.float32)
+    e[rng.integers(0, k, n), np.arange(n)] = 1.0
+    return e
+
+
+@pytest.mark.parametrize("m,n,k", [(256, 200, 512), (130, 60, 1100), (700, 330, 320)])
+def test_sums_of_one_term_keep_every_bit(be, m, n, k):
+    """Columns of ones and zeros pick values of all lengths and sizes out of a row, unchanged; with one factor in the ones' place the
+    product is a fused multiply-add's: rounded once, here within 2^-24 (half a unit in the last place) and what the sum of the parts'
+    products adds, 2^-8 of that."""
+    rng = np.random.default_rng(m + k)
+    a = (rng.standard_normal((m, k)) * 10.0 ** rng.uniform(-30, 15, (m, k))).astype(np.float32)
+    a[:, ::4] = np.ldexp(1.0 - 2.0 ** -24 * rng.integers(1, 9, a[:, ::4].shape), rng.integers(-90, 60, a[:, ::4].shape))  # below powers of two
+    a[::2] *= -1.0
+    e = hits(rng, k, n)
+    ob, ov = dense(be, np.zeros((m, n), np.float32))
+    be.call("gemm", dense(be, a)[1], dense(be, e)[1], ov)
+    assert np.array_equal(read(ob, ov), a[:, e.argmax(0)])
+    et, at = np.ascontiguousarray(e.T), np.ascontiguousarray(a.T)
+    ob, ov = dense(be, np.zeros((n, m), np.float32))
+    be.call("gemm", dense(be, et)[1], dense(be, at)[1], ov)
+    assert np.array_equal(read(ob, ov), a[:, e.argmax(0)].T)
+    f = e * rng.standard_normal((1, n)).astype(np.float32)
+    ob, ov = dense(be, np.zeros((m, n), np.float32))
+    be.call("gemm", dense(be, a)[1], dense(be, f)[1], ov)
+    want = a.astype(np.float64) @ f.astype(np.float64)
+    assert (np.abs(read(ob, ov) - want) <= 2.0 ** -24 * (1 + 2.0 ** -8) * np.abs(want)).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(200, 130, 256), (64, 300, 2048)])
+@pytest.mark.parametrize("of", ["normal", "positive", "uneven"])
+def test_error_not_above_sums_in_32_bits(be, m, n, k, of):
+    """Against 64-bit sums, in the 2-norm: no further off than multiplied and added one after another in 32 bits."""
+    rng = np.random.default_rng(k)
+    a, b = rng.standard_normal((m, k)), rng.standard_normal((k, n))
+    if of == "positive":
+        a, b = np.abs(a), np.abs(b)
+    if of == "uneven":
+        a, b = a * 10.0 ** rng.uniform(-5, 5, a.shape), b * 10.0 ** rng.uniform(-5, 5, b.shape)
+    a, b = a.astype(np.float32), b.astype(np.float32)
+    ob, ov = dense(be, np.zeros((m, n), np.float32))
+    be.call("gemm", dense(be, a)[1], dense(be, b)[1], ov)
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    plain = np.zeros((m, n), np.float32)
+    for i in range(k):
+        plain += a[:, i:i + 1] * b[i:i + 1]
+    assert np.linalg.norm(read(ob, ov) - want) <= np.linalg.norm(plain - want)
+
+
+def test_values_near_the_smallest(be):
+    """Operands down to the smallest normal numbers: nothing of them is lost."""
+    rng = np.random.default_rng(9)
+    a = (rng.standard_normal((256, 512)) * 1e-37).astype(np.float32)
+    b = (rng.standard_normal((512, 256)) * 1e17).astype(np.float32)
+    ob, ov = dense(be, np.zeros((256, 256), np.float32))
+    be.call("gemm", dense(be, a)[1], dense(be, b)[1], ov)
+    assert (np.abs(read(ob, ov) - a.astype(np.float64) @ b.astype(np.float64)) <= bound(a, b)).all()
+    a[np.abs(a) < 2.0 ** -126] = 2.0 ** -126
+    e = hits(rng, 512, 256)
+    be.call("gemm", dense(be, a)[1], dense(be, e)[1], ov)
+    assert np.array_equal(read(ob, ov), a[:, e.argmax(0)])
