@@ -157,6 +157,7 @@ void *api_create(uint32_t device_kind) {
   try {
     b->device = dev;
     b->split.pdl = true;
+    b->split.least = 64 << 20;
     if (const char *env = std::getenv("LITNICE_B200_READ_AHEAD")) b->read_ahead = env[0] != '0';
     if (const char *env = std::getenv("LITNICE_B200_ABI_QUEUE")) b->queue_on = env[0] != '0';
     bind(b);

@@ -230,6 +230,7 @@ void launch_gemm_simt(const MatView &a, const MatView &bmat, const MatView &c, l
 struct SplitScratch {
   void *p = nullptr;
   size_t bytes = 0;
+  size_t least = 0;  // bytes of the first allocation at least
   bool pdl = false;  // launch dependent kernels early although the thread's PdlScope does not say so
   SplitScratch() = default;
   SplitScratch(const SplitScratch &) = delete;

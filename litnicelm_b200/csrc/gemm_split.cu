@@ -669,17 +669,22 @@ bool SplitScratch::ensure(size_t need, cudaStream_t st) {
   if (need <= bytes) return true;
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) return false;
+  // Products come in all sizes: with room for the largest so far alone, a first training step stopped for a new allocation a
+  // dozen times (each waits for the stream). So the first is generous and the others double, up to a gigabyte.
+  size_t grown = need + need / 4;
+  const size_t room = bytes ? (bytes < (size_t)512 << 20 ? 2 * bytes : (size_t)1 << 30) : least;
+  if (grown < room) grown = room;
   if (p) {
     LB_CUDA(cudaStreamSynchronize(st));
     cudaFree(p);
     p = nullptr;
     bytes = 0;
   }
-  const size_t grown = need + need / 4;
-  if (cudaMalloc(&p, grown) != cudaSuccess) {
+  while (cudaMalloc(&p, grown) != cudaSuccess) {
     p = nullptr;
     (void)cudaGetLastError();
-    return false;
+    if (grown == need) return false;
+    grown = need;
   }
   bytes = grown;
   LB_CUDA(cudaMemsetAsync(p, 0, 256, st));

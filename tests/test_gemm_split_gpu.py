@@ -286,3 +286,23 @@ def test_values_near_the_smallest(be):
     e = hits(rng, 512, 256)
     be.call("gemm", dense(be, a)[1], dense(be, e)[1], ov)
     assert np.array_equal(read(ob, ov), a[:, e.argmax(0)])
+
+
+def free_bytes():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_products_of_a_first_step_share_one_allocation():
+    """Each larger than the one before, as a first training step has them: the memory for their operands' parts is there from the
+    first on."""
+    with Backend() as fresh:
+        sizes = [(256, 256, 256), (300, 512, 512), (1000, 512, 512), (2000, 512, 512), (512, 512, 2000), (2000, 2048, 512)]
+        views = [(dense(fresh, np.ones((m, k), np.float32))[1], dense(fresh, np.ones((k, n), np.float32))[1],
+                  dense(fresh, np.ones((m, n), np.float32))[1]) for m, n, k in sizes]
+        held = set()
+        for a, b, c in views:
+            fresh.call("gemm", a, b, c)
+            held.add(free_bytes())
+    assert len(held) == 1
