@@ -313,7 +313,9 @@ int litnice_b200_gemv_noalloc(const float *x, int32_t m, const float *w, int32_t
 
 /* Runs one step at context length seq_len for n_streams streams with CUDA
  * events around each projection and attention launch, `repeats` times, and
- * fills the gemm_* / attn_* fields of the stats. Measurement aid. */
+ * fills the gemm_* / attn_* fields of the stats. A small model whose layers
+ * the token loop runs in one launch has that launch counted under gemm_*, with
+ * the flops of its projections, and nothing under attn_*. Measurement aid. */
 int litnice_b200_profile_step(litnice_b200_session *s, int32_t n_streams, int32_t seq_len,
                               int32_t repeats);
 

@@ -381,7 +381,7 @@ void ensure_rows(litnice_b200_session *s, long long rows) {
 // behind that (width 128 and 128 positions 0.6 to 0.9, 16 streams of 128 positions 0.6 to 0.9).
 bool small_body_taken(const litnice_b200_session *s, int B, int sl) {
   const litnice_b200_dims &d = s->dims;
-  if (!s->small || s->kv_store || s->profiling || s->stamping) return false;
+  if (!s->small || s->kv_store) return false;
   return B <= 15 && sl <= (d.d_model <= 96 ? 128 : 64) && small_body_supports(B, sl, d.n_layers, d.n_heads, d.d_model, d.d_ff);
 }
 
@@ -565,6 +565,8 @@ void enqueue_body(litnice_b200_session *s, int B, int sl, const LoopState *dstat
   const int D = d.d_model, F = d.d_ff;
   const LoopState *rows_state = newest ? nullptr : dstate;  // what shortens a launch's row count
   if (!newest && small_body_taken(s, B, sl)) {
+    ClassTimer t(s, &s->gemm_ev);  // products and attention are one launch
+    if (s->profiling) s->gemm_flops += 2.0 * (double)R * D * (4.0 * D + 2.0 * F) * d.n_layers;
     launch_small_body(s->params, s->pk_offsets, d.n_layers, d.n_heads, D, F, d.vocab_size, s->ids, d.max_seq_len, B, sl, dstate,
                       s->small_kv, s->x, s->err_dev, s->st);
     ++s->launches;

@@ -1,5 +1,7 @@
 """All layers of a small model in one launch against the oracle: row counts around a block of eight and a cluster's share, every
 head dimension, several streams, contexts that grow through a graph's bucket and past what the launch is used for."""
+import os
+
 import numpy as np
 import pytest
 
@@ -85,3 +87,21 @@ def test_values_that_are_not_finite_stay_visible(oracle, value, place):
     assert np.isnan(oracle.forward(d, arena, ids)[4:]).all() and np.isnan(got[4:]).all()
     before = oracle.forward(d, arena, ids[:4])
     assert float(np.abs(got[:4] - before).max() / np.abs(before).max()) < 2e-5
+
+
+def test_profile_of_the_path_that_runs():
+    """profile_step times what the token loop launches: all layers at once, or operator by operator where that is asked for."""
+    d = formats.ModelDims(2, 2, 64, 256, 8, 64)
+    stats = {}
+    for small in ("1", "0"):
+        os.environ["LITNICE_B200_SMALL"] = small
+        try:
+            with Session(d, 2) as s:
+                s.load_params(formats.make_param_arena(d, 5))
+                stats[small] = s.profile_step(2, 40, 3)
+        finally:
+            del os.environ["LITNICE_B200_SMALL"]
+    head = stats["0"].gemm_launches - 3 * 2 * 4  # of the operators' run, beside four projections per layer
+    assert stats["0"].attn_launches == 3 * 2 and stats["1"].attn_launches == 0
+    assert stats["1"].gemm_launches == 3 + head and stats["1"].gemm_flops == stats["0"].gemm_flops
+    assert 0 < stats["1"].gemm_ms < stats["0"].gemm_ms + stats["0"].attn_ms
