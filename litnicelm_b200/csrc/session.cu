@@ -1382,6 +1382,10 @@ static int session_create_impl(const litnice_b200_dims *dims, int32_t max_stream
     const char *tc_env = std::getenv("LITNICE_B200_TC");
     s->tc = !(tc_env && tc_env[0] == '0') && tc_runtime_available() && d.d_model % 64 == 0 &&
             d.d_ff % 64 == 0;
+    // Cached mode with few streams: only the pass over the prompt would run there. Below width 128 sums in 32 bits are as
+    // exact as pairs of 22 are (width 64, 200 positions: 1.8e-7 against 1.9e-7 from the 64-bit logits; width 256 2.6e-7 and
+    // 2.2e-7), and the weights need no pairs.
+    if (s->kv && max_streams <= 8 && d.d_model < 128) s->tc = false;
     // Attention on the tensor cores needs head dimension 64; LITNICE_B200_TC_ATTN=0
     // keeps the fp32 SIMT attention kernel.
     const char *ta_env = std::getenv("LITNICE_B200_TC_ATTN");

@@ -169,3 +169,58 @@ def test_contexts_between_the_buckets(oracle, dims, streams, prompt, new):
         n = agreed_prefix(toks[b], ref_tokens, gaps)
         assert rel_err(lg[:n, b, :], ref_logits[:n]) < 2e-5  # as above
         agreed_prefix(fast[b], ref_tokens, gaps)
+
+
+def logits_64(d, arena, ids):
+    """Logits [rows, vocab] of one text in 64 bits."""
+    p = {k: formats.ParamLayout.build(d).view(arena, k).astype(np.float64) for k in formats.ParamLayout.build(d).slices}
+
+    def norm(x, name):
+        m = x.mean(-1, keepdims=True)
+        return (x - m) / np.sqrt(((x - m) ** 2).mean(-1, keepdims=True) + np.float32(1e-5)) * p[name + "_gamma"] + p[name + "_beta"]
+
+    x = p["tok_embedding"][ids] + p["pos_embedding"][:len(ids)]
+    dh = d.d_model // d.n_heads
+    for l in range(d.n_layers):
+        n = f"layer{l}."
+        h = norm(x, n + "ln1") @ p[n + "attn_qkv_w"] + p[n + "attn_qkv_b"]
+        q, k, v = (t.reshape(len(ids), d.n_heads, dh).transpose(1, 0, 2) for t in np.split(h, 3, -1))
+        s = np.where(np.tri(len(ids), dtype=bool), q @ k.transpose(0, 2, 1) / np.sqrt(dh), -np.inf)
+        w = np.exp(s - s.max(-1, keepdims=True))
+        o = (w / w.sum(-1, keepdims=True)) @ v
+        x = x + o.transpose(1, 0, 2).reshape(len(ids), -1) @ p[n + "attn_out_w"] + p[n + "attn_out_b"]
+        h = norm(x, n + "ln2")
+        x = x + np.maximum(h @ p[n + "ffn_w1"] + p[n + "ffn_b1"], 0.0) @ p[n + "ffn_w2"] + p[n + "ffn_b2"]
+    return norm(x, "lnf") @ p["lm_head_w"]
+
+
+@pytest.mark.parametrize("dims,streams,prompt,new", [
+    ((2, 4, 256, 512, 40, 200), 12, 70, 6),     # steps and prompt on fp16 pairs
+    ((2, 8, 256, 1024, 96, 120), 40, 20, 6),    # head dimension 32: TF32 pairs
+    ((1, 8, 512, 2048, 96, 300), 9, 200, 4),
+    ((2, 4, 256, 1024, 30, 300), 2, 230, 12),   # the prompt alone
+    ((2, 2, 64, 256, 24, 300), 7, 200, 12),     # narrow, few streams: 32-bit throughout
+])
+def test_error_not_above_the_32_bit_kernels(dims, streams, prompt, new):
+    """Step logits against 64 bits, in the 2-norm: where operands are split in two 16- or 19-bit parts, no further off than the
+    same run on the fp32 kernels."""
+    d = formats.ModelDims(*dims)
+    arena = formats.make_param_arena(d, 7, bias_std=0.02, ln_std=0.1)
+    prompts = np.stack([formats.zipf_prompt(d.vocab, prompt, 70 + i) for i in range(streams)])
+    off = []
+    for tc in ("1", "0"):
+        os.environ["LITNICE_B200_TC"] = tc
+        try:
+            with Session(d, streams) as s:
+                s.load_params(arena)
+                s.keep_step_logits(True)
+                toks = s.generate(prompts, new)
+                lg = s.read_step_logits(new, streams)
+        finally:
+            del os.environ["LITNICE_B200_TC"]
+        total = 0.0
+        for b in sorted({0, streams // 2, streams - 1}):
+            want = logits_64(d, arena, np.concatenate([prompts[b], toks[b][:-1]]))[prompt - 1:]
+            total += ((lg[:, b] - want) ** 2).sum() / (want ** 2).sum()
+        off.append(total)
+    assert off[0] <= off[1]
