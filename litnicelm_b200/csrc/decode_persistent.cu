@@ -325,7 +325,7 @@ __device__ __forceinline__ float pk_join(const float *pp, int chunks, int dh, in
   float oo = 0.f;
 #pragma unroll
   for (int q = 0; q < N; ++q) {
-    if (mq[q] != -INFINITY) {  // not an empty chunk
+    if (mq[q] != -INFINITY) {  // not past the chunks there are
       const float w = expf(mq[q] - mm);
       ll += (double)lq[q] * (double)w;
       oo = fmaf(oq[q], w, oo);
@@ -430,13 +430,6 @@ __global__ void __launch_bounds__(PK_THREADS, 1) decode_persistent_kernel(PkPara
           const int c = u % chunks, h = (u / chunks) % H, b = u / (chunks * H);
           const int c0 = c * keys_per_chunk, c1 = min(s, c0 + keys_per_chunk);
           float *out = P.part_attn + (((long long)b * H + h) * P.attn_chunks_max + c) * (DH + 2);
-          if (c0 >= s) {
-            if (tid == 0) {
-              out[DH] = -INFINITY;
-              out[DH + 1] = 0.f;
-            }
-            continue;
-          }
           // Keys and values of earlier positions do not depend on this token: the first trip of keys
           // (four per thread group) and the first sixteen values per thread are requested before the
           // partial sums of q are gathered, so that all three reads are in flight together.
