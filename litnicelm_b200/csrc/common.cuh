@@ -160,8 +160,8 @@ struct MatView {
 };
 
 // a / b of two non-negative numbers: in 32 bits where both fit, which is nearly always (a 64-bit division is a call of
-// about a hundred instructions, and an element of a view costs up to eight of them; a training step of 265 launches
-// went from 3.28 to 3.24 ms).
+// about a hundred instructions, and an element of a view costs up to eight of them; 1 % of a training step of 265
+// launches).
 __host__ __device__ __forceinline__ long long div_index(long long a, long long b) {
   return (unsigned long long)(a | b) >> 32 == 0 ? (long long)((unsigned)a / (unsigned)b) : a / b;
 }

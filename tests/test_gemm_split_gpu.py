@@ -1,5 +1,5 @@
 """The plugin table's products at sizes that run on the tensor cores, against 64-bit sums: tile edges and remainders, strides
-of every kind, summed and batched operands, cut k ranges, epilogues, values that no operand pair holds."""
+of every kind, summed and batched operands, cut k ranges, epilogues, values that no operand parts hold, and what the parts keep of those they hold."""
 import time
 
 import numpy as np
@@ -38,8 +38,9 @@ def operand(be, a, layout):
 
 
 def bound(a, b):
-    """Pairs leave 2^-22 of each product's size, a sum of k such parts rounded in chains of 32: below 2^-21 |a| |b| in all. Short
-    sums run one after another in 32 bits: 2^-24 a step."""
+    """What the operands' parts leave out is below 2^-32 of a product; a chain of 64 k loses up to 2^-23 of its sum at each of four
+    truncations, every chain 2^-24 at each of two roundings: below 2^-21 |a| |b| in all. Short sums run one after another in 32 bits:
+    2^-24 a step."""
     k = a.shape[-1]
     return max(2.0 ** -21, k * 2.0 ** -24 if k < 128 else 0.0) * (np.abs(a.astype(np.float64)) @ np.abs(b.astype(np.float64))) + 1e-30
 
@@ -83,6 +84,7 @@ def test_batches_sums_and_epilogues(be, batch, m, n, k):
 
 @pytest.mark.parametrize("m,n,k", [(300, 200, 512), (64, 96, 2048)])
 def test_values_no_pair_holds(be, m, n, k):
+    """Several kinds in one product, and the product after it (each kind alone: below)."""
     rng = np.random.default_rng(m)
     a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
     a[3, 7], a[5, 9], a[6, 1], a[9, :] = np.inf, np.nan, -np.inf, 0.0
