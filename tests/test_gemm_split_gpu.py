@@ -308,3 +308,38 @@ def test_products_of_a_first_step_share_one_allocation():
             fresh.call("gemm", a, b, c)
             held.add(free_bytes())
     assert len(held) == 1
+
+
+@pytest.mark.parametrize("order,gap,offset", [((0, 1, 2), 0, 1), ((0, 2, 1), 0, 0), ((0, 2, 1), 3, 4), ((1, 0, 2), 0, 0),
+                                              ((1, 0, 2), 4, 0), ((2, 1, 0), 1, 7), ((0, 1, 2), 5, 0)])
+def test_results_and_operands_in_any_order(be, order, gap, offset):
+    """Batches of matrices whose three axes lie in memory in every order, with and without gaps and 16-byte rows, operands and
+    results alike; what lies between the results stays as it was."""
+    rng = np.random.default_rng(gap + offset)
+    batch, m, n, k = 3, 130, 94, 260
+
+    def placed(values):
+        strides, at = [0, 0, 0], 1
+        for axis in reversed(order):
+            strides[axis] = at
+            at = at * values.shape[axis] + gap
+        buf = Buffer(be, (at + offset) * 4, fill=-7.0)
+        view = buf.view(values.shape, [4 * x for x in strides], 4 * offset)
+        buf.np_view(view)[...] = values
+        buf.push()
+        return buf, view
+
+    a, b = (rng.standard_normal(x).astype(np.float32) for x in ((batch, m, k), (batch, k, n)))
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    (_, av), (_, bv), (ob, ov) = placed(a), placed(b), placed(np.zeros((batch, m, n), np.float32))
+    be.call("gemm_batched", av, bv, ov)
+    assert (np.abs(read(ob, ov) - want) <= bound(a, b)).all()
+    ob.np_view(ov)[...] = -7.0
+    assert (ob.host.view(np.float32) == -7.0).all()
+    _, wv = placed(b[:1])
+    be.call("gemm_ranked_matrix_rhs", av, type(wv)(wv.ptr, wv.shape[1:], wv.strides[1:], wv.dtype, wv.device), ov)
+    assert (np.abs(read(ob, ov) - a.astype(np.float64) @ b[0].astype(np.float64)) <= bound(a, b[0])).all()
+    sb, sv = placed(np.zeros((1, m, n), np.float32))
+    tv = type(av)(av.ptr, (batch, k, m), (av.strides[0], av.strides[2], av.strides[1]), av.dtype, av.device)
+    be.call("gemm_ranked_reduce_lhs_t", tv, bv, type(sv)(sv.ptr, sv.shape[1:], sv.strides[1:], sv.dtype, sv.device))
+    assert (np.abs(read(sb, sv)[0] - want.sum(0)) <= bound(a, b).sum(0)).all()
