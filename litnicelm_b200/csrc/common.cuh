@@ -391,6 +391,14 @@ struct DecodePersistentArgs {
 bool decode_persistent_supports(int n_streams, int n_heads, int d_model, int d_ff, int vocab);
 size_t decode_persistent_scratch_floats(int n_streams, int n_heads, int d_model, int d_ff, int vocab, int sm_count);
 void launch_decode_persistent(const DecodePersistentArgs &a, cudaStream_t st);
+// decode_cluster.cu: the same for models with up to eight heads, a cluster of CTAs per head; any vocabulary. packed: the
+// weights in the order of use (decode_cluster_packed_floats, written by launch_decode_cluster_pack once per load); words:
+// decode_cluster_words 64-bit words; scratch and sm_count of the arguments are not used.
+bool decode_cluster_supports(int n_streams, int n_layers, int n_heads, int d_model, int d_ff, int vocab);
+size_t decode_cluster_packed_floats(int n_layers, int n_heads, int d_model, int d_ff, int vocab);
+size_t decode_cluster_words(int n_heads, int d_model);
+void launch_decode_cluster_pack(const DecodePersistentArgs &a, float *packed, cudaStream_t st);
+void launch_decode_cluster(const DecodePersistentArgs &a, const float *packed, unsigned long long *words, cudaStream_t st);
 
 // sampler.cu
 struct SamplerParams {

@@ -223,11 +223,16 @@ struct litnice_b200_session {
   // greedy runs of up to 8 streams: all steps after the first in one resident kernel
   // (decode_persistent.cu; LITNICE_B200_KV_PERSIST=0 keeps one graph replay per token)
   bool kv_persist = true;
+  bool kv_cluster = true;  // with a cluster per head where the model allows it; off once there was no memory for it
   int sm_count = 0;
   unsigned long long *pk_offsets = nullptr;  // device table of parameter offsets
   float *pk_scratch = nullptr;
   size_t pk_scratch_floats = 0;
   unsigned *pk_barrier = nullptr;
+  // decode_cluster.cu: weights in that kernel's order, laid out at the first run after a load, and its words
+  float *cl_packed = nullptr;
+  bool cl_packed_valid = false;
+  unsigned long long *cl_words = nullptr;
 
   // Registered decoder design served instead of the litnicelm transformer (null: the transformer).
   std::unique_ptr<DecoderModel> model;
@@ -827,6 +832,32 @@ void enqueue_decode_step(litnice_b200_session *s, int B, int sl, const LoopState
 
 // Cached mode: caches for n_streams streams of up to cap positions, and the scratch of the
 // attention over key chunks for every context length up to cap.
+// The resident kernel that runs the steps of B greedy streams of the cached mode: a cluster per head where the model allows
+// it, which was 2.4 to 6 times as fast over widths 64 to 512, 1 to 8 streams, contexts of 8 to 960 and vocabularies of 24 to 32000
+// (6 layers of 512, one stream 157 -> 57 us a token; figures in decode_cluster.cu); else one CTA per SM behind grid-wide
+// barriers; else none (a graph replay per token).
+enum Resident { RESIDENT_NONE, RESIDENT_GRID, RESIDENT_CLUSTER };
+Resident resident_kernel(const litnice_b200_session *s, int B) {
+  const litnice_b200_dims &d = s->dims;
+  if (!s->kv || !s->kv_persist || B > 8) return RESIDENT_NONE;
+  if (s->kv_cluster && decode_cluster_supports(B, d.n_layers, d.n_heads, d.d_model, d.d_ff, d.vocab_size)) return RESIDENT_CLUSTER;
+  return decode_persistent_supports(B, d.n_heads, d.d_model, d.d_ff, d.vocab_size) ? RESIDENT_GRID : RESIDENT_NONE;
+}
+
+// Memory of the cluster kernel; without it the run takes the grid's kernel or a graph replay per token.
+bool ensure_cluster(litnice_b200_session *s) {
+  const litnice_b200_dims &d = s->dims;
+  const size_t floats = decode_cluster_packed_floats(d.n_layers, d.n_heads, d.d_model, d.d_ff, d.vocab_size);
+  for (auto &[p, bytes] : {std::pair<void **, size_t>{reinterpret_cast<void **>(&s->cl_packed), floats * 4},
+                           {reinterpret_cast<void **>(&s->cl_words), decode_cluster_words(d.n_heads, d.d_model) * 8}})
+    if (*p == nullptr && cudaMalloc(p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      *p = nullptr;
+      return false;
+    }
+  return true;
+}
+
 void ensure_kv(litnice_b200_session *s, int B, int cap) {
   const litnice_b200_dims &d = s->dims;
   if (B > s->kv_streams || cap > s->kv_cap) {
@@ -846,7 +877,8 @@ void ensure_kv(litnice_b200_session *s, int B, int cap) {
     ++s->generation;
   }
   const size_t need = attn_decode_scratch_floats(B, cap, d.n_heads, d.d_model / d.n_heads);
-  if (s->kv_persist && B <= 8 && decode_persistent_supports(B, d.n_heads, d.d_model, d.d_ff, d.vocab_size)) {
+  if (resident_kernel(s, B) == RESIDENT_CLUSTER && !ensure_cluster(s)) s->kv_cluster = false;
+  if (resident_kernel(s, B) == RESIDENT_GRID) {
     const size_t need_pk = decode_persistent_scratch_floats(B, d.n_heads, d.d_model, d.d_ff, d.vocab_size, s->sm_count);
     if (need_pk > s->pk_scratch_floats) {
       LB_CUDA(cudaStreamSynchronize(s->st));
@@ -1458,6 +1490,8 @@ void litnice_b200_session_destroy(litnice_b200_session *s) {
   if (s->small_kv) cudaFree(s->small_kv);
   if (s->pk_scratch) cudaFree(s->pk_scratch);
   if (s->pk_barrier) cudaFree(s->pk_barrier);
+  if (s->cl_packed) cudaFree(s->cl_packed);
+  if (s->cl_words) cudaFree(s->cl_words);
   if (s->xl_lo) cudaFree(s->xl_lo);
   if (s->tc_scratch) cudaFree(s->tc_scratch);
   if (s->attn_timeline) cudaFree(s->attn_timeline);
@@ -1501,6 +1535,7 @@ int litnice_b200_load_params(litnice_b200_session *s, const void *host_arena, ui
     if (host_arena == nullptr || bytes != s->lay.total)
       throw std::invalid_argument("parameter arena must be " + std::to_string(s->lay.total) + " bytes, got " +
                                   std::to_string(bytes));
+    s->cl_packed_valid = false;
     LB_CUDA(cudaMemcpyAsync(s->params, host_arena, bytes, cudaMemcpyHostToDevice, s->st));
     if (s->tc) prepare_tc_weights(s);
     LB_CUDA(cudaStreamSynchronize(s->st));
@@ -1551,6 +1586,7 @@ int litnice_b200_load_checkpoint(litnice_b200_session *s, const char *path) {
   }
   return guarded(s, [&]() {
     s->params_loaded = false;
+    s->cl_packed_valid = false;
     try {
       file_to_device(path, sizeof(Header), s->lay.total, s->params, s->st, true);
     } catch (const std::domain_error &) {
@@ -1745,8 +1781,8 @@ int litnice_b200_run(litnice_b200_session *s, int32_t max_new, const litnice_b20
       // cached mode: a step on one new row per stream when the caches hold every earlier
       // position, else a whole-context pass that also fills them (the first step of a batch)
       const bool decode = (s->kv || s->model) && s->kv_len == sl - 1;
-      if (decode && s->kv && s->kv_persist && greedy && !s->keep_logits && B <= 8 && s->pk_scratch != nullptr &&
-          decode_persistent_supports(B, s->dims.n_heads, s->dims.d_model, s->dims.d_ff, V)) {
+      const Resident resident = decode && greedy && !s->keep_logits ? resident_kernel(s, B) : RESIDENT_NONE;
+      if (resident != RESIDENT_NONE) {
         // every remaining step in one resident kernel
         DecodePersistentArgs a{};
         a.params = s->params;
@@ -1781,7 +1817,16 @@ int litnice_b200_run(litnice_b200_session *s, int32_t max_new, const litnice_b20
           LB_CUDA(cudaMemsetAsync(tl, 0, 64 * 8, s->st));
         }
         a.timeline = tl;
-        launch_decode_persistent(a, s->st);
+        if (resident == RESIDENT_CLUSTER) {
+          if (!s->cl_packed_valid) {
+            launch_decode_cluster_pack(a, s->cl_packed, s->st);
+            ++s->launches;
+            s->cl_packed_valid = true;
+          }
+          launch_decode_cluster(a, s->cl_packed, s->cl_words, s->st);
+        } else {
+          launch_decode_persistent(a, s->st);
+        }
         if (tl != nullptr) {  // measurement aid: the phases of one token of CTA 0, ns from the token's start
           unsigned long long h[64];
           LB_CUDA(cudaMemcpyAsync(h, tl, sizeof(h), cudaMemcpyDeviceToHost, s->st));

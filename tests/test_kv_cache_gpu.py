@@ -224,3 +224,51 @@ def test_error_not_above_the_32_bit_kernels(dims, streams, prompt, new):
             total += ((lg[:, b] - want) ** 2).sum() / (want ** 2).sum()
         off.append(total)
     assert off[0] <= off[1]
+
+
+# Greedy steps in one resident kernel: a cluster per head (1, 2, 4 or 8 heads of 32 or 64), else a CTA per SM (three heads).
+# Every number of streams its rows are compiled for and those between; contexts of one and several batches of keys per warp,
+# shorter than the cluster; one and several passes of every product, vocabularies of one column, with a remainder, of several
+# tiles per CTA; hidden widths at both ends of what a cluster takes.
+@pytest.mark.parametrize("dims,streams,prompt,new", [
+    ((2, 2, 64, 256, 8, 64), 1, 3, 60),
+    ((1, 1, 32, 32, 1, 40), 1, 1, 12),
+    ((2, 1, 64, 1024, 33, 90), 3, 5, 30),
+    ((2, 2, 128, 64, 51, 330), 8, 300, 25),
+    ((3, 4, 128, 512, 1000, 200), 5, 130, 40),
+    ((2, 4, 256, 512, 96, 1300), 1, 1240, 30),
+    ((2, 8, 256, 1024, 7, 260), 2, 200, 50),
+    ((2, 8, 512, 2048, 96, 400), 1, 250, 40),
+    ((1, 8, 512, 2048, 9000, 300), 4, 60, 12),
+    ((2, 8, 512, 1024, 130, 160), 7, 100, 24),
+    ((2, 3, 96, 256, 52, 120), 2, 40, 20),
+])
+def test_resident_steps(dims, streams, prompt, new):
+    d = formats.ModelDims(*dims)
+    arena = formats.make_param_arena(d, 7, bias_std=0.02, ln_std=0.1)
+    prompts = np.stack([formats.zipf_prompt(d.vocab, prompt, 70 + i) for i in range(streams)])
+    with Session(d, streams) as s:
+        s.load_params(arena)
+        whole = s.generate(prompts, new)
+        s.upload_prompts(prompts)
+        first = new // 2
+        assert s.run(first) == first
+        s.keep_step_logits(True)
+        assert s.run(new - first) == new  # launched one by one, on the keys and values that the resident kernel left
+        toks = s.download_tokens(new)
+        lg = s.read_step_logits(new, streams)[first:]
+    # sums of up to 1024 terms in fp32 on either side: as in the tests above
+    for b in range(streams):
+        for run in (whole, toks):
+            want = logits_64(d, arena, np.concatenate([prompts[b], run[b][:-1]]))[prompt - 1:]
+            srt = np.sort(want, axis=1)
+            gaps = srt[:, -1] - srt[:, -2] if d.vocab > 1 else np.ones(new)
+            agreed_prefix(run[b], want.argmax(1), gaps)
+        assert rel_err(lg[:, b], want[first:]) < 2e-5
+    if streams > 1:  # a stream's tokens do not depend on its neighbours
+        with Session(d, streams) as s:
+            s.load_params(arena)
+            alone = s.generate(prompts[1:2], new)[0]
+        want = logits_64(d, arena, np.concatenate([prompts[1], alone[:-1]]))[prompt - 1:]
+        srt = np.sort(want, axis=1)
+        agreed_prefix(alone, want.argmax(1), srt[:, -1] - srt[:, -2])
