@@ -40,19 +40,20 @@ struct Backend {
   // (self_attention_fused_inplace.cpp:82-94: three calls per head; transformer_layer.cpp:79-86 and
   // the FFN variants: a product, then its bias). Calls that can be merged with their neighbours are
   // recorded instead of launched and issued together at the next call that is anything else:
-  // a projection with the bias (and ReLU) that follows it becomes one launch, and the score product,
-  // causal softmax and context product of all heads of a layer become three launches instead of
-  // three per head. Nothing is reordered against other calls and every buffer the host's sequence
-  // writes is written with the same values, so the host cannot tell the difference
+  // a projection with the bias (and ReLU) that follows it becomes one launch, and the calls of all heads of a layer,
+  // forward (score product, causal softmax, context product) or backward (four products, softmax gradient, scale),
+  // become one launch per call of a head instead of one per call and head. Nothing is reordered against other calls and
+  // every buffer the host's sequence writes is written with the same values, so the host cannot tell the difference
   // (LITNICE_B200_ABI_QUEUE=0 issues every call at once).
   struct Pending {
-    enum Kind { PROJECTION, BIAS, BIAS_RELU, SCORES, SOFTMAX, CONTEXT } kind;
+    // from SCORES on: calls of a head (products a b^T, a b, a^T b; the softmax and its gradient; x * scale)
+    enum Kind { PROJECTION, BIAS, BIAS_RELU, SCORES, SOFTMAX, CONTEXT, LHS_T, SOFTMAX_BWD, SCALE } kind;
     BackendTensorView a, b, c;  // copies: the host's views are only valid during its call
     float scale = 0.f;
   };
   std::vector<Pending> queue;
   bool queue_on = true;
-  float *queue_scratch = nullptr;  // scores of all heads when the host gives every head the same buffer
+  float *queue_scratch = nullptr;  // what heads keep in one buffer of the host, for all heads
   size_t queue_scratch_floats = 0;
   long long fused_projections = 0, grouped_heads = 0;
 
@@ -406,6 +407,24 @@ bool same_view(const BackendTensorView &p, const BackendTensorView &q) {
   return true;
 }
 
+// Calls of heads, recorded: a product a b^T or a^T b opens a run of them, every kind of them continues it.
+constexpr size_t MAX_RECORDED = 1024;
+bool heads_recorded(const Backend *b) { return !b->queue.empty() && b->queue[0].kind >= Backend::Pending::SCORES; }
+// True: recorded. Else whatever was recorded has been issued and the call is to run now.
+bool record_head_call(Backend *b, bool opens, Backend::Pending::Kind kind, LitniceView x, LitniceView y, LitniceView out,
+                      float scale = 0.f) {
+  if (!b->queue.empty() && (!heads_recorded(b) || b->queue.size() >= MAX_RECORDED)) flush_queue(b);
+  if (b->queue.empty() && !(opens && b->queue_on)) return false;
+  Backend::Pending p;
+  p.kind = kind;
+  p.a = *x;
+  if (y != nullptr) p.b = *y;
+  p.c = *out;
+  p.scale = scale;
+  b->queue.push_back(p);
+  return true;
+}
+
 void bias_op(void *h, EwOp op, LitniceView x, LitniceView bias, LitniceView out, const char *who) {
   Backend *b = self_recording(h);
   require_gpu_f32(x, who);
@@ -469,7 +488,15 @@ void unary_op(void *h, EwOp op, LitniceView x, float s, LitniceView out, const c
 
 // device_backend.cpp:942-964, :978-1001
 void api_mul_scalar(void *h, LitniceView x, float s, LitniceView out) {
-  unary_op(h, EW_MUL_SCALAR, x, s, out, "litnice_b200::mul_scalar");
+  const char *who = "litnice_b200::mul_scalar";
+  Backend *b = self_recording(h);
+  require_gpu_f32(x, who);
+  require_gpu_f32(out, who);
+  if (heads_recorded(b)) {
+    const RowView rx = make_row_view(x, who), ro = make_row_view(out, who);
+    if (rx.cols == ro.cols && rx.rows == ro.rows && record_head_call(b, false, Backend::Pending::SCALE, x, nullptr, out, s)) return;
+  }
+  unary_op(h, EW_MUL_SCALAR, x, s, out, who);
 }
 void api_relu(void *h, LitniceView x, LitniceView out) {
   unary_op(h, EW_RELU, x, 0.f, out, "litnice_b200::relu");
@@ -571,17 +598,7 @@ void api_causal_softmax(void *h, LitniceView scores, float scale, LitniceView ou
     if (rx.rows != ro.rows || rx.cols != ro.cols)
       throw std::runtime_error("litnice_b200::scaled_causal_softmax_rows: shape mismatch");
   }
-  // the softmax of the score product recorded just before: part of a head's three calls
-  if (!b->queue.empty() && b->queue.back().kind == Backend::Pending::SCORES && same_view(b->queue.back().c, *scores)) {
-    Backend::Pending p;
-    p.kind = Backend::Pending::SOFTMAX;
-    p.a = *scores;
-    p.c = *out;
-    p.scale = scale;
-    b->queue.push_back(p);
-    return;
-  }
-  if (!b->queue.empty()) flush_queue(b);
+  if (record_head_call(b, false, Backend::Pending::SOFTMAX, scores, nullptr, out, scale)) return;
   run_causal_softmax(b, scores, scale, out);
 }
 
@@ -653,18 +670,8 @@ void api_gemm_batched(void *h, LitniceView a, LitniceView bb, LitniceView out) {
   require_gpu_f32(out, "litnice_b200::gemm_batched(out)");
   const MatView av = make_mat_view(a, "gemm_batched(a)"), bv = make_mat_view(bb, "gemm_batched(b)"),
                 ov = make_mat_view(out, "gemm_batched(out)");
-  // the context product of the softmax recorded just before: completes a head's three calls
-  if (!b->queue.empty() && b->queue.back().kind == Backend::Pending::SOFTMAX && same_view(b->queue.back().c, *a)) {
-    check_gemm(av, bv, ov, "litnice_b200::gemm_batched");
-    Backend::Pending p;
-    p.kind = Backend::Pending::CONTEXT;
-    p.a = *a;
-    p.b = *bb;
-    p.c = *out;
-    b->queue.push_back(p);
-    return;
-  }
-  if (!b->queue.empty()) flush_queue(b);
+  check_gemm(av, bv, ov, "litnice_b200::gemm_batched");
+  if (record_head_call(b, false, Backend::Pending::CONTEXT, a, bb, out)) return;
   run_gemm(b, av, bv, ov, "litnice_b200::gemm_batched");
 }
 
@@ -677,19 +684,8 @@ void api_gemm_batched_rhs_t(void *h, LitniceView a, LitniceView bb, LitniceView 
   const MatView av = make_mat_view(a, "gemm_batched_rhs_t(a)"),
                 bv = transposed(make_mat_view(bb, "gemm_batched_rhs_t(b)")),
                 ov = make_mat_view(out, "gemm_batched_rhs_t(out)");
-  // a score product opens a head's three calls; it may follow the completed calls of earlier heads
-  const bool heads_pending = !b->queue.empty() && b->queue.back().kind == Backend::Pending::CONTEXT;
-  if (!b->queue.empty() && !heads_pending) flush_queue(b);
-  if (b->queue_on) {
-    check_gemm(av, bv, ov, "litnice_b200::gemm_batched_rhs_t");
-    Backend::Pending p;
-    p.kind = Backend::Pending::SCORES;
-    p.a = *a;
-    p.b = *bb;
-    p.c = *out;
-    b->queue.push_back(p);
-    return;
-  }
+  check_gemm(av, bv, ov, "litnice_b200::gemm_batched_rhs_t");
+  if (record_head_call(b, true, Backend::Pending::SCORES, a, bb, out)) return;
   run_gemm(b, av, bv, ov, "litnice_b200::gemm_batched_rhs_t");
 }
 
@@ -725,6 +721,17 @@ bool same_shape(const BackendTensorView &p, const BackendTensorView &q) {
   return true;
 }
 
+void run_softmax_backward(Backend *b, const RowView &sm, const RowView &dout, const RowView &dx, float scale) {
+  bind(b);
+  launch_softmax_backward(sm, dout, dx, true, scale, b->st);
+  ++b->launches;
+}
+void run_scale(Backend *b, const RowView &x, const RowView &out, float scale) {
+  bind(b);
+  launch_rowwise(EW_MUL_SCALAR, x, nullptr, 0, scale, out, b->st);
+  ++b->launches;
+}
+
 void issue_one(Backend *b, const Backend::Pending &p) {
   switch (p.kind) {
     case Backend::Pending::PROJECTION:
@@ -742,103 +749,230 @@ void issue_one(Backend *b, const Backend::Pending &p) {
       run_gemm(b, make_mat_view(&p.a, "gemm_batched(a)"), make_mat_view(&p.b, "gemm_batched(b)"),
                make_mat_view(&p.c, "gemm_batched(out)"), "litnice_b200::gemm_batched");
       break;
+    case Backend::Pending::LHS_T:
+      run_gemm(b, transposed(make_mat_view(&p.a, "gemm_batched_lhs_t(a)")), make_mat_view(&p.b, "gemm_batched_lhs_t(b)"),
+               make_mat_view(&p.c, "gemm_batched_lhs_t(out)"), "litnice_b200::gemm_batched_lhs_t");
+      break;
+    case Backend::Pending::SOFTMAX_BWD:
+      run_softmax_backward(b, make_row_view(&p.a, "softmax_backward_causal_rows"), make_row_view(&p.b, "softmax_backward_causal_rows"),
+                           make_row_view(&p.c, "softmax_backward_causal_rows"), 1.0f);
+      break;
+    case Backend::Pending::SCALE:
+      run_scale(b, make_row_view(&p.a, "mul_scalar"), make_row_view(&p.c, "mul_scalar"), p.scale);
+      break;
     default:
       throw std::logic_error("litnice_b200: a recorded bias has no projection");
   }
 }
 
-// The three calls of heads [0, n) starting at queue index `at` as three launches over all heads, when
-// every head's views have the same shape and their addresses advance by one constant per operand.
-bool issue_heads_grouped(Backend *b, size_t at, long long n) {
-  const Backend::Pending *q = b->queue.data() + at;
-  auto delta = [&](int op, int which) -> long long {  // address step from head 0 to head 1
-    auto pick = [&](const Backend::Pending &p) { return which == 0 ? p.a.data : which == 1 ? p.b.data : p.c.data; };
-    return (long long)(static_cast<char *>(pick(q[3 + op])) - static_cast<char *>(pick(q[op])));
+// The bytes a tensor touches, heads included: addresses base + sum of index * stride, each four bytes long.
+struct Footprint {
+  uintptr_t base;
+  int n = 0;
+  long long dims[8], strides[8];
+  bool sound = true;  // only non-negative strides are reasoned about
+  Footprint(const BackendTensorView &v, long long heads, long long delta) : base(reinterpret_cast<uintptr_t>(v.data)) {
+    for (uint32_t i = 0; i < v.rank; ++i) axis((long long)v.dims[i], (long long)v.strides_bytes[i]);
+    axis(heads, delta);
+  }
+  void axis(long long d, long long s) {
+    if (d <= 1) return;
+    if (s < 0 || n == 8) sound = false;
+    if (!sound) return;
+    dims[n] = d;
+    strides[n++] = s;
+  }
+  // Length of the part that axes of strides no multiple of g span: modulo g the tensor lies in [base, base + length).
+  long long span(long long g) const {
+    long long len = 4;
+    for (int i = 0; i < n; ++i)
+      if (strides[i] % g != 0) len += (dims[i] - 1) * strides[i];
+    return len;
+  }
+  long long bytes() const {
+    long long len = 4;
+    for (int i = 0; i < n; ++i) len += (dims[i] - 1) * strides[i];
+    return len;
+  }
+};
+// True only if no byte belongs to both: their ranges are apart, or they lie in different columns of a common pitch (one of the
+// strides: what is a multiple of it moves no address modulo it).
+bool disjoint(const Footprint &p, const Footprint &q) {
+  if (!p.sound || !q.sound) return false;
+  if (p.base + (uintptr_t)p.bytes() <= q.base || q.base + (uintptr_t)q.bytes() <= p.base) return true;
+  auto apart = [&](long long g) {
+    if (g <= 4) return false;
+    const long long lp = p.span(g), lq = q.span(g);
+    if (lp > g || lq > g) return false;
+    const long long from_p = (long long)((q.base % (uintptr_t)g + (uintptr_t)g - p.base % (uintptr_t)g) % (uintptr_t)g);  // p's start to q's, onwards
+    return from_p >= lp && from_p + lq <= g;
   };
-  const long long dq = delta(0, 0), dk = delta(0, 1), ds = delta(0, 2), dw = delta(1, 2), dv = delta(2, 1),
-                  dc = delta(2, 2);
-  for (long long h = 0; h < n; ++h)
-    for (int op = 0; op < 3; ++op) {
-      const Backend::Pending &p = q[3 * h + op], &p0 = q[op];
-      if (!same_shape(p.a, p0.a) || !same_shape(p.c, p0.c) || (op != 1 && !same_shape(p.b, p0.b))) return false;
-      if (op == 1 && p.scale != p0.scale) return false;
-      auto at_step = [&](void *ptr, void *base, long long d) {
-        return static_cast<char *>(ptr) == static_cast<char *>(base) + h * d;
-      };
-      if (op == 0 && !(at_step(p.a.data, p0.a.data, dq) && at_step(p.b.data, p0.b.data, dk) &&
-                       at_step(p.c.data, p0.c.data, ds)))
-        return false;
-      if (op == 1 && !at_step(p.c.data, p0.c.data, dw)) return false;
-      if (op == 2 && !(at_step(p.b.data, p0.b.data, dv) && at_step(p.c.data, p0.c.data, dc))) return false;
+  for (int i = 0; i < p.n; ++i)
+    if (apart(p.strides[i])) return true;
+  for (int i = 0; i < q.n; ++i)
+    if (apart(q.strides[i])) return true;
+  return false;
+}
+
+// The calls of `heads` heads, n each, recorded head by head, as n launches over all heads (the head index becomes one more
+// batch axis). False, with nothing issued, unless that provably writes what the recorded order writes:
+// - every head makes the same calls on views of one shape, whose addresses advance by a constant per operand;
+// - what one head writes no other head reads or writes (a head's own calls keep their order). A buffer that all heads share
+//   is given to each head separately where every head first fills it with a product and only uses it as that one view; the
+//   host's buffer then receives the last head's content, which is what it holds after the host's own sequence.
+// Beyond this a single head's calls fill the GPU by themselves (512 MB over 8 heads: 64 MB each).
+constexpr size_t MAX_HEAD_FLOATS = (size_t)128 << 20;
+bool issue_heads_grouped(Backend *b, const Backend::Pending *q, int n, long long heads) {
+  using P = Backend::Pending;
+  struct Operand {
+    const BackendTensorView *v;
+    int op;
+    bool written;
+    long long delta;
+    bool temp = false;
+  };
+  auto product = [](P::Kind k) { return k == P::SCORES || k == P::CONTEXT || k == P::LHS_T; };
+  auto view = [](const P &p, int which) -> const BackendTensorView & { return which == 0 ? p.a : which == 1 ? p.b : p.c; };
+  std::vector<Operand> all;
+  std::vector<int> index((size_t)n * 3, -1);
+  for (int i = 0; i < n; ++i) {
+    for (long long h = 0; h < heads; ++h)
+      if (q[h * n + i].kind != q[i].kind || q[h * n + i].scale != q[i].scale) return false;
+    for (int w = 0; w < 3; ++w) {
+      if (w == 1 && !product(q[i].kind) && q[i].kind != P::SOFTMAX_BWD) continue;
+      const BackendTensorView &v0 = view(q[i], w);
+      const long long d = static_cast<char *>(view(q[n + i], w).data) - static_cast<char *>(v0.data);
+      for (long long h = 1; h < heads; ++h) {
+        const BackendTensorView &v = view(q[h * n + i], w);
+        if (!same_shape(v, v0) || static_cast<char *>(v.data) != static_cast<char *>(v0.data) + h * d) return false;
+      }
+      index[(size_t)i * 3 + w] = (int)all.size();
+      all.push_back(Operand{&v0, i, w == 2, d});
     }
-  if (dw == 0 || dc == 0) return false;  // heads must not share their outputs
-  MatView qa = make_mat_view(&q[0].a, "gemm_batched_rhs_t(a)"),
-          kb = transposed(make_mat_view(&q[0].b, "gemm_batched_rhs_t(b)")),
-          sc = make_mat_view(&q[0].c, "gemm_batched_rhs_t(out)");
-  RowView sx = make_row_view(&q[1].a, "scaled_causal_softmax_rows(scores)"),
-          so = make_row_view(&q[1].c, "scaled_causal_softmax_rows(out)");
-  MatView wa = make_mat_view(&q[2].a, "gemm_batched(a)"), vb = make_mat_view(&q[2].b, "gemm_batched(b)"),
-          co = make_mat_view(&q[2].c, "gemm_batched(out)");
-  if (qa.nb > 2 || sx.np > 3) return false;
-  bind(b);
-  const bool shared_scores = ds == 0;  // every head's scores land in one buffer of the host
-  MatView sc_all = with_heads(sc, n, ds);
-  RowView sx_all = with_heads(sx, n, ds);
-  if (shared_scores) {
-    // Scores of all heads side by side in scratch; the host's buffer receives the last head's, which is
-    // what it holds after the host's own sequence.
-    if (sc.batch != 1) return false;
-    const size_t per_head = (size_t)sc.rows * sc.cols;
-    if (per_head * n > b->queue_scratch_floats) {
+  }
+  // the shared buffer, if there is one
+  const BackendTensorView *temp = nullptr;
+  for (const Operand &o : all)
+    if (o.written && o.delta == 0) {
+      if (temp != nullptr && !same_view(*temp, *o.v)) return false;
+      if (temp == nullptr && !product(q[o.op].kind)) return false;
+      temp = o.v;
+    }
+  if (temp != nullptr) {
+    bool filled = false;
+    for (Operand &o : all) {  // in the order of the calls, inputs before the result
+      if (o.delta != 0 || o.v->data != temp->data) continue;
+      if (!same_view(*temp, *o.v) || (!filled && !o.written)) return false;
+      o.temp = filled = true;
+    }
+  }
+  for (size_t i = 0; i < all.size(); ++i) {
+    const Operand &x = all[i];
+    const Footprint fx(*x.v, heads, x.delta);
+    if (x.temp) {  // the host's buffer is written behind all calls
+      for (const Operand &y : all)
+        if (!y.temp && !disjoint(fx, Footprint(*y.v, heads, y.delta))) return false;
+      continue;
+    }
+    if (!x.written) continue;
+    for (long long k = 1; k < heads; ++k) {  // head h against head h + k
+      BackendTensorView other = *x.v;
+      other.data = static_cast<char *>(other.data) + k * x.delta;
+      if (!disjoint(Footprint(*x.v, 1, 0), Footprint(other, 1, 0))) return false;
+    }
+    for (const Operand &y : all) {
+      if (y.temp || (y.delta == x.delta && same_view(*x.v, *y.v))) continue;
+      if (!disjoint(fx, Footprint(*y.v, heads, y.delta))) return false;
+    }
+  }
+  // the views of all heads
+  MatView temp_m{};
+  RowView temp_r{};
+  if (temp != nullptr) {
+    const MatView m = make_mat_view(temp, "head buffer");
+    const RowView r = make_row_view(temp, "head buffer");
+    if (r.rows != m.batch * m.rows || r.cols != m.cols) return false;
+    const size_t per_head = (size_t)m.batch * m.rows * m.cols;
+    if (per_head * heads > MAX_HEAD_FLOATS) return false;
+    if (per_head * heads > b->queue_scratch_floats) {
+      bind(b);
       LB_CUDA(cudaStreamSynchronize(b->st));
       if (b->queue_scratch) cudaFree(b->queue_scratch);
       b->queue_scratch = nullptr;
       b->queue_scratch_floats = 0;
-      if (cudaMalloc(reinterpret_cast<void **>(&b->queue_scratch), per_head * n * 4) != cudaSuccess) {
+      if (cudaMalloc(reinterpret_cast<void **>(&b->queue_scratch), per_head * heads * 4) != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
       }
-      b->queue_scratch_floats = per_head * n;
+      b->queue_scratch_floats = per_head * heads;
     }
-    MatView dense_sc{};
-    dense_sc.data = reinterpret_cast<char *>(b->queue_scratch);
-    dense_sc.nb = 0;
-    dense_sc.batch = 1;
-    dense_sc.rows = sc.rows;
-    dense_sc.cols = sc.cols;
-    dense_sc.rs = sc.cols * 4;
-    dense_sc.cs = 4;
-    sc_all = with_heads(dense_sc, n, (long long)per_head * 4);
-    RowView dense_sx{};
-    dense_sx.data = reinterpret_cast<char *>(b->queue_scratch);
-    dense_sx.np = 1;
-    dense_sx.pd[0] = sc.rows;
-    dense_sx.ps[0] = sc.cols * 4;
-    dense_sx.rows = sc.rows;
-    dense_sx.cols = sc.cols;
-    dense_sx.cs = 4;
-    sx_all = with_heads(dense_sx, n, (long long)per_head * 4);
+    // dense, head by head: [heads * batch][rows][cols]
+    temp_m.data = temp_r.data = reinterpret_cast<char *>(b->queue_scratch);
+    temp_m.rows = m.rows;
+    temp_m.cols = temp_r.cols = m.cols;
+    temp_m.rs = m.cols * 4;
+    temp_m.cs = temp_r.cs = 4;
+    temp_m.nb = 1;
+    temp_m.bd[0] = temp_m.batch = m.batch * heads;
+    temp_m.bs[0] = m.rows * m.cols * 4;
+    temp_r.np = 1;
+    temp_r.pd[0] = temp_r.rows = r.rows * heads;
+    temp_r.ps[0] = m.cols * 4;
   }
-  b->launches += launch_gemm_f32(with_heads(qa, n, dq), with_heads(kb, n, dk), sc_all, false, GemmEpilogue{}, b->split, b->st,
-                                 b->err_dev);
-  launch_softmax_rows(sx_all, with_heads(so, n, dw), 1, q[1].scale, b->st);
-  b->launches += 1 + launch_gemm_f32(with_heads(wa, n, dw), with_heads(vb, n, dv), with_heads(co, n, dc), false,
-                                     GemmEpilogue{}, b->split, b->st, b->err_dev);
-  if (shared_scores) {
-    RowView last{};
-    last.data = reinterpret_cast<char *>(b->queue_scratch + (size_t)(n - 1) * sc.rows * sc.cols);
-    last.np = 1;
-    last.pd[0] = sc.rows;
-    last.ps[0] = sc.cols * 4;
-    last.rows = sc.rows;
-    last.cols = sc.cols;
-    last.cs = 4;
-    launch_rowwise(EW_COPY, last, nullptr, 0, 0.f, sx, b->st);
+  auto operand = [&](int i, int w) -> const Operand & { return all[(size_t)index[(size_t)i * 3 + w]]; };
+  auto mat = [&](int i, int w, const char *who) {
+    const Operand &o = operand(i, w);
+    return o.temp ? temp_m : with_heads(make_mat_view(o.v, who), heads, o.delta);
+  };
+  auto rows = [&](int i, int w, const char *who) {
+    const Operand &o = operand(i, w);
+    return o.temp ? temp_r : with_heads(make_row_view(o.v, who), heads, o.delta);
+  };
+  for (const Operand &o : all)
+    if (!o.temp && (make_mat_view(o.v, "head operand").nb > 2 || make_row_view(o.v, "head operand").np > 3)) return false;
+  for (int i = 0; i < n; ++i) {
+    switch (q[i].kind) {
+      case P::SCORES:
+        run_gemm(b, mat(i, 0, "gemm_batched_rhs_t(a)"), transposed(mat(i, 1, "gemm_batched_rhs_t(b)")), mat(i, 2, "gemm_batched_rhs_t(out)"),
+                 "litnice_b200::gemm_batched_rhs_t");
+        break;
+      case P::CONTEXT:
+        run_gemm(b, mat(i, 0, "gemm_batched(a)"), mat(i, 1, "gemm_batched(b)"), mat(i, 2, "gemm_batched(out)"), "litnice_b200::gemm_batched");
+        break;
+      case P::LHS_T:
+        run_gemm(b, transposed(mat(i, 0, "gemm_batched_lhs_t(a)")), mat(i, 1, "gemm_batched_lhs_t(b)"), mat(i, 2, "gemm_batched_lhs_t(out)"),
+                 "litnice_b200::gemm_batched_lhs_t");
+        break;
+      case P::SOFTMAX:
+        bind(b);
+        launch_softmax_rows(rows(i, 0, "scaled_causal_softmax_rows(scores)"), rows(i, 2, "scaled_causal_softmax_rows(out)"), 1, q[i].scale, b->st);
+        ++b->launches;
+        break;
+      case P::SOFTMAX_BWD: {
+        // a scale in place right behind it joins it
+        const bool scaled = i + 1 < n && q[i + 1].kind == P::SCALE && same_view(q[i].c, q[i + 1].a) && same_view(q[i].c, q[i + 1].c) &&
+                            operand(i, 2).delta == operand(i + 1, 0).delta && operand(i, 2).delta == operand(i + 1, 2).delta;
+        run_softmax_backward(b, rows(i, 0, "softmax_backward_causal_rows"), rows(i, 1, "softmax_backward_causal_rows"),
+                             rows(i, 2, "softmax_backward_causal_rows"), scaled ? q[i + 1].scale : 1.0f);
+        if (scaled) ++i;
+        break;
+      }
+      default:
+        run_scale(b, rows(i, 0, "mul_scalar"), rows(i, 2, "mul_scalar"), q[i].scale);
+    }
+  }
+  if (temp != nullptr) {
+    RowView last = temp_r;
+    last.rows = last.pd[0] = temp_r.rows / heads;
+    last.data += (heads - 1) * last.rows * temp_r.cols * 4;
+    launch_rowwise(EW_COPY, last, nullptr, 0, 0.f, make_row_view(temp, "head buffer"), b->st);
     ++b->launches;
   }
-  b->grouped_heads += n;
+  b->grouped_heads += heads;
   return true;
 }
+
+constexpr int MAX_HEAD_CALLS = 8;
 
 void flush_queue(Backend *b) {
   std::vector<Backend::Pending> q;
@@ -858,19 +992,18 @@ void flush_queue(Backend *b) {
     }
     return;
   }
-  const long long heads = (long long)(q.size() / 3);  // complete (scores, softmax, context) triples
+  // The shortest run of calls that the heads repeat; a last head that is not complete is issued call by call.
   size_t done = 0;
-  if (heads >= 2) {
-    b->queue.swap(q);  // issue_heads_grouped reads the recorded calls through the instance
-    bool grouped = false;
-    try {
-      grouped = issue_heads_grouped(b, 0, heads);
-    } catch (...) {
-      b->queue.clear();
-      throw;
-    }
-    q.swap(b->queue);
-    if (grouped) done = (size_t)heads * 3;
+  for (int n = 1; n <= MAX_HEAD_CALLS && done == 0; ++n) {
+    long long heads = 1;
+    auto repeats = [&](size_t at) {
+      if (at + n > q.size()) return false;
+      for (int i = 0; i < n; ++i)
+        if (q[at + i].kind != q[i].kind) return false;
+      return true;
+    };
+    while (repeats((size_t)heads * n)) ++heads;
+    if (heads >= 2 && q.size() - (size_t)heads * n < (size_t)n && issue_heads_grouped(b, q.data(), n, heads)) done = (size_t)heads * n;
   }
   for (size_t i = done; i < q.size(); ++i) issue_one(b, q[i]);
 }
@@ -1032,12 +1165,15 @@ void api_gemm_ranked_reduce_lhs_t(void *h, LitniceView a, LitniceView bb, Litnic
 
 // device_backend.cpp:1195-1214: out[p] = a[p]^T * b[p]
 void api_gemm_batched_lhs_t(void *h, LitniceView a, LitniceView bb, LitniceView out) {
-  Backend *b = self(h);
+  Backend *b = self_recording(h);
   require_gpu_f32(a, "litnice_b200::gemm_batched_lhs_t(a)");
   require_gpu_f32(bb, "litnice_b200::gemm_batched_lhs_t(b)");
   require_gpu_f32(out, "litnice_b200::gemm_batched_lhs_t(out)");
-  run_gemm(b, transposed(make_mat_view(a, "gemm_batched_lhs_t(a)")), make_mat_view(bb, "gemm_batched_lhs_t(b)"),
-           make_mat_view(out, "gemm_batched_lhs_t(out)"), "litnice_b200::gemm_batched_lhs_t");
+  const MatView av = transposed(make_mat_view(a, "gemm_batched_lhs_t(a)")), bv = make_mat_view(bb, "gemm_batched_lhs_t(b)"),
+                ov = make_mat_view(out, "gemm_batched_lhs_t(out)");
+  check_gemm(av, bv, ov, "litnice_b200::gemm_batched_lhs_t");
+  if (record_head_call(b, true, Backend::Pending::LHS_T, a, bb, out)) return;
+  run_gemm(b, av, bv, ov, "litnice_b200::gemm_batched_lhs_t");
 }
 void api_gemm_batched_lhs_t_ctx(void *h, LitniceView a, LitniceView bb, LitniceView out) {
   require_group(h, "litnice_b200::gemm_batched_lhs_t_exec_context");
@@ -1121,15 +1257,17 @@ void api_backward_from_logits_targets(void *h, LitniceView logits, LitniceView t
 
 // device_backend.cpp:1519-1552, :1649-1673
 void softmax_backward_op(void *h, LitniceView sm, LitniceView dout, LitniceView dx, bool causal, const char *who) {
-  Backend *b = self(h);
+  Backend *b = self_recording(h);
   require_gpu_f32(sm, who);
   require_gpu_f32(dout, who);
   require_gpu_f32(dx, who);
-  bind(b);
   RowView rs = make_row_view(sm, who), rd = make_row_view(dout, who), rx = make_row_view(dx, who);
   if (rs.rows != rd.rows || rs.cols != rd.cols || rs.rows != rx.rows || rs.cols != rx.cols)
     throw std::runtime_error(std::string(who) + ": shape mismatch");
-  launch_softmax_backward(rs, rd, rx, causal, b->st);
+  if (causal && record_head_call(b, false, Backend::Pending::SOFTMAX_BWD, sm, dout, dx)) return;
+  if (!b->queue.empty()) flush_queue(b);
+  bind(b);
+  launch_softmax_backward(rs, rd, rx, causal, 1.0f, b->st);
   ++b->launches;
 }
 void api_softmax_backward_rows(void *h, LitniceView sm, LitniceView dout, LitniceView dx) {

@@ -374,7 +374,7 @@ __global__ void cross_entropy_kernel(const __grid_constant__ RowView logits, con
 
 template <bool CAUSAL>
 __global__ void softmax_bwd_kernel(const __grid_constant__ RowView sm, const __grid_constant__ RowView dout,
-                                   const __grid_constant__ RowView dx) {
+                                   const __grid_constant__ RowView dx, float scale) {
   const long long row = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= sm.rows) return;
   const int lane = threadIdx.x & 31;
@@ -386,7 +386,7 @@ __global__ void softmax_bwd_kernel(const __grid_constant__ RowView sm, const __g
   dot = warp_sum(dot);
   for (long long c = lane; c < cols; c += 32) {
     float g = 0.f;
-    if (c < live) g = ld(sm, so, c) * (ld(dout, go, c) - dot);
+    if (c < live) g = ld(sm, so, c) * (ld(dout, go, c) - dot) * scale;
     st(dx, xo, c, g);
   }
 }
@@ -395,7 +395,7 @@ __global__ void softmax_bwd_kernel(const __grid_constant__ RowView sm, const __g
 template <bool CAUSAL, int NP>
 __global__ void __launch_bounds__(256)
 softmax_bwd_row_kernel(const __grid_constant__ RowView sm, const __grid_constant__ RowView dout,
-                       const __grid_constant__ RowView dx) {
+                       const __grid_constant__ RowView dx, float scale) {
   const long long row = blockIdx.x * 8LL + (threadIdx.x >> 5);
   if (row >= sm.rows) return;
   const int lane = threadIdx.x & 31, cols = (int)sm.cols, live = CAUSAL ? (int)(row % cols) + 1 : cols;
@@ -414,7 +414,7 @@ softmax_bwd_row_kernel(const __grid_constant__ RowView sm, const __grid_constant
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
     const int c = lane + 32 * i;
-    if (c < cols) st(dx, xo, c, c < live ? s[i] * (g[i] - dot) : 0.f);
+    if (c < cols) st(dx, xo, c, c < live ? s[i] * (g[i] - dot) * scale : 0.f);
   }
 }
 
@@ -542,19 +542,19 @@ void launch_cross_entropy(const RowView &logits, const char *targets, int target
   }
 }
 
-void launch_softmax_backward(const RowView &sm, const RowView &dout, const RowView &dx, bool causal, cudaStream_t st) {
+void launch_softmax_backward(const RowView &sm, const RowView &dout, const RowView &dx, bool causal, float scale, cudaStream_t st) {
   if (sm.rows <= 0 || sm.cols <= 0) return;
   const unsigned grid = (unsigned)((sm.rows + 7) / 8);
   if (sm.cols >= 1 && sm.cols <= 512) {
-    if (sm.cols <= 256 && causal) softmax_bwd_row_kernel<true, 8><<<grid, 256, 0, st>>>(sm, dout, dx);
-    else if (sm.cols <= 256) softmax_bwd_row_kernel<false, 8><<<grid, 256, 0, st>>>(sm, dout, dx);
-    else if (causal) softmax_bwd_row_kernel<true, 16><<<grid, 256, 0, st>>>(sm, dout, dx);
-    else softmax_bwd_row_kernel<false, 16><<<grid, 256, 0, st>>>(sm, dout, dx);
+    if (sm.cols <= 256 && causal) softmax_bwd_row_kernel<true, 8><<<grid, 256, 0, st>>>(sm, dout, dx, scale);
+    else if (sm.cols <= 256) softmax_bwd_row_kernel<false, 8><<<grid, 256, 0, st>>>(sm, dout, dx, scale);
+    else if (causal) softmax_bwd_row_kernel<true, 16><<<grid, 256, 0, st>>>(sm, dout, dx, scale);
+    else softmax_bwd_row_kernel<false, 16><<<grid, 256, 0, st>>>(sm, dout, dx, scale);
     LB_LAUNCH_CHECK();
     return;
   }
-  if (causal) softmax_bwd_kernel<true><<<grid, 256, 0, st>>>(sm, dout, dx);
-  else softmax_bwd_kernel<false><<<grid, 256, 0, st>>>(sm, dout, dx);
+  if (causal) softmax_bwd_kernel<true><<<grid, 256, 0, st>>>(sm, dout, dx, scale);
+  else softmax_bwd_kernel<false><<<grid, 256, 0, st>>>(sm, dout, dx, scale);
   LB_LAUNCH_CHECK();
 }
 

@@ -1,0 +1,158 @@
+"""Calls that a host makes head by head (attention, forward and backward) are recorded and issued over all heads at once where
+that writes the same values: every buffer of a run must hold the same bits as when each call is issued at once."""
+import os
+
+import numpy as np
+import pytest
+import torch
+
+from litnicelm_b200.plugin import Backend, DevTensor
+
+pytestmark = pytest.mark.gpu
+
+B, S, H, DH = 2, 24, 4, 16   # below the extents of the tensor-core products: sums in the order of k on either route
+D = H * DH
+
+
+class Arena:
+    """Buffers of one instance, filled alike in every instance."""
+
+    def __init__(self, be):
+        self.be, self.buffers = be, {}
+
+    def buffer(self, name, floats):
+        rng = np.random.default_rng(sum(map(ord, name)))
+        values = (rng.standard_normal(floats) * 0.5).astype(np.float32)
+        ptr = self.be.alloc(values.nbytes, 64)
+        self.be.upload(ptr, values.view(np.uint8))
+        self.buffers[name] = (ptr, values.nbytes)
+        return ptr
+
+    def read(self):
+        return {k: self.be.download(p, n) for k, (p, n) in self.buffers.items()}
+
+
+def view(ptr, shape, strides=None):
+    if strides is None:
+        strides = [4 * int(np.prod(shape[i + 1:])) for i in range(len(shape))]
+    return DevTensor(ptr, tuple(shape), tuple(strides), 0, 1)
+
+
+def third(ptr, i, h):
+    return view(ptr + 4 * (i * D + h * DH), (B, S, DH), (12 * S * D, 12 * D, 4))
+
+
+def head(ptr, h):
+    return view(ptr + 4 * h * DH, (B, S, DH), (4 * S * D, 4 * D, 4))
+
+
+def square(ptr, h):
+    return view(ptr + 4 * h * S * S, (B, S, S), (4 * H * S * S, 4 * S, 4))
+
+
+def forward(be, a, shared, scale=0.25):
+    qkv, w, ctx, tmp = a.buffer("qkv", 3 * B * S * D), a.buffer("w", B * H * S * S), a.buffer("ctx", B * S * D), a.buffer("tmp", B * S * S)
+    for h in range(H):
+        s = view(tmp, (B, S, S)) if shared else square(w, h)
+        be.call("gemm_batched_rhs_t", third(qkv, 0, h), third(qkv, 1, h), s)
+        be.call("scaled_causal_softmax_rows", s, scale, square(w, h))
+        be.call("gemm_batched", square(w, h), third(qkv, 2, h), head(ctx, h))
+
+
+def backward(be, a, variant):
+    qkv, w, dctx = a.buffer("qkv", 3 * B * S * D), a.buffer("w", B * H * S * S), a.buffer("dctx", B * S * D)
+    dqkv, tmp, more = a.buffer("dqkv", 3 * B * S * D), a.buffer("tmp", B * S * S), a.buffer("more", B * H * S * S)
+    for h in range(H):
+        dw = square(more, h) if variant == "own" else view(tmp, (B, S, S))
+        scale = 0.25 + 0.125 * h if variant == "scales" else 0.25
+        dv = third(dqkv, 2, 0 if variant == "one gradient" else h)
+        k = third(qkv, 1, h)
+        if variant == "next head reads":   # a head's key is what the head before it wrote
+            k = third(dqkv, 0, max(h - 1, 0))
+        be.call("gemm_batched_lhs_t", square(w, h), head(dctx, h), dv)
+        if variant == "not filled":        # what the shared buffer holds is used before a head fills it
+            be.call("mul_scalar", dw, 0.5, dw)
+            be.call("gemm_batched", dw, third(qkv, 0, h), third(dqkv, 1, h))
+        if variant == "exec":
+            be.call("gemm_batched_rhs_t_exec_context", head(dctx, h), third(qkv, 2, h), dw)
+            be.call("softmax_backward_causal_rows_exec_context", square(w, h), dw, dw)
+        else:
+            be.call("gemm_batched_rhs_t", head(dctx, h), third(qkv, 2, h), dw)
+            be.call("softmax_backward_causal_rows", square(w, h), dw, dw)
+        if variant == "last incomplete" and h == H - 1:
+            break
+        if variant != "not scaled":
+            be.call("mul_scalar", dw, scale, dw)
+        if variant == "other view":        # the shared buffer through another view of itself
+            be.call("gemm_batched", view(tmp, (B, S, S), (4 * S * S, 4, 4 * S)), k, third(dqkv, 0, h))
+        else:
+            be.call("gemm_batched", dw, k, third(dqkv, 0, h))
+        be.call("gemm_batched_lhs_t", dw, third(qkv, 0, h), third(dqkv, 1, h))
+
+
+def uneven(be, a):
+    """Two heads of the usual pitch and one somewhere else."""
+    x, y = a.buffer("x", 4 * S * S), a.buffer("y", 8 * S * S)
+    for at in (0, 1, 3):
+        v = view(x + 4 * at * S * S, (1, S, S))
+        be.call("gemm_batched_rhs_t", v, v, view(y + 4 * (at if at < 2 else 7) * S * S, (1, S, S)))
+
+
+def running(be, a):
+    """Each product reads what the one before it wrote."""
+    x = a.buffer("x", 6 * S * S)
+    for at in range(5):
+        v = view(x + 4 * at * S * S, (1, S, S))
+        be.call("gemm_batched_rhs_t", v, v, view(x + 4 * (at + 1) * S * S, (1, S, S)))
+
+
+def overlapping(be, a):
+    """Results half over their neighbours'."""
+    x, y = a.buffer("x", 4 * S * S), a.buffer("y", 4 * S * S)
+    for at in range(4):
+        v = view(x + 4 * at * S * S, (1, S, S))
+        be.call("gemm_batched_lhs_t", v, v, view(y + 2 * at * S * S, (1, S, S)))
+
+
+def backwards(be, a):
+    """Addresses that fall from head to head."""
+    x, y = a.buffer("x", 4 * S * S), a.buffer("y", 4 * S * S)
+    for at in (3, 2, 1, 0):
+        v = view(x + 4 * at * S * S, (1, S, S))
+        be.call("gemm_batched_lhs_t", v, v, view(y + 4 * at * S * S, (1, S, S)))
+
+
+def lanes(be, a):
+    be.call("start_exec_context_iteration")
+    be.call("start_exec_context_group")
+    backward(be, a, "exec")
+    be.call("finish_exec_context_group")
+    be.call("finish_exec_context_iteration")
+
+
+RUNS = {"forward": lambda be, a: forward(be, a, False), "forward, one score buffer": lambda be, a: forward(be, a, True),
+        "uneven": uneven, "running": running, "overlapping": overlapping, "backwards": backwards, "exec": lanes}
+for name in ("shared", "own", "scales", "one gradient", "next head reads", "not filled", "not scaled", "other view", "last incomplete"):
+    RUNS["backward, " + name] = lambda be, a, name=name: backward(be, a, name)
+GROUPED = {"forward", "forward, one score buffer", "exec", "backward, shared", "backward, own", "backward, not scaled",
+           "backward, last incomplete"}
+
+
+@pytest.mark.parametrize("name", RUNS)
+def test_same_bits_as_call_by_call(name):
+    left, launches = [], []
+    for queue in ("1", "0"):
+        os.environ["LITNICE_B200_ABI_QUEUE"] = queue
+        try:
+            be = Backend()
+        finally:
+            del os.environ["LITNICE_B200_ABI_QUEUE"]
+        with be:
+            a = Arena(be)
+            with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+                RUNS[name](be, a)
+                left.append(a.read())
+            launches.append(sum("kernel" in e.name for e in prof.events()))
+    for k in left[0]:
+        assert np.array_equal(left[0][k], left[1][k]), k
+    assert (launches[0] < launches[1]) == (name in GROUPED), launches
