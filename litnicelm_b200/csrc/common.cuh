@@ -297,12 +297,18 @@ void launch_gather_last_ln(const float *x, const float *gamma, const float *beta
                            float *out_lo, cudaStream_t st);
 // small_body.cu: every layer of a small model (width up to 128) in one launch, from the ids to x [streams * s, d].
 // offsets: device table of byte offsets into params, [layers][12] in the order of a layer's parameters, then the
-// token and position embeddings. kv: small_body_kv_floats floats. state as elsewhere: s is then a bound.
+// token and position embeddings, the final norm's scale and shift and the head. kv: small_body_kv_floats floats. state as elsewhere: s is then a bound.
 bool small_body_supports(int streams, int s, int layers, int n_heads, int d, int f);
 size_t small_body_kv_floats(int streams, int s, int d);
 void launch_small_body(const char *params, const unsigned long long *offsets, int layers, int n_heads, int d, int f, int vocab,
                        const int *ids, int ids_ld, int streams, int s, const LoopState *state, float *kv, float *x, DevErr *err,
                        cudaStream_t st);
+// The same for a greedy run of `steps` tokens (at least one) behind contexts of s0 positions, with the tail of every step: ids,
+// out_tokens and state as head_greedy.cu leaves them; logits [streams, vocab] of the last step.
+bool small_loop_supports(int streams, int s, int layers, int n_heads, int d, int f, int vocab);
+void launch_small_loop(const char *params, const unsigned long long *offsets, int layers, int n_heads, int d, int f, int vocab,
+                       int *ids, int ids_ld, int *out_tokens, int out_ld, int streams, int s0, int step0, int steps, LoopState *state,
+                       float *logits, float *kv, DevErr *err, cudaStream_t st);
 // out_lo != nullptr: out receives the TF32 high part and out_lo the low part.
 // state != nullptr: the launch covers `rows` as an upper bound and the kernel
 // takes n_streams * state->s as the actual row count.

@@ -1720,8 +1720,8 @@ int litnice_b200_run(litnice_b200_session *s, int32_t max_new, const litnice_b20
     // the device-side LoopState) and replayed for every step in the bucket, so
     // the host issues one launch per token instead of ~50.
     const bool graphs = s->use_graphs && !s->keep_logits;
-    const bool fused_tail =
-        greedy && !s->keep_logits && s->fused_tail && !s->kv && !s->model && head_greedy_supports(B, s->dims.d_model, V);
+    const bool fused_tail_on = greedy && !s->keep_logits && s->fused_tail && !s->kv && !s->model;
+    const bool fused_tail = fused_tail_on && head_greedy_supports(B, s->dims.d_model, V);
     // cached mode, greedy, few streams, small vocabulary: the step ends in the one-launch tail too
     const bool decode_tail = s->kv && s->kv_fuse && greedy && !s->keep_logits && s->fused_tail &&
                              head_greedy_supports(B, s->dims.d_model, V);
@@ -1776,7 +1776,15 @@ int litnice_b200_run(litnice_b200_session *s, int32_t max_new, const litnice_b20
       s->launches += 2;
     };
     LB_CUDA(cudaEventRecord(s->ev0, s->st));
-    for (int step = 0; step < steps; ++step) {
+    const bool small_loop = fused_tail_on && steps > 0 && small_body_taken(s, B, s_last) &&
+                            small_loop_supports(B, s_last, s->dims.n_layers, s->dims.n_heads, s->dims.d_model, s->dims.d_ff, V);
+    if (small_loop) {
+      launch_small_loop(s->params, s->pk_offsets, s->dims.n_layers, s->dims.n_heads, s->dims.d_model, s->dims.d_ff, V, s->ids,
+                        s->dims.max_seq_len, s->out_tokens, s->out_cap, B, s0, s->cur_tokens, steps, s->state, s->logits, s->small_kv,
+                        s->err_dev, s->st);
+      ++s->launches;
+    }
+    for (int step = small_loop ? steps : 0; step < steps; ++step) {
       const int sl = s0 + step;
       // cached mode: a step on one new row per stream when the caches hold every earlier
       // position, else a whole-context pass that also fills them (the first step of a batch)

@@ -13,6 +13,11 @@
 // the next product, and the vectors of the next layer, are requested before the work in front of them; all
 // loads of a phase are in flight together. The ranges' sums meet in shared memory, in range order.
 // 32-bit products and sums; LayerNorm sums and the softmax's sum in double, expf, as in the host code.
+//
+// Greedy runs of small vocabularies go through all their tokens in one launch (small_loop_supports): the CTA that has the last row
+// finishes it (final norm, head out of shared memory, first maximum; output_head.cpp:58-70, inference.cpp:188-198) and a barrier
+// of the stream's cluster hands the token on; every token still computes its whole context. Two layers of width 64, one stream, contexts of 6 to 63: 47 us a token with a
+// launch for the body and one for the tail, replayed from a graph, 37 in one launch.
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
@@ -28,6 +33,14 @@ constexpr int SB_PARTIALS = SB_THREADS * 4 * SB_ROWS;  // floats: every thread's
 
 struct SmallShape {
   int layers, heads, d, f, vocab, streams, s_cap;
+};
+
+// A run of `steps` tokens behind contexts of s0 positions; steps == 0: the body of one step, rows to x_out.
+struct SmallRun {
+  int s0, steps, step0, out_ld;
+  int *ids, *out_tokens;
+  float *logits;  // [streams][vocab] of the last step
+  LoopState *state;
 };
 
 // One product's cut: groups of four columns, ranges of k; a thread's range and group.
@@ -155,9 +168,11 @@ __device__ __forceinline__ void sb_attention(const float *qr, const float *ks, i
 // offsets: [layers][12] byte offsets into params: ln1_g, ln1_b, qkv_w, qkv_b, out_w, out_b, ln2_g, ln2_b, w1, b1, w2,
 // b2; then tok_emb, pos_emb. kv: [2][streams][s_cap][2 d]. x: [streams * s][d], rows as the other kernels pack them.
 __global__ void __launch_bounds__(SB_THREADS)
-small_body_kernel(SmallShape g, const char *__restrict__ params, const unsigned long long *__restrict__ offsets, const int *ids,
+small_body_kernel(SmallShape g, SmallRun run, const char *__restrict__ params, const unsigned long long *__restrict__ offsets, const int *ids,
                   int ids_ld, const LoopState *state, float *kv, float *x_out, DevErr *err) {
   extern __shared__ __align__(16) float sm[];
+  __shared__ float s_best[SB_WARPS];
+  __shared__ int s_at[SB_WARPS];
   const int tid = threadIdx.x, wid = tid >> 5;
   const int b = blockIdx.y, me = blockIdx.x, D = g.d, F = g.f, H = g.heads, dh = D / H;
   const int blocks_max = ((g.s_cap + SB_ROWS - 1) / SB_ROWS + SB_CTAS - 1) / SB_CTAS;
@@ -173,7 +188,8 @@ small_body_kernel(SmallShape g, const char *__restrict__ params, const unsigned 
   float *vs = ks + g.s_cap * kp;                    // [s][D]
   float *vecs = vs + g.s_cap * D;                   // [2][9 D + F] a layer's vectors: LayerNorms and biases
   const int nvec = 9 * D + F;
-  unsigned long long *offs = reinterpret_cast<unsigned long long *>(vecs + 2 * nvec);  // the table of offsets
+  float *tail = vecs + 2 * nvec;                    // of a run: final norm [2][D], head [D][vocab]
+  unsigned long long *offs = reinterpret_cast<unsigned long long *>(tail + (run.steps ? D * (g.vocab + 2) : 0));  // the table of offsets
   auto P = [&](int l, int i) { return reinterpret_cast<const float *>(params + offs[l * 12 + i]); };
   enum { LN1G, LN1B, QKVW, QKVB, OUTW, OUTB, LN2G, LN2B, W1, B1, W2, B2 };
   auto weight_of = [](int op) { return op == 0 ? (int)QKVW : op == 1 ? (int)OUTW : op == 2 ? (int)W1 : (int)W2; };
@@ -188,13 +204,13 @@ small_body_kernel(SmallShape g, const char *__restrict__ params, const unsigned 
       vr[i] = e < nvec ? __ldg(P(l, which) + e - (at >= 6 && at < 9 ? 6 : at) * D) : 0.f;
     }
   };
-  auto store_vectors = [&](int l) {
+  auto store_vectors = [&](int turn) {
 #pragma unroll
     for (int i = 0; i < SB_VECTORS; ++i)
-      if (tid + i * SB_THREADS < nvec) vecs[(l & 1) * nvec + tid + i * SB_THREADS] = vr[i];
+      if (tid + i * SB_THREADS < nvec) vecs[turn * nvec + tid + i * SB_THREADS] = vr[i];
   };
   pdl_launch_dependents();
-  for (int i = tid; i < g.layers * 12 + 2; i += SB_THREADS) offs[i] = offsets[i];
+  for (int i = tid; i < g.layers * 12 + 5; i += SB_THREADS) offs[i] = offsets[i];
   __syncthreads();
   SbWeights wt;
   SbCut cut[4];  // QKV, out-projection, W1, W2
@@ -207,8 +223,20 @@ small_body_kernel(SmallShape g, const char *__restrict__ params, const unsigned 
   wt.request(P(0, QKVW), cut[0]);
   request_vectors(0);  // (all of this never changes: before the wait)
   store_vectors(0);
+  if (run.steps) {
+    const float *gamma = P(g.layers, 2), *beta = P(g.layers, 3), *w = P(g.layers, 4);
+    for (int c = tid; c < D; c += SB_THREADS) {
+      tail[c] = __ldg(gamma + c);
+      tail[D + c] = __ldg(beta + c);
+    }
+    for (int e = tid; e < D * g.vocab; e += SB_THREADS) tail[2 * D + e] = __ldg(w + e);
+  }
   pdl_wait();
-  const int s = state ? state->s : g.s_cap;
+  int turn = 0;  // of the two buffers, for keys and values and for a layer's vectors
+#pragma unroll 1
+  for (int step = 0; step == 0 || step < run.steps; ++step) {
+  const bool another = step + 1 < run.steps;
+  const int s = run.steps ? run.s0 + step : state ? state->s : g.s_cap;
   const int blocks = (s + SB_ROWS - 1) / SB_ROWS;
   const int mine = blocks > me ? (blocks - me + SB_CTAS - 1) / SB_CTAS : 0;
   auto row_of = [&](int j, int r) { return (j * SB_CTAS + me) * SB_ROWS + r; };
@@ -218,7 +246,7 @@ small_body_kernel(SmallShape g, const char *__restrict__ params, const unsigned 
     const int i = e / D, c = e - i * D, t = row_of(i / SB_ROWS, i % SB_ROWS);
     float v = 0.f;
     if (t < s) {
-      int id = ids[(long long)b * ids_ld + t];
+      int id = __ldcg(ids + (long long)b * ids_ld + t);
       if (id < 0 || id >= g.vocab) {
         if (c == 0) {
           err->code = DEVERR_BAD_TOKEN_ID;
@@ -234,21 +262,27 @@ small_body_kernel(SmallShape g, const char *__restrict__ params, const unsigned 
   const float scale = 1.0f / sqrtf((float)dh);
   const int last = mine > 0 ? min(s, row_of(mine - 1, SB_ROWS)) : 0;  // keys this CTA's rows see
   enum { QKV = 0, WO, FF1, FF2 };
-  for (int l = 0; l < g.layers; ++l) {
-    const float *vec = vecs + (l & 1) * nvec;
-    float *kvl = kv + ((long long)(l & 1) * g.streams + b) * g.s_cap * 2 * D;
+  for (int l = 0; l < g.layers; ++l, turn ^= 1) {
+    const float *vec = vecs + turn * nvec;
+    float *kvl = kv + ((long long)turn * g.streams + b) * g.s_cap * 2 * D;
+    const bool more = l + 1 < g.layers || another;  // a layer follows: nl
+    const int nl = l + 1 < g.layers ? l + 1 : 0;
     if (mine == 0) {
       __syncwarp();
       cluster_sync_all();
+      if (more) {  // this CTA may have rows in the next step
+        request_vectors(nl);
+        store_vectors(turn ^ 1);
+      }
       continue;
     }
-    if (l + 1 < g.layers) request_vectors(l + 1);
+    if (more) request_vectors(nl);
     // the operators as steps of one loop, with one instance of the product, the LayerNorm and the attention
 #pragma unroll 1
-    for (int step = 0; step < 4 * mine; ++step) {
-      const int op = step < mine ? QKV : WO + (step - mine) % 3, j = step < mine ? step : (step - mine) / 3;
+    for (int at = 0; at < 4 * mine; ++at) {
+      const int op = at < mine ? QKV : WO + (at - mine) % 3, j = at < mine ? at : (at - mine) / 3;
       const float *xj = x + j * SB_ROWS * D;
-      if (step == mine) {  // every CTA's keys and values of this layer
+      if (at == mine) {  // every CTA's keys and values of this layer
         __syncwarp();
         cluster_sync_all();
         const int pieces = last * (D / 2);  // float4s: a position's keys, then its values
@@ -264,7 +298,7 @@ small_body_kernel(SmallShape g, const char *__restrict__ params, const unsigned 
             if (e < pieces) *reinterpret_cast<float4 *>(c < D ? ks + t * kp + c : vs + t * D + c - D) = v[i];
           }
         }
-        if (l + 1 < g.layers) store_vectors(l + 1);
+        if (more) store_vectors(turn ^ 1);
         __syncthreads();
       }
       if (op == QKV || op == FF1) {
@@ -307,11 +341,11 @@ small_body_kernel(SmallShape g, const char *__restrict__ params, const unsigned 
         }
       }
       {  // the first weights of the step that follows
-        const int after = step + 1;
+        const int after = at + 1;
         const bool over = after == 4 * mine;
-        if (!over || l + 1 < g.layers) {
+        if (!over || more) {
           const int nop = over || after < mine ? QKV : WO + (after - mine) % 3;
-          wt.request(P(over ? l + 1 : l, weight_of(nop)), cut_of(nop));
+          wt.request(P(over ? nl : l, weight_of(nop)), cut_of(nop));
         }
       }
       if (c.q < c.ranges) {
@@ -354,9 +388,75 @@ small_body_kernel(SmallShape g, const char *__restrict__ params, const unsigned 
       __syncthreads();
     }
   }
-  for (int e = tid; e < mine * SB_ROWS * D; e += SB_THREADS) {
-    const int i = e / D, t = row_of(i / SB_ROWS, i % SB_ROWS);
-    if (t < s) x_out[((long long)b * s + t) * D + (e - i * D)] = x[e];
+  if (run.steps == 0) {
+    for (int e = tid; e < mine * SB_ROWS * D; e += SB_THREADS) {
+      const int i = e / D, t = row_of(i / SB_ROWS, i % SB_ROWS);
+      if (t < s) x_out[((long long)b * s + t) * D + (e - i * D)] = x[e];
+    }
+    return;
+  }
+  // ---- the last row's token: a strict '>' scan from index 0 ----
+  if (me == (blocks - 1) % SB_CTAS) {
+    const int V = g.vocab, r = (s - 1) % SB_ROWS;
+    sb_layernorm(x + (mine - 1) * SB_ROWS * D, tail, tail + D, D, inv_d, in);
+    int wide = 1;  // columns side by side, the threads left over share k
+    while (wide < V && wide < SB_THREADS) wide *= 2;
+    const int ranges = SB_THREADS / wide, q = tid / wide;
+#pragma unroll 1
+    for (int c = tid % wide; c < V; c += wide) {
+      const float *w = tail + 2 * D + c;
+      float v = 0.f;
+#pragma unroll 4
+      for (int k = q; k < D; k += ranges) v = fmaf(in[k * SB_ROWS + r], w[k * V], v);
+      part[q * V + c] = v;
+    }
+    __syncthreads();
+    float best = -3.402823466e+38f;
+    int best_at = 0x7fffffff;
+#pragma unroll 1
+    for (int c = tid; c < V; c += SB_THREADS) {
+      float v = 0.f;
+      for (int z = 0; z < ranges; ++z) v += part[z * V + c];
+      if (!another) run.logits[(long long)b * V + c] = v;
+      if (v > best || (v == best && c < best_at)) {
+        best = v;
+        best_at = c;
+      }
+    }
+    auto first = [&]() {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, best_at, o);
+        if (ov > best || (ov == best && oi < best_at)) {
+          best = ov;
+          best_at = oi;
+        }
+      }
+    };
+    first();
+    if ((tid & 31) == 0) {
+      s_best[wid] = best;
+      s_at[wid] = best_at;
+    }
+    __syncthreads();
+    if (wid == 0) {
+      best = tid < SB_WARPS ? s_best[tid] : -3.402823466e+38f;
+      best_at = tid < SB_WARPS ? s_at[tid] : 0x7fffffff;
+      first();
+      if (tid == 0) {
+        const int token = best_at == 0x7fffffff ? 0 : best_at;  // every entry NaN or below the sentinel
+        run.ids[(long long)b * ids_ld + s] = token;
+        run.out_tokens[(long long)b * run.out_ld + run.step0 + step] = token;
+      }
+    }
+  }
+  __syncthreads();
+  cluster_sync_all();  // the token is there for every CTA of the stream
+  }
+  if (b == 0 && me == 0 && tid == 0) {
+    run.state->s = run.s0 + run.steps;
+    run.state->step = run.step0 + run.steps;
   }
 }
 
@@ -364,7 +464,16 @@ size_t small_smem(int layers, int d, int f, int s) {
   const size_t blocks = ((size_t)(s + SB_ROWS - 1) / SB_ROWS + SB_CTAS - 1) / SB_CTAS;
   return 4 * (SB_PARTIALS + (size_t)(d > f ? d : f) * SB_ROWS + SB_ROWS * (size_t)d + 2 * blocks * SB_ROWS * d +
               (size_t)SB_WARPS * ((s + 3) & ~3) + (size_t)s * (2 * d + 4) + 2 * (9 * (size_t)d + f)) +
-         8 * ((size_t)layers * 12 + 2);
+         8 * ((size_t)layers * 12 + 5);
+}
+
+void small_launch(const SmallShape &g, const SmallRun &run, const char *params, const unsigned long long *offsets, const int *ids,
+                  int ids_ld, const LoopState *state, float *kv, float *x, DevErr *err, cudaStream_t st) {
+  const size_t smem = small_smem(g.layers, g.d, g.f, g.s_cap) + (run.steps ? (size_t)4 * g.d * (g.vocab + 2) : 0);
+  if (smem > 48 * 1024)
+    LB_CUDA(cudaFuncSetAttribute(small_body_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  launch_pdl_cluster_x(small_body_kernel, dim3(SB_CTAS, (unsigned)g.streams), dim3(SB_THREADS), smem, st, g_pdl_enabled,
+                       (unsigned)SB_CTAS, g, run, params, offsets, ids, ids_ld, state, kv, x, err);
 }
 
 }  // namespace
@@ -379,12 +488,20 @@ size_t small_body_kv_floats(int streams, int s, int d) { return (size_t)2 * stre
 void launch_small_body(const char *params, const unsigned long long *offsets, int layers, int n_heads, int d, int f, int vocab,
                        const int *ids, int ids_ld, int streams, int s, const LoopState *state, float *kv, float *x, DevErr *err,
                        cudaStream_t st) {
-  const SmallShape g{layers, n_heads, d, f, vocab, streams, s};
-  const size_t smem = small_smem(layers, d, f, s);
-  if (smem > 48 * 1024)
-    LB_CUDA(cudaFuncSetAttribute(small_body_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  launch_pdl_cluster_x(small_body_kernel, dim3(SB_CTAS, (unsigned)streams), dim3(SB_THREADS), smem, st, g_pdl_enabled,
-                       (unsigned)SB_CTAS, g, params, offsets, ids, ids_ld, state, kv, x, err);
+  small_launch(SmallShape{layers, n_heads, d, f, vocab, streams, s}, SmallRun{}, params, offsets, ids, ids_ld, state, kv, x, err, st);
+}
+
+// The head stays in shared memory for the run: vocabularies beyond what is left there go token by token.
+bool small_loop_supports(int streams, int s, int layers, int n_heads, int d, int f, int vocab) {
+  return small_body_supports(streams, s, layers, n_heads, d, f) && vocab >= 1 && vocab <= 1024 &&
+         small_smem(layers, d, f, s) + (size_t)4 * d * (vocab + 2) <= 220 * 1024;
+}
+
+void launch_small_loop(const char *params, const unsigned long long *offsets, int layers, int n_heads, int d, int f, int vocab,
+                       int *ids, int ids_ld, int *out_tokens, int out_ld, int streams, int s0, int step0, int steps, LoopState *state,
+                       float *logits, float *kv, DevErr *err, cudaStream_t st) {
+  const SmallShape g{layers, n_heads, d, f, vocab, streams, s0 + steps - 1};
+  small_launch(g, SmallRun{s0, steps, step0, out_ld, ids, out_tokens, logits, state}, params, offsets, ids, ids_ld, nullptr, kv, nullptr, err, st);
 }
 
 }  // namespace lb

@@ -44,6 +44,40 @@ def test_small_models_against_the_oracle(oracle, dims, streams, prompt, new):
         assert float((np.abs(every[b] - whole) / np.abs(whole).max()).max()) < 2e-5
 
 
+# Greedy runs in one launch: vocabularies of any size up to what shared memory holds of the head, then token by token; texts that
+# start shorter than the cluster's share; one layer and three (the two buffers change roles from step to step); runs resumed.
+@pytest.mark.parametrize("dims,streams,prompt,new", [
+    ((1, 2, 64, 128, 1, 40), 1, 2, 30),
+    ((3, 2, 64, 256, 37, 70), 4, 6, 60),
+    ((1, 2, 32, 64, 300, 128), 15, 60, 60),
+    ((2, 2, 64, 256, 400, 60), 2, 20, 30),
+    ((2, 4, 128, 256, 130, 64), 1, 1, 62),
+])
+def test_runs_in_one_launch(oracle, dims, streams, prompt, new):
+    d = formats.ModelDims(*dims)
+    arena = formats.make_param_arena(d, 5, bias_std=0.02, ln_std=0.1)
+    prompts = np.stack([formats.zipf_prompt(d.vocab, prompt, 90 + i) for i in range(streams)])
+    with Session(d, streams) as s:
+        s.load_params(arena)
+        whole = s.generate(prompts, new)
+        s.upload_prompts(prompts)
+        assert s.run(new // 3) == new // 3 and s.run(new - new // 3) == new
+        parts = s.download_tokens(new)
+        s.keep_step_logits(True)
+        toks = s.generate(prompts, new)
+        lg = s.read_step_logits(new, streams)
+    assert np.array_equal(whole, parts)
+    for b in range(streams):
+        ties = np.flatnonzero(whole[b] != toks[b])
+        if len(ties):
+            srt = np.sort(lg[ties[0], b].astype(np.float64))
+            assert srt[-1] - srt[-2] < 1e-4
+    ref_tokens, ref_logits = oracle.generate(d, arena, prompts[-1], new, want_logits=True)
+    srt = np.sort(ref_logits.astype(np.float64), axis=1)
+    ties = np.flatnonzero(whole[-1] != ref_tokens)
+    assert not len(ties) or srt[ties[0], -1] - srt[ties[0], -2] < 1e-4
+
+
 def test_bad_ids_are_errors():
     d = formats.ModelDims(1, 2, 64, 128, 9, 32)
     with Session(d, 1) as s:
