@@ -7,7 +7,7 @@
 // dot product is free, so a lane loads 16 consecutive bytes (8 k) of its W row and of its activation
 // row and feeds them to two k-steps as they lie: no shared memory, no shuffles, whole 128-byte lines
 // of W per warp and row. Up to two products with inputs of their own share a launch. Where the columns
-// alone give too few CTAs, k is cut over the CTAs of a thread-block cluster, whose sums meet in the shared
+// alone give too few CTAs, the rows go to several CTAs, and of long rows k is cut over the CTAs of a thread-block cluster, whose sums meet in the shared
 // memory of the rank that stores them (rank order, so results do not depend on scheduling).
 #include "activation.cuh"
 #include "model.cuh"
@@ -47,14 +47,15 @@ __device__ __forceinline__ uint4 ld_stream(const bf16 *p) {  // weights: read on
 // NT: tiles of 8 activation rows; UNROLL: blocks of 32 k in flight per lane and row.
 template <int NT, int UNROLL>
 __global__ void __launch_bounds__(FR_WARPS * 32)
-few_row_bf16_kernel(FewRowPair pair, int m, int ranks) {
+few_row_bf16_kernel(FewRowPair pair, int rows, int ranks) {
   __shared__ __align__(16) float red[FR_WARPS][NT][FR_COLS][8];
   const bool second = (int)blockIdx.x >= pair.blocks0;
   const Bf16Product &p = pair.p[second ? 1 : 0];
   const int n0 = ((int)blockIdx.x - (second ? pair.blocks0 : 0)) * FR_COLS;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int k8 = (p.k + 7) & ~7;  // rows end on a multiple of 8, zeros behind k
-  const bf16 *w = static_cast<const bf16 *>(p.w), *a = static_cast<const bf16 *>(p.a);
+  const int first = (int)blockIdx.y * NT * 8, m = min(NT * 8, rows - first);  // this CTA's activation rows
+  const bf16 *w = static_cast<const bf16 *>(p.w), *a = static_cast<const bf16 *>(p.a) + (long long)first * p.a_ld;
   const bool v0 = n0 + g < p.n, v1 = n0 + g + 8 < p.n;
   const bf16 *w0 = w + (long long)(n0 + g) * p.w_ld + t * 8, *w1 = w0 + (long long)8 * p.w_ld;
   constexpr int SPAN = 32 * UNROLL;  // k per warp and trip
@@ -161,14 +162,14 @@ few_row_bf16_kernel(FewRowPair pair, int m, int ranks) {
     if (p.gated && col < p.n_half) {  // a pair's columns are neighbours in one share: its even one finishes both
       if (c & 1) continue;
       const float z = activate(total(c, row), p.act) * total(c + 1, row);
-      static_cast<bf16 *>(p.half_out)[(long long)row * p.half_ld + (col >> 1)] = __float2bfloat16_rn(z);
+      static_cast<bf16 *>(p.half_out)[(long long)(first + row) * p.half_ld + (col >> 1)] = __float2bfloat16_rn(z);
       continue;
     }
     const float v = total(c, row);
     if (col < p.n_half) {
-      static_cast<bf16 *>(p.half_out)[(long long)row * p.half_ld + col] = __float2bfloat16_rn(activate(v, p.act));
+      static_cast<bf16 *>(p.half_out)[(long long)(first + row) * p.half_ld + col] = __float2bfloat16_rn(activate(v, p.act));
     } else {
-      float *o = p.float_out + (long long)row * p.float_ld + (col - p.n_half);
+      float *o = p.float_out + (long long)(first + row) * p.float_ld + (col - p.n_half);
       *o = p.accumulate ? *o + v : v;
     }
   }
@@ -189,25 +190,29 @@ void launch_few_row_bf16(const Bf16Product *p, int count, int m, cudaStream_t st
   }
   int k_max = 0;
   for (int i = 0; i < count; ++i) k_max = p[i].k > k_max ? p[i].k : k_max;
-  // ranks of a cluster that share a tile's k: enough CTAs for two per SM, at least 512 k each
+  const int tiles = (m + 7) / 8;
+  // Tiles of activation rows a CTA takes. Bound by latency, a launch wants its loads spread over many CTAs, and the weights
+  // that several read come out of L2: as few as give no more than four CTAs an SM (64 rows, us with all rows in one CTA and with
+  // this: n 512 k 512 4.9, 3.4; n 1040 k 512 5.1, 3.1; n 2816 k 512 5.6, 4.7; n 512 k 1408 6.8, 4.4; n 1024 k 1024 6.6, 3.7). Not for
+  // long rows, where reading the weights again costs as much (n 1024 k 5120: 10.1 in one, 12.2 in eight).
+  int nt = 1;
+  while (nt < 8 && nt < tiles && (k_max > 1536 || (long long)blocks * ((tiles + nt - 1) / nt) > 4 * 148)) nt *= 2;
+  const unsigned row_ctas = (unsigned)((tiles + nt - 1) / nt);
+  // Ranks of a cluster that share a tile's k: enough CTAs for two per SM, but a range of less than 1024 (of long rows 640) k costs
+  // more in the exchange than it saves (8 rows, n 1024 k 1024: one rank 2.8, two 4.0; 64 rows, n 2048 k 2048: two ranks 8.0, four 12.8).
   int ranks = 1;
   const int ranks_max = m > 16 ? 4 : 8;  // many rows: a CTA's share of the sums is work too
-  while (ranks < ranks_max && blocks * ranks < 2 * 148 && k_max >= 1024 * ranks) ranks *= 2;
-  const dim3 grid(blocks, 1, (unsigned)ranks), block(FR_WARPS * 32);
+  while (ranks < ranks_max && blocks * row_ctas * ranks < 2 * 148 && k_max >= 2 * ranks * (ranks == 1 ? 1024 : 640)) ranks *= 2;
+  const dim3 grid(blocks, row_ctas, (unsigned)ranks), block(FR_WARPS * 32);
   auto go = [&](auto kernel) {
     launch_pdl_cluster(kernel, grid, block, 0, st, g_pdl_enabled, (unsigned)ranks, pair, m, ranks);
   };
-  const int nt = (m + 7) / 8;
-  if (ranks > 1) {  // shorter ranges: two blocks of 32 k per lane and trip keep every warp busy
-    if (nt <= 1) go(few_row_bf16_kernel<1, 2>);
-    else if (nt <= 2) go(few_row_bf16_kernel<2, 2>);
-    else if (nt <= 4) go(few_row_bf16_kernel<4, 2>);
-    else go(few_row_bf16_kernel<8, 4>);
-    return;
-  }
-  if (nt <= 1) go(few_row_bf16_kernel<1, 4>);
-  else if (nt <= 2) go(few_row_bf16_kernel<2, 4>);
-  else if (nt <= 4) go(few_row_bf16_kernel<4, 4>);
+  // Two blocks of 32 k per lane and trip where the range would leave warps idle with four (n 1040 k 512: 3.1, 3.7 with one); with
+  // eight tiles the activations of a trip outweigh that (n 8192 k 512: 13.2 with two, 10.2 with four).
+  const bool two = k_max <= 512 * ranks;
+  if (nt == 1) two ? go(few_row_bf16_kernel<1, 2>) : go(few_row_bf16_kernel<1, 4>);
+  else if (nt == 2) two ? go(few_row_bf16_kernel<2, 2>) : go(few_row_bf16_kernel<2, 4>);
+  else if (nt == 4) two ? go(few_row_bf16_kernel<4, 2>) : go(few_row_bf16_kernel<4, 4>);
   else go(few_row_bf16_kernel<8, 4>);
 }
 

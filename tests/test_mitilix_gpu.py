@@ -63,6 +63,23 @@ def test_product(engine, m, n, k):
     assert np.abs(got[:, half:] - (want + c)[:, half:]).max() < 2e-5 * max(1.0, k ** 0.5)
 
 
+# rows over several CTAs (one, two, four tiles each, the last not full), all in one, and long rows over the ranks of a cluster
+@pytest.mark.parametrize("m,n,k", [(64, 520, 512), (37, 1300, 300), (20, 4000, 600), (61, 2900, 512), (64, 9600, 136), (3, 40, 1300),
+                                   (5, 64, 2100), (9, 40, 5200), (50, 130, 2600), (8, 1000, 5120)])
+def test_few_rows_by_tiles_and_ranks(m, n, k):
+    rng = np.random.default_rng(m + n + k)
+    a, w = rounded(rng.standard_normal((m, k))), rounded(rng.standard_normal((n, k)) * k ** -0.5)
+    want = a.astype(np.float64) @ w.T.astype(np.float64)
+    c = rng.standard_normal((m, n)).astype(np.float32)
+    # exact products, sums in 32 bits: as above
+    assert np.abs(bf16_product_host(a, w, 0, c=c) - (want + c)).max() < 2e-5 * max(1.0, k ** 0.5)
+    pairs = n // 4 * 2
+    got = bf16_product_host(a, w, 0, n_half=pairs, act="gelu", gated=True)
+    gated = om.gelu_exact(want[:, 0:pairs:2]) * want[:, 1:pairs:2]
+    assert np.abs(got[:, :pairs // 2] - gated).max() < 2 ** -7 * np.abs(gated).max()
+    assert np.abs(got[:, pairs // 2:] - want[:, pairs:]).max() < 2e-5 * max(1.0, k ** 0.5)
+
+
 def test_product_over_many_tiles_and_a_long_k():
     rng = np.random.default_rng(5)
     for m, n, k in ((900, 4100, 192), (2300, 2056, 72), (200, 130, 5000)):
