@@ -4,10 +4,13 @@
 //   h  = x / sqrt(mean(x^2) + eps) * before           (the next sublayer's input)
 //
 // One CTA per row, the row in registers between the two reductions (four consecutive columns per thread and
-// piece); rows of any other width go through a loop over columns that each thread owns. All 32-bit.
+// piece), or a warp per row where there are many; rows of any other width go through a loop over columns that each thread owns.
+// All 32-bit.
 #include "model.cuh"
 
 #include <cuda_bf16.h>
+
+#include <algorithm>
 
 namespace lb {
 
@@ -94,6 +97,74 @@ residual_norm_kernel(float *x, const float *y, RmsWeight after, T *h, int h_ld, 
                                            v[i].w * inv * gb[i].w));
 }
 
+// The same for many rows: a warp per row, so that no barrier stands between a row's loads and its stores and every lane has all of
+// its share (PIECES float4s of x and of y) in flight at once; both gains in shared memory.
+template <typename T, int PIECES>
+__global__ void __launch_bounds__(RN_THREADS)
+residual_norm_rows_kernel(float *x, const float *y, RmsWeight after, T *h, int h_ld, RmsWeight before, int d, int rows, float eps) {
+  extern __shared__ __align__(16) float gains[];  // [2][d]
+  pdl_launch_dependents();
+  const int lane = threadIdx.x & 31;
+  for (int c = threadIdx.x * 4; c < d; c += RN_THREADS * 4) {
+    if (y) put4(gains + c, gain4(after, c));
+    if (h) put4(gains + d + c, gain4(before, c));
+  }
+  __syncthreads();
+  pdl_wait();
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto row_sum = [](float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  };
+  for (int row = blockIdx.x * (RN_THREADS / 32) + (threadIdx.x >> 5); row < rows; row += gridDim.x * (RN_THREADS / 32)) {
+    float *xr = x + (long long)row * d;
+    float4 v[PIECES];
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+      const int c = (i * 32 + lane) * 4;
+      v[i] = c < d ? *reinterpret_cast<const float4 *>(xr + c) : zero;
+    }
+    if (y) {
+      const float *yr = y + (long long)row * d;
+      float4 w[PIECES];
+      float s = 0.f;
+#pragma unroll
+      for (int i = 0; i < PIECES; ++i) {
+        const int c = (i * 32 + lane) * 4;
+        w[i] = c < d ? *reinterpret_cast<const float4 *>(yr + c) : zero;
+      }
+#pragma unroll
+      for (int i = 0; i < PIECES; ++i) s += squares(w[i]);
+      const float inv = 1.0f / sqrtf(row_sum(s) / (float)d + eps);
+#pragma unroll
+      for (int i = 0; i < PIECES; ++i) {
+        const int c = (i * 32 + lane) * 4;
+        if (c >= d) continue;
+        const float4 g = *reinterpret_cast<const float4 *>(gains + c);
+        v[i].x += w[i].x * inv * g.x;
+        v[i].y += w[i].y * inv * g.y;
+        v[i].z += w[i].z * inv * g.z;
+        v[i].w += w[i].w * inv * g.w;
+        put4(xr + c, v[i]);
+      }
+    }
+    if (h == nullptr) continue;
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) s += squares(v[i]);
+    const float inv = 1.0f / sqrtf(row_sum(s) / (float)d + eps);
+    T *hr = h + (long long)row * h_ld;
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+      const int c = (i * 32 + lane) * 4;
+      if (c >= d) continue;
+      const float4 g = *reinterpret_cast<const float4 *>(gains + d + c);
+      put4(hr + c, make_float4(v[i].x * inv * g.x, v[i].y * inv * g.y, v[i].z * inv * g.z, v[i].w * inv * g.w));
+    }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(RN_THREADS)
 residual_norm_any_kernel(float *x, const float *y, RmsWeight after, T *h, int h_ld, RmsWeight before, int d, float eps) {
@@ -124,6 +195,17 @@ void launch_t(float *x, const float *y, const RmsWeight &after, T *h, int h_ld, 
                eps);
   };
   const int quads = d / 4;
+  // A warp per row from about a thousand rows on: 8188 rows x 1024 in bfloat16 25.0 us with a CTA per row, 14.0 with a warp (32.9
+  // and 26.6 with x and y out of HBM), 2048 rows 7.6 and 4.6; 613 rows 3.7 and 3.5; 256 rows 2.7 and 3.3. Up to width 1024: at 2048 a
+  // lane's share of x and y leaves room for one CTA an SM, and both take as long.
+  if (rows >= 1024 && d % 4 == 0 && h_ld % 4 == 0 && quads <= 256) {
+    auto many = [&](auto kernel, int per_sm) {
+      const long long blocks = (rows + RN_THREADS / 32 - 1) / (RN_THREADS / 32);
+      launch_pdl(kernel, dim3((unsigned)std::min<long long>(blocks, 148ll * per_sm)), dim3(RN_THREADS), (size_t)2 * d * 4, st, g_pdl_enabled, x, y,
+                 after, h, h_ld, before, d, (int)rows, eps);
+    };
+    return quads <= 128 ? many(residual_norm_rows_kernel<T, 4>, 5) : many(residual_norm_rows_kernel<T, 8>, 3);
+  }
   if (d % 4 != 0 || h_ld % 4 != 0 || quads > 8 * RN_THREADS) return go(residual_norm_any_kernel<T>, RN_THREADS);
   auto threads = [&](int pieces) { return ((quads + pieces - 1) / pieces + 31) / 32 * 32; };
   if (quads <= RN_THREADS) go(residual_norm_kernel<T, 1>, threads(1));

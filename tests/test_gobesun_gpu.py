@@ -82,6 +82,23 @@ def test_residual_norm(d):
     assert gh is None and not np.array_equal(gx, x)
 
 
+@pytest.mark.parametrize("rows,d", [(1024, 4), (1030, 132), (5000, 512), (1100, 516), (2500, 1024), (1025, 1028)])
+def test_residual_norm_of_many_rows(rows, d):
+    """A warp per row, every CTA several rows, up to width 1024; a CTA per row beyond."""
+    rng = np.random.default_rng(rows + d)
+    x, y = (3.0 * rng.standard_normal((2, rows, d))).astype(np.float32)
+    after, before = (0.3 * rng.standard_normal((2, d))).astype(np.float32)
+    wx = x + om.rms_normalise(y.astype(np.float64), 1e-2) * (1.0 + after)
+    wh = om.rms_normalise(wx, 1e-2) * (1.0 + before)
+    for dtype, near in (("float32", 1e-5), ("bfloat16", 2 ** -8)):
+        gx, gh = residual_norm_host(x, y, after, before, 1.0, 1e-2, dtype=dtype)
+        assert np.abs(gx - wx).max() < 1e-5 * np.abs(wx).max() and np.abs(gh - wh).max() < near * np.abs(wh).max()
+    gx, gh = residual_norm_host(x, None, None, before, 1.0, 1e-6)
+    assert np.array_equal(gx, x) and np.abs(gh - og.centred_rms_norm(x.astype(np.float64), before, 1e-6)).max() < 1e-5 * np.abs(gh).max()
+    gx, gh = residual_norm_host(x, y, after, None, 1.0, 1e-2)
+    assert gh is None and np.abs(gx - wx).max() < 1e-5 * np.abs(wx).max()
+
+
 def delta_case(seed, streams, n, heads, groups, dim, vdim, taps):
     rng = np.random.default_rng(seed)
     c = 2 * groups * dim + heads * vdim
