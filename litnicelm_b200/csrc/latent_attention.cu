@@ -205,6 +205,20 @@ __device__ __forceinline__ void ldmatrix_x2_trans(unsigned &r0, unsigned &r1, co
   const unsigned addr = (unsigned)__cvta_generic_to_shared(p);
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
 }
+__device__ __forceinline__ void ldmatrix_x4(unsigned (&r)[4], const void *p) {
+  const unsigned addr = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ float2 ld_cluster_f2(unsigned cluster_addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(cluster_addr) : "memory");
+  return v;
+}
+// Pitch of value rows in shared memory, in halves: 64 bytes beside a multiple of 128, so that 16-byte reads of two rows' quarters
+// by eight lanes hit all banks.
+__host__ __device__ constexpr int uv_pitch(int w_ld) { return (w_ld * 2 + 127) / 128 * 64 + 32; }
 // 16 bytes to shared memory in the background; bytes = 0 stores zeros.
 __device__ __forceinline__ void copy16(void *dst, const void *src, int bytes) {
   const unsigned addr = (unsigned)__cvta_generic_to_shared(dst);
@@ -334,18 +348,28 @@ latent_chunk_kernel(LdShape g, const bf16 *q_hi, const bf16 *q_lo, const bf16 *c
   constexpr int PP = LD_KEYS + 8, SP = LD_KEYS + 4;
   bf16 *ph = ql + LD_HEADS * pitch;                  // [16][PP] high and low terms of the weights
   bf16 *pl = ph + LD_HEADS * PP;
-  float *sc = reinterpret_cast<float *>(pl + LD_HEADS * PP);  // [16][SP]
-  float *fac = sc + LD_HEADS * SP;                   // [16] factors of what has been summed so far
+  float *sc = reinterpret_cast<float *>(pl + LD_HEADS * PP);  // [2][16][SP] of both halves of the columns
+  float *fac = sc + 2 * LD_HEADS * SP;               // [16] factors of what has been summed so far
   bf16 *tiles = reinterpret_cast<bf16 *>(fac + LD_HEADS);     // [stages][LD_KEYS][pitch]
   pdl_launch_dependents();
-  bf16 *uv = tiles + stages * LD_KEYS * pitch;       // [share][vdim][w_ld] value rows, where uv_resident
+  bf16 *uv = tiles + stages * LD_KEYS * pitch;       // [share][vdim][uv_pitch] value rows, where uv_resident
   if constexpr (CLUSTER) {  // the value rows this CTA maps its heads through depend on nothing: on their way now
     const int nh = min(LD_HEADS, g.heads - (int)blockIdx.y * LD_HEADS);
     for (int hh = blockIdx.x; hh < nh; hh += g.splits) {
       const char *rows = reinterpret_cast<const char *>(w_uv + (long long)(blockIdx.y * LD_HEADS + hh) * g.vdim * w_ld);
       if (uv_resident) {
-        char *to = reinterpret_cast<char *>(uv) + (size_t)(hh / g.splits) * g.vdim * w_ld * 2;
-        for (int at = threadIdx.x * 16; at < g.vdim * w_ld * 2; at += LD_THREADS * 16) copy16(to + at, rows + at, 16);
+        const int per = w_ld >> 3;  // pieces of a row
+        int e = threadIdx.x / per, c = threadIdx.x - e * per;
+        bf16 *to = uv + (size_t)(hh / g.splits) * g.vdim * uv_pitch(w_ld);
+        while (e < g.vdim) {
+          copy16(to + e * uv_pitch(w_ld) + c * 8, rows + ((size_t)e * w_ld + c * 8) * 2, 16);
+          e += LD_THREADS / per;
+          c += LD_THREADS % per;
+          if (c >= per) {
+            c -= per;
+            ++e;
+          }
+        }
         continue;
       }
       for (int at = threadIdx.x * 128; at < g.vdim * w_ld * 2; at += LD_THREADS * 128)
@@ -403,34 +427,39 @@ latent_chunk_kernel(LdShape g, const bf16 *q_hi, const bf16 *q_lo, const bf16 *c
     __syncthreads();
     const bf16 *ck = tiles + (tile % stages) * LD_KEYS * pitch;
     const int nk = min(LD_KEYS, total - tile * LD_KEYS);
-    {  // scores: warp w takes keys 8w .. 8w + 7; two accumulators keep the products of the terms apart
-      float d[4] = {0.f, 0.f, 0.f, 0.f}, d2[4] = {0.f, 0.f, 0.f, 0.f};
-      const bf16 *kr = ck + (wid * 8 + gr) * pitch + tq * 2;
-      const bf16 *ah = qh + gr * pitch + tq * 2, *al = ql + gr * pitch + tq * 2;
+    {  // scores: warp w takes sixteen keys and half of the columns, so that the queries are read four times and not eight; two
+       // accumulators keep the products of the terms apart
+      float d[2][4] = {}, d2[2][4] = {};
+      const int keys = (wid & 3) * 16, half = (rk / 16 + 1) / 2 * 16, k_end = wid < 4 ? half : rk;
+      // (of the queries rows by lanes 0 .. 15, their second eight k by lanes 16 .. 31; of the keys eight rows by eight lanes, their
+      // second eight k by the next, eight more rows by lanes 16 .. 31)
+      const bf16 *kr = ck + (keys + (lane & 7) + (lane >> 4) * 8) * pitch + (lane >> 3 & 1) * 8;
+      const bf16 *ah = qh + (lane & 15) * pitch + (lane >> 4) * 8, *al = ql + (lane & 15) * pitch + (lane >> 4) * 8;
 #pragma unroll 4
-      for (int k = 0; k < rk; k += 16) {
-        const unsigned b0 = *reinterpret_cast<const unsigned *>(kr + k), b1 = *reinterpret_cast<const unsigned *>(kr + k + 8);
-        const unsigned a[4] = {*reinterpret_cast<const unsigned *>(ah + k),
-                               *reinterpret_cast<const unsigned *>(ah + k + 8 * pitch),
-                               *reinterpret_cast<const unsigned *>(ah + k + 8),
-                               *reinterpret_cast<const unsigned *>(ah + k + 8 * pitch + 8)};
-        const unsigned a2[4] = {*reinterpret_cast<const unsigned *>(al + k),
-                                *reinterpret_cast<const unsigned *>(al + k + 8 * pitch),
-                                *reinterpret_cast<const unsigned *>(al + k + 8),
-                                *reinterpret_cast<const unsigned *>(al + k + 8 * pitch + 8)};
-        mma_bf16(d2, a2, b0, b1);
-        mma_bf16(d, a, b0, b1);
+      for (int k = wid < 4 ? 0 : half; k < k_end; k += 16) {
+        unsigned bk[4], a[4], a2[4];
+        ldmatrix_x4(bk, kr + k);
+        ldmatrix_x4(a, ah + k);
+        ldmatrix_x4(a2, al + k);
+        mma_bf16(d2[0], a2, bk[0], bk[1]);
+        mma_bf16(d2[1], a2, bk[2], bk[3]);
+        mma_bf16(d[0], a, bk[0], bk[1]);
+        mma_bf16(d[1], a, bk[2], bk[3]);
       }
-      const int j = wid * 8 + tq * 2;
-      *reinterpret_cast<float2 *>(sc + gr * SP + j) = make_float2(d[0] + d2[0], d[1] + d2[1]);
-      *reinterpret_cast<float2 *>(sc + (gr + 8) * SP + j) = make_float2(d[2] + d2[2], d[3] + d2[3]);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float *to = sc + (wid >> 2) * LD_HEADS * SP + gr * SP + keys + u * 8 + tq * 2;
+        *reinterpret_cast<float2 *>(to) = make_float2(d[u][0] + d2[u][0], d[u][1] + d2[u][1]);
+        *reinterpret_cast<float2 *>(to + 8 * SP) = make_float2(d[u][2] + d2[u][2], d[u][3] + d2[u][3]);
+      }
     }
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < 2; ++i) {  // weights: a lane takes two keys
       const int hh = wid * 2 + i;
-      const float s0 = lane < nk ? sc[hh * SP + lane] : -INFINITY;
-      const float s1 = lane + 32 < nk ? sc[hh * SP + lane + 32] : -INFINITY;
+      const float *of = sc + hh * SP + lane;
+      const float s0 = lane < nk ? of[0] + of[LD_HEADS * SP] : -INFINITY;
+      const float s1 = lane + 32 < nk ? of[32] + of[LD_HEADS * SP + 32] : -INFINITY;
       const float mn = fmaxf(m[i], warp_max(fmaxf(s0, s1)));
       const float p0 = exp2f(s0 - mn), p1 = exp2f(s1 - mn), keep = exp2f(m[i] - mn);
       l[i] = l[i] * keep + warp_sum(p0 + p1);
@@ -448,15 +477,8 @@ latent_chunk_kernel(LdShape g, const bf16 *q_hi, const bf16 *q_lo, const bf16 *c
     unsigned a[LD_KEYS / 16][4], a2[LD_KEYS / 16][4];
 #pragma unroll
     for (int k = 0; k < LD_KEYS / 16; ++k) {
-      const bf16 *x = ph + gr * PP + tq * 2 + k * 16, *y = pl + gr * PP + tq * 2 + k * 16;
-      a[k][0] = *reinterpret_cast<const unsigned *>(x);
-      a[k][1] = *reinterpret_cast<const unsigned *>(x + 8 * PP);
-      a[k][2] = *reinterpret_cast<const unsigned *>(x + 8);
-      a[k][3] = *reinterpret_cast<const unsigned *>(x + 8 * PP + 8);
-      a2[k][0] = *reinterpret_cast<const unsigned *>(y);
-      a2[k][1] = *reinterpret_cast<const unsigned *>(y + 8 * PP);
-      a2[k][2] = *reinterpret_cast<const unsigned *>(y + 8);
-      a2[k][3] = *reinterpret_cast<const unsigned *>(y + 8 * PP + 8);
+      ldmatrix_x4(a[k], ph + (lane & 15) * PP + (lane >> 4) * 8 + k * 16);
+      ldmatrix_x4(a2[k], pl + (lane & 15) * PP + (lane >> 4) * 8 + k * 16);
     }
     const float f0 = fac[gr], f1 = fac[gr + 8];
 #pragma unroll
@@ -491,7 +513,6 @@ latent_chunk_kernel(LdShape g, const bf16 *q_hi, const bf16 *q_lo, const bf16 *c
     const int r8 = (g.rank + 7) & ~7, ranks = g.splits;
     const int share = (nh - (int)blockIdx.x + ranks - 1) / ranks;  // heads blockIdx.x, blockIdx.x + ranks, ... are this CTA's
     float *ol = reinterpret_cast<float *>(qh);                     // [share][r8] weighted latents, over the queries
-    float *join = sc;                                              // [share][8] factors of the splits, over the scores
 #pragma unroll
     for (int i = 0; i < 2; ++i)
       if (lane == 0) mls[wid * 2 + i] = make_float2(m[i], l[i]);
@@ -505,69 +526,78 @@ latent_chunk_kernel(LdShape g, const bf16 *q_hi, const bf16 *q_lo, const bf16 *c
     __syncwarp();
     cluster_sync_all();
     const unsigned os_at = smem_u32(os), ml_at = smem_u32(mls);
-    for (int i = wid; i < share; i += LD_THREADS / 32) {  // lane q looks at split q
-      const unsigned at = ml_at + (unsigned)((int)blockIdx.x + i * ranks) * 8u;
-      const float mq = lane < ranks ? ld_cluster_f32(cluster_map(at, (unsigned)lane)) : -INFINITY;
-      const float lq = lane < ranks ? ld_cluster_f32(cluster_map(at + 4u, (unsigned)lane)) : 0.f;
-      const float e = exp2f(mq - warp_max(mq));
-      const float sum = warp_sum(lq * e);
-      if (lane < ranks) join[i * LD_CLUSTER + lane] = e / sum;
-    }
-    __syncthreads();
     const int cols = r8 >> 2;
-    for (int k = tid; k < share * cols; k += LD_THREADS) {
+    for (int k = tid; k < share * cols; k += LD_THREADS) {  // maxima, sums and outputs of all splits in one round trip
       const int i = k / cols, c = (k - i * cols) * 4;
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
       if (c < g.rank4) {
-        const unsigned at = os_at + (unsigned)(((int)blockIdx.x + i * ranks) * g.rank4 + c) * 4u;
+        const int hh = (int)blockIdx.x + i * ranks;
+        const unsigned at = os_at + (unsigned)(hh * g.rank4 + c) * 4u;
         float4 v[LD_CLUSTER];
+        float2 ml[LD_CLUSTER];
 #pragma unroll
-        for (int q = 0; q < LD_CLUSTER; ++q)
-          v[q] = q < ranks ? ld_cluster_f4(cluster_map(at, (unsigned)q)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int q = 0; q < LD_CLUSTER; ++q) {
+          v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+          ml[q] = make_float2(-INFINITY, 0.f);
+          if (q < ranks) {
+            ml[q] = ld_cluster_f2(cluster_map(ml_at + (unsigned)hh * 8u, (unsigned)q));
+            v[q] = ld_cluster_f4(cluster_map(at, (unsigned)q));
+          }
+        }
+        float mx = ml[0].x, sum = 0.f;
+#pragma unroll
+        for (int q = 1; q < LD_CLUSTER; ++q) mx = fmaxf(mx, ml[q].x);
+#pragma unroll
+        for (int q = 0; q < LD_CLUSTER; ++q) {
+          ml[q].x = exp2f(ml[q].x - mx);
+          sum = fmaf(ml[q].y, ml[q].x, sum);
+        }
+        const float inv = 1.0f / sum;
 #pragma unroll
         for (int q = 0; q < LD_CLUSTER; ++q)
           if (q < ranks) {
-            const float f = join[i * LD_CLUSTER + q];
+            const float f = ml[q].x * inv;
             acc = make_float4(fmaf(f, v[q].x, acc.x), fmaf(f, v[q].y, acc.y), fmaf(f, v[q].z, acc.z), fmaf(f, v[q].w, acc.w));
           }
       }
       *reinterpret_cast<float4 *>(ol + i * r8 + c) = acc;
     }
     __syncthreads();
-    // the value rows of all the CTA's heads, four per warp and trip; a row's loads precede their use
-    const int n_rows = share * g.vdim;
-    for (int k0 = wid * 4; k0 < n_rows; k0 += LD_THREADS / 32 * 4) {
-      float sum[4] = {};
-      const bf16 *wr[4];
-      const float *x[4];
+    // the value rows of all the CTA's heads: four lanes a row, eight columns each in turn (a warp a row, its sums over 32 lanes by
+    // shuffles, took 10 000 of the 21 000 cycles that this kernel did; now 2 900 of 14 600: 8 rows, 16 heads of 64, rank 256, 300 keys,
+    // 16.0 us a layer for query and chunk kernels together, now 11.4; 64 rows 32.1, now 22.7)
+    const int n_rows = share * g.vdim, quarter = lane & 3;
+    auto map_rows = [&](auto resident) {
+      for (int k0 = wid * 8; k0 < n_rows; k0 += LD_THREADS / 32 * 8) {
+        const int k = k0 + (lane >> 2), kk = min(k, n_rows - 1), i = kk / g.vdim, e = kk - i * g.vdim;
+        const long long col = (long long)(h0 + (int)blockIdx.x + i * ranks) * g.vdim + e;
+        const bf16 *wr = resident.value ? uv + kk * uv_pitch(w_ld) : w_uv + col * w_ld;
+        const float *x = ol + i * r8;
+        float sum[2] = {0.f, 0.f};
+        for (int c0 = quarter * 8; c0 < r8; c0 += 256) {
+          uint4 w8[8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int k = min(k0 + u, n_rows - 1), i = k / g.vdim, e = k - i * g.vdim;
-        wr[u] = uv_resident ? uv + (i * g.vdim + e) * w_ld
-                            : w_uv + ((long long)(h0 + (int)blockIdx.x + i * ranks) * g.vdim + e) * w_ld;
-        x[u] = ol + i * r8;
-      }
-      for (int c = lane * 8; c < r8; c += 256) {
-        uint4 w4[4];
+          for (int u = 0; u < 8; ++u)
+            w8[u] = c0 + u * 32 < r8 ? *reinterpret_cast<const uint4 *>(wr + c0 + u * 32) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) w4[u] = *reinterpret_cast<const uint4 *>(wr[u] + c);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          float f[8];
-          unpack8(w4[u], f);
-          const float4 y = *reinterpret_cast<const float4 *>(x[u] + c), z = *reinterpret_cast<const float4 *>(x[u] + c + 4);
-          sum[u] = fmaf(f[0], y.x, fmaf(f[1], y.y, fmaf(f[2], y.z, fmaf(f[3], y.w, sum[u]))));
-          sum[u] = fmaf(f[4], z.x, fmaf(f[5], z.y, fmaf(f[6], z.z, fmaf(f[7], z.w, sum[u]))));
+          for (int u = 0; u < 8; ++u) {
+            const int c = c0 + u * 32;
+            if (c >= r8) break;
+            float f[8];
+            unpack8(w8[u], f);
+            const float4 y = *reinterpret_cast<const float4 *>(x + c), z = *reinterpret_cast<const float4 *>(x + c + 4);
+            sum[0] = fmaf(f[0], y.x, fmaf(f[1], y.y, fmaf(f[2], y.z, fmaf(f[3], y.w, sum[0]))));
+            sum[1] = fmaf(f[4], z.x, fmaf(f[5], z.y, fmaf(f[6], z.z, fmaf(f[7], z.w, sum[1]))));
+          }
         }
+        float v = sum[0] + sum[1];
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        if (quarter == 0 && k < n_rows) out[r * out_ld + col] = __float2bfloat16_rn(v);
       }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float v = warp_sum(sum[u]);
-        const int k = k0 + u, i = k / g.vdim;
-        if (lane == 0 && k < n_rows)
-          out[r * out_ld + (long long)(h0 + (int)blockIdx.x + i * ranks) * g.vdim + (k - i * g.vdim)] = __float2bfloat16_rn(v);
-      }
-    }
+    };
+    if (uv_resident) map_rows(std::integral_constant<bool, true>());
+    else map_rows(std::integral_constant<bool, false>());
     __syncwarp();
     cluster_sync_all();  // a split's shared memory stays until every other has read it
   } else {
@@ -688,7 +718,7 @@ latent_join_kernel(LdShape g, const float *part_o, const float2 *part_ml, const 
 size_t chunk_smem(int rank, int stages) {
   const int pitch = ((rank + 15) & ~15) + 8;
   return (size_t)(stages * LD_KEYS + 2 * LD_HEADS) * pitch * 2 + (size_t)2 * LD_HEADS * (LD_KEYS + 8) * 2 +
-         (size_t)LD_HEADS * (LD_KEYS + 4) * 4 + LD_HEADS * 4;
+         (size_t)2 * LD_HEADS * (LD_KEYS + 4) * 4 + LD_HEADS * 4;
 }
 constexpr size_t LD_SMEM_LIMIT = 220 * 1024;
 
@@ -805,7 +835,7 @@ int launch_latent_decode(const LatentAttention &a, const LatentFresh &fresh, flo
   // Where every CTA has an SM to itself, the value rows of its heads come to shared memory while the queries and scores
   // are formed (and while the predecessor ends); read from L2 behind them, four rows a warp at a time, they cost 4 us of a
   // layer's 37 (8 rows, 16 heads of 64, rank 256, 350 keys: 459 -> 410 us a token in 12 layers).
-  const size_t uv = (size_t)((a.heads < LD_HEADS ? a.heads : LD_HEADS) + g.splits - 1) / g.splits * a.vdim * a.w_ld * 2;
+  const size_t uv = (size_t)((a.heads < LD_HEADS ? a.heads : LD_HEADS) + g.splits - 1) / g.splits * a.vdim * uv_pitch(a.w_ld) * 2;
   const bool uv_resident = cluster && (long long)g.splits * (g.heads16 / LD_HEADS) * rows <= 148 && smem + uv <= LD_SMEM_LIMIT;
   if (uv_resident) smem += uv;
   auto chunk = [&](auto kernel) {
