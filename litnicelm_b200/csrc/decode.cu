@@ -131,10 +131,11 @@ __device__ __forceinline__ void store_context(const DecodeCtx &o, float v, int b
 // and V (this step's QKV row) to the caches. With one chunk the normalised context row is
 // written directly; otherwise (o, max, sum) go to `part` and the chunk that finishes last joins them.
 //
-// Bound by the cache bytes (8 * s * d_model per layer and stream), so what counts is bytes in
-// flight: both products read 16 bytes per lane and issue DEC_UNROLL keys' loads before the first
-// is used (DEC_UNROLL x 32 bytes per thread of keys, x 16 of values): 64 streams of 128 .. 191
-// positions at d_model 512 take 19.5 us, 27.4 us with 4-byte loads of values and one key at a time.
+// Bound by the cache bytes (8 * s * d_model per layer and stream), so what counts is bytes in flight: the chunk's lines are asked for
+// towards L2 before the predecessor has ended, and a warp has eight keys and values in use and eight more on their way, without a
+// barrier before the warps' results meet. 64 streams of 128 .. 191 positions at d_model 512: 12.6 us; 19.5 with scores, weights
+// and values as three phases of the CTA, four loads in flight in each (which heads of 16 columns still do); prefetching alone
+// makes those 15.3 with eight loads. A cached step of 6 layers: 392 -> 320 us.
 constexpr int DEC_UNROLL = 4;
 template <int DH>
 __global__ void __launch_bounds__(128)
@@ -151,10 +152,19 @@ attn_decode_kernel(const float *__restrict__ qkv, float *kc, float *vc, int cap,
   __shared__ __align__(16) float o_part[512];  // [VPI][DH]
   __shared__ int is_last;
   pdl_launch_dependents();
+  const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, chunks = gridDim.x;
+  {  // the chunk's keys and values of earlier positions, on their way to L2 while the predecessor ends and scores are formed
+    const int early = min(state ? *static_cast<const volatile int *>(&state->s) : s_host, cap);  // (of the step before, perhaps)
+    const int first = c * keys_per_chunk, lines = max(0, min(early, first + keys_per_chunk) - first) * (DH / 32);
+    for (int i = threadIdx.x; i < 2 * lines; i += 128) {
+      const int at = i < lines ? i : i - lines;
+      const float *line = (i < lines ? kc : vc) + ((long long)b * cap + first + at / (DH / 32)) * d_model + h * DH + at % (DH / 32) * 32;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
+    }
+  }
   pdl_wait();
   const int s = state ? state->s : s_host;  // context length including the newest token
   const int p = s - 1;
-  const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, chunks = gridDim.x;
   const int c0 = c * keys_per_chunk, c1 = min(s, c0 + keys_per_chunk);
   float *out = part ? part + (((long long)b * gridDim.y + h) * chunks + c) * (DH + 2) : nullptr;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -166,90 +176,200 @@ attn_decode_kernel(const float *__restrict__ qkv, float *kc, float *vc, int cap,
     }
   } else {
     const float *row = qkv + (long long)b * 3 * d_model;
+    float t = 0.f, m = -INFINITY;
+    double l = 0.0;
     if (p >= c0 && p < c1 && tid < DH / 4) {
       const float4 k4 = *reinterpret_cast<const float4 *>(row + d_model + h * DH + tid * 4);
       const float4 v4 = *reinterpret_cast<const float4 *>(row + 2 * d_model + h * DH + tid * 4);
       *reinterpret_cast<float4 *>(kc + ((long long)b * cap + p) * d_model + h * DH + tid * 4) = k4;
       *reinterpret_cast<float4 *>(vc + ((long long)b * cap + p) * d_model + h * DH + tid * 4) = v4;
     }
-    __syncthreads();
-    const int sub = tid % LPK;
-    const float4 q0 = *reinterpret_cast<const float4 *>(row + h * DH + sub * 8);
-    const float4 q1 = *reinterpret_cast<const float4 *>(row + h * DH + sub * 8 + 4);
-    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float *kb = kc + (long long)b * cap * d_model + h * DH + sub * 8;
-    for (int base = c0; base < c1; base += DEC_UNROLL * KPI) {  // uniform trip count: the shuffles need whole warps
-      float4 k0[DEC_UNROLL], k1[DEC_UNROLL];
+    if constexpr (DH >= 32) {
+      // A warp takes every fourth key, eight at a time: their scores over LPK lanes a key, the running maximum and sum, the weighted
+      // values with a lane per DH / 32 columns. The next eight keys and values are on their way while eight are used.
+      constexpr int KB = 8, KPP = 32 / LPK, NP = KB / KPP, VW = DH / 32;
+      const int sub = lane % LPK, grp = lane / LPK;
+      const int mine = (c1 - c0 - wid + 3) / 4;  // keys of this warp: positions c0 + wid + 4 n
+      const float4 q0 = *reinterpret_cast<const float4 *>(row + h * DH + sub * 8);
+      const float4 q1 = *reinterpret_cast<const float4 *>(row + h * DH + sub * 8 + 4);
+      const long long at0 = ((long long)b * cap + c0 + wid) * d_model + h * DH;
+      struct Batch {
+        float4 k0[NP], k1[NP];
+        float v[KB][VW];
+      };
+      Batch next;
+      auto load = [&](int n0) {
 #pragma unroll
-      for (int u = 0; u < DEC_UNROLL; ++u) {
-        const int j = base + u * KPI + tid / LPK;
-        const float4 *kp = reinterpret_cast<const float4 *>(kb + (long long)j * d_model);
-        k0[u] = j < c1 ? kp[0] : zero4;
-        k1[u] = j < c1 ? kp[1] : zero4;
+        for (int u = 0; u < NP; ++u) {
+          const int n = n0 + u * KPP + grp;
+          next.k0[u] = next.k1[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (n < mine) {  // (the newest position's key and value are this step's own)
+            const float *kp = c0 + wid + 4 * n == p ? row + d_model + h * DH : kc + at0 + (long long)(4 * n) * d_model;
+            next.k0[u] = *reinterpret_cast<const float4 *>(kp + sub * 8);
+            next.k1[u] = *reinterpret_cast<const float4 *>(kp + sub * 8 + 4);
+          }
+        }
+#pragma unroll
+        for (int x = 0; x < KB; ++x) {
+          const int n = n0 + x;
+#pragma unroll
+          for (int y = 0; y < VW; ++y) next.v[x][y] = 0.f;
+          if (n < mine) {
+            const float *vp = (c0 + wid + 4 * n == p ? row + 2 * d_model + h * DH : vc + at0 + (long long)(4 * n) * d_model) + lane * VW;
+            if constexpr (VW == 4) {
+              const float4 f = *reinterpret_cast<const float4 *>(vp);
+              next.v[x][0] = f.x;
+              next.v[x][1] = f.y;
+              next.v[x][2] = f.z;
+              next.v[x][3] = f.w;
+            } else if constexpr (VW == 2) {
+              const float2 f = *reinterpret_cast<const float2 *>(vp);
+              next.v[x][0] = f.x;
+              next.v[x][1] = f.y;
+            } else {
+              next.v[x][0] = *vp;
+            }
+          }
+        }
+      };
+      float o[VW];
+#pragma unroll
+      for (int y = 0; y < VW; ++y) o[y] = 0.f;
+      load(0);
+#pragma unroll 1
+      for (int n0 = 0; n0 < mine; n0 += KB) {
+        const Batch now = next;
+        if (n0 + KB < mine) load(n0 + KB);
+        float e[NP], bm = -INFINITY;
+#pragma unroll
+        for (int u = 0; u < NP; ++u) {
+          float dot = q0.x * now.k0[u].x;
+          dot = fmaf(q0.y, now.k0[u].y, dot);
+          dot = fmaf(q0.z, now.k0[u].z, dot);
+          dot = fmaf(q0.w, now.k0[u].w, dot);
+          dot = fmaf(q1.x, now.k1[u].x, dot);
+          dot = fmaf(q1.y, now.k1[u].y, dot);
+          dot = fmaf(q1.z, now.k1[u].z, dot);
+          dot = fmaf(q1.w, now.k1[u].w, dot);
+#pragma unroll
+          for (int x = LPK >> 1; x > 0; x >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, x);
+          e[u] = n0 + u * KPP + grp < mine ? dot * scale : -INFINITY;
+          bm = fmaxf(bm, e[u]);
+        }
+#pragma unroll
+        for (int x = LPK; x < 32; x <<= 1) bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, x));
+        const float mn = fmaxf(m, bm), keep = m == -INFINITY ? 0.f : expf(m - mn);
+        m = mn;
+        l *= (double)keep;
+#pragma unroll
+        for (int y = 0; y < VW; ++y) o[y] *= keep;
+#pragma unroll
+        for (int u = 0; u < NP; ++u) {
+          e[u] = e[u] == -INFINITY ? 0.f : expf(e[u] - m);
+          l += (double)e[u];
+        }
+#pragma unroll
+        for (int x = 0; x < KB; ++x) {
+          const float w = __shfl_sync(0xffffffffu, e[x / KPP], x % KPP * LPK);
+#pragma unroll
+          for (int y = 0; y < VW; ++y) o[y] = fmaf(w, now.v[x][y], o[y]);
+        }
       }
 #pragma unroll
-      for (int u = 0; u < DEC_UNROLL; ++u) {
-        const int j = base + u * KPI + tid / LPK;
-        float dot = q0.x * k0[u].x;
-        dot = fmaf(q0.y, k0[u].y, dot);
-        dot = fmaf(q0.z, k0[u].z, dot);
-        dot = fmaf(q0.w, k0[u].w, dot);
-        dot = fmaf(q1.x, k1[u].x, dot);
-        dot = fmaf(q1.y, k1[u].y, dot);
-        dot = fmaf(q1.z, k1[u].z, dot);
-        dot = fmaf(q1.w, k1[u].w, dot);
+      for (int x = LPK; x < 32; x <<= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
 #pragma unroll
-        for (int o = LPK >> 1; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        if (j < c1 && sub == 0) sc[j - c0] = dot * scale;
+      for (int y = 0; y < VW; ++y) o_part[wid * DH + lane * VW + y] = o[y];
+      if (lane == 0) {
+        red_f[wid] = m;
+        red_d[wid] = l;
       }
-    }
-    __syncthreads();
-    const int nk = c1 - c0;
-    float m = -INFINITY;
-    for (int i = tid; i < nk; i += 128) m = fmaxf(m, sc[i]);
+      __syncthreads();
+      m = fmaxf(fmaxf(red_f[0], red_f[1]), fmaxf(red_f[2], red_f[3]));
+      l = 0.0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0) red_f[wid] = m;
-    __syncthreads();
-    m = fmaxf(fmaxf(red_f[0], red_f[1]), fmaxf(red_f[2], red_f[3]));
-    double l = 0.0;
-    for (int i = tid; i < nk; i += 128) {
-      const float e = expf(sc[i] - m);
-      sc[i] = e;
-      l += (double)e;
-    }
-    l = warp_sum_d(l);
-    if (lane == 0) red_d[wid] = l;
-    __syncthreads();
-    l = ((red_d[0] + red_d[1]) + red_d[2]) + red_d[3];
-    // second product: thread -> (four columns of the head, every VPI-th key)
-    const int vr = tid / VPR, vq = tid % VPR;
-    float4 o = zero4;
-    const float *vp = vc + ((long long)b * cap + c0) * d_model + h * DH + vq * 4;
-    for (int i0 = vr; i0 < nk; i0 += DEC_UNROLL * VPI) {
-      float4 v[DEC_UNROLL];
-#pragma unroll
-      for (int u = 0; u < DEC_UNROLL; ++u) {
-        const int i = i0 + u * VPI;
-        v[u] = i < nk ? *reinterpret_cast<const float4 *>(vp + (long long)i * d_model) : zero4;
+      for (int w = 0; w < 4; ++w) {
+        const float f = red_f[w] == -INFINITY ? 0.f : expf(red_f[w] - m);
+        l += red_d[w] * (double)f;
+        if (tid < DH) t = fmaf(o_part[w * DH + tid], f, t);
       }
+      __syncthreads();  // (red_f is used again below)
+    } else {
+      __syncthreads();
+      const int sub = tid % LPK;
+      const float4 q0 = *reinterpret_cast<const float4 *>(row + h * DH + sub * 8);
+      const float4 q1 = *reinterpret_cast<const float4 *>(row + h * DH + sub * 8 + 4);
+      const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float *kb = kc + (long long)b * cap * d_model + h * DH + sub * 8;
+      for (int base = c0; base < c1; base += DEC_UNROLL * KPI) {  // uniform trip count: the shuffles need whole warps
+        float4 k0[DEC_UNROLL], k1[DEC_UNROLL];
 #pragma unroll
-      for (int u = 0; u < DEC_UNROLL; ++u) {
-        const int i = i0 + u * VPI;
-        const float e = i < nk ? sc[i] : 0.f;
-        o.x = fmaf(e, v[u].x, o.x);
-        o.y = fmaf(e, v[u].y, o.y);
-        o.z = fmaf(e, v[u].z, o.z);
-        o.w = fmaf(e, v[u].w, o.w);
+        for (int u = 0; u < DEC_UNROLL; ++u) {
+          const int j = base + u * KPI + tid / LPK;
+          const float4 *kp = reinterpret_cast<const float4 *>(kb + (long long)j * d_model);
+          k0[u] = j < c1 ? kp[0] : zero4;
+          k1[u] = j < c1 ? kp[1] : zero4;
+        }
+#pragma unroll
+        for (int u = 0; u < DEC_UNROLL; ++u) {
+          const int j = base + u * KPI + tid / LPK;
+          float dot = q0.x * k0[u].x;
+          dot = fmaf(q0.y, k0[u].y, dot);
+          dot = fmaf(q0.z, k0[u].z, dot);
+          dot = fmaf(q0.w, k0[u].w, dot);
+          dot = fmaf(q1.x, k1[u].x, dot);
+          dot = fmaf(q1.y, k1[u].y, dot);
+          dot = fmaf(q1.z, k1[u].z, dot);
+          dot = fmaf(q1.w, k1[u].w, dot);
+#pragma unroll
+          for (int o = LPK >> 1; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+          if (j < c1 && sub == 0) sc[j - c0] = dot * scale;
+        }
       }
-    }
-    *reinterpret_cast<float4 *>(o_part + vr * DH + vq * 4) = o;
-    __syncthreads();
-    float t = 0.f;
-    if (tid < DH) {
-      t = o_part[tid];
+      __syncthreads();
+      const int nk = c1 - c0;
+      for (int i = tid; i < nk; i += 128) m = fmaxf(m, sc[i]);
 #pragma unroll
-      for (int q = 1; q < VPI; ++q) t += o_part[q * DH + tid];
+      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if (lane == 0) red_f[wid] = m;
+      __syncthreads();
+      m = fmaxf(fmaxf(red_f[0], red_f[1]), fmaxf(red_f[2], red_f[3]));
+      for (int i = tid; i < nk; i += 128) {
+        const float e = expf(sc[i] - m);
+        sc[i] = e;
+        l += (double)e;
+      }
+      l = warp_sum_d(l);
+      if (lane == 0) red_d[wid] = l;
+      __syncthreads();
+      l = ((red_d[0] + red_d[1]) + red_d[2]) + red_d[3];
+      // second product: thread -> (four columns of the head, every VPI-th key)
+      const int vr = tid / VPR, vq = tid % VPR;
+      float4 o = zero4;
+      const float *vp = vc + ((long long)b * cap + c0) * d_model + h * DH + vq * 4;
+      for (int i0 = vr; i0 < nk; i0 += DEC_UNROLL * VPI) {
+        float4 v[DEC_UNROLL];
+#pragma unroll
+        for (int u = 0; u < DEC_UNROLL; ++u) {
+          const int i = i0 + u * VPI;
+          v[u] = i < nk ? *reinterpret_cast<const float4 *>(vp + (long long)i * d_model) : zero4;
+        }
+#pragma unroll
+        for (int u = 0; u < DEC_UNROLL; ++u) {
+          const int i = i0 + u * VPI;
+          const float e = i < nk ? sc[i] : 0.f;
+          o.x = fmaf(e, v[u].x, o.x);
+          o.y = fmaf(e, v[u].y, o.y);
+          o.z = fmaf(e, v[u].z, o.z);
+          o.w = fmaf(e, v[u].w, o.w);
+        }
+      }
+      *reinterpret_cast<float4 *>(o_part + vr * DH + vq * 4) = o;
+      __syncthreads();
+      if (tid < DH) {
+        t = o_part[tid];
+#pragma unroll
+        for (int q = 1; q < VPI; ++q) t += o_part[q * DH + tid];
+      }
     }
     if (out == nullptr) {
       store_context<DH>(ctx, t * (float)(1.0 / l), b, h, d_model, tid, red_f);
