@@ -16,8 +16,9 @@
 //
 // Greedy runs of small vocabularies go through all their tokens in one launch (small_loop_supports): the CTA that has the last row
 // finishes it (final norm, head out of shared memory, first maximum; output_head.cpp:58-70, inference.cpp:188-198) and a barrier
-// of the stream's cluster hands the token on; every token still computes its whole context. Two layers of width 64, one stream, contexts of 6 to 63: 47 us a token with a
-// launch for the body and one for the tail, replayed from a graph, 37 in one launch.
+// of the stream's cluster hands the token on; every token still computes its whole context. Two layers of width 64, one
+// stream, contexts of 6 to 63: 47 us a token with a launch for the body and one for the tail, replayed from a graph, 37 in
+// one launch. (RUN: such a run; the body of one step is compiled without what only a run needs, which cost it 1 %.)
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
@@ -167,6 +168,7 @@ __device__ __forceinline__ void sb_attention(const float *qr, const float *ks, i
 
 // offsets: [layers][12] byte offsets into params: ln1_g, ln1_b, qkv_w, qkv_b, out_w, out_b, ln2_g, ln2_b, w1, b1, w2,
 // b2; then tok_emb, pos_emb. kv: [2][streams][s_cap][2 d]. x: [streams * s][d], rows as the other kernels pack them.
+template <bool RUN>
 __global__ void __launch_bounds__(SB_THREADS)
 small_body_kernel(SmallShape g, SmallRun run, const char *__restrict__ params, const unsigned long long *__restrict__ offsets, const int *ids,
                   int ids_ld, const LoopState *state, float *kv, float *x_out, DevErr *err) {
@@ -189,7 +191,7 @@ small_body_kernel(SmallShape g, SmallRun run, const char *__restrict__ params, c
   float *vecs = vs + g.s_cap * D;                   // [2][9 D + F] a layer's vectors: LayerNorms and biases
   const int nvec = 9 * D + F;
   float *tail = vecs + 2 * nvec;                    // of a run: final norm [2][D], head [D][vocab]
-  unsigned long long *offs = reinterpret_cast<unsigned long long *>(tail + (run.steps ? D * (g.vocab + 2) : 0));  // the table of offsets
+  unsigned long long *offs = reinterpret_cast<unsigned long long *>(tail + (RUN ? D * (g.vocab + 2) : 0));  // the table of offsets
   auto P = [&](int l, int i) { return reinterpret_cast<const float *>(params + offs[l * 12 + i]); };
   enum { LN1G, LN1B, QKVW, QKVB, OUTW, OUTB, LN2G, LN2B, W1, B1, W2, B2 };
   auto weight_of = [](int op) { return op == 0 ? (int)QKVW : op == 1 ? (int)OUTW : op == 2 ? (int)W1 : (int)W2; };
@@ -223,7 +225,7 @@ small_body_kernel(SmallShape g, SmallRun run, const char *__restrict__ params, c
   wt.request(P(0, QKVW), cut[0]);
   request_vectors(0);  // (all of this never changes: before the wait)
   store_vectors(0);
-  if (run.steps) {
+  if constexpr (RUN) {
     const float *gamma = P(g.layers, 2), *beta = P(g.layers, 3), *w = P(g.layers, 4);
     for (int c = tid; c < D; c += SB_THREADS) {
       tail[c] = __ldg(gamma + c);
@@ -234,9 +236,9 @@ small_body_kernel(SmallShape g, SmallRun run, const char *__restrict__ params, c
   pdl_wait();
   int turn = 0;  // of the two buffers, for keys and values and for a layer's vectors
 #pragma unroll 1
-  for (int step = 0; step == 0 || step < run.steps; ++step) {
-  const bool another = step + 1 < run.steps;
-  const int s = run.steps ? run.s0 + step : state ? state->s : g.s_cap;
+  for (int step = 0; step < (RUN ? run.steps : 1); ++step) {
+  const bool another = RUN && step + 1 < run.steps;
+  const int s = RUN ? run.s0 + step : state ? state->s : g.s_cap;
   const int blocks = (s + SB_ROWS - 1) / SB_ROWS;
   const int mine = blocks > me ? (blocks - me + SB_CTAS - 1) / SB_CTAS : 0;
   auto row_of = [&](int j, int r) { return (j * SB_CTAS + me) * SB_ROWS + r; };
@@ -246,7 +248,7 @@ small_body_kernel(SmallShape g, SmallRun run, const char *__restrict__ params, c
     const int i = e / D, c = e - i * D, t = row_of(i / SB_ROWS, i % SB_ROWS);
     float v = 0.f;
     if (t < s) {
-      int id = __ldcg(ids + (long long)b * ids_ld + t);
+      int id = RUN ? __ldcg(ids + (long long)b * ids_ld + t) : ids[(long long)b * ids_ld + t];
       if (id < 0 || id >= g.vocab) {
         if (c == 0) {
           err->code = DEVERR_BAD_TOKEN_ID;
@@ -388,13 +390,13 @@ small_body_kernel(SmallShape g, SmallRun run, const char *__restrict__ params, c
       __syncthreads();
     }
   }
-  if (run.steps == 0) {
+  if constexpr (!RUN) {
     for (int e = tid; e < mine * SB_ROWS * D; e += SB_THREADS) {
       const int i = e / D, t = row_of(i / SB_ROWS, i % SB_ROWS);
       if (t < s) x_out[((long long)b * s + t) * D + (e - i * D)] = x[e];
     }
-    return;
   }
+  if constexpr (RUN) {
   // ---- the last row's token: a strict '>' scan from index 0 ----
   if (me == (blocks - 1) % SB_CTAS) {
     const int V = g.vocab, r = (s - 1) % SB_ROWS;
@@ -454,7 +456,8 @@ small_body_kernel(SmallShape g, SmallRun run, const char *__restrict__ params, c
   __syncthreads();
   cluster_sync_all();  // the token is there for every CTA of the stream
   }
-  if (b == 0 && me == 0 && tid == 0) {
+  }
+  if (RUN && b == 0 && me == 0 && tid == 0) {
     run.state->s = run.s0 + run.steps;
     run.state->step = run.step0 + run.steps;
   }
@@ -470,9 +473,9 @@ size_t small_smem(int layers, int d, int f, int s) {
 void small_launch(const SmallShape &g, const SmallRun &run, const char *params, const unsigned long long *offsets, const int *ids,
                   int ids_ld, const LoopState *state, float *kv, float *x, DevErr *err, cudaStream_t st) {
   const size_t smem = small_smem(g.layers, g.d, g.f, g.s_cap) + (run.steps ? (size_t)4 * g.d * (g.vocab + 2) : 0);
-  if (smem > 48 * 1024)
-    LB_CUDA(cudaFuncSetAttribute(small_body_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  launch_pdl_cluster_x(small_body_kernel, dim3(SB_CTAS, (unsigned)g.streams), dim3(SB_THREADS), smem, st, g_pdl_enabled,
+  auto kernel = run.steps ? small_body_kernel<true> : small_body_kernel<false>;
+  if (smem > 48 * 1024) LB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  launch_pdl_cluster_x(kernel, dim3(SB_CTAS, (unsigned)g.streams), dim3(SB_THREADS), smem, st, g_pdl_enabled,
                        (unsigned)SB_CTAS, g, run, params, offsets, ids, ids_ld, state, kv, x, err);
 }
 
