@@ -194,6 +194,23 @@ __device__ __forceinline__ void f16_store_block(float4 v, bool active, __half *h
   }
 }
 
+// few_row_pair.cu: products of up to 64 fp32 rows [rows, k] on a weight's fp16 pair, fp32 rows out. ln_u != nullptr: the folded
+// LayerNorm of the row comes first, bias is then v[n]. n a multiple of 16, k of 64.
+struct FewRowPairProduct {
+  const float *x = nullptr;
+  const __half *w_hi = nullptr, *w_lo = nullptr;  // [n, k]
+  const float *w_inv = nullptr;                   // device: the inverse of the matrix's scale
+  const float *bias = nullptr, *ln_u = nullptr, *residual = nullptr;
+  float *out = nullptr;
+  // [rows, k / 16] sums and sums of squares of 16 columns of x each, as a product that made x left them in its sums_out (of out);
+  // without them a folded LayerNorm takes its own
+  const double2 *sums_in = nullptr;
+  double2 *sums_out = nullptr;
+  int n = 0, k = 0, relu = 0;
+};
+bool few_row_pair_supports(int rows, int n, int k);
+void launch_few_row_pair(const FewRowPairProduct &p, int rows, cudaStream_t st);
+
 // attention_tc.cu: fused causal attention on the tensor cores for head
 // dimension 64. qk: maps (box 128 rows x 32) over the split [rows, 3*d_model]
 // output of the QKV projection; vt: maps (box 64 rows x 32) over the split V^T

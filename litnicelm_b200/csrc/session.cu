@@ -578,6 +578,43 @@ void enqueue_body(litnice_b200_session *s, int B, int sl, const LoopState *dstat
     return;
   }
   const size_t cache_layer = (size_t)s->kv_streams * s->kv_cap * D;
+  // Few rows and k that one span a warp covers: on the weights' pairs, everything between the products in fp32 (beyond, the tiles of
+  // gemm_tc.cu are as fast or faster: 64 rows, n 3072 k 1024 take 20 us on the pairs). 512 / 16 sums a row fit row_stats.
+  if (newest && s->f16 && D <= 512 && few_row_pair_supports(B, D, D) && few_row_pair_supports(B, F, D)) {
+    launch_embed_last_ln(P(s, s->lay.tok_emb), P(s, s->lay.pos_emb), s->ids, d.max_seq_len, dstate, sl, B, D, d.vocab_size,
+                         P(s, s->lay.layer[0].ln1_g), P(s, s->lay.layer[0].ln1_b), s->x, nullptr, s->err_dev, s->st);
+    ++s->launches;
+    auto product = [&](const TcWeight &w, const float *x, const float *bias, const float *u, const float *residual, int relu, float *out,
+                       const double2 *sums_in, double2 *sums_out) {
+      FewRowPairProduct p;
+      p.x = x;
+      p.w_hi = w.h_hi;
+      p.w_lo = w.h_lo;
+      p.w_inv = w.h_inv_scale;
+      p.bias = bias;
+      p.ln_u = u;
+      p.residual = residual;
+      p.out = out;
+      p.sums_in = sums_in;
+      p.sums_out = sums_out;
+      p.n = w.n;
+      p.k = w.k;
+      p.relu = relu;
+      launch_few_row_pair(p, B, s->st);
+      ++s->launches;
+    };
+    for (int l = 0; l < d.n_layers; ++l) {
+      const LayerOff &o = s->lay.layer[l];
+      const std::array<TcWeight, 4> &w = s->tcw[l];
+      product(w[0], s->x, w[0].ln_v, w[0].ln_u, nullptr, 0, s->dqkv, l > 0 ? s->row_stats : nullptr, nullptr);
+      s->launches += launch_attn_decode(s->dqkv, s->kcache + l * cache_layer, s->vcache + l * cache_layer, s->kv_cap, D, d.n_heads, B,
+                                        dstate, sl, s->dec_part, s->dec_counters, s->dctx, s->st);
+      product(w[1], s->dctx, P(s, o.out_b), nullptr, s->x, 0, s->y, nullptr, s->row_stats);
+      product(w[2], s->y, w[2].ln_v, w[2].ln_u, nullptr, 1, s->dh, s->row_stats, nullptr);
+      product(w[3], s->dh, P(s, o.b2), nullptr, s->y, 0, s->x, nullptr, s->row_stats);
+    }
+    return;
+  }
   // With the LayerNorms folded into the QKV and W1 products, the kernels that
   // produce x and y also store them as TF32 pairs in (ln, ln_lo) with per-row
   // partial sums in row_stats, and no LayerNorm kernel runs in the layers.
@@ -797,8 +834,8 @@ void decode_projection(litnice_b200_session *s, const float *a, int B, int k, co
 void enqueue_decode_step(litnice_b200_session *s, int B, int sl, const LoopState *dstate, bool with_head) {
   const litnice_b200_dims &d = s->dims;
   const int D = d.d_model, F = d.d_ff, V = d.vocab_size;
-  // Beyond the few-row products' 8 rows: 64 streams at 6 layers of width 512 take 0.33 ms a step here
-  // (a product 10 us), 1.77 ms on the fp32 tile kernel (55 us: few tiles, a serial k loop).
+  // Beyond the few-row products' 8 rows: 64 streams at 6 layers of width 512 take 0.27 ms a step here, 1.77 ms on the fp32 tile
+  // kernel (55 us a product: few tiles, a serial k loop).
   if (s->tc && B > 8) {
     enqueue_body(s, B, sl, dstate, true);
     if (with_head) enqueue_head_last(s, B, 1);

@@ -272,3 +272,32 @@ def test_resident_steps(dims, streams, prompt, new):
         want = logits_64(d, arena, np.concatenate([prompts[1], alone[:-1]]))[prompt - 1:]
         srt = np.sort(want, axis=1)
         agreed_prefix(alone, want.argmax(1), srt[:, -1] - srt[:, -2])
+
+
+# Up to 64 rows a step on the weights' pairs: tiles of rows that are not full, one, two and four of them a CTA, one span of k for a
+# part of the warps, for all of them and several; past 64 rows and past width 512 the tiles of the large products.
+@pytest.mark.parametrize("dims,streams,prompt,new", [
+    ((2, 1, 64, 64, 30, 60), 9, 20, 5),
+    ((2, 3, 192, 576, 50, 60), 23, 30, 4),
+    ((2, 8, 512, 2048, 96, 70), 64, 40, 4),
+    ((1, 8, 512, 512, 40, 70), 41, 20, 4),
+    ((1, 4, 256, 1024, 40, 70), 65, 20, 3),
+    ((1, 10, 640, 1280, 40, 60), 12, 20, 3),
+])
+def test_steps_of_tens_of_rows(dims, streams, prompt, new):
+    d = formats.ModelDims(*dims)
+    arena = formats.make_param_arena(d, 7, bias_std=0.02, ln_std=0.1)
+    prompts = np.stack([formats.zipf_prompt(d.vocab, prompt, 70 + i) for i in range(streams)])
+    with Session(d, streams) as s:
+        s.load_params(arena)
+        fast = s.generate(prompts, new)
+        s.keep_step_logits(True)
+        toks = s.generate(prompts, new)
+        lg = s.read_step_logits(new, streams)
+    for b in sorted({0, 7, 8, streams // 2, streams - 1}):
+        want = logits_64(d, arena, np.concatenate([prompts[b], toks[b][:-1]]))[prompt - 1:]
+        # operands of 22 bits, sums of at most 2048 terms in fp32: as above
+        assert rel_err(lg[:, b], want) < 2e-5
+        same = np.flatnonzero(fast[b] != toks[b])
+        srt = np.sort(want, axis=1)
+        assert not len(same) or srt[same[0], -1] - srt[same[0], -2] < NEAR_TIE
