@@ -309,7 +309,7 @@ void launch_bn(const Bf16Product &p, int m, cudaStream_t st, DevErr *err) {
   const int mt = (m + TC_BM - 1) / TC_BM, nt = (p.n + BN - 1) / BN;
   const long long tiles = (long long)mt * nt;
   const unsigned grid = (unsigned)(tiles < device_sms() ? tiles : device_sms());
-  launch_pdl(gemm_bf16_kernel<BN, GATED>, dim3(grid), dim3(GB_THREADS), L::TOTAL, st, false, ma, mw, mh, mf, half_tma ? 1 : 0,
+  launch_pdl(gemm_bf16_kernel<BN, GATED>, dim3(grid), dim3(GB_THREADS), L::TOTAL, st, g_pdl_enabled, ma, mw, mh, mf, half_tma ? 1 : 0,
              float_tma ? 1 : 0, p, m, mt, nt, err);
 }
 

@@ -309,7 +309,7 @@ void lp_launch(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &
   const size_t smem = lp_smem(a.dim, a.vdim, V_ROWS);
   LB_CUDA(cudaFuncSetAttribute(prefill_attention_kernel<V_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   launch_pdl(prefill_attention_kernel<V_ROWS>, dim3((unsigned)((a.n + LP_BQ - 1) / LP_BQ), (unsigned)heads, (unsigned)streams),
-             dim3(LP_THREADS), smem, st, false, mq, mk, mv, a, err);
+             dim3(LP_THREADS), smem, st, g_pdl_enabled, mq, mk, mv, a, err);
 }
 
 }  // namespace
