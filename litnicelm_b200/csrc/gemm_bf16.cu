@@ -12,9 +12,16 @@
 // padded patch, residuals read back inside it: about 12 us a tile of 128 x 256 whatever the activation, against 1 us of
 // products at k = 256 and 4 us at k = 1024. Prompts of 4 x 2048 tokens through six Mitilix layers of width 1024, 30 of these
 // products: 3.06 ms a pass before, 1.97 ms with eight warps and TMA stores.
+// Long k is bound by shared memory too: an instruction of 128 x 256 reads 384 operand rows of its SM for 128 x 256 products a k.
+// A pair of CTAs (cta_group::2) takes tiles of 256 x 256 instead, each CTA loading its 128 rows of A and 128 of W's 256, two
+// thirds of the operand bytes, with six stages in place of four; each stores its own 128 rows. The even CTA issues the
+// instructions of both and owns the barriers they wait on; commits arrive in both. Where activations make the store the longer
+// part, sixteen warps store. Mitilix 4 x 2048 (above) 1.897 -> 1.801 ms, Gobesun 4 x 2047 2.571 -> 2.471 ms.
+// A launch may begin while its predecessor ends (its dependents are let go behind the allocation of tensor memory, so a CTA
+// never waits for tensor memory that a later launch holds).
 // Rows and columns outside the operands load as zeros (k need not be a multiple of 64) and are not
 // stored. Every mbarrier wait is bounded; a wait that runs out sets the error word and ends the kernel
-// after its copies have landed and tensor memory is freed. No clusters, no multicast.
+// after its copies have landed and tensor memory is freed. No load is multicast.
 #include "activation.cuh"
 #include "model.cuh"
 #include "gemm_tc.cuh"
@@ -30,29 +37,55 @@ namespace {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int GB_STORE_WARPS = 8;
-constexpr int GB_THREADS = 64 + 32 * GB_STORE_WARPS;
 constexpr int GB_PATCH = 32 * 32 * 4;  // a warp's staging patch: 32 rows of 32 floats, or two buffers of 32 rows of 32 bfloat16
 constexpr int GB_GROUP = 16;     // row tiles that share a sweep over the columns (W tiles stay in L2)
 
-template <int BN>
+template <int BN, bool PAIR, int WARPS>
 struct GbSmem {
-  static constexpr int STAGES = BN == 256 ? 4 : BN == 128 ? 6 : 8;
+  static constexpr int THREADS = 64 + 32 * WARPS;
+  static constexpr int STAGES = PAIR ? (WARPS == 8 ? 6 : 5) : BN == 256 ? 4 : BN == 128 ? 6 : 8;
   static constexpr int A_BYTES = TC_BM * 128;
-  static constexpr int B_BYTES = BN * 128;
+  static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * 128;
   static constexpr int STAGE = A_BYTES + B_BYTES;
   static constexpr int PATCH_OFF = STAGES * STAGE;
-  static constexpr int BAR_OFF = PATCH_OFF + GB_STORE_WARPS * GB_PATCH;
+  static constexpr int BAR_OFF = PATCH_OFF + WARPS * GB_PATCH;
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
-template <int BN, int GATED>
-__global__ void __launch_bounds__(GB_THREADS, 1)
+// Instructions of a pair of CTAs (cta_group::2): the even one's thread issues them for both, operands at the same places of both
+// shared memories, rows 128 .. 255 of the result in the odd one's tensor memory.
+__device__ __forceinline__ void gb_pair_load(unsigned dst, const CUtensorMap *map, int x, int y, unsigned leader_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(leader_bar)
+      : "memory");
+}
+__device__ __forceinline__ void gb_pair_mma(unsigned d, unsigned long long a, unsigned long long b, unsigned idesc,
+                                            unsigned accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void gb_pair_commit(unsigned bar) {  // the barrier at this place in both CTAs
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"((unsigned short)3)
+               : "memory");
+}
+__device__ __forceinline__ void gb_arrive_cluster(unsigned cluster_bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+
+template <int BN, int GATED, bool PAIR, int WARPS>
+__global__ void __launch_bounds__(64 + 32 * WARPS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                  const __grid_constant__ CUtensorMap map_half, const __grid_constant__ CUtensorMap map_float, int half_tma,
                  int float_tma, const __grid_constant__ Bf16Product p, int m, int m_tiles, int n_tiles, DevErr *err) {
-  using L = GbSmem<BN>;
-  constexpr int S = L::STAGES;
+  using L = GbSmem<BN, PAIR, WARPS>;
+  constexpr int S = L::STAGES, CTAS = PAIR ? 2 : 1, GROUP = GB_GROUP / CTAS;  // m_tiles counts tiles of CTAS * 128 rows
+  const int rank = PAIR ? (int)blockIdx.x & 1 : 0, cta = (int)blockIdx.x / CTAS, ctas = (int)gridDim.x / CTAS;
   extern __shared__ unsigned char smem_raw[];
   const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char *base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -66,10 +99,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles = m_tiles * n_tiles, kblocks = (p.k + 63) / 64;
   auto place = [&](int tile, int &m0, int &n0) {
-    const int per = GB_GROUP * n_tiles, grp = tile / per, rest = tile - grp * per;
-    const int gm = min(GB_GROUP, m_tiles - grp * GB_GROUP);
+    const int per = GROUP * n_tiles, grp = tile / per, rest = tile - grp * per;
+    const int gm = min(GROUP, m_tiles - grp * GROUP);
     n0 = rest / gm * BN;
-    m0 = (grp * GB_GROUP + rest % gm) * TC_BM;
+    m0 = ((grp * GROUP + rest % gm) * CTAS + rank) * TC_BM;
   };
 
   if (threadIdx.x == 0) {
@@ -79,29 +112,41 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull(b), 1);
-      mbar_init(tempty(b), GB_STORE_WARPS);
+      mbar_init(tempty(b), CTAS * WARPS);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void *)tmem_holder)),
-                 "r"((unsigned)(2 * BN))
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void *)tmem_holder)),
+                   "r"((unsigned)(2 * BN))
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void *)tmem_holder)),
+                   "r"((unsigned)(2 * BN))
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();  // both CTAs' barriers are there
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const unsigned tmem = *tmem_holder;
   pdl_launch_dependents();  // behind the allocation: a dependent's CTA must not take tensor memory first
   pdl_wait();
 
+  auto commit = [](unsigned bar) {
+    if constexpr (PAIR) gb_pair_commit(bar);
+    else tc_commit(bar);
+  };
   if (warp == 0) {
     int it = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+    for (int tile = cta; tile < tiles && ok; tile += ctas) {
       int m0, n0;
       place(tile, m0, n0);
       for (int kb = 0; kb < kblocks; ++kb, ++it) {
@@ -111,14 +156,25 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         if (!ok) break;
         if (lane == 0) {
           const unsigned st = base + (unsigned)(s * L::STAGE);
-          mbar_expect_tx(full(s), (unsigned)L::STAGE);
-          tma_load_2d(st, &map_a, kb * 64, m0, full(s));
-          tma_load_2d(st + L::A_BYTES, &map_w, kb * 64, n0, full(s));
+          if constexpr (PAIR) {  // this CTA's rows of A and half of W's; the even one's barrier counts both CTAs' bytes
+            if (rank == 0) mbar_expect_tx(full(s), 2u * (unsigned)L::STAGE);
+            const unsigned bar = cluster_map(full(s), 0);
+            gb_pair_load(st, &map_a, kb * 64, m0, bar);
+            gb_pair_load(st + L::A_BYTES, &map_w, kb * 64, n0 + rank * (BN / 2), bar);
+          } else {
+            mbar_expect_tx(full(s), (unsigned)L::STAGE);
+            tma_load_2d(st, &map_a, kb * 64, m0, full(s));
+            tma_load_2d(st + L::A_BYTES, &map_w, kb * 64, n0, full(s));
+          }
         }
         __syncwarp();
       }
     }
-    if (*abort_flag) {  // copies in flight must land before the shared memory goes away
+    if (PAIR && *abort_flag) {  // copies in flight must land (only the even CTA's barriers know: a millisecond is ample)
+      const unsigned long long t0 = global_timer();
+      while (global_timer() - t0 < 1000000ull) {
+      }
+    } else if (*abort_flag) {  // copies in flight must land before the shared memory goes away
       for (int j = it > S ? it - S : 0; j < it; ++j) {
         const unsigned long long t0 = global_timer();
         while (!mbar_try_wait(full(j % S), (unsigned)(j / S) & 1u))
@@ -126,10 +182,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    constexpr unsigned idesc = umma_idesc_bf16(BN);
+    constexpr unsigned idesc = umma_idesc_bf16(BN) + (PAIR ? (unsigned)(TC_BM >> 4) << 24 : 0u);  // 256 rows of a pair
     int it = 0, use = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++use) {
+    for (int tile = rank == 0 ? cta : tiles; tile < tiles && ok; tile += ctas, ++use) {
       const int buf = use & 1;
       ok = mbar_wait(tempty(buf), ((unsigned)(use >> 1) & 1u) ^ 1u, abort_flag, err, 12);
       __syncwarp();
@@ -145,30 +201,33 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           const unsigned st = base + (unsigned)(s * L::STAGE);
           const unsigned long long da = umma_desc_k128(st), db = umma_desc_k128(st + L::A_BYTES);
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            tc_mma_f16(tmem + (unsigned)(buf * BN), da + (unsigned long long)(ks * 2), db + (unsigned long long)(ks * 2), idesc,
-                       (kb | ks) ? 1u : 0u);
-          tc_commit(empty(s));
+          for (int ks = 0; ks < 4; ++ks) {
+            const unsigned d = tmem + (unsigned)(buf * BN), more = (kb | ks) ? 1u : 0u;
+            if constexpr (PAIR) gb_pair_mma(d, da + (unsigned long long)(ks * 2), db + (unsigned long long)(ks * 2), idesc, more);
+            else tc_mma_f16(d, da + (unsigned long long)(ks * 2), db + (unsigned long long)(ks * 2), idesc, more);
+          }
+          commit(empty(s));
         }
         __syncwarp();
       }
-      if (ok && lane == 0) tc_commit(tfull(buf));
+      if (ok && lane == 0) commit(tfull(buf));
       __syncwarp();
     }
     if (!ok) {  // give the tensor pipe a bounded chance to finish before tensor memory is freed
       const unsigned long long t0 = global_timer();
-      if (lane == 0) tc_commit(tfull(use & 1));
+      if (lane == 0) commit(tfull(use & 1));
       __syncwarp();
       while (!mbar_try_wait(tfull(use & 1), (unsigned)(use >> 1) & 1u))
         if (global_timer() - t0 > WAIT_LIMIT_NS) break;
     }
   } else {
+    constexpr int COLS = BN / (WARPS / 4);
     const int q = warp & 3, part = (warp - 2) >> 2;  // lanes of tensor memory, share of the columns
     unsigned char *patch = base_ptr + L::PATCH_OFF + (warp - 2) * GB_PATCH;
     const unsigned patch_u = base + (unsigned)(L::PATCH_OFF + (warp - 2) * GB_PATCH);
     int use = 0, turn = 0;
     bool wide = false;  // the last store read the whole patch
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++use) {
+    for (int tile = cta; tile < tiles; tile += ctas, ++use) {
       const int buf = use & 1;
       if (!mbar_wait_warp(tfull(buf), (unsigned)(use >> 1) & 1u, abort_flag, err, 14)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -176,14 +235,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       place(tile, m0, n0);
       const int row0 = m0 + q * 32;
 #pragma unroll 1
-      for (int c0 = part * (BN / 2); c0 < (part + 1) * (BN / 2); c0 += 32) {
+      for (int c0 = part * COLS; c0 < (part + 1) * COLS; c0 += 32) {
         unsigned r[32];
         tc_ld32(tmem + ((unsigned)(q * 32) << 16) + (unsigned)(buf * BN + c0), r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (c0 + 32 == (part + 1) * (BN / 2)) {
+        if (c0 + 32 == (part + 1) * COLS) {
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
-          if (lane == 0) mbar_arrive(tempty(buf));
+          if (lane == 0) {
+            if constexpr (PAIR) gb_arrive_cluster(cluster_map(tempty(buf), 0));
+            else mbar_arrive(tempty(buf));
+          }
         }
         const int col = n0 + c0;
         if (col >= p.n || row0 >= m) continue;
@@ -274,9 +336,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();  // nothing of the pair's is on its way to the other CTA
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((unsigned)(2 * BN)));
+    if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((unsigned)(2 * BN)));
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((unsigned)(2 * BN)));
   }
 }
 
@@ -291,12 +355,12 @@ int device_sms() {
   return n;
 }
 
-template <int BN, int GATED>
+template <int BN, int GATED, bool PAIR, int WARPS>
 void launch_bn(const Bf16Product &p, int m, cudaStream_t st, DevErr *err) {
-  using L = GbSmem<BN>;
+  using L = GbSmem<BN, PAIR, WARPS>;
   CUtensorMap ma, mw, mh{}, mf{};
   tc_make_map_bf16(&ma, p.a, (unsigned long long)m, (unsigned long long)p.k, (unsigned long long)p.a_ld, TC_BM);
-  tc_make_map_bf16(&mw, p.w, (unsigned long long)p.n, (unsigned long long)p.k, (unsigned long long)p.w_ld, BN);
+  tc_make_map_bf16(&mw, p.w, (unsigned long long)p.n, (unsigned long long)p.k, (unsigned long long)p.w_ld, PAIR ? BN / 2 : BN);
   const int halves = GATED ? p.n_half / 2 : p.n_half, floats = p.n - p.n_half;
   const bool half_tma = halves > 0 && p.half_ld % 8 == 0 && (reinterpret_cast<uintptr_t>(p.half_out) & 15) == 0;
   const bool float_tma = floats > 0 && p.float_ld % 4 == 0 && p.n_half % 4 == 0 &&
@@ -305,18 +369,19 @@ void launch_bn(const Bf16Product &p, int m, cudaStream_t st, DevErr *err) {
                                   (unsigned long long)p.half_ld, GATED ? 16 : 32);
   if (float_tma) tc_make_store_map(&mf, p.float_out, false, (unsigned long long)m, (unsigned long long)floats,
                                    (unsigned long long)p.float_ld, 32);
-  LB_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<BN, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
-  const int mt = (m + TC_BM - 1) / TC_BM, nt = (p.n + BN - 1) / BN;
+  LB_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<BN, GATED, PAIR, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+  constexpr int CTAS = PAIR ? 2 : 1;
+  const int mt = (m + CTAS * TC_BM - 1) / (CTAS * TC_BM), nt = (p.n + BN - 1) / BN;
   const long long tiles = (long long)mt * nt;
-  const unsigned grid = (unsigned)(tiles < device_sms() ? tiles : device_sms());
-  launch_pdl(gemm_bf16_kernel<BN, GATED>, dim3(grid), dim3(GB_THREADS), L::TOTAL, st, g_pdl_enabled, ma, mw, mh, mf, half_tma ? 1 : 0,
-             float_tma ? 1 : 0, p, m, mt, nt, err);
+  const unsigned grid = CTAS * (unsigned)(tiles < device_sms() / CTAS ? tiles : device_sms() / CTAS);
+  launch_pdl_cluster_x(gemm_bf16_kernel<BN, GATED, PAIR, WARPS>, dim3(grid), dim3(L::THREADS), L::TOTAL, st, g_pdl_enabled,
+                       (unsigned)CTAS, ma, mw, mh, mf, half_tma ? 1 : 0, float_tma ? 1 : 0, p, m, mt, nt, err);
 }
 
-template <int BN>
+template <int BN, bool PAIR = false, int WARPS = 8>
 void launch_form(const Bf16Product &p, int m, cudaStream_t st, DevErr *err) {
-  if (p.gated) launch_bn<BN, 1>(p, m, st, err);
-  else launch_bn<BN, 0>(p, m, st, err);
+  if (p.gated) launch_bn<BN, 1, PAIR, WARPS>(p, m, st, err);
+  else launch_bn<BN, 0, PAIR, WARPS>(p, m, st, err);
 }
 
 }  // namespace
@@ -327,8 +392,17 @@ void launch_gemm_bf16(const Bf16Product &p, int m, cudaStream_t st, DevErr *err)
   // the widest tile that still gives most SMs one
   const long long mt = (m + TC_BM - 1) / TC_BM;
   const long long sms = device_sms();
-  if (p.n > 128 && mt * ((p.n + 255) / 256) >= sms * 3 / 4) launch_form<256>(p, m, st, err);
-  else if (p.n > 64 && mt * ((p.n + 127) / 128) >= sms * 3 / 4) launch_form<128>(p, m, st, err);
+  const long long nt = (p.n + 255) / 256, turns = (mt * nt + sms - 1) / sms, pair_turns = ((mt + 1) / 2 * nt + sms / 2 - 1) / (sms / 2);
+  if (p.n > 128 && mt * nt >= sms * 3 / 4) {
+    // A pair starts about 2 us later (its CTAs meet before and after) and then gains a share of each 64 k of each tile: 5 % at
+    // 6 tiles of 1024 k a CTA, 11 % at 2 of 5120, 17 % at 6 of 5120, against 4 to 8 % lost at 2 of 2048 and at one tile.
+    // With an activation, sixteen storing warps: without them a pair gains nothing (gated 8192 x 8192 x 1024: 90 us alone, 96 a
+    // pair with eight, 79 with sixteen; plain results prefer the sixth operand stage, 8192 x 1024 x 5120 74, 65 and 69).
+    const bool pair = turns >= 2 && turns * p.k >= 5120 && pair_turns <= turns;
+    if (pair && p.act != ACT_NONE && p.n_half > 0) launch_form<256, true, 16>(p, m, st, err);
+    else if (pair) launch_form<256, true>(p, m, st, err);
+    else launch_form<256>(p, m, st, err);
+  } else if (p.n > 64 && mt * ((p.n + 127) / 128) >= sms * 3 / 4) launch_form<128>(p, m, st, err);
   else launch_form<64>(p, m, st, err);
 }
 

@@ -87,6 +87,26 @@ def test_product_over_many_tiles_and_a_long_k():
         assert rms_rel(bf16_product_host(a, w, 1), a.astype(np.float64) @ w.T.astype(np.float64)) < 1e-4
 
 
+# tiles of pairs of CTAs: last pairs of which one CTA has no rows, or no columns to load, each way a tile is stored
+@pytest.mark.parametrize("m,n,k,n_half", [(1300, 3900, 2570, 3900), (1281, 4090, 2600, 2024), (2047, 3329, 2568, 0), (8190, 1030, 5128, 1030),
+                                          (4095, 3073, 1736, 1536)])
+@pytest.mark.parametrize("form", ["plain", "act", "gated"])
+def test_product_by_pairs(m, n, k, n_half, form):
+    rng = np.random.default_rng(m + n + k + n_half)
+    a, w = rounded(rng.standard_normal((m, k))), rounded(rng.standard_normal((n, k)) * k ** -0.5)
+    c = a.astype(np.float64) @ w.T.astype(np.float64)
+    act = om.gelu_exact if form != "plain" else lambda x: x
+    first = act(c[:, :n_half])
+    if form == "gated":
+        first = act(c[:, 0:n_half:2]) * c[:, 1:n_half:2]
+    old = rng.standard_normal((m, first.shape[1] + n - n_half)).astype(np.float32)
+    got = bf16_product_host(a, w, 1, n_half=n_half, act=None if form == "plain" else "gelu", gated=form == "gated", c=old)
+    rest = c[:, n_half:] + old[:, first.shape[1]:]
+    # exact products, sums in 32 bits as above; bfloat16's half unit in the last place
+    assert n_half == 0 or np.abs(got[:, :first.shape[1]] - first).max() < 2 ** -8 * np.abs(first).max()
+    assert n_half == n or np.abs(got[:, first.shape[1]:] - rest).max() < 2e-5 * k ** 0.5
+
+
 @pytest.mark.parametrize("m,n,n_half", [(1000, 3600, 3600), (1000, 3600, 1808), (1000, 3601, 2008), (1025, 3590, 36),
                                         (2080, 1030, 0), (1999, 1040, 520)])
 @pytest.mark.parametrize("gated", [False, True])
