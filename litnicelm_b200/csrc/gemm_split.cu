@@ -89,69 +89,87 @@ __device__ __forceinline__ void gs_split(float x, __nv_bfloat16 (&part)[3]) {
 // the product, in range.
 __device__ __forceinline__ bool gs_no_parts(float x) { return (__float_as_uint(x) & 0x7fffffffu) >= 0x5f000000u; }
 
-// One tile of 32 rows x 64 k of one operand: read along whichever axis is contiguous, written as rows of k.
+// One tile of 64 rows x 64 k of one operand: read along whichever axis is contiguous, written as rows of k, 16 bytes of a part at a
+// time.
+constexpr int GS_SPLIT_ROWS = 32;
 __global__ void __launch_bounds__(256) split_operands_kernel(const __grid_constant__ GsArgs g, int a_blocks) {
-  __shared__ float tile[32][65];
+  __shared__ float tile[GS_SPLIT_ROWS][65];
   pdl_launch_dependents();
   pdl_wait();
   const bool first = (int)blockIdx.x < a_blocks;
   const GsOperand &o = first ? g.a : g.b;
-  const int k_tiles = (g.kp + 63) / 64, r_tiles = (o.n + 31) / 32;
+  const int k_tiles = (g.kp + 63) / 64, r_tiles = (o.n + GS_SPLIT_ROWS - 1) / GS_SPLIT_ROWS;
   int at = (int)blockIdx.x - (first ? 0 : a_blocks);
   const int k0 = at % k_tiles * 64;
   at /= k_tiles;
-  const int r0 = at % r_tiles * 32, batch = at / r_tiles, tid = threadIdx.x;
+  const int r0 = at % r_tiles * GS_SPLIT_ROWS, batch = at / r_tiles, tid = threadIdx.x;
   const float *src = reinterpret_cast<const float *>(reinterpret_cast<const char *>(o.p) + batch_offset(o.view, batch));
   const long long ld = (long long)g.kp * g.sums;
   const long long to0 = g.sums > 1 ? (long long)batch * g.kp : (long long)batch * o.n * ld;
-  float4 x[2];
-  const int piece = tid & 15, k = k0 + piece * 4;
+  constexpr int N = GS_SPLIT_ROWS / 32;  // rows of a thread, 8 k of each
+  float x[N][8];
+  const int row = tid >> 3, k = k0 + (tid & 7) * 8;
   if (o.vec && o.k == 1) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int r = r0 + (tid >> 4) + i * 16;
-      x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (r < o.n) {
-        const float *p = src + (long long)r * o.outer + k;
-        if (k + 4 <= g.k) {
-          x[i] = *reinterpret_cast<const float4 *>(p);
-        } else {
-          if (k < g.k) x[i].x = p[0];
-          if (k + 1 < g.k) x[i].y = p[1];
-          if (k + 2 < g.k) x[i].z = p[2];
+    for (int i = 0; i < N; ++i) {
+      const int r = r0 + row + i * 32;
+      const float *p = src + (long long)r * o.outer + k;
+#pragma unroll
+      for (int h = 0; h < 8; h += 4) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < o.n) {
+          if (k + h + 4 <= g.k) {
+            v = *reinterpret_cast<const float4 *>(p + h);
+          } else {
+            if (k + h < g.k) v.x = p[h];
+            if (k + h + 1 < g.k) v.y = p[h + 1];
+            if (k + h + 2 < g.k) v.z = p[h + 2];
+          }
         }
+        x[i][h] = v.x; x[i][h + 1] = v.y; x[i][h + 2] = v.z; x[i][h + 3] = v.w;
       }
     }
   } else {
+    const bool along_k = o.k == 1;
+    float t[GS_SPLIT_ROWS / 4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < GS_SPLIT_ROWS / 4; ++i) {
       const int e = tid + i * 256;
-      const int r = o.k == 1 ? e >> 6 : e & 31, kk = o.k == 1 ? e & 63 : e >> 5;
-      tile[r][kk] = r0 + r < o.n && k0 + kk < g.k ? src[(long long)(r0 + r) * o.outer + (long long)(k0 + kk) * o.k] : 0.f;
+      const int r = along_k ? e >> 6 : e % GS_SPLIT_ROWS, kk = along_k ? e & 63 : e / GS_SPLIT_ROWS;
+      t[i] = r0 + r < o.n && k0 + kk < g.k ? src[(long long)(r0 + r) * o.outer + (long long)(k0 + kk) * o.k] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < GS_SPLIT_ROWS / 4; ++i) {
+      const int e = tid + i * 256;
+      tile[along_k ? e >> 6 : e % GS_SPLIT_ROWS][along_k ? e & 63 : e / GS_SPLIT_ROWS] = t[i];
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float *p = &tile[(tid >> 4) + i * 16][piece * 4];
-      x[i] = make_float4(p[0], p[1], p[2], p[3]);
-    }
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[i][j] = tile[row + i * 32][(tid & 7) * 8 + j];
   }
   bool bad = false;
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int r = r0 + (tid >> 4) + i * 16;
-    if (r >= o.n || k >= g.kp) continue;
-    bad |= gs_no_parts(x[i].x) | gs_no_parts(x[i].y) | gs_no_parts(x[i].z) | gs_no_parts(x[i].w);
-    const float v[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
-    __nv_bfloat16 part[4][3];
+  for (int i = 0; i < N; ++i) {
+    const int r = r0 + row + i * 32;
+    if (r >= o.n) continue;
+    __nv_bfloat16 part[8][3];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) gs_split(v[j], part[j]);
+    for (int j = 0; j < 8; ++j) {
+      bad |= gs_no_parts(x[i][j]);
+      gs_split(x[i][j], part[j]);
+    }
     const long long to = to0 + (long long)r * ld + k;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      const __nv_bfloat162 lo{part[0][q], part[1][q]}, hi{part[2][q], part[3][q]};
-      *reinterpret_cast<uint2 *>(o.part + q * o.each + to) =
-          make_uint2(*reinterpret_cast<const unsigned *>(&lo), *reinterpret_cast<const unsigned *>(&hi));
+      unsigned w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const __nv_bfloat162 two{part[2 * j][q], part[2 * j + 1][q]};
+        w[j] = *reinterpret_cast<const unsigned *>(&two);
+      }
+      *reinterpret_cast<uint4 *>(o.part + q * o.each + to) = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
   if (bad) *g.bad = 1;
@@ -653,7 +671,8 @@ void launch_gemm_split(MatView a, MatView b, MatView c, bool sum_batches, const 
   g.m_tiles = (g.m + GS_BM - 1) / GS_BM;
   g.n_tiles = (g.n + plan.bn - 1) / plan.bn;
   const long long k_tiles = (g.kp + 63) / 64;
-  const long long a_blocks = (g.m + 31) / 32 * k_tiles * g.a.batch, b_blocks = (g.n + 31) / 32 * k_tiles * g.b.batch;
+  const long long a_blocks = (g.m + GS_SPLIT_ROWS - 1) / GS_SPLIT_ROWS * k_tiles * g.a.batch;
+  const long long b_blocks = (g.n + GS_SPLIT_ROWS - 1) / GS_SPLIT_ROWS * k_tiles * g.b.batch;
   launch_pdl(split_operands_kernel, dim3((unsigned)(a_blocks + b_blocks)), dim3(256), 0, st, pdl, g, (int)a_blocks);
   if (plan.bn == 128) launch_tile<128>(g, pdl, st, err);
   else launch_tile<64>(g, pdl, st, err);
