@@ -226,10 +226,13 @@ __device__ __forceinline__ void store_cols(float *p, const float (&s)[VPT]) {
   else *p = s[0];
 }
 
+// Bound by the latency of its chain (state and history in, two barriers, state out), so as many CTAs as the SM holds: the compiler
+// takes 95 registers where it may, two CTAs an SM, and does without spills with 64, four. 64 streams of 8 heads of 64 x 64: 512 CTAs
+// in one wave instead of two, 10.6 -> 8.9 us.
 // WARPS warps share the state's rows, DPW each; a lane holds VPT value columns. The CTAs of a head are a
 // cluster (one CTA: none); the squares of its outputs meet in shared memory while each stores its part of the state.
 template <typename T, int WARPS, int DPW, int VPT>
-__global__ void __launch_bounds__(WARPS * 32, 512 / (WARPS * 32))
+__global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : DPW * VPT <= 16 ? 4 : DPW * VPT <= 32 ? 3 : 2)
 delta_step_kernel(StepArgs a, const T *in, T *history, T *out, DeltaRows g) {
   constexpr int THREADS = WARPS * 32, VT = 32 * VPT, DIMS = WARPS * DPW;
   constexpr int FILL = (2 * DIMS + VT + THREADS - 1) / THREADS;
