@@ -1,4 +1,5 @@
-// Cached mode, greedy, up to 8 streams: the whole token loop as ONE resident kernel.
+// Cached mode, greedy, up to 8 streams, models that decode_cluster.cu does not take: the whole token loop as ONE resident
+// kernel.
 //
 // The one-row steps of the cached mode are chains of small dependent operators
 // (per layer: LayerNorm + QKV product, attention over the cached keys,
