@@ -389,11 +389,15 @@ void launch_form(const Bf16Product &p, int m, cudaStream_t st, DevErr *err) {
 void launch_gemm_bf16(const Bf16Product &p, int m, cudaStream_t st, DevErr *err) {
   if (m < 1 || p.n < 1 || p.k < 1) throw std::invalid_argument("launch_gemm_bf16: empty product");
   if (p.gated && ((p.n_half | p.half_ld) & 1) != 0) throw std::invalid_argument("launch_gemm_bf16: a gated product needs pairs");
-  // the widest tile that still gives most SMs one
+  // The widest tile of which the next narrower would need a second turn: a turn costs about what its tile's k loop does, 1 : 0.6 :
+  // 0.4 from 256 to 64 columns. 2368 x 1024 (76 tiles of 256 columns), by 64, 128 and 256: k 512 12.4, 10.4, 8.6 us, k 5120 74, 51, 29;
+  // 613 x 2048 (80 of 128): k 512 10.4, 8.3, 8.4, k 5120 51, 29, 29; 613 x 1600 (65 of 128, 125 of 64): k 512 8.3 each, with GELU 8.3,
+  // 10.4, 12.5. Mitilix, 8 streams of 256 + 96 tokens: 31.51 ms with 256 columns from 111 tiles on (and so 128), 31.24.
   const long long mt = (m + TC_BM - 1) / TC_BM;
   const long long sms = device_sms();
-  const long long nt = (p.n + 255) / 256, turns = (mt * nt + sms - 1) / sms, pair_turns = ((mt + 1) / 2 * nt + sms / 2 - 1) / (sms / 2);
-  if (p.n > 128 && mt * nt >= sms * 3 / 4) {
+  const long long nt = (p.n + 255) / 256, turns = (mt * nt + sms - 1) / sms;
+  const long long pair_turns = ((mt + 1) / 2 * nt + sms / 2 - 1) / (sms / 2);
+  if (p.n > 128 && mt * ((p.n + 127) / 128) > sms) {
     // A pair starts about 2 us later (its CTAs meet before and after) and then gains a share of each 64 k of each tile: 5 % at
     // 6 tiles of 1024 k a CTA, 11 % at 2 of 5120, 17 % at 6 of 5120, against 4 to 8 % lost at 2 of 2048 and at one tile.
     // With an activation, sixteen storing warps: without them a pair gains nothing (gated 8192 x 8192 x 1024: 90 us alone, 96 a
@@ -402,7 +406,7 @@ void launch_gemm_bf16(const Bf16Product &p, int m, cudaStream_t st, DevErr *err)
     if (pair && p.act != ACT_NONE && p.n_half > 0) launch_form<256, true, 16>(p, m, st, err);
     else if (pair) launch_form<256, true>(p, m, st, err);
     else launch_form<256>(p, m, st, err);
-  } else if (p.n > 64 && mt * ((p.n + 127) / 128) >= sms * 3 / 4) launch_form<128>(p, m, st, err);
+  } else if (p.n > 64 && mt * ((p.n + 63) / 64) > sms) launch_form<128>(p, m, st, err);
   else launch_form<64>(p, m, st, err);
 }
 

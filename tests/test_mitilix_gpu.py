@@ -108,7 +108,7 @@ def test_product_by_pairs(m, n, k, n_half, form):
 
 
 @pytest.mark.parametrize("m,n,n_half", [(1000, 3600, 3600), (1000, 3600, 1808), (1000, 3601, 2008), (1025, 3590, 36),
-                                        (2080, 1030, 0), (1999, 1040, 520)])
+                                        (2080, 1030, 0), (1999, 1040, 520), (2350, 1020, 1020), (613, 1700, 800), (613, 2040, 1024)])
 @pytest.mark.parametrize("gated", [False, True])
 def test_product_stored_by_tile(m, n, n_half, gated):
     """Every way a tile's columns leave: bfloat16, pairs, floats stored and added, the border between them inside a group of
