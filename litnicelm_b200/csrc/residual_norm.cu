@@ -45,6 +45,11 @@ __device__ __forceinline__ float4 gain4(const RmsWeight &w, int c) {
   return make_float4(w.base + v.x, w.base + v.y, w.base + v.z, w.base + v.w);
 }
 __device__ __forceinline__ float squares(float4 v) { return v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; }
+// The same with the products fused into the sums as they are in residual_norm_kernel<T, 1>: left to the compiler, the order of x
+// and y was another one in the kernel for many rows.
+__device__ __forceinline__ float squares_fused(float4 v) {
+  return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, __fmul_rn(v.x, v.x))));
+}
 
 template <typename T, int PIECES>
 __global__ void __launch_bounds__(RN_THREADS)
@@ -112,10 +117,29 @@ residual_norm_rows_kernel(float *x, const float *y, RmsWeight after, T *h, int h
   __syncthreads();
   pdl_wait();
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto row_sum = [](float v) {
+  // A row's sum in the other kernel's order, its bits the same however many rows a call has: each piece over the lanes (which
+  // pass half of their pieces on as long as they have several; piece i ends in lane i * 32 / PIECES), then piece after piece.
+  auto row_sum = [lane](float (&u)[PIECES]) {
+    int held = PIECES;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    for (int o = 16; o > 0; o >>= 1) {
+      if (held > 1) {
+        held >>= 1;
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < PIECES / 2; ++i)
+          if (i < held) {
+            const float pass_on = up ? u[i] : u[i + held], keep = up ? u[i + held] : u[i];
+            u[i] = keep + __shfl_xor_sync(0xffffffffu, pass_on, o);
+          }
+      } else {
+        u[0] += __shfl_xor_sync(0xffffffffu, u[0], o);
+      }
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) s += __shfl_sync(0xffffffffu, u[0], i * (32 / PIECES));
+    return s;
   };
   for (int row = blockIdx.x * (RN_THREADS / 32) + (threadIdx.x >> 5); row < rows; row += gridDim.x * (RN_THREADS / 32)) {
     float *xr = x + (long long)row * d;
@@ -128,14 +152,14 @@ residual_norm_rows_kernel(float *x, const float *y, RmsWeight after, T *h, int h
     if (y) {
       const float *yr = y + (long long)row * d;
       float4 w[PIECES];
-      float s = 0.f;
+      float s[PIECES];
 #pragma unroll
       for (int i = 0; i < PIECES; ++i) {
         const int c = (i * 32 + lane) * 4;
         w[i] = c < d ? *reinterpret_cast<const float4 *>(yr + c) : zero;
       }
 #pragma unroll
-      for (int i = 0; i < PIECES; ++i) s += squares(w[i]);
+      for (int i = 0; i < PIECES; ++i) s[i] = squares_fused(w[i]);
       const float inv = 1.0f / sqrtf(row_sum(s) / (float)d + eps);
 #pragma unroll
       for (int i = 0; i < PIECES; ++i) {
@@ -150,9 +174,9 @@ residual_norm_rows_kernel(float *x, const float *y, RmsWeight after, T *h, int h
       }
     }
     if (h == nullptr) continue;
-    float s = 0.f;
+    float s[PIECES];
 #pragma unroll
-    for (int i = 0; i < PIECES; ++i) s += squares(v[i]);
+    for (int i = 0; i < PIECES; ++i) s[i] = squares_fused(v[i]);
     const float inv = 1.0f / sqrtf(row_sum(s) / (float)d + eps);
     T *hr = h + (long long)row * h_ld;
 #pragma unroll

@@ -99,6 +99,21 @@ def test_residual_norm_of_many_rows(rows, d):
     assert gh is None and np.abs(gx - wx).max() < 1e-5 * np.abs(wx).max()
 
 
+@pytest.mark.parametrize("d", [4, 128, 132, 500, 512, 516, 768, 1000, 1024])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_residual_norm_of_a_row_does_not_depend_on_the_others(d, dtype):
+    """A warp per row adds what a CTA per row adds, in its order: the same bits for a row among many and among few."""
+    rng = np.random.default_rng(d)
+    x, y = (3.0 * rng.standard_normal((2, 1100, d))).astype(np.float32)
+    after, before = (0.3 * rng.standard_normal((2, d))).astype(np.float32)
+    for used in ((y, after, before), (None, None, before), (y, after, None)):
+        many = residual_norm_host(x, *used, 1.0, 1e-2, dtype=dtype)
+        for at in (0, 550):
+            few = residual_norm_host(x[at:at + 550], None if used[0] is None else y[at:at + 550], *used[1:], 1.0, 1e-2, dtype=dtype)
+            for m, f in zip(many, few):
+                assert (m is None) == (f is None) and (m is None or np.array_equal(m[at:at + 550].view(np.int32), f.view(np.int32)))
+
+
 def delta_case(seed, streams, n, heads, groups, dim, vdim, taps):
     rng = np.random.default_rng(seed)
     c = 2 * groups * dim + heads * vdim
