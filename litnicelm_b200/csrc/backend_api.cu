@@ -885,6 +885,13 @@ bool issue_heads_grouped(Backend *b, const Backend::Pending *q, int n, long long
       if (!disjoint(fx, Footprint(*y.v, heads, y.delta))) return false;
     }
   }
+  // A causal row's limit is its number among the rows of the call modulo the columns: over all heads the same only where one
+  // head's rows are whole squares.
+  for (int i = 0; i < n; ++i)
+    if (q[i].kind == P::SOFTMAX || q[i].kind == P::SOFTMAX_BWD) {
+      const RowView r = make_row_view(&q[i].a, "head operand");
+      if (r.rows % r.cols != 0) return false;
+    }
   // the views of all heads
   MatView temp_m{};
   RowView temp_r{};

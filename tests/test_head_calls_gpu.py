@@ -138,6 +138,32 @@ GROUPED = {"forward", "forward, one score buffer", "exec", "backward, shared", "
            "backward, last incomplete"}
 
 
+def rectangular(be, a, rows, cols, batch):
+    """A causal row's limit is its number among the rows of its call, modulo the columns: heads whose rows are no whole squares."""
+    def mat(name, h, m, n):
+        return view(a.buffers[name][0] + 4 * h * batch * m * n, (batch, m, n))
+    for name, floats in (("q", rows * DH), ("k", cols * DH), ("w", rows * cols), ("ctx", rows * DH), ("dw", rows * cols), ("dq", rows * DH)):
+        a.buffer(name, H * batch * floats)
+    for h in range(H):
+        w = mat("w", h, rows, cols)
+        be.call("gemm_batched_rhs_t", mat("q", h, rows, DH), mat("k", h, cols, DH), w)
+        be.call("scaled_causal_softmax_rows", w, 0.25, w)
+        be.call("gemm_batched", w, mat("k", h, cols, DH), mat("ctx", h, rows, DH))
+    be.download(*a.buffers["q"])         # (a run ends at any other call)
+    for h in range(H):
+        dw = mat("dw", h, rows, cols)
+        be.call("gemm_batched_rhs_t", mat("ctx", h, rows, DH), mat("k", h, cols, DH), dw)
+        be.call("softmax_backward_causal_rows", mat("w", h, rows, cols), dw, dw)
+        be.call("gemm_batched", dw, mat("k", h, cols, DH), mat("dq", h, rows, DH))
+
+
+for rows, cols, batch in ((24, 32, 1), (32, 24, 1), (24, 32, 2), (3, 5, 1), (48, 24, 1), (24, 48, 2)):
+    name = f"causal {batch} x {rows} x {cols}"
+    RUNS[name] = lambda be, a, size=(rows, cols, batch): rectangular(be, a, *size)
+    if batch * rows % cols == 0:
+        GROUPED.add(name)
+
+
 @pytest.mark.parametrize("name", RUNS)
 def test_same_bits_as_call_by_call(name):
     left, launches = [], []
