@@ -885,6 +885,9 @@ bool issue_heads_grouped(Backend *b, const Backend::Pending *q, int n, long long
       if (!disjoint(fx, Footprint(*y.v, heads, y.delta))) return false;
     }
   }
+  // room for one more axis, in the form the call takes its views in (rows may be a vector, which no product takes)
+  for (const Operand &o : all)
+    if (product(q[o.op].kind) ? make_mat_view(o.v, "head operand").nb > 2 : make_row_view(o.v, "head operand").np > 3) return false;
   // A causal row's limit is its number among the rows of the call modulo the columns: over all heads the same only where one
   // head's rows are whole squares.
   for (int i = 0; i < n; ++i)
@@ -935,8 +938,6 @@ bool issue_heads_grouped(Backend *b, const Backend::Pending *q, int n, long long
     const Operand &o = operand(i, w);
     return o.temp ? temp_r : with_heads(make_row_view(o.v, who), heads, o.delta);
   };
-  for (const Operand &o : all)
-    if (!o.temp && (make_mat_view(o.v, "head operand").nb > 2 || make_row_view(o.v, "head operand").np > 3)) return false;
   for (int i = 0; i < n; ++i) {
     switch (q[i].kind) {
       case P::SCORES:

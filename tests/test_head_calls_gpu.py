@@ -122,6 +122,21 @@ def backwards(be, a):
         be.call("gemm_batched_lhs_t", v, v, view(y + 4 * at * S * S, (1, S, S)))
 
 
+def vectors(be, a, op):
+    """Row calls on views of rank 1 between the products."""
+    x, y, z = a.buffer("x", H * S * S), a.buffer("y", H * S * S), a.buffer("z", 3 * H * S)
+    for h in range(H):
+        m, out = view(x + 4 * h * S * S, (1, S, S)), view(y + 4 * h * S * S, (1, S, S))
+        u, v, w = (view(z + 4 * (i * H + h) * S, (S,)) for i in range(3))
+        be.call("gemm_batched_lhs_t", m, m, out)
+        if op == "mul_scalar":
+            be.call(op, u, 0.5, v)
+        elif op == "scaled_causal_softmax_rows":
+            be.call(op, u, 0.5, v)
+        else:
+            be.call(op, u, v, w)
+
+
 def lanes(be, a):
     be.call("start_exec_context_iteration")
     be.call("start_exec_context_group")
@@ -162,6 +177,11 @@ for rows, cols, batch in ((24, 32, 1), (32, 24, 1), (24, 32, 2), (3, 5, 1), (48,
     RUNS[name] = lambda be, a, size=(rows, cols, batch): rectangular(be, a, *size)
     if batch * rows % cols == 0:
         GROUPED.add(name)
+
+
+for op in ("mul_scalar", "scaled_causal_softmax_rows", "softmax_backward_causal_rows"):
+    RUNS[op + " of vectors"] = lambda be, a, op=op: vectors(be, a, op)
+GROUPED.add("mul_scalar of vectors")
 
 
 @pytest.mark.parametrize("name", RUNS)
