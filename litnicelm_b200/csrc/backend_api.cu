@@ -888,6 +888,9 @@ bool issue_heads_grouped(Backend *b, const Backend::Pending *q, int n, long long
   // room for one more axis, in the form the call takes its views in (rows may be a vector, which no product takes)
   for (const Operand &o : all)
     if (product(q[o.op].kind) ? make_mat_view(o.v, "head operand").nb > 2 : make_row_view(o.v, "head operand").np > 3) return false;
+  // A right operand that a head's batch shares has no axis to put the heads beside.
+  for (int i = 0; i < n; ++i)
+    if (product(q[i].kind) && make_mat_view(&q[i].b, "head operand").batch != make_mat_view(&q[i].c, "head operand").batch) return false;
   // A causal row's limit is its number among the rows of the call modulo the columns: over all heads the same only where one
   // head's rows are whole squares.
   for (int i = 0; i < n; ++i)

@@ -137,6 +137,14 @@ def vectors(be, a, op):
             be.call(op, u, v, w)
 
 
+def one_right_operand(be, a, op):
+    """A head's batch shares its right operand, which has no batch axis, or one of extent 1."""
+    x, y, z = a.buffer("x", H * B * S * S), a.buffer("y", H * S * S), a.buffer("z", H * B * S * S)
+    for h in range(H):
+        shape = (S, S) if op == "gemm_batched_rhs_t" else (1, S, S)
+        be.call(op, view(x + 4 * h * B * S * S, (B, S, S)), view(y + 4 * h * S * S, shape), view(z + 4 * h * B * S * S, (B, S, S)))
+
+
 def lanes(be, a):
     be.call("start_exec_context_iteration")
     be.call("start_exec_context_group")
@@ -182,6 +190,10 @@ for rows, cols, batch in ((24, 32, 1), (32, 24, 1), (24, 32, 2), (3, 5, 1), (48,
 for op in ("mul_scalar", "scaled_causal_softmax_rows", "softmax_backward_causal_rows"):
     RUNS[op + " of vectors"] = lambda be, a, op=op: vectors(be, a, op)
 GROUPED.add("mul_scalar of vectors")
+
+
+for op in ("gemm_batched_rhs_t", "gemm_batched_lhs_t"):
+    RUNS[op + ", one right operand"] = lambda be, a, op=op: one_right_operand(be, a, op)
 
 
 @pytest.mark.parametrize("name", RUNS)
