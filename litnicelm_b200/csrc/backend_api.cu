@@ -12,6 +12,7 @@
 
 #include <cmath>
 #include <cstdlib>
+#include <algorithm>
 #include <cstring>
 #include <fstream>
 #include <map>
@@ -819,7 +820,8 @@ bool disjoint(const Footprint &p, const Footprint &q) {
 // - every head makes the same calls on views of one shape, whose addresses advance by a constant per operand;
 // - what one head writes no other head reads or writes (a head's own calls keep their order). A buffer that all heads share
 //   is given to each head separately where every head first fills it with a product and only uses it as that one view; the
-//   host's buffer then receives the last head's content, which is what it holds after the host's own sequence.
+//   host's buffer then receives the last head's content, which is what it holds after the host's own sequence;
+// - one launch can hold all heads, by the kernel that a head's own call takes.
 // Beyond this a single head's calls fill the GPU by themselves (512 MB over 8 heads: 64 MB each).
 constexpr size_t MAX_HEAD_FLOATS = (size_t)128 << 20;
 bool issue_heads_grouped(Backend *b, const Backend::Pending *q, int n, long long heads) {
@@ -901,26 +903,14 @@ bool issue_heads_grouped(Backend *b, const Backend::Pending *q, int n, long long
   // the views of all heads
   MatView temp_m{};
   RowView temp_r{};
+  size_t temp_floats = 0;
   if (temp != nullptr) {
     const MatView m = make_mat_view(temp, "head buffer");
     const RowView r = make_row_view(temp, "head buffer");
     if (r.rows != m.batch * m.rows || r.cols != m.cols) return false;
-    const size_t per_head = (size_t)m.batch * m.rows * m.cols;
-    if (per_head * heads > MAX_HEAD_FLOATS) return false;
-    if (per_head * heads > b->queue_scratch_floats) {
-      bind(b);
-      LB_CUDA(cudaStreamSynchronize(b->st));
-      if (b->queue_scratch) cudaFree(b->queue_scratch);
-      b->queue_scratch = nullptr;
-      b->queue_scratch_floats = 0;
-      if (cudaMalloc(reinterpret_cast<void **>(&b->queue_scratch), per_head * heads * 4) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
-      }
-      b->queue_scratch_floats = per_head * heads;
-    }
+    temp_floats = (size_t)m.batch * m.rows * m.cols * heads;
+    if (temp_floats > MAX_HEAD_FLOATS) return false;
     // dense, head by head: [heads * batch][rows][cols]
-    temp_m.data = temp_r.data = reinterpret_cast<char *>(b->queue_scratch);
     temp_m.rows = m.rows;
     temp_m.cols = temp_r.cols = m.cols;
     temp_m.rs = m.cols * 4;
@@ -933,29 +923,63 @@ bool issue_heads_grouped(Backend *b, const Backend::Pending *q, int n, long long
     temp_r.ps[0] = m.cols * 4;
   }
   auto operand = [&](int i, int w) -> const Operand & { return all[(size_t)index[(size_t)i * 3 + w]]; };
-  auto mat = [&](int i, int w, const char *who) {
-    const Operand &o = operand(i, w);
-    return o.temp ? temp_m : with_heads(make_mat_view(o.v, who), heads, o.delta);
-  };
   auto rows = [&](int i, int w, const char *who) {
     const Operand &o = operand(i, w);
     return o.temp ? temp_r : with_heads(make_row_view(o.v, who), heads, o.delta);
   };
+  struct Product {
+    MatView a, b, c;
+  };
+  auto product_of = [&](int i, bool of_all, const char *who) {
+    MatView v[3];
+    for (int w = 0; w < 3; ++w) {
+      const Operand &o = operand(i, w);
+      v[w] = of_all && o.temp ? temp_m : make_mat_view(o.v, who);
+      if (of_all && !o.temp) v[w] = with_heads(v[w], heads, o.delta);
+    }
+    return Product{q[i].kind == P::LHS_T ? transposed(v[0]) : v[0], q[i].kind == P::SCORES ? transposed(v[1]) : v[1], v[2]};
+  };
+  // What one head's call is launched with has to hold all heads: a batch in the grid's z, rows in its x, and a product that has
+  // room for its parts on the tensor cores must not lose them (launch_gemm_f32 takes plain tiles instead, slower and less exact).
+  size_t parts = 0;
+  for (int i = 0; i < n; ++i) {
+    if (!product(q[i].kind)) {
+      if (rows(i, 0, "head operand").rows > 0x7fffffff) return false;
+      continue;
+    }
+    const Product one = product_of(i, false, "head operand"), every = product_of(i, true, "head operand");
+    if (every.c.batch > 65535) return false;
+    const size_t need = gemm_f32_scratch_bytes(every.a, every.b, every.c);
+    if (gemm_f32_scratch_bytes(one.a, one.b, one.c) == 0) continue;
+    if (need == 0) return false;
+    parts = std::max(parts, need);
+  }
+  bind(b);
+  if (temp_floats > b->queue_scratch_floats) {
+    LB_CUDA(cudaStreamSynchronize(b->st));
+    if (b->queue_scratch) cudaFree(b->queue_scratch);
+    b->queue_scratch = nullptr;
+    b->queue_scratch_floats = 0;
+    if (cudaMalloc(reinterpret_cast<void **>(&b->queue_scratch), temp_floats * 4) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return false;
+    }
+    b->queue_scratch_floats = temp_floats;
+  }
+  if (parts > 0 && !b->split.ensure(parts, b->st)) return false;
+  temp_m.data = temp_r.data = reinterpret_cast<char *>(b->queue_scratch);
   for (int i = 0; i < n; ++i) {
     switch (q[i].kind) {
       case P::SCORES:
-        run_gemm(b, mat(i, 0, "gemm_batched_rhs_t(a)"), transposed(mat(i, 1, "gemm_batched_rhs_t(b)")), mat(i, 2, "gemm_batched_rhs_t(out)"),
-                 "litnice_b200::gemm_batched_rhs_t");
-        break;
       case P::CONTEXT:
-        run_gemm(b, mat(i, 0, "gemm_batched(a)"), mat(i, 1, "gemm_batched(b)"), mat(i, 2, "gemm_batched(out)"), "litnice_b200::gemm_batched");
+      case P::LHS_T: {
+        const char *who = q[i].kind == P::SCORES ? "litnice_b200::gemm_batched_rhs_t"
+                                                 : q[i].kind == P::CONTEXT ? "litnice_b200::gemm_batched" : "litnice_b200::gemm_batched_lhs_t";
+        const Product p = product_of(i, true, who);
+        run_gemm(b, p.a, p.b, p.c, who);
         break;
-      case P::LHS_T:
-        run_gemm(b, transposed(mat(i, 0, "gemm_batched_lhs_t(a)")), mat(i, 1, "gemm_batched_lhs_t(b)"), mat(i, 2, "gemm_batched_lhs_t(out)"),
-                 "litnice_b200::gemm_batched_lhs_t");
-        break;
+      }
       case P::SOFTMAX:
-        bind(b);
         launch_softmax_rows(rows(i, 0, "scaled_causal_softmax_rows(scores)"), rows(i, 2, "scaled_causal_softmax_rows(out)"), 1, q[i].scale, b->st);
         ++b->launches;
         break;

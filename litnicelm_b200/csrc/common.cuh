@@ -240,6 +240,7 @@ struct SplitScratch {
 };
 // Bytes that launch_gemm_f32 uses for a product of these extents (0: it runs on launch_gemm_simt).
 size_t gemm_f32_scratch_bytes(long long m, long long n, long long k, long long a_batch, long long b_batch, bool sum_batches);
+size_t gemm_f32_scratch_bytes(MatView a, const MatView &b, MatView c);  // C[b] = A[b] B[b]
 // C[b] = A[b] B[b], or with sum_batches C = sum over b of A[b] B[b], by the kernel that suits the extents; falls back to
 // launch_gemm_simt where there is no memory for the parts. Returns the kernels launched.
 int launch_gemm_f32(const MatView &a, const MatView &b, const MatView &c, bool sum_batches, const GemmEpilogue &ep,

@@ -733,6 +733,11 @@ size_t gemm_f32_scratch_bytes(long long m, long long n, long long k, long long a
   return (size_t)parts * 2 + 256;
 }
 
+size_t gemm_f32_scratch_bytes(MatView a, const MatView &b, MatView c) {
+  if (b.batch == 1) fold(a, c);
+  return gemm_f32_scratch_bytes(a.rows, b.cols, a.cols, a.batch, b.batch, false);
+}
+
 int launch_gemm_f32(const MatView &a, const MatView &b, const MatView &c, bool sum_batches, const GemmEpilogue &ep,
                     SplitScratch &scratch, cudaStream_t st, DevErr *err) {
   if (a.rows <= 0 || b.cols <= 0) return 0;

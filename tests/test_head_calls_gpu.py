@@ -145,6 +145,15 @@ def one_right_operand(be, a, op):
         be.call(op, view(x + 4 * h * B * S * S, (B, S, S)), view(y + 4 * h * S * S, shape), view(z + 4 * h * B * S * S, (B, S, S)))
 
 
+def small_products(be, a):
+    """More products of 2 x 2 than a grid has layers, each call alone within them."""
+    batch = 20000
+    x, y = a.buffer("x", H * batch * 4), a.buffer("y", H * batch * 4)
+    for h in range(H):
+        m = view(x + 16 * h * batch, (batch, 2, 2))
+        be.call("gemm_batched_rhs_t", m, m, view(y + 16 * h * batch, (batch, 2, 2)))
+
+
 def lanes(be, a):
     be.call("start_exec_context_iteration")
     be.call("start_exec_context_group")
@@ -154,10 +163,10 @@ def lanes(be, a):
 
 
 RUNS = {"forward": lambda be, a: forward(be, a, False), "forward, one score buffer": lambda be, a: forward(be, a, True),
-        "uneven": uneven, "running": running, "overlapping": overlapping, "backwards": backwards, "exec": lanes}
+        "uneven": uneven, "running": running, "small products": small_products, "overlapping": overlapping, "backwards": backwards, "exec": lanes}
 for name in ("shared", "own", "scales", "one gradient", "next head reads", "not filled", "not scaled", "other view", "last incomplete"):
     RUNS["backward, " + name] = lambda be, a, name=name: backward(be, a, name)
-GROUPED = {"forward", "forward, one score buffer", "exec", "backward, shared", "backward, own", "backward, not scaled",
+GROUPED = {"small products", "forward", "forward, one score buffer", "exec", "backward, shared", "backward, own", "backward, not scaled",
            "backward, last incomplete"}
 
 
@@ -214,3 +223,28 @@ def test_same_bits_as_call_by_call(name):
     for k in left[0]:
         assert np.array_equal(left[0][k], left[1][k]), k
     assert (launches[0] < launches[1]) == (name in GROUPED), launches
+
+
+def test_long_sums_stay_on_the_tensor_cores():
+    """Heads whose operands in parts pass the 4 GB up to which a product has room for them, each alone far below: no head may go
+    to the plain tiles for the others' sake. Blocks of 64 k are added with rounding, in ranges that need not be the same: errors of
+    2^-24 that add up like a walk."""
+    heads, k = 32, 163840
+    left = []
+    for queue in ("1", "0"):
+        os.environ["LITNICE_B200_ABI_QUEUE"] = queue
+        try:
+            be = Backend()
+        finally:
+            del os.environ["LITNICE_B200_ABI_QUEUE"]
+        with be:
+            a = Arena(be)
+            x, y = a.buffer("x", (heads + 64) * k), a.buffer("y", heads * 64 * 64)
+            with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+                for h in range(heads):
+                    m = view(x + 4 * h * k, (1, 64, k))
+                    be.call("gemm_batched_rhs_t", m, m, view(y + 4 * h * 64 * 64, (1, 64, 64)))
+                left.append(be.download(*a.buffers["y"]).view(np.float32))
+            names = {e.name for e in prof.events()}
+            assert any("gemm_split" in n for n in names) and not any("gemm_simt" in n for n in names), names
+    assert np.linalg.norm(left[0] - left[1]) < 2 ** -24 * (k / 64) ** 0.5 * np.linalg.norm(left[0])
