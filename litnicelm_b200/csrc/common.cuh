@@ -266,7 +266,7 @@ void launch_embedding_grads(const char *ids, int ids_is_f32, const RowView &ids_
 void launch_cross_entropy(const RowView &logits, const char *targets, int targets_is_f32, const RowView &targets_rows,
                           bool want_loss, bool want_backward, float *loss_out, void *scratch, DevErr *err,
                           cudaStream_t st);
-// scale: factor of the finished gradient, a rounding of its own
+// scale: factor of the finished gradient, a rounding of its own; of its zeros too, which a negative or infinite one changes
 void launch_softmax_backward(const RowView &sm, const RowView &dout, const RowView &dx, bool causal, float scale, cudaStream_t st);
 void launch_adamw(float *params, const float *grads, float *m, float *v, long long n, float lr, float beta1,
                   float beta2, float b1_corr, float b2_corr, float weight_decay, int apply_decay, cudaStream_t st);

@@ -386,8 +386,8 @@ __global__ void softmax_bwd_kernel(const __grid_constant__ RowView sm, const __g
   dot = warp_sum(dot);
   for (long long c = lane; c < cols; c += 32) {
     float g = 0.f;
-    if (c < live) g = ld(sm, so, c) * (ld(dout, go, c) - dot) * scale;
-    st(dx, xo, c, g);
+    if (c < live) g = ld(sm, so, c) * (ld(dout, go, c) - dot);
+    st(dx, xo, c, g * scale);
   }
 }
 
@@ -414,7 +414,7 @@ softmax_bwd_row_kernel(const __grid_constant__ RowView sm, const __grid_constant
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
     const int c = lane + 32 * i;
-    if (c < cols) st(dx, xo, c, c < live ? s[i] * (g[i] - dot) * scale : 0.f);
+    if (c < cols) st(dx, xo, c, (c < live ? s[i] * (g[i] - dot) : 0.f) * scale);
   }
 }
 

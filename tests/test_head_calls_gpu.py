@@ -64,7 +64,7 @@ def backward(be, a, variant):
     dqkv, tmp, more = a.buffer("dqkv", 3 * B * S * D), a.buffer("tmp", B * S * S), a.buffer("more", B * H * S * S)
     for h in range(H):
         dw = square(more, h) if variant == "own" else view(tmp, (B, S, S))
-        scale = 0.25 + 0.125 * h if variant == "scales" else 0.25
+        scale = 0.25 + 0.125 * h if variant == "scales" else {"negative scale": -0.25, "infinite scale": np.inf}.get(variant, 0.25)
         dv = third(dqkv, 2, 0 if variant == "one gradient" else h)
         k = third(qkv, 1, h)
         if variant == "next head reads":   # a head's key is what the head before it wrote
@@ -164,10 +164,11 @@ def lanes(be, a):
 
 RUNS = {"forward": lambda be, a: forward(be, a, False), "forward, one score buffer": lambda be, a: forward(be, a, True),
         "uneven": uneven, "running": running, "small products": small_products, "overlapping": overlapping, "backwards": backwards, "exec": lanes}
-for name in ("shared", "own", "scales", "one gradient", "next head reads", "not filled", "not scaled", "other view", "last incomplete"):
+for name in ("shared", "own", "scales", "one gradient", "next head reads", "not filled", "not scaled", "other view", "last incomplete", "negative scale",
+             "infinite scale"):
     RUNS["backward, " + name] = lambda be, a, name=name: backward(be, a, name)
 GROUPED = {"small products", "forward", "forward, one score buffer", "exec", "backward, shared", "backward, own", "backward, not scaled",
-           "backward, last incomplete"}
+           "backward, last incomplete", "backward, negative scale", "backward, infinite scale"}
 
 
 def rectangular(be, a, rows, cols, batch):
