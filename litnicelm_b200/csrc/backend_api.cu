@@ -201,23 +201,39 @@ uint32_t api_device(void *h) {
   return 1u;
 }
 
+// Device memory for the host. What the calls of heads and the large products keep for the next of them is given back where there
+// is none left.
+void *device_memory(Backend *b, uint64_t bytes) {
+  void *p = nullptr;
+  cudaError_t e = cudaMalloc(&p, bytes);
+  if (e == cudaErrorMemoryAllocation && (b->queue_scratch != nullptr || b->split.p != nullptr)) {
+    (void)cudaGetLastError();
+    LB_CUDA(cudaStreamSynchronize(b->st));
+    if (b->queue_scratch) cudaFree(b->queue_scratch);
+    b->queue_scratch = nullptr;
+    b->queue_scratch_floats = 0;
+    b->split.give_back();
+    e = cudaMalloc(&p, bytes);
+  }
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    throw std::runtime_error(std::string("litnice_b200::alloc failed: ") + cudaGetErrorString(e));
+  }
+  return p;
+}
+
 void *api_alloc(void *h, uint64_t bytes, uint32_t alignment) {
   Backend *b = self(h);
   if (bytes == 0) return nullptr;
   if (alignment == 0 || (alignment & (alignment - 1)) != 0)
     throw std::invalid_argument("litnice_b200::alloc: invalid alignment");
   bind(b);
-  void *p = nullptr;
   if (alignment <= 256) {  // cudaMalloc returns 256-byte aligned memory
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess)
-      throw std::runtime_error(std::string("litnice_b200::alloc failed: ") + cudaGetErrorString(e));
+    void *p = device_memory(b, bytes);
     b->allocs[reinterpret_cast<uintptr_t>(p)] = bytes;
     return p;
   }
-  cudaError_t e = cudaMalloc(&p, bytes + alignment);
-  if (e != cudaSuccess)
-    throw std::runtime_error(std::string("litnice_b200::alloc failed: ") + cudaGetErrorString(e));
+  void *p = device_memory(b, bytes + alignment);
   const uintptr_t a = (reinterpret_cast<uintptr_t>(p) + alignment - 1) & ~(uintptr_t)(alignment - 1);
   b->over_aligned[reinterpret_cast<void *>(a)] = p;
   b->allocs[a] = bytes;

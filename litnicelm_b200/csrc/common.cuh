@@ -237,6 +237,7 @@ struct SplitScratch {
   SplitScratch &operator=(const SplitScratch &) = delete;
   ~SplitScratch();
   bool ensure(size_t need, cudaStream_t st);  // true: there are `need` bytes
+  void give_back();                           // behind the last product that used them
 };
 // Bytes that launch_gemm_f32 uses for a product of these extents (0: it runs on launch_gemm_simt).
 size_t gemm_f32_scratch_bytes(long long m, long long n, long long k, long long a_batch, long long b_batch, bool sum_batches);

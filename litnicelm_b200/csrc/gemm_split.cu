@@ -680,8 +680,12 @@ void launch_gemm_split(MatView a, MatView b, MatView c, bool sum_batches, const 
 
 }  // namespace
 
-SplitScratch::~SplitScratch() {
+SplitScratch::~SplitScratch() { give_back(); }
+
+void SplitScratch::give_back() {
   if (p) cudaFree(p);
+  p = nullptr;
+  bytes = 0;
 }
 
 bool SplitScratch::ensure(size_t need, cudaStream_t st) {
@@ -695,9 +699,7 @@ bool SplitScratch::ensure(size_t need, cudaStream_t st) {
   if (grown < room) grown = room;
   if (p) {
     LB_CUDA(cudaStreamSynchronize(st));
-    cudaFree(p);
-    p = nullptr;
-    bytes = 0;
+    give_back();
   }
   while (cudaMalloc(&p, grown) != cudaSuccess) {
     p = nullptr;

@@ -249,3 +249,17 @@ def test_long_sums_stay_on_the_tensor_cores():
             names = {e.name for e in prof.events()}
             assert any("gemm_split" in n for n in names) and not any("gemm_simt" in n for n in names), names
     assert np.linalg.norm(left[0] - left[1]) < 2 ** -24 * (k / 64) ** 0.5 * np.linalg.norm(left[0])
+
+
+def test_kept_memory_is_given_back():
+    """What the calls of heads keep (here 256 MB) does not stand in the way of the host's own allocations."""
+    heads, n = 8, 2048 * 4
+    with Backend() as be:
+        x, y = be.alloc(heads * n * 2 * 4, 64), be.alloc(n * n // 8 * 4, 64)
+        be.call("fill", view(x, (heads * n * 2,)), 1.0)
+        out = view(y, (1, n // 8, n))
+        for h in range(heads):
+            be.call("gemm_batched_rhs_t", view(x + 8 * n * h, (1, n // 8, 2)), view(x + 8 * n * h, (1, n, 2)), out)
+        be.download(y, 4)
+        whole = be.api.memory_info(be.h).free_bytes + (128 << 20)
+        be.api.free(be.h, be.api.alloc(be.h, whole, 64))
