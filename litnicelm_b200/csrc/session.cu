@@ -223,7 +223,7 @@ struct litnice_b200_session {
   // greedy runs of up to 8 streams: all steps after the first in one resident kernel
   // (decode_persistent.cu; LITNICE_B200_KV_PERSIST=0 keeps one graph replay per token)
   bool kv_persist = true;
-  bool kv_cluster = true;  // with a cluster per head where the model allows it; off once there was no memory for it
+  signed char cl_fits[4] = {-1, -1, -1, -1};  // whether its form with a cluster per head takes 1, 2, 4, 8 streams: -1 not asked yet
   int sm_count = 0;
   unsigned long long *pk_offsets = nullptr;  // device table of parameter offsets
   float *pk_scratch = nullptr;
@@ -869,32 +869,6 @@ void enqueue_decode_step(litnice_b200_session *s, int B, int sl, const LoopState
 
 // Cached mode: caches for n_streams streams of up to cap positions, and the scratch of the
 // attention over key chunks for every context length up to cap.
-// The resident kernel that runs the steps of B greedy streams of the cached mode: a cluster per head where the model allows
-// it, which was 2.4 to 6 times as fast over widths 64 to 512, 1 to 8 streams, contexts of 8 to 960 and vocabularies of 24 to 32000
-// (6 layers of 512, one stream 157 -> 57 us a token; figures in decode_cluster.cu); else one CTA per SM behind grid-wide
-// barriers; else none (a graph replay per token).
-enum Resident { RESIDENT_NONE, RESIDENT_GRID, RESIDENT_CLUSTER };
-Resident resident_kernel(const litnice_b200_session *s, int B) {
-  const litnice_b200_dims &d = s->dims;
-  if (!s->kv || !s->kv_persist || B > 8) return RESIDENT_NONE;
-  if (s->kv_cluster && decode_cluster_supports(B, d.n_layers, d.n_heads, d.d_model, d.d_ff, d.vocab_size)) return RESIDENT_CLUSTER;
-  return decode_persistent_supports(B, d.n_heads, d.d_model, d.d_ff, d.vocab_size) ? RESIDENT_GRID : RESIDENT_NONE;
-}
-
-// Memory of the cluster kernel; without it the run takes the grid's kernel or a graph replay per token.
-bool ensure_cluster(litnice_b200_session *s) {
-  const litnice_b200_dims &d = s->dims;
-  const size_t floats = decode_cluster_packed_floats(d.n_layers, d.n_heads, d.d_model, d.d_ff, d.vocab_size);
-  for (auto &[p, bytes] : {std::pair<void **, size_t>{reinterpret_cast<void **>(&s->cl_packed), floats * 4},
-                           {reinterpret_cast<void **>(&s->cl_words), decode_cluster_words(d.n_heads, d.d_model) * 8}})
-    if (*p == nullptr && cudaMalloc(p, bytes) != cudaSuccess) {
-      cudaGetLastError();
-      *p = nullptr;
-      return false;
-    }
-  return true;
-}
-
 void ensure_kv(litnice_b200_session *s, int B, int cap) {
   const litnice_b200_dims &d = s->dims;
   if (B > s->kv_streams || cap > s->kv_cap) {
@@ -914,18 +888,6 @@ void ensure_kv(litnice_b200_session *s, int B, int cap) {
     ++s->generation;
   }
   const size_t need = attn_decode_scratch_floats(B, cap, d.n_heads, d.d_model / d.n_heads);
-  if (resident_kernel(s, B) == RESIDENT_CLUSTER && !ensure_cluster(s)) s->kv_cluster = false;
-  if (resident_kernel(s, B) == RESIDENT_GRID) {
-    const size_t need_pk = decode_persistent_scratch_floats(B, d.n_heads, d.d_model, d.d_ff, d.vocab_size, s->sm_count);
-    if (need_pk > s->pk_scratch_floats) {
-      LB_CUDA(cudaStreamSynchronize(s->st));
-      if (s->pk_scratch) cudaFree(s->pk_scratch);
-      s->pk_scratch = nullptr;
-      s->pk_scratch_floats = 0;
-      if (cudaMalloc(reinterpret_cast<void **>(&s->pk_scratch), need_pk * 4) != cudaSuccess) throw std::bad_alloc();
-      s->pk_scratch_floats = need_pk;
-    }
-  }
   if (s->dec_counters == nullptr) {
     const size_t n = (size_t)s->max_streams * d.n_heads;
     if (cudaMalloc(reinterpret_cast<void **>(&s->dec_counters), n * 4) != cudaSuccess) throw std::bad_alloc();
@@ -940,6 +902,51 @@ void ensure_kv(litnice_b200_session *s, int B, int cap) {
     s->dec_part_floats = need;
     ++s->generation;
   }
+}
+
+// The occupancy is a matter of the model and the row class alone, and asking for it costs a run of few tokens something.
+bool cluster_takes(litnice_b200_session *s, int B) {
+  const litnice_b200_dims &d = s->dims;
+  signed char &fits = s->cl_fits[B <= 1 ? 0 : B <= 2 ? 1 : B <= 4 ? 2 : 3];
+  if (fits < 0) fits = decode_cluster_supports(B, d.n_layers, d.n_heads, d.d_model, d.d_ff, d.vocab_size) ? 1 : 0;
+  return fits > 0;
+}
+
+// Memory of the cluster kernel: another copy of the weights, and its words.
+bool ensure_cluster(litnice_b200_session *s) {
+  const litnice_b200_dims &d = s->dims;
+  if (s->cl_words != nullptr) return true;
+  const size_t floats = decode_cluster_packed_floats(d.n_layers, d.n_heads, d.d_model, d.d_ff, d.vocab_size);
+  if (cudaMalloc(reinterpret_cast<void **>(&s->cl_packed), floats * 4) == cudaSuccess &&
+      cudaMalloc(reinterpret_cast<void **>(&s->cl_words), decode_cluster_words(d.n_heads, d.d_model) * 8) == cudaSuccess)
+    return true;
+  cudaGetLastError();
+  if (s->cl_packed) cudaFree(s->cl_packed);
+  s->cl_packed = nullptr;
+  s->cl_words = nullptr;
+  return false;
+}
+
+// The resident kernel that runs the steps of B greedy streams of the cached mode, its memory there: a cluster per head where the
+// model allows it, which was 2.4 to 6 times as fast over widths 64 to 512, 1 to 8 streams, contexts of 8 to 960 and vocabularies
+// of 24 to 32000 (6 layers of 512, one stream 157 -> 57 us a token; figures in decode_cluster.cu); else, or where there is no
+// memory for it, one CTA per SM behind grid-wide barriers; else none (a graph replay per token).
+enum Resident { RESIDENT_NONE, RESIDENT_GRID, RESIDENT_CLUSTER };
+Resident ensure_resident(litnice_b200_session *s, int B) {
+  const litnice_b200_dims &d = s->dims;
+  if (!s->kv || !s->kv_persist || B > 8) return RESIDENT_NONE;
+  if (cluster_takes(s, B) && ensure_cluster(s)) return RESIDENT_CLUSTER;
+  if (!decode_persistent_supports(B, d.n_heads, d.d_model, d.d_ff, d.vocab_size)) return RESIDENT_NONE;
+  const size_t need = decode_persistent_scratch_floats(B, d.n_heads, d.d_model, d.d_ff, d.vocab_size, s->sm_count);
+  if (need > s->pk_scratch_floats) {
+    LB_CUDA(cudaStreamSynchronize(s->st));
+    if (s->pk_scratch) cudaFree(s->pk_scratch);
+    s->pk_scratch = nullptr;
+    s->pk_scratch_floats = 0;
+    if (cudaMalloc(reinterpret_cast<void **>(&s->pk_scratch), need * 4) != cudaSuccess) throw std::bad_alloc();
+    s->pk_scratch_floats = need;
+  }
+  return RESIDENT_GRID;
 }
 
 // Weights are immutable during inference: build, once per load, the K-major
@@ -1750,6 +1757,10 @@ int litnice_b200_run(litnice_b200_session *s, int32_t max_new, const litnice_b20
       }
     }
 
+    // behind everything that a run cannot do without, and only where a step is left for it once the caches are filled
+    const bool decodes = steps > (s->kv_len == s0 - 1 ? 0 : 1);
+    const Resident resident = s->kv && greedy && !s->keep_logits && decodes ? ensure_resident(s, B) : RESIDENT_NONE;
+
     const long long launches0 = s->launches;
     // One step = whole-context forward + head + selector + state advance. With
     // graph replay the step of a 64-token context bucket is captured once (its
@@ -1826,8 +1837,7 @@ int litnice_b200_run(litnice_b200_session *s, int32_t max_new, const litnice_b20
       // cached mode: a step on one new row per stream when the caches hold every earlier
       // position, else a whole-context pass that also fills them (the first step of a batch)
       const bool decode = (s->kv || s->model) && s->kv_len == sl - 1;
-      const Resident resident = decode && greedy && !s->keep_logits ? resident_kernel(s, B) : RESIDENT_NONE;
-      if (resident != RESIDENT_NONE) {
+      if (decode && resident != RESIDENT_NONE) {
         // every remaining step in one resident kernel
         DecodePersistentArgs a{};
         a.params = s->params;

@@ -11,6 +11,7 @@ import os
 
 import numpy as np
 import pytest
+import torch
 
 from litnicelm_b200 import formats
 from litnicelm_b200.plugin import Session
@@ -272,6 +273,20 @@ def test_resident_steps(dims, streams, prompt, new):
         want = logits_64(d, arena, np.concatenate([prompts[1], alone[:-1]]))[prompt - 1:]
         srt = np.sort(want, axis=1)
         agreed_prefix(alone, want.argmax(1), srt[:, -1] - srt[:, -2])
+
+
+def test_only_greedy_runs_hold_the_resident_kernels_weights():
+    """The kernel's copy of the weights (44 MB here) is made for the first run that uses it."""
+    d = formats.ModelDims(1, 8, 512, 2048, 16000, 64)
+    prompts = np.stack([formats.zipf_prompt(d.vocab, 20, 70 + i) for i in range(2)])
+    free = []
+    with Session(d, 2) as s:
+        s.load_params(formats.make_param_arena(d, 7, bias_std=0.02, ln_std=0.1))
+        for more in (dict(temp=0.8, top_k=20, seeds=[1, 2]), dict()):
+            for _ in range(2):
+                s.generate(prompts, 8, **more)
+            free.append(torch.cuda.mem_get_info()[0])
+    assert 40 << 20 < free[0] - free[1] < 64 << 20
 
 
 # Up to 64 rows a step on the weights' pairs: tiles of rows that are not full, one, two and four of them a CTA, one span of k for a
