@@ -720,7 +720,7 @@ size_t chunk_smem(int rank, int stages) {
   return (size_t)(stages * LD_KEYS + 2 * LD_HEADS) * pitch * 2 + (size_t)2 * LD_HEADS * (LD_KEYS + 8) * 2 +
          (size_t)2 * LD_HEADS * (LD_KEYS + 4) * 4 + LD_HEADS * 4;
 }
-constexpr size_t LD_SMEM_LIMIT = 220 * 1024;
+constexpr size_t LD_SMEM_LIMIT = 225 * 1024;  // two stages up to rank 656
 
 // How a window of `window` keys (contexts up to s_cap) is cut for so many rows: about two CTAs per SM.
 int most_splits(int heads, int window, int s_cap, long long rows) {

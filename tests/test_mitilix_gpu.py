@@ -196,6 +196,15 @@ def test_latent_attention(engine, streams, t, n, heads, dim, vdim, rank, window)
     assert np.abs(got - want).max() < 10 * ATT_TOL[engine] * np.abs(want).max()
 
 
+@pytest.mark.parametrize("rank", [640, 656, 672, 1024])
+def test_latent_attention_of_few_rows_with_wide_latents(rank):
+    """The widest latents of which shared memory holds two tiles of keys, and those of which it holds one."""
+    dkv, gain, uk, uv, q = attention_case(rank, 1, 900, 2, 3, 32, 48, rank)
+    want = plain_attention(q, dkv, gain, 1e-3, uk, uv, 3, 32, 48, 0.3, 850)
+    got = latent_attention_host(2, q, dkv, gain, 1e-3, uk, uv, 3, 32, 48, 0.3, 850)
+    assert rms_rel(got, want) < ATT_TOL[2] and np.abs(got - want).max() < 10 * ATT_TOL[2] * np.abs(want).max()
+
+
 @pytest.mark.parametrize("engine", [0, 1, 2, 3])
 @pytest.mark.parametrize("window", [1, 2, 7, 63, 64, 65, 127, 128, 129, 200])
 @pytest.mark.parametrize("back", ["newest", "inside", "outside"])
