@@ -146,14 +146,14 @@ attn_decode_kernel(const float *__restrict__ qkv, float *kc, float *vc, int cap,
   constexpr int KPI = 128 / LPK;   // keys per trip of the CTA
   constexpr int VPR = DH / 4;      // lanes that share one row of values: 4 floats each
   constexpr int VPI = 128 / VPR;   // rows of values per trip of the CTA
-  extern __shared__ float sc[];    // scores, then e, of the chunk's keys
+  extern __shared__ float sc[];    // heads of 16 columns: scores, then e, of the chunk's keys
   __shared__ float red_f[4];
   __shared__ double red_d[4];
   __shared__ __align__(16) float o_part[512];  // [VPI][DH]
   __shared__ int is_last;
   pdl_launch_dependents();
   const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, chunks = gridDim.x;
-  {  // the chunk's keys and values of earlier positions, on their way to L2 while the predecessor ends and scores are formed
+  if constexpr (DH >= 32) {  // the chunk's keys and values of earlier positions, on their way to L2 while the predecessor ends and scores are formed
     const int early = min(state ? *static_cast<const volatile int *>(&state->s) : s_host, cap);  // (of the step before, perhaps)
     const int first = c * keys_per_chunk, lines = max(0, min(early, first + keys_per_chunk) - first) * (DH / 32);
     for (int i = threadIdx.x; i < 2 * lines; i += 128) {
@@ -465,8 +465,9 @@ static void launch_attn_decode_dh(const float *qkv, float *kc, float *vc, int ca
   const float scale = 1.0f / sqrtf((float)DH);
   dim3 grid((unsigned)plan.chunks, (unsigned)n_heads, (unsigned)n_streams);
   float *pp = plan.chunks > 1 ? part : nullptr;
-  launch_pdl(attn_decode_kernel<DH>, grid, dim3(128), (size_t)plan.keys_per_chunk * sizeof(float), st, g_pdl_enabled,
-             qkv, kc, vc, cap, d_model, state, s_host, plan.keys_per_chunk, scale, pp, ctx, counters);
+  const size_t smem = DH < 32 ? (size_t)plan.keys_per_chunk * sizeof(float) : 0;
+  launch_pdl(attn_decode_kernel<DH>, grid, dim3(128), smem, st, g_pdl_enabled, qkv, kc, vc, cap, d_model, state, s_host,
+             plan.keys_per_chunk, scale, pp, ctx, counters);
 }
 
 int launch_attn_decode(const float *qkv, float *kc, float *vc, int cap, int d_model, int n_heads, int n_streams,

@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) decode_cluster_kernel(const __g
           for (int tile = wid; tile < groups; tile += CL_WARPS * G) {
             float v[4 * MB * G];
 #pragma unroll
-            for (int c = 0; c < 4 * MB * G; ++c) v[c] = 0.f;
+            for (int x = 0; x < 4 * MB * G; ++x) v[x] = 0.f;
 #pragma unroll 1
             for (int r0 = 0; r0 < k; r0 += CL_ROWS * AHEAD) {
               float4 wv[G][AHEAD][4];
@@ -626,13 +626,13 @@ __global__ void __launch_bounds__(CL_THREADS, 1) decode_cluster_kernel(const __g
               const int col = (blockIdx.x * S.head_tiles + ph) * c + group * 4;
               const float x[4] = {sum.x, sum.y, sum.z, sum.w};
 #pragma unroll
-              for (int c = 0; c < 4; ++c)
-                if (col + c < V) {
-                  if (x[c] > best || (x[c] == best && best_at == CL_NO_INDEX)) {
-                    best = x[c];
-                    best_at = (unsigned)(col + c);
+              for (int y = 0; y < 4; ++y)
+                if (col + y < V) {
+                  if (x[y] > best || (x[y] == best && best_at == CL_NO_INDEX)) {
+                    best = x[y];
+                    best_at = (unsigned)(col + y);
                   }
-                  if (j == 0 && t + 1 == P.steps && b < B) P.logits[(long long)b * V + col + c] = x[c];
+                  if (j == 0 && t + 1 == P.steps && b < B) P.logits[(long long)b * V + col + y] = x[y];
                 }
             } else if (second) {  // this head's, or slice's, part of columns rank * SL ..
               if (j == 0) {
