@@ -45,7 +45,8 @@ struct FpShape {
 };
 enum { FP_PLAIN, FP_FOLD, FP_FOLD_SUMS };  // no LayerNorm; one whose sums are taken here; one whose sums there are
 
-// MORE: k longer than one span per warp, the next span's weights come ahead. CTAs an SM without spills.
+// MORE: k longer than one span per warp, the next span's weights come ahead. CTAs an SM with next to no spills (4 and 24 bytes in two
+// of the eighteen forms).
 constexpr int fp_ctas(int nt, int fold, bool more) { return more ? (nt == 1 ? 2 : 1) : nt == 1 ? (fold ? 3 : 4) : nt == 2 ? 3 : 2; }
 template <int NT, int FOLD, bool MORE>
 __global__ void __launch_bounds__(FP_WARPS * 32, fp_ctas(NT, FOLD, MORE)) few_row_pair_kernel(const __grid_constant__ FpShape g) {

@@ -89,8 +89,8 @@ __device__ __forceinline__ void gs_split(float x, __nv_bfloat16 (&part)[3]) {
 // the product, in range.
 __device__ __forceinline__ bool gs_no_parts(float x) { return (__float_as_uint(x) & 0x7fffffffu) >= 0x5f000000u; }
 
-// One tile of 64 rows x 64 k of one operand: read along whichever axis is contiguous, written as rows of k, 16 bytes of a part at a
-// time.
+// One tile of 32 rows x 64 k of one operand: read along whichever axis is contiguous, written as rows of k, 16 bytes of a part at a
+// time (a thread: eight k of one row).
 constexpr int GS_SPLIT_ROWS = 32;
 __global__ void __launch_bounds__(256) split_operands_kernel(const __grid_constant__ GsArgs g, int a_blocks) {
   __shared__ float tile[GS_SPLIT_ROWS][65];
@@ -106,28 +106,23 @@ __global__ void __launch_bounds__(256) split_operands_kernel(const __grid_consta
   const float *src = reinterpret_cast<const float *>(reinterpret_cast<const char *>(o.p) + batch_offset(o.view, batch));
   const long long ld = (long long)g.kp * g.sums;
   const long long to0 = g.sums > 1 ? (long long)batch * g.kp : (long long)batch * o.n * ld;
-  constexpr int N = GS_SPLIT_ROWS / 32;  // rows of a thread, 8 k of each
-  float x[N][8];
-  const int row = tid >> 3, k = k0 + (tid & 7) * 8;
+  float x[8];
+  const int row = tid >> 3, k = k0 + (tid & 7) * 8, r = r0 + row;
   if (o.vec && o.k == 1) {
+    const float *p = src + (long long)r * o.outer + k;
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const int r = r0 + row + i * 32;
-      const float *p = src + (long long)r * o.outer + k;
-#pragma unroll
-      for (int h = 0; h < 8; h += 4) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < o.n) {
-          if (k + h + 4 <= g.k) {
-            v = *reinterpret_cast<const float4 *>(p + h);
-          } else {
-            if (k + h < g.k) v.x = p[h];
-            if (k + h + 1 < g.k) v.y = p[h + 1];
-            if (k + h + 2 < g.k) v.z = p[h + 2];
-          }
+    for (int h = 0; h < 8; h += 4) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < o.n) {
+        if (k + h + 4 <= g.k) {
+          v = *reinterpret_cast<const float4 *>(p + h);
+        } else {
+          if (k + h < g.k) v.x = p[h];
+          if (k + h + 1 < g.k) v.y = p[h + 1];
+          if (k + h + 2 < g.k) v.z = p[h + 2];
         }
-        x[i][h] = v.x; x[i][h + 1] = v.y; x[i][h + 2] = v.z; x[i][h + 3] = v.w;
       }
+      x[h] = v.x; x[h + 1] = v.y; x[h + 2] = v.z; x[h + 3] = v.w;
     }
   } else {
     const bool along_k = o.k == 1;
@@ -135,8 +130,8 @@ __global__ void __launch_bounds__(256) split_operands_kernel(const __grid_consta
 #pragma unroll
     for (int i = 0; i < GS_SPLIT_ROWS / 4; ++i) {
       const int e = tid + i * 256;
-      const int r = along_k ? e >> 6 : e % GS_SPLIT_ROWS, kk = along_k ? e & 63 : e / GS_SPLIT_ROWS;
-      t[i] = r0 + r < o.n && k0 + kk < g.k ? src[(long long)(r0 + r) * o.outer + (long long)(k0 + kk) * o.k] : 0.f;
+      const int rr = along_k ? e >> 6 : e % GS_SPLIT_ROWS, kk = along_k ? e & 63 : e / GS_SPLIT_ROWS;
+      t[i] = r0 + rr < o.n && k0 + kk < g.k ? src[(long long)(r0 + rr) * o.outer + (long long)(k0 + kk) * o.k] : 0.f;
     }
 #pragma unroll
     for (int i = 0; i < GS_SPLIT_ROWS / 4; ++i) {
@@ -145,20 +140,15 @@ __global__ void __launch_bounds__(256) split_operands_kernel(const __grid_consta
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) x[i][j] = tile[row + i * 32][(tid & 7) * 8 + j];
+    for (int j = 0; j < 8; ++j) x[j] = tile[row][(tid & 7) * 8 + j];
   }
   bool bad = false;
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const int r = r0 + row + i * 32;
-    if (r >= o.n) continue;
+  if (r < o.n) {
     __nv_bfloat16 part[8][3];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      bad |= gs_no_parts(x[i][j]);
-      gs_split(x[i][j], part[j]);
+      bad |= gs_no_parts(x[j]);
+      gs_split(x[j], part[j]);
     }
     const long long to = to0 + (long long)r * ld + k;
 #pragma unroll
