@@ -250,7 +250,11 @@ bool batch_aligned16(const MatView &v) {
 template <int BM, int BN, int TM, int TN, int AMODE, int BMODE>
 void launch_cfg(const GemmArgs &g, long long batch, cudaStream_t st) {
   dim3 grid((g.n + BN - 1) / BN, (g.m + BM - 1) / BM, (unsigned)batch);
-  launch_pdl(gemm_simt_kernel<BM, BN, TM, TN, AMODE, BMODE>, grid, dim3((BM / TM) * (BN / TN)), 0, st, g_pdl_enabled, g);
+  // Begun while its predecessor ends, a launch of few CTAs lands on the few SMs that are free by then, several to one, where each
+  // takes the time of them all: a head of 40 rows x 1000 columns 38 us, 16 behind its predecessor's end. Cached steps of 9 to 64
+  // streams with such products: 8 % less on average, up to a third.
+  const bool early = g_pdl_enabled && (long long)grid.x * grid.y * grid.z >= 148;
+  launch_pdl(gemm_simt_kernel<BM, BN, TM, TN, AMODE, BMODE>, grid, dim3((BM / TM) * (BN / TN)), 0, st, early, g);
 }
 
 template <int AMODE, int BMODE>
