@@ -132,13 +132,17 @@ __device__ __forceinline__ void store_context(const DecodeCtx &o, float v, int b
 // written directly; otherwise (o, max, sum) go to `part` and the chunk that finishes last joins them.
 //
 // Bound by the cache bytes (8 * s * d_model per layer and stream), so what counts is bytes in flight: the chunk's lines are asked for
-// towards L2 before the predecessor has ended, and a warp has eight keys and values in use and eight more on their way, without a
-// barrier before the warps' results meet. 64 streams of 128 .. 191 positions at d_model 512: 12.6 us; 19.5 with scores, weights
-// and values as three phases of the CTA, four loads in flight in each (which heads of 16 columns still do); prefetching alone
-// makes those 15.3 with eight loads. A cached step of 6 layers: 392 -> 320 us.
+// towards L2 before the predecessor has ended, and a warp has a batch of 4 KB of keys and values in use and as much on its way, without
+// a barrier before the warps' results meet. With scores, weights and values as three phases of the CTA, four loads in flight in each
+// (which heads of 16 columns still do), and now, us a launch: 64 streams, 8 heads of 64, 160 positions 16.6, 9.4, 250 positions 27.1,
+// 16.9; 40 streams, 8 heads of 32, 250 positions 7.9, 6.6 (9.9 with values read four bytes a lane).
+// The batch on its way costs registers: five CTAs an SM, eight without. More CTAs than five an SM hold run without, and chunks that
+// are one batch a warp: 40 streams, 16 heads of 64, 4 positions 3.5 in three phases, 4.6 always ahead, 3.4 so; 64 streams, 60 positions
+// 8.0, 9.1, 7.2; 64 streams, 16 heads of 32, 100 positions 6.2, 8.9, 6.9.
 constexpr int DEC_UNROLL = 4;
-template <int DH>
-__global__ void __launch_bounds__(128)
+__host__ __device__ constexpr int dec_batch(int dh) { return dh <= 32 ? 16 : dh == 64 ? 8 : 4; }  // keys of a warp's batch: 2 KB, and 2 KB of values
+template <int DH, bool MORE>
+__global__ void __launch_bounds__(128, DH < 32 ? 0 : MORE ? 5 : 8)
 attn_decode_kernel(const float *__restrict__ qkv, float *kc, float *vc, int cap, int d_model, const LoopState *state,
                    int s_host, int keys_per_chunk, float scale, float *__restrict__ part, DecodeCtx ctx,
                    int *__restrict__ counters) {
@@ -185,17 +189,17 @@ attn_decode_kernel(const float *__restrict__ qkv, float *kc, float *vc, int cap,
       *reinterpret_cast<float4 *>(vc + ((long long)b * cap + p) * d_model + h * DH + tid * 4) = v4;
     }
     if constexpr (DH >= 32) {
-      // A warp takes every fourth key, eight at a time: their scores over LPK lanes a key, the running maximum and sum, the weighted
-      // values with a lane per DH / 32 columns. The next eight keys and values are on their way while eight are used.
-      constexpr int KB = 8, KPP = 32 / LPK, NP = KB / KPP, VW = DH / 32;
-      const int sub = lane % LPK, grp = lane / LPK;
+      // A warp takes every fourth key, a batch at a time: their scores over LPK lanes a key, the running maximum and sum, the weighted
+      // values with a lane per four columns of every KPV-th key. MORE: the next batch is on its way while one is used.
+      constexpr int KB = dec_batch(DH), KPP = 32 / LPK, NP = KB / KPP;  // keys of a load of keys, such loads
+      constexpr int KPV = 32 / VPR, NV = KB / KPV;                      // of a load of values: a lane has four columns of one key
+      const int sub = lane % LPK, grp = lane / LPK, vq = lane % VPR, vr = lane / VPR;
       const int mine = (c1 - c0 - wid + 3) / 4;  // keys of this warp: positions c0 + wid + 4 n
       const float4 q0 = *reinterpret_cast<const float4 *>(row + h * DH + sub * 8);
       const float4 q1 = *reinterpret_cast<const float4 *>(row + h * DH + sub * 8 + 4);
       const long long at0 = ((long long)b * cap + c0 + wid) * d_model + h * DH;
       struct Batch {
-        float4 k0[NP], k1[NP];
-        float v[KB][VW];
+        float4 k0[NP], k1[NP], v[NV];
       };
       Batch next;
       auto load = [&](int n0) {
@@ -210,36 +214,22 @@ attn_decode_kernel(const float *__restrict__ qkv, float *kc, float *vc, int cap,
           }
         }
 #pragma unroll
-        for (int x = 0; x < KB; ++x) {
-          const int n = n0 + x;
-#pragma unroll
-          for (int y = 0; y < VW; ++y) next.v[x][y] = 0.f;
+        for (int x = 0; x < NV; ++x) {
+          const int n = n0 + x * KPV + vr;
+          next.v[x] = make_float4(0.f, 0.f, 0.f, 0.f);
           if (n < mine) {
-            const float *vp = (c0 + wid + 4 * n == p ? row + 2 * d_model + h * DH : vc + at0 + (long long)(4 * n) * d_model) + lane * VW;
-            if constexpr (VW == 4) {
-              const float4 f = *reinterpret_cast<const float4 *>(vp);
-              next.v[x][0] = f.x;
-              next.v[x][1] = f.y;
-              next.v[x][2] = f.z;
-              next.v[x][3] = f.w;
-            } else if constexpr (VW == 2) {
-              const float2 f = *reinterpret_cast<const float2 *>(vp);
-              next.v[x][0] = f.x;
-              next.v[x][1] = f.y;
-            } else {
-              next.v[x][0] = *vp;
-            }
+            const float *vp = c0 + wid + 4 * n == p ? row + 2 * d_model + h * DH : vc + at0 + (long long)(4 * n) * d_model;
+            next.v[x] = *reinterpret_cast<const float4 *>(vp + vq * 4);
           }
         }
       };
-      float o[VW];
-#pragma unroll
-      for (int y = 0; y < VW; ++y) o[y] = 0.f;
+      float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
       load(0);
 #pragma unroll 1
       for (int n0 = 0; n0 < mine; n0 += KB) {
+        if (!MORE && n0 > 0) load(n0);
         const Batch now = next;
-        if (n0 + KB < mine) load(n0 + KB);
+        if (MORE && n0 + KB < mine) load(n0 + KB);
         float e[NP], bm = -INFINITY;
 #pragma unroll
         for (int u = 0; u < NP; ++u) {
@@ -261,24 +251,31 @@ attn_decode_kernel(const float *__restrict__ qkv, float *kc, float *vc, int cap,
         const float mn = fmaxf(m, bm), keep = m == -INFINITY ? 0.f : expf(m - mn);
         m = mn;
         l *= (double)keep;
-#pragma unroll
-        for (int y = 0; y < VW; ++y) o[y] *= keep;
+        o = make_float4(o.x * keep, o.y * keep, o.z * keep, o.w * keep);
 #pragma unroll
         for (int u = 0; u < NP; ++u) {
           e[u] = e[u] == -INFINITY ? 0.f : expf(e[u] - m);
           l += (double)e[u];
         }
 #pragma unroll
-        for (int x = 0; x < KB; ++x) {
-          const float w = __shfl_sync(0xffffffffu, e[x / KPP], x % KPP * LPK);
-#pragma unroll
-          for (int y = 0; y < VW; ++y) o[y] = fmaf(w, now.v[x][y], o[y]);
+        for (int x = 0; x < NV; ++x) {
+          const float w = __shfl_sync(0xffffffffu, e[x * KPV / KPP], (x * KPV % KPP + vr) * LPK);
+          o.x = fmaf(w, now.v[x].x, o.x);
+          o.y = fmaf(w, now.v[x].y, o.y);
+          o.z = fmaf(w, now.v[x].z, o.z);
+          o.w = fmaf(w, now.v[x].w, o.w);
         }
       }
 #pragma unroll
       for (int x = LPK; x < 32; x <<= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
 #pragma unroll
-      for (int y = 0; y < VW; ++y) o_part[wid * DH + lane * VW + y] = o[y];
+      for (int x = VPR; x < 32; x <<= 1) {
+        o.x += __shfl_xor_sync(0xffffffffu, o.x, x);
+        o.y += __shfl_xor_sync(0xffffffffu, o.y, x);
+        o.z += __shfl_xor_sync(0xffffffffu, o.z, x);
+        o.w += __shfl_xor_sync(0xffffffffu, o.w, x);
+      }
+      if (lane < VPR) *reinterpret_cast<float4 *>(o_part + wid * DH + lane * 4) = o;
       if (lane == 0) {
         red_f[wid] = m;
         red_d[wid] = l;
@@ -466,8 +463,14 @@ static void launch_attn_decode_dh(const float *qkv, float *kc, float *vc, int ca
   dim3 grid((unsigned)plan.chunks, (unsigned)n_heads, (unsigned)n_streams);
   float *pp = plan.chunks > 1 ? part : nullptr;
   const size_t smem = DH < 32 ? (size_t)plan.keys_per_chunk * sizeof(float) : 0;
-  launch_pdl(attn_decode_kernel<DH>, grid, dim3(128), smem, st, g_pdl_enabled, qkv, kc, vc, cap, d_model, state, s_host,
-             plan.keys_per_chunk, scale, pp, ctx, counters);
+  auto go = [&](auto kernel) {
+    launch_pdl(kernel, grid, dim3(128), smem, st, g_pdl_enabled, qkv, kc, vc, cap, d_model, state, s_host, plan.keys_per_chunk, scale, pp, ctx,
+               counters);
+  };
+  if constexpr (DH >= 32) {
+    if (plan.keys_per_chunk <= 4 * dec_batch(DH) || (long long)plan.chunks * n_heads * n_streams > 5 * 148) return go(attn_decode_kernel<DH, false>);
+  }
+  go(attn_decode_kernel<DH, true>);
 }
 
 int launch_attn_decode(const float *qkv, float *kc, float *vc, int cap, int d_model, int n_heads, int n_streams,

@@ -316,3 +316,18 @@ def test_steps_of_tens_of_rows(dims, streams, prompt, new):
         same = np.flatnonzero(fast[b] != toks[b])
         srt = np.sort(want, axis=1)
         assert not len(same) or srt[same[0], -1] - srt[same[0], -2] < NEAR_TIE
+
+
+# The step's attention by batches of keys a warp: one that is not full, one that is, several with the next on its way, several without
+# (more CTAs than are resident with it); heads of 32, 64 and 128; chunks joined, and one that writes its context by itself.
+@pytest.mark.parametrize("dims,streams,prompt,new", [
+    ((1, 16, 512, 128, 24, 150), 64, 62, 5),
+    ((1, 16, 512, 128, 24, 150), 64, 124, 5),
+    ((1, 16, 1024, 128, 24, 60), 64, 31, 4),
+    ((1, 16, 1024, 128, 24, 80), 48, 62, 5),
+    ((1, 8, 1024, 128, 24, 100), 9, 14, 5),
+    ((1, 8, 1024, 128, 24, 100), 60, 70, 5),
+    ((1, 4, 128, 128, 24, 700), 12, 640, 5),
+])
+def test_attention_of_a_step_by_batches(dims, streams, prompt, new):
+    test_steps_of_tens_of_rows(dims, streams, prompt, new)
