@@ -44,8 +44,11 @@ __device__ __forceinline__ uint4 ld_stream(const bf16 *p) {  // weights: read on
   return v;
 }
 
-// NT: tiles of 8 activation rows; UNROLL: blocks of 32 k in flight per lane and row.
-template <int NT, int UNROLL>
+// NT: tiles of 8 activation rows; UNROLL: blocks of 32 k in flight per lane and row. SPLIT: the rows may go to several CTAs. Where they
+// do not, the form without takes 16 registers less with four tiles (24 rows, n 3072 k 2048 by two ranks 9.4 us, 9.9 with). With fewer
+// or more it is the slower, though by the launch alone it is not (12 layers of width 1024, 8 streams: 324 us a token with, 344
+// without; 9 layers, 64 streams 537 and 544), and there is none.
+template <int NT, int UNROLL, bool SPLIT>
 __global__ void __launch_bounds__(FR_WARPS * 32)
 few_row_bf16_kernel(FewRowPair pair, int rows, int ranks) {
   __shared__ __align__(16) float red[FR_WARPS][NT][FR_COLS][8];
@@ -54,7 +57,7 @@ few_row_bf16_kernel(FewRowPair pair, int rows, int ranks) {
   const int n0 = ((int)blockIdx.x - (second ? pair.blocks0 : 0)) * FR_COLS;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int k8 = (p.k + 7) & ~7;  // rows end on a multiple of 8, zeros behind k
-  const int first = (int)blockIdx.y * NT * 8, m = min(NT * 8, rows - first);  // this CTA's activation rows
+  const int first = SPLIT ? (int)blockIdx.y * NT * 8 : 0, m = SPLIT ? min(NT * 8, rows - first) : rows;  // this CTA's activation rows
   const bf16 *w = static_cast<const bf16 *>(p.w), *a = static_cast<const bf16 *>(p.a) + (long long)first * p.a_ld;
   const bool v0 = n0 + g < p.n, v1 = n0 + g + 8 < p.n;
   const bf16 *w0 = w + (long long)(n0 + g) * p.w_ld + t * 8, *w1 = w0 + (long long)8 * p.w_ld;
@@ -193,27 +196,46 @@ void launch_few_row_bf16(const Bf16Product *p, int count, int m, cudaStream_t st
   const int tiles = (m + 7) / 8;
   // Tiles of activation rows a CTA takes. Bound by latency, a launch wants its loads spread over many CTAs, and the weights
   // that several read come out of L2: as few as give no more than four CTAs an SM (64 rows, us with all rows in one CTA and with
-  // this: n 512 k 512 4.9, 3.4; n 1040 k 512 5.1, 3.1; n 2816 k 512 5.6, 4.7; n 512 k 1408 6.8, 4.4; n 1024 k 1024 6.6, 3.7). Not for
-  // long rows, where reading the weights again costs as much (n 1024 k 5120: 10.1 in one, 12.2 in eight).
+  // this: n 512 k 512 5.7, 2.9; n 1040 k 512 5.3, 3.5; n 2816 k 512 7.1, 5.8; n 512 k 1408 6.8, 4.1; n 1024 k 1024 6.9, 4.8). Not for
+  // long rows, where reading the weights again costs as much (n 1024 k 5120: 11.4 in one, 13.0 in eight).
   int nt = 1;
   while (nt < 8 && nt < tiles && (k_max > 1536 || (long long)blocks * ((tiles + nt - 1) / nt) > 4 * 148)) nt *= 2;
   const unsigned row_ctas = (unsigned)((tiles + nt - 1) / nt);
-  // Ranks of a cluster that share a tile's k: enough CTAs for two per SM, but a range of less than 1024 (of long rows 640) k costs
-  // more in the exchange than it saves (8 rows, n 1024 k 1024: one rank 2.8, two 4.0; 64 rows, n 2048 k 2048: two ranks 8.0, four 12.8).
+  // Ranks of a cluster that share a tile's k: enough CTAs for two per SM, but a range of less than 1024 (of more than two, 512, with many
+  // rows 640) k costs more in the exchange than it saves (us by one, two, four: 8 rows, n 1024 k 1024 3.3, 4.0, 4.2, n 2048 k 2048 5.9,
+  // 6.0, 5.4; 64 rows, n 2048 k 2048 two 8.0, four 12.8).
   int ranks = 1;
   const int ranks_max = m > 16 ? 4 : 8;  // many rows: a CTA's share of the sums is work too
-  while (ranks < ranks_max && blocks * row_ctas * ranks < 2 * 148 && k_max >= 2 * ranks * (ranks == 1 ? 1024 : 640)) ranks *= 2;
+  while (ranks < ranks_max && blocks * row_ctas * ranks < 2 * 148 && k_max >= 2 * ranks * (ranks == 1 ? 1024 : m > 16 ? 640 : 512)) ranks *= 2;
+  const long long ctas = (long long)blocks * row_ctas * ranks;
   const dim3 grid(blocks, row_ctas, (unsigned)ranks), block(FR_WARPS * 32);
   auto go = [&](auto kernel) {
     launch_pdl_cluster(kernel, grid, block, 0, st, g_pdl_enabled, (unsigned)ranks, pair, m, ranks);
   };
-  // Two blocks of 32 k per lane and trip where the range would leave warps idle with four (n 1040 k 512: 3.1, 3.7 with one); with
-  // eight tiles the activations of a trip outweigh that (n 8192 k 512: 13.2 with two, 10.2 with four).
-  const bool two = k_max <= 512 * ranks;
-  if (nt == 1) two ? go(few_row_bf16_kernel<1, 2>) : go(few_row_bf16_kernel<1, 4>);
-  else if (nt == 2) two ? go(few_row_bf16_kernel<2, 2>) : go(few_row_bf16_kernel<2, 4>);
-  else if (nt == 4) two ? go(few_row_bf16_kernel<4, 2>) : go(few_row_bf16_kernel<4, 4>);
-  else go(few_row_bf16_kernel<8, 4>);
+  // Two blocks of 32 k per lane and trip instead of four: where the range would leave warps idle with four, where a cluster's CTAs are
+  // more than the registers of four hold at once (16 rows, us with four and two: n 2048 k 5504 18.4, 10.9, n 1024 k 5120 12.1, 8.3;
+  // a token of 4 layers of width 2048, 16 streams, 214 and 196), and where CTAs are few and the range takes several trips anyway
+  // (6 layers of width 512, one stream 123 and 118 a token). Four where one tile's range is then a single trip, all of it requested
+  // before the predecessor has ended, though by the launch alone two take less (9 layers of width 1024, 8 streams 241 and 262 a
+  // token); and for eight tiles, whose activations outweigh that.
+  const int range = (k_max + ranks - 1) / ranks;
+  bool two = range <= 512;
+  if (range > 1024 && ranks == 1) two = ctas <= 3 * 148 / 2;
+  else if (range > 512 && ranks > 1) two = ctas > 2 * 148 && !(nt == 1 && range <= 1024);
+  auto by_split = [&](auto nt_c, auto unroll_c) {
+    constexpr int NT = nt_c.value, UNROLL = unroll_c.value;
+    constexpr bool ONE_FORM = NT != 4;
+    if (ONE_FORM || row_ctas > 1) go(few_row_bf16_kernel<NT, UNROLL, true>);
+    else go(few_row_bf16_kernel<NT, UNROLL, ONE_FORM>);
+  };
+  auto by_unroll = [&](auto nt_c) {
+    if (two) by_split(nt_c, std::integral_constant<int, 2>());
+    else by_split(nt_c, std::integral_constant<int, 4>());
+  };
+  if (nt == 1) by_unroll(std::integral_constant<int, 1>());
+  else if (nt == 2) by_unroll(std::integral_constant<int, 2>());
+  else if (nt == 4) by_unroll(std::integral_constant<int, 4>());
+  else by_split(std::integral_constant<int, 8>(), std::integral_constant<int, 4>());
 }
 
 }  // namespace lb
