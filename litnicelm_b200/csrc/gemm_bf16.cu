@@ -389,19 +389,19 @@ void launch_form(const Bf16Product &p, int m, cudaStream_t st, DevErr *err) {
 void launch_gemm_bf16(const Bf16Product &p, int m, cudaStream_t st, DevErr *err) {
   if (m < 1 || p.n < 1 || p.k < 1) throw std::invalid_argument("launch_gemm_bf16: empty product");
   if (p.gated && ((p.n_half | p.half_ld) & 1) != 0) throw std::invalid_argument("launch_gemm_bf16: a gated product needs pairs");
-  // The widest tile of which the next narrower would need a second turn: a turn costs about what its tile's k loop does, 1 : 0.6 :
-  // 0.4 from 256 to 64 columns. 2368 x 1024 (76 tiles of 256 columns), by 64, 128 and 256: k 512 12.4, 10.4, 8.6 us, k 5120 74, 51, 29;
-  // 613 x 2048 (80 of 128): k 512 10.4, 8.3, 8.4, k 5120 51, 29, 29; 613 x 1600 (65 of 128, 125 of 64): k 512 8.3 each, with GELU 8.3,
-  // 10.4, 12.5. Mitilix, 8 streams of 256 + 96 tokens: 31.51 ms with 256 columns from 111 tiles on (and so 128), 31.24.
+  // The widest tile of which the next narrower would need a second turn: a turn costs about what its tile's k loop does, 1 : 0.8 :
+  // 0.7 from 256 to 64 columns. 2368 x 1024 (76 tiles of 256 columns), by 64, 128 and 256: k 512 11.7, 9.4, 8.0 us, k 5120 74, 51, 29;
+  // 613 x 2048 (80 of 128): k 512 9.1, 6.9, 7.8, k 5120 51, 29, 28; 613 x 1600 (65 of 128, 125 of 64): k 512 6.4, 6.9, 7.8, with GELU 7.5,
+  // 8.9, 11.9. Mitilix, 8 streams of 256 + 96 tokens: 31.51 ms with 256 columns from 111 tiles on (and so 128), 31.24.
   const long long mt = (m + TC_BM - 1) / TC_BM;
   const long long sms = device_sms();
   const long long nt = (p.n + 255) / 256, turns = (mt * nt + sms - 1) / sms;
   const long long pair_turns = ((mt + 1) / 2 * nt + sms / 2 - 1) / (sms / 2);
   if (p.n > 128 && mt * ((p.n + 127) / 128) > sms) {
-    // A pair starts about 2 us later (its CTAs meet before and after) and then gains a share of each 64 k of each tile: 5 % at
-    // 6 tiles of 1024 k a CTA, 11 % at 2 of 5120, 17 % at 6 of 5120, against 4 to 8 % lost at 2 of 2048 and at one tile.
-    // With an activation, sixteen storing warps: without them a pair gains nothing (gated 8192 x 8192 x 1024: 90 us alone, 96 a
-    // pair with eight, 79 with sixteen; plain results prefer the sixth operand stage, 8192 x 1024 x 5120 74, 65 and 69).
+    // A pair starts 1.5 to 2 us later (its CTAs meet before and after) and then gains a share of each 64 k of each tile: 6 % at 7
+    // tiles of 1024 k a CTA, 6 to 9 % at 2 of 5120, 9 to 12 % at 4 and 7 of 5120, against 1 to 4 % lost at 2 of 2048 and more below.
+    // With an activation, sixteen storing warps: with eight a pair gains nothing (gated 8192 x 4096 x 1024: 64 us alone, 69 a
+    // pair with eight, 57 with sixteen; plain results prefer the sixth operand stage, 8192 x 4096 x 1024 60.5, 56.9 and 58.8).
     const bool pair = turns >= 2 && turns * p.k >= 5120 && pair_turns <= turns;
     if (pair && p.act != ACT_NONE && p.n_half > 0) launch_form<256, true, 16>(p, m, st, err);
     else if (pair) launch_form<256, true>(p, m, st, err);
